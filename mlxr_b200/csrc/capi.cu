@@ -432,7 +432,7 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
   const size_t i_bytes = align_up((size_t)M * inter * es, 256);
   Workspace* ws = nullptr;
   const void* wgu[2] = {w_gate, w_up};
-  // batches 3..64 of Q4_K: RMSNorm, then gate/up with the SiLU(gate) * up epilogue and down on the
+  // batches 3..64: RMSNorm, then gate/up with the SiLU(gate) * up epilogue and down on the
   // small-batch tensor-core kernel (three launches; the decode kernel is built for batch 1-2)
   const bool small = M >= 3 && smallm_supported(qt, M, inter, hidden, dtype, x, w_gate) &&
                      smallm_supported(qt, M, inter, hidden, dtype, x, w_up) &&

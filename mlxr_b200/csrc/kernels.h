@@ -116,7 +116,7 @@ bool stream_gemv_supported(int qt, int M, int K, const void* const* w, int nmat)
 int launch_stream_gemv(const DecodeLinear& L, int M, int dtype, int* status, cudaStream_t st,
                        const void* next_w = nullptr, size_t next_bytes = 0);
 
-// ---- small-batch tensor-core linear (smallm.cu): Q4_K / Q4_0, 1 <= M <= 64, fp16 / bf16 --------------
+// ---- small-batch tensor-core linear (smallm.cu): Q4_K, Q4_0, Q8_0, NF4, canonical Q4_K; 1 <= M <= 64, fp16 / bf16 ----
 bool smallm_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w);
 void smallm_partition(long long units, int ctas, int cta, long long unit, long long* begin, long long* end, int* owner);
 // grid size, the most CTAs that share one output tile, and the bytes of fp32 partial sums needed;

@@ -113,3 +113,52 @@ def test_bit_identical_over_many_launches():
             assert torch.equal(mx.q_gemm_dequant(x, w, M, N, K, mx.QuantType(3), 256, None), first)
     torch.cuda.synchronize()
     assert _status() == 0
+
+
+@pytest.mark.parametrize("qt", [2, 16, 33])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("M,N,K", [(3, 2, 256), (8, 129, 768), (9, 131, 1280), (17, 200, 512), (64, 385, 768)])
+def test_other_formats(oracle, qt, dt, M, N, K):
+    """Q8_0, NF4 and canonical ggml Q4_K: odd row counts and odd numbers of super-blocks (NF4 rows are
+    then only 8-byte aligned).  Against float32 products of the dequantized weights.  Up to batch 8,
+    and for canonical Q4_K at any, the weights keep 16 (bf16) or 22 (fp16) significant bits, so the
+    result's own rounding is what is left: at most 2^-9 (2^-12) of each value, about 0.6 of that in the
+    2-norm; 2^-9 and 2^-11 leave room for sums that cancel.  Wider batches round the weight once more:
+    twice that."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    if qt == 33:
+        rng = np.random.Generator(np.random.PCG64(M + N))
+        raw = rng.integers(0, 256, size=(N * (K // 256), 144), dtype=np.uint8)
+        raw[:, 0:2] = (rng.random(raw.shape[0]) * 0.002 + 0.0005).astype(np.float16).view(np.uint8).reshape(-1, 2)
+        raw[:, 2:4] = (rng.random(raw.shape[0]) * 0.004 + 0.0005).astype(np.float16).view(np.uint8).reshape(-1, 2)
+        packed = raw.reshape(-1)
+        import gguf
+        import gguf.quants as gq
+        w = gq.dequantize(packed.reshape(N, -1), gguf.GGMLQuantizationType.Q4_K).astype(np.float64)
+    else:
+        packed = quantize(make_weights(N, K, 100 + M), qt)
+        w = oracle.dequantize(packed, N, K, qt)[0].astype(np.float64).reshape(N, K)
+    xt, xf = make_acts(M, K, 200 + M, DT[dt])
+    bt, bf = make_acts(1, N, 300, DT[dt])
+    want = xf.astype(np.float64) @ w.T + bf[0]
+    args = (xt.cuda(), torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt), bt[0].contiguous().cuda())
+    y = mx.q_gemm_dequant(*args)
+    assert torch.equal(y, mx.q_gemm_dequant(*args))
+    assert _status() == 0
+    bound = {"bf16": 2.0 ** -9, "f16": 2.0 ** -11}[dt] * (1 if M <= 8 or qt == 33 else 2)
+    assert oracle.rel_l2(y.float().cpu().numpy(), want) <= bound
+
+
+@pytest.mark.parametrize("qt", [2, 16])
+@pytest.mark.parametrize("M,H,I", [(5, 256, 768), (33, 768, 1280)])
+def test_gate_up_other_formats(oracle, qt, M, H, I):
+    """The SiLU(gate) * up form of Q8_0 and NF4, with odd numbers of super-blocks, inside the block."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    g, u, d = (quantize(make_weights(n, k, s), qt) for n, k, s in ((I, H, 1), (I, H, 2), (H, I, 3)))
+    xt, xf = make_acts(M, H, 4, torch.bfloat16)
+    nt, nf = make_acts(1, H, 5, torch.bfloat16)
+    y = mx.mlp_block(xt.cuda(), nt[0].contiguous().cuda(), *(torch.from_numpy(w).cuda() for w in (g, u, d)), I, mx.QuantType(qt), 1e-5)
+    assert _status() == 0
+    assert oracle.rel_l2(y.float().cpu().numpy(), oracle.mlp_block(xf, nf[0], g, u, d, I, qt, 1e-5, oracle.BF16)) <= TIGHT["bf16"]
