@@ -100,3 +100,29 @@ def check(status: int) -> None:
     if status == ERR_INVALID_ARGUMENT:
         raise MlxrInvalidArgument(status, msg)
     raise MlxrError(status, msg)
+
+
+def _load_ops():
+    """lib/mlxr_torch_ops.so: the operators' call path for plainly valid arguments (cpp/torch_ops.cpp)."""
+    import importlib.machinery
+    import importlib.util
+
+    import torch  # noqa: F401  (its libraries must be loaded first)
+    path = os.path.join(_HERE, "lib", "mlxr_torch_ops.so")
+    if not os.path.exists(path):
+        raise ImportError(f"{path} not found: build it with python -m mlxr_b200.build")
+    loader = importlib.machinery.ExtensionFileLoader("mlxr_torch_ops", path)
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("mlxr_torch_ops", path, loader=loader))
+    loader.exec_module(mod)
+    mod.bind({n: C.cast(getattr(lib, n), _vp).value for n in PROTOTYPES if n.startswith("mlxr_")})
+    return mod
+
+
+fast = _load_ops()
+
+
+def done(r):
+    """The result of a `fast` call that returned one: a status is raised."""
+    if type(r) is int:
+        check(r)
+    return r

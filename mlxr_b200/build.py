@@ -1,5 +1,6 @@
 """Build recipe: compiles the CUDA sources under csrc/ for sm_100a with nvcc and links
-them in-tree into lib/libmlxr_b200.so (the C ABI of include/mlxr_b200.h).
+them in-tree into lib/libmlxr_b200.so (the C ABI of include/mlxr_b200.h), and the call path from
+torch tensors to it into lib/mlxr_torch_ops.so.
 
     python -m mlxr_b200.build            # build what is out of date
     python -m mlxr_b200.build --force    # rebuild everything
@@ -23,6 +24,8 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "lib")
 OBJ = os.path.join(OUT, "obj")
 LIB = os.path.join(OUT, "libmlxr_b200.so")
+OPS_SRC = os.path.join(HERE, "cpp", "torch_ops.cpp")
+OPS = os.path.join(OUT, "mlxr_torch_ops.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -53,6 +56,24 @@ def _deps_mtime() -> float:
 
 def sources() -> list[str]:
     return sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
+
+
+def _build_ops(force: bool) -> None:
+    """lib/mlxr_torch_ops.so: the Python-to-C-ABI call path of ops.py (g++ against torch's headers)."""
+    if not force and os.path.exists(OPS) and os.path.getmtime(OPS) >= max(os.path.getmtime(OPS_SRC), os.path.getmtime(os.path.join(ROOT, "include", "mlxr_b200.h"))):
+        return
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    inc = [f"-I{d}" for d in cpp_extension.include_paths() + [sysconfig.get_paths()["include"], "/usr/local/cuda/include"]]
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *inc, OPS_SRC, "-o", OPS, f"-L{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        sys.stderr.write(p.stdout + p.stderr)
+        raise RuntimeError("building mlxr_torch_ops.so failed")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -105,6 +126,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if p.returncode != 0:
             sys.stderr.write(p.stdout + p.stderr)
             raise RuntimeError("link failed")
+    _build_ops(force)
     return LIB
 
 

@@ -79,7 +79,7 @@ int get_workspace(cudaStream_t st, size_t need, Workspace** out, size_t need_sta
     MLXR_CUDA_TRY(cudaMalloc(&ws.status, 64));
     MLXR_CUDA_TRY(cudaMemset(ws.status, 0, 64));
     MLXR_CUDA_TRY(cudaMallocHost(&ws.status_host, 64));
-    ws.status_host[0] = 0;
+    memset(ws.status_host, 0, 64);
   }
   if (int r = grow(&ws.buf, &ws.bytes, need, st)) return r;
   if (int r = grow(&ws.stage, &ws.stage_bytes, need_stage, st)) return r;
@@ -133,6 +133,29 @@ static int check_quant(int qt, int K, int group_size, bool check_group) {
 // Kernel selection for one linear.  Fast kernels need 16-byte aligned rows.
 // The first kDecodeScratchBytes of a workspace's scratch belong to the decode kernel's
 // split-K partial sums; intermediates of the fused entry points start after them.
+// Y = X W^T (+ bias), or SiLU(X w^T) * (X w2^T), on the tensor-core kernels that keep the weight tile in
+// tensor memory: up to 64 tokens the small-batch kernel, above that the wide one.
+static bool weight_tile_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w) {
+  return M <= 64 ? smallm_supported(qt, M, N, K, dtype, x, w) : widem_supported(qt, M, N, K, dtype, x, w);
+}
+static int run_weight_tile(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K,
+                           int qt, int dtype, cudaStream_t st) {
+  const int rows = w2 ? 2 * N : N;
+  int grid = 0, maxc = 0;
+  size_t part = 0;
+  WidePlan plan;
+  if (M <= 64) { if (int r = smallm_plan(M, rows, K, &grid, &maxc, &part)) return r; }
+  else { if (int r = widem_plan(M, rows, K, &plan)) return r; part = plan.partial_bytes; }
+  Workspace* ws = nullptr;
+  if (int r = get_workspace(st, 0, &ws)) return r;
+  {
+    std::lock_guard<std::mutex> lk(g_ws_mu);
+    if (int r = grow(&ws->part, &ws->part_bytes, part, st)) return r;
+  }
+  if (M <= 64) return launch_smallm(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, grid, maxc, st);
+  return launch_widem(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, plan, st);
+}
+
 static int run_linear(const void* x, const void* w, const void* bias, void* y, int M, int N, int K,
                       int qt, int dtype, cudaStream_t st) {
   if (M > 0 && N > 0 && stream_gemv_supported(qt, M, K, &w, 1) && !tune_env("MLXR_NO_STREAM")) {
@@ -143,18 +166,8 @@ static int run_linear(const void* x, const void* w, const void* bias, void* y, i
     L.w[0] = w; L.rows[0] = N; L.nmat = 1; L.K = K; L.x = x; L.y[0] = y; L.bias[0] = bias;
     return launch_stream_gemv(L, M, dtype, ws->status, st);
   }
-  if (M >= 3 && N > 0 && smallm_supported(qt, M, N, K, dtype, x, w) && !tune_env("MLXR_NO_SMALLM")) {
-    int grid = 0, maxc = 0;
-    size_t part = 0;
-    if (int r = smallm_plan(M, N, K, &grid, &maxc, &part)) return r;
-    Workspace* ws = nullptr;
-    if (int r = get_workspace(st, 0, &ws)) return r;
-    {
-      std::lock_guard<std::mutex> lk(g_ws_mu);
-      if (int r = grow(&ws->part, &ws->part_bytes, part, st)) return r;
-    }
-    return launch_smallm(x, w, nullptr, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, grid, maxc, st);
-  }
+  if (M >= 3 && N > 0 && weight_tile_supported(qt, M, N, K, dtype, x, w))
+    return run_weight_tile(x, w, nullptr, bias, y, M, N, K, qt, dtype, st);
   if (M > 0 && N > 0 && decode_supported(qt, M, K, &w, 1)) {
     Workspace* ws = nullptr;
     if (int r = get_workspace(st, kDecodeScratchBytes, &ws)) return r;
@@ -353,14 +366,17 @@ int mlxr_rope_apply(const void* x, const uint16_t* cos_f16, const uint16_t* sin_
   cudaStream_t st = (cudaStream_t)stream;
   Workspace* ws = nullptr;
   if (int r = get_workspace(st, 0, &ws)) return r;
+  // With `check` the kernel records a violation straight in pinned host memory (under unified addressing the
+  // host address is the device address), which saves a copy and a memset per call; the word is only
+  // read and cleared while the stream is idle.
+  int* const violation = ws->status_host + 8;
   if (int r = launch_rope(x, cos_f16, sin_f16, positions, y, tokens, heads, head_dim, max_seq_len, mode,
-                          scale_factor, position_offset, dtype, ws->status, st))
+                          scale_factor, position_offset, dtype, check ? violation : ws->status, st))
     return r;
   if (check) {
-    MLXR_CUDA_TRY(cudaMemcpyAsync(ws->status_host, ws->status, sizeof(int), cudaMemcpyDeviceToHost, st));
-    MLXR_CUDA_TRY(cudaMemsetAsync(ws->status, 0, sizeof(int), st));
     MLXR_CUDA_TRY(cudaStreamSynchronize(st));
-    if (ws->status_host[0] != 0) {
+    if (*reinterpret_cast<volatile int*>(violation) != 0) {
+      *reinterpret_cast<volatile int*>(violation) = 0;
       set_error("rope_apply: a position (+offset) lies outside [0, max_seq_len)");
       return MLXR_ERR_SHAPE;
     }
@@ -432,12 +448,12 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
   const size_t i_bytes = align_up((size_t)M * inter * es, 256);
   Workspace* ws = nullptr;
   const void* wgu[2] = {w_gate, w_up};
-  // batches 3..64: RMSNorm, then gate/up with the SiLU(gate) * up epilogue and down on the
-  // small-batch tensor-core kernel (three launches; the decode kernel is built for batch 1-2)
-  const bool small = M >= 3 && smallm_supported(qt, M, inter, hidden, dtype, x, w_gate) &&
-                     smallm_supported(qt, M, inter, hidden, dtype, x, w_up) &&
-                     smallm_supported(qt, M, hidden, inter, dtype, x, w_down) &&
-                     (2 * inter + 127) / 128 <= kSyncWords - 16 && !tune_env("MLXR_NO_SMALLM");
+  // more than two tokens: RMSNorm, then gate/up with the SiLU(gate) * up epilogue and down on the
+  // tensor-core kernels (three launches; the decode kernel is built for batch 1-2)
+  const bool small = M >= 3 && weight_tile_supported(qt, M, inter, hidden, dtype, x, w_gate) &&
+                     weight_tile_supported(qt, M, inter, hidden, dtype, x, w_up) &&
+                     weight_tile_supported(qt, M, hidden, inter, dtype, x, w_down) &&
+                     (2 * inter + 127) / 128 <= kSyncWords - 16;
   const bool decode = !small && decode_supported(qt, M, hidden, wgu, 2) && decode_supported(qt, M, inter, &w_down, 1);
   if (int r = get_workspace(st, decode ? kDecodeScratchBytes : kDecodeScratchBytes + n_bytes + 2 * i_bytes, &ws, 0,
                             decode ? decode_tagged_bytes(M, inter, dtype) : 0))
@@ -465,16 +481,7 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
     n = nbuf;
   }
   if (small) {
-    int grid = 0, maxc = 0;
-    size_t part = 0;
-    if (int r = smallm_plan(M, 2 * inter, hidden, &grid, &maxc, &part)) return r;
-    {
-      std::lock_guard<std::mutex> lk(g_ws_mu);
-      if (int r = grow(&ws->part, &ws->part_bytes, part, st)) return r;
-    }
-    if (int r = launch_smallm(n, w_gate, w_up, nullptr, gbuf, M, inter, hidden, qt, dtype, ws->status, (float*)ws->part,
-                              ws->sync + 16, grid, maxc, st))
-      return r;
+    if (int r = run_weight_tile(n, w_gate, w_up, nullptr, gbuf, M, inter, hidden, qt, dtype, st)) return r;
     if (!y_f32) return run_linear(gbuf, w_down, nullptr, y, M, hidden, inter, qt, dtype, st);
     if (int r = run_linear(gbuf, w_down, nullptr, nbuf, M, hidden, inter, qt, dtype, st)) return r;
     return launch_cast_to_f32(nbuf, (float*)y, (size_t)M * hidden, dtype, st);

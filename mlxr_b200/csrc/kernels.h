@@ -126,6 +126,18 @@ int smallm_plan(int M, int rows, int K, int* grid, int* maxc, size_t* partial_by
 int launch_smallm(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K, int qt, int dtype,
                   int* status, float* partials, uint32_t* counters, int grid, int maxc, cudaStream_t st);
 
+// ---- the same form for more tokens (widem.cu): Q4_K, Q4_0, Q8_0, NF4, fp16 / bf16 ---------------------
+struct WidePlan {
+  int nt, ntt, ntiles;     // tokens per tile, token tiles, tiles in all
+  int grid, whole;         // CTAs; 1: whole tiles per CTA, 0: equal ranges of work units
+  size_t partial_bytes;    // fp32 partial sums needed
+  double cost_us;          // the plan's own estimate
+};
+bool widem_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w);
+int widem_plan(int M, int rows, int K, WidePlan* out);     // rows = weight rows streamed (N, or 2 N for the gate/up form)
+int launch_widem(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K, int qt, int dtype,
+                 int* status, float* partials, uint32_t* counters, const WidePlan& plan, cudaStream_t st);
+
 // ---- tensor-core GEMM for batch >= 9 on Q4_K with 16-bit activations (prefill.cu) -------------
 bool prefill_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w, const void* y);
 int prefill_slices(int M, int N, int K);     // K-slices (grid z); S > 1 needs S*M*N floats of scratch

@@ -48,6 +48,7 @@
 #include "kernels.h"
 #include "tc_common.cuh"
 #include "weight_convert.cuh"
+#include "weight_maps.h"
 
 namespace mlxr {
 namespace smallm {
@@ -522,38 +523,6 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
 }  // namespace smallm
 
 // ---- host side -----------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static int tensor_map_encoder(EncodeTiledFn* out) {
-  static std::mutex mu;
-  static EncodeTiledFn encode = nullptr;
-  std::lock_guard<std::mutex> lk(mu);
-  if (!encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    MLXR_CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
-    if (!fn || q != cudaDriverEntryPointSuccess) { set_error("cuTensorMapEncodeTiled is not available in this driver"); return MLXR_ERR_CUDA; }
-    encode = (EncodeTiledFn)fn;
-  }
-  *out = encode;
-  return MLXR_OK;
-}
-
-static int device_sms(int* out) {
-  static std::atomic<int> sms[64];
-  int dev = 0;
-  MLXR_CUDA_TRY(cudaGetDevice(&dev));
-  int n = sms[dev & 63].load();
-  if (!n) {
-    MLXR_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-    sms[dev & 63].store(n);
-  }
-  *out = n;
-  return MLXR_OK;
-}
-
 static int smallm_npad(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 
 void smallm_partition(long long units, int ctas, int cta, long long unit, long long* begin, long long* end, int* owner) {
@@ -624,64 +593,21 @@ static int launch_inst(const smallm::Maps& maps, const smallm::Params& P, int gr
   return MLXR_OK;
 }
 
-// Rows of `stride` bytes as 8-byte elements, boxes of `box_bytes` x `box_rows`; rows past the end
-// and bytes past `inner` read as zero.
-static int weight_map(EncodeTiledFn encode, const void* base, int rows, size_t inner, size_t stride, int box_bytes, int box_rows, CUtensorMap* out) {
-  const cuuint64_t dims[2] = {(cuuint64_t)(inner / 8), (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)stride};
-  const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 8), (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void*>(base), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed (%d) for W [%d rows of %zu bytes]", (int)r, rows, inner); return MLXR_ERR_CUDA; }
-  return MLXR_OK;
-}
-
-// The maps of one packed matrix [N, K] for tiles of `tile_rows` of its rows.  NF4 rows are 136 bytes
-// per 256 weights, so with an odd number of super-blocks every other row starts 8 bytes off a
-// 16-byte boundary: even and odd rows get a map each, with twice the row stride, the odd one starting
-// at the 16-byte boundary at or below row 1 (*odd_shift bytes before it).
-static int weight_maps(EncodeTiledFn encode, int qt, const void* w, int N, int K, int tile_rows, CUtensorMap* out, int* odd_shift) {
-  if (qt != MLXR_NF4) {
-    const int unit = qt == MLXR_Q8_0 ? 272 : 144;
-    const size_t rb = (size_t)(K / 256) * unit;
-    return weight_map(encode, w, N, rb, rb, unit, tile_rows, out);
-  }
-  const size_t rb = (size_t)(K / 256) * 136;
-  const int sh = (int)(rb & 8);
-  *odd_shift = sh;
-  if (int r = weight_map(encode, w, (N + 1) / 2, rb, 2 * rb, 144, tile_rows / 2, out)) return r;
-  return weight_map(encode, (const char*)w + rb - sh, N / 2, rb + sh, 2 * rb, 144, tile_rows / 2, out + 1);
-}
-
 // w2 == nullptr: Y[M, N] = X W^T (+ bias).  Otherwise w = gate, w2 = up (both [N, K]) and
 // Y[M, N] = SiLU(X gate^T) * (X up^T), the two products rounded to the activation dtype first.
 int launch_smallm(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K, int qt, int dtype,
                   int* status, float* partials, uint32_t* counters, int grid, int maxc, cudaStream_t st) {
-  EncodeTiledFn encode = nullptr;
-  if (int r = tensor_map_encoder(&encode)) return r;
   const int npad = smallm_npad(M);
   const bool swiglu = w2 != nullptr;
   smallm::Maps maps;
   smallm::Params P;
   memset(&maps, 0, sizeof(maps));
   memset(&P, 0, sizeof(P));
-  {
-    // X [M, K] of a 16-bit type (K inner), boxes of 64 x NPAD with the 128-byte swizzle; rows past M read as zero
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)smallm::kBK, (cuuint32_t)npad};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(&maps.x, dtype == MLXR_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                              const_cast<void*>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed (%d) for X [%d, %d]", (int)r, M, K); return MLXR_ERR_CUDA; }
-  }
+  if (int r = activation_map(x, M, K, dtype, npad, &maps.x)) return r;
   const int tile_rows = swiglu ? 64 : smallm::kRows;
-  if (int r = weight_maps(encode, qt, w, N, K, tile_rows, maps.w, &P.odd_shift)) return r;
+  if (int r = weight_maps(qt, w, N, K, tile_rows, maps.w, &P.odd_shift)) return r;
   if (swiglu)
-    if (int r = weight_maps(encode, qt, w2, N, K, tile_rows, maps.w + (qt == MLXR_NF4 ? 2 : 1), &P.odd_shift)) return r;
+    if (int r = weight_maps(qt, w2, N, K, tile_rows, maps.w + (qt == MLXR_NF4 ? 2 : 1), &P.odd_shift)) return r;
   P.bias = bias;
   P.y = y;
   P.M = M; P.N = N; P.K = K;

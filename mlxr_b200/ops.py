@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from . import _capi
-from ._capi import check, lib
+from ._capi import check, done, fast, lib
 from .types import QuantType, RoPEScalingMode
 
 _DT = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}
@@ -101,6 +101,9 @@ def q_gemm_dequant(input: torch.Tensor, weights: torch.Tensor, M: int, N: int, K
                    ) -> torch.Tensor:
     """q_gemm_dequant(), q_gemm_dequant_primitive.h:211-215 / .mm:478-522.
     input [M, K]; weights: packed uint8; bias [N] optional -> [M, N] of input's dtype."""
+    r = fast.q_gemm_dequant(input, weights, M, N, K, quant_type, group_size, bias)
+    if r is not None:
+        return done(r)
     if input.dim() != 2 or input.shape[0] != M or input.shape[1] != K:
         raise _capi.MlxrError(_capi.ERR_SHAPE, "Input shape must be [M, K]")
     if bias is not None and (bias.dim() != 1 or bias.shape[0] != N):
@@ -121,6 +124,9 @@ def rmsnorm_fused(input: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
                   residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     """rmsnorm_fused(), rmsnorm_primitive.h:123-126 / .mm:302-359.  A non-contiguous
     input is made contiguous first, as the reference does (:332-346)."""
+    r = fast.rmsnorm_fused(input, weight, eps, residual)
+    if r is not None:
+        return done(r)
     if input.dim() < 1:
         raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, "RMSNorm input must have at least 1 dimension")
     if weight.dim() != 1:
@@ -150,6 +156,9 @@ def swish(x: torch.Tensor) -> torch.Tensor:
 
 def swiglu(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     """swiglu(), swiglu_mlp_primitive.mm:311-318"""
+    r = fast.swiglu(gate, up)
+    if r is not None:
+        return done(r)
     if gate.shape != up.shape or gate.dtype != up.dtype:
         raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, "gate and up must match")
     out = torch.empty_like(gate)
@@ -189,6 +198,10 @@ def rope_apply(input: torch.Tensor, cos_table: torch.Tensor, sin_table: torch.Te
                check_positions: bool = True) -> torch.Tensor:
     """rope_apply(), rope_apply_primitive.h:192-197 / .mm:399-475.  input is
     [tokens, heads, d] or [batch, seq, heads, d]; tables fp16 [max_seq, d/2]."""
+    r = fast.rope_apply(input, cos_table, sin_table, positions, scaling_mode, scale_factor, position_offset, inplace, check_positions)
+    if r is not None:
+        done(r)
+        return input if inplace else r
     if input.dim() not in (3, 4):
         raise _capi.MlxrError(_capi.ERR_SHAPE, "Input must be 3D [tokens, num_heads, head_dim] or 4D [batch, seq_len, num_heads, head_dim]")
     if input.dim() == 4:
@@ -283,6 +296,9 @@ def mlp_block(x: torch.Tensor, norm_weight: Optional[torch.Tensor], w_gate: torc
     """y = down(SiLU(gate(n)) * up(n)), n = rmsnorm(x) when norm_weight is given: the
     quantized form of swiglu_mlp() (swiglu_mlp_primitive.h:169-176) with the RMSNorm
     prologue of TransformerBlock::forward (core/graph/layers.cpp:451-452)."""
+    r = fast.mlp_block(x, norm_weight, w_gate, w_up, w_down, inter, quant_type, eps)
+    if r is not None:
+        return done(r)
     if x.dim() != 2:
         raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, "Input must be 2D [M, hidden_size]")
     M, hidden = x.shape
@@ -325,6 +341,9 @@ def qkv_rope(x: torch.Tensor, norm_weight: Optional[torch.Tensor], wq: torch.Ten
              quant_type: QuantType, eps: float = 1e-5, position_offset: int = 0
              ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """RMSNorm -> q/k/v projections -> rope_apply on q and k (see mlxr_qkv_rope)."""
+    r = fast.qkv_rope(x, norm_weight, wq, wk, wv, cos_table, sin_table, positions, q_heads, kv_heads, head_dim, quant_type, eps, position_offset)
+    if r is not None:
+        return done(r)
     M, hidden = x.shape
     q = torch.empty((M, q_heads, head_dim), dtype=x.dtype, device=x.device)
     k = torch.empty((M, kv_heads, head_dim), dtype=x.dtype, device=x.device)
