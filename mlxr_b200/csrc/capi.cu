@@ -44,6 +44,8 @@ struct Workspace {
   size_t stage_bytes = 0;
   void* part = nullptr;      // split-K partial sums of the tensor-core GEMM (never aliases buf)
   size_t part_bytes = 0;
+  void* w16 = nullptr;       // 16-bit weights of the dense path, at most 256 MB
+  size_t w16_bytes = 0;
   void* tagged = nullptr;    // h of the decode MLP block as {payload, sequence number} words; zero-filled when
   size_t tagged_bytes = 0;   // allocated and written by nothing else, so a stale word never carries a live number
   uint32_t* sync = nullptr;  // kSyncWords zero-initialised words (counters, barriers)
@@ -130,32 +132,47 @@ static int check_quant(int qt, int K, int group_size, bool check_group) {
   return MLXR_OK;
 }
 
-// Kernel selection for one linear.  Fast kernels need 16-byte aligned rows.
-// The first kDecodeScratchBytes of a workspace's scratch belong to the decode kernel's
-// split-K partial sums; intermediates of the fused entry points start after them.
-// Y = X W^T (+ bias), or SiLU(X w^T) * (X w2^T), on the tensor-core kernels that keep the weight tile in
-// tensor memory: up to 64 tokens the small-batch kernel, above that the wide one.
-static bool weight_tile_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w) {
-  return M <= 64 ? smallm_supported(qt, M, N, K, dtype, x, w) : widem_supported(qt, M, N, K, dtype, x, w);
+// The tensor-core linears for 16-bit activations: Y = X W^T (+ bias), or SiLU(X w^T) * (X w2^T).
+// Up to 64 tokens the small-batch kernel.  Above that the wide kernel, which converts the weights beside the
+// MMAs once per 256 tokens, or the dense path, which converts them once in a pass of its own: whichever
+// their plans estimate to be faster (for 14336 x 4096 they meet near 1800 tokens).  The dense path also takes what the others
+// do not: K that is not a multiple of 256, rows that do not start on 16 bytes.
+enum TcPath { kTcNone = 0, kTcSmall, kTcWide, kTcDense };
+static int tc_path(int qt, int M, int N, int K, int dtype, const void* x, const void* w, const void* w2, WidePlan* wide, DensePlan* dense, TcPath* out) {
+  *out = kTcNone;
+  const int rows = w2 ? 32 * ((N + 15) / 16) : N;
+  auto both = [&](auto&& ok) { return ok(w) && (!w2 || ok(w2)); };
+  if (M <= 64 && both([&](const void* p) { return smallm_supported(qt, M, N, K, dtype, x, p); })) { *out = kTcSmall; return MLXR_OK; }
+  if (M > 64 && both([&](const void* p) { return widem_supported(qt, M, N, K, dtype, x, p); })) {
+    if (int r = widem_plan(M, rows, K, wide)) return r;
+    *out = kTcWide;
+  }
+  if (both([&](const void* p) { return dense_supported(qt, M, N, K, dtype, x, p); })) {
+    if (int r = dense_plan(M, rows, K, dense)) return r;
+    if (*out == kTcNone || dense->cost_us < wide->cost_us) *out = kTcDense;
+  }
+  return MLXR_OK;
 }
-static int run_weight_tile(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K,
-                           int qt, int dtype, cudaStream_t st) {
-  const int rows = w2 ? 2 * N : N;
+static int run_tc(TcPath path, const WidePlan& wide, const DensePlan& dense, const void* x, const void* w, const void* w2, const void* bias, void* y,
+                  int M, int N, int K, int qt, int dtype, cudaStream_t st) {
   int grid = 0, maxc = 0;
-  size_t part = 0;
-  WidePlan plan;
-  if (M <= 64) { if (int r = smallm_plan(M, rows, K, &grid, &maxc, &part)) return r; }
-  else { if (int r = widem_plan(M, rows, K, &plan)) return r; part = plan.partial_bytes; }
+  size_t part = path == kTcWide ? wide.partial_bytes : 0;
+  if (path == kTcSmall) { if (int r = smallm_plan(M, w2 ? 2 * N : N, K, &grid, &maxc, &part)) return r; }
   Workspace* ws = nullptr;
   if (int r = get_workspace(st, 0, &ws)) return r;
   {
     std::lock_guard<std::mutex> lk(g_ws_mu);
     if (int r = grow(&ws->part, &ws->part_bytes, part, st)) return r;
+    if (path == kTcDense) if (int r = grow(&ws->w16, &ws->w16_bytes, dense.bytes, st)) return r;
   }
-  if (M <= 64) return launch_smallm(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, grid, maxc, st);
-  return launch_widem(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, plan, st);
+  if (path == kTcSmall) return launch_smallm(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, grid, maxc, st);
+  if (path == kTcWide) return launch_widem(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, wide, st);
+  return launch_dense(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, ws->w16, dense, st);
 }
 
+// Kernel selection for one linear.  Fast kernels need 16-byte aligned rows.
+// The first kDecodeScratchBytes of a workspace's scratch belong to the decode kernel's
+// split-K partial sums; intermediates of the fused entry points start after them.
 static int run_linear(const void* x, const void* w, const void* bias, void* y, int M, int N, int K,
                       int qt, int dtype, cudaStream_t st) {
   if (M > 0 && N > 0 && stream_gemv_supported(qt, M, K, &w, 1) && !tune_env("MLXR_NO_STREAM")) {
@@ -166,8 +183,13 @@ static int run_linear(const void* x, const void* w, const void* bias, void* y, i
     L.w[0] = w; L.rows[0] = N; L.nmat = 1; L.K = K; L.x = x; L.y[0] = y; L.bias[0] = bias;
     return launch_stream_gemv(L, M, dtype, ws->status, st);
   }
-  if (M >= 3 && N > 0 && weight_tile_supported(qt, M, N, K, dtype, x, w))
-    return run_weight_tile(x, w, nullptr, bias, y, M, N, K, qt, dtype, st);
+  if (M >= 3 && N > 0) {
+    TcPath path;
+    WidePlan wide;
+    DensePlan dense;
+    if (int r = tc_path(qt, M, N, K, dtype, x, w, nullptr, &wide, &dense, &path)) return r;
+    if (path != kTcNone) return run_tc(path, wide, dense, x, w, nullptr, bias, y, M, N, K, qt, dtype, st);
+  }
   if (M > 0 && N > 0 && decode_supported(qt, M, K, &w, 1)) {
     Workspace* ws = nullptr;
     if (int r = get_workspace(st, kDecodeScratchBytes, &ws)) return r;
@@ -178,16 +200,6 @@ static int run_linear(const void* x, const void* w, const void* bias, void* y, i
   }
   if (M > 0 && N > 0 && gemv_rows_supported(qt, M, K, x, w) && !tune_env("MLXR_NO_GEMV"))
     return launch_gemv_rows(x, w, bias, y, M, N, K, qt, dtype, st);
-  if (M > 0 && N > 0 && prefill_supported(qt, M, N, K, dtype, x, w, y) && !tune_env("MLXR_NO_TC")) {
-    const int S = prefill_slices(M, N, K);
-    Workspace* ws = nullptr;
-    if (int r = get_workspace(st, 0, &ws)) return r;
-    if (S > 1) {
-      std::lock_guard<std::mutex> lk(g_ws_mu);
-      if (int r = grow(&ws->part, &ws->part_bytes, (size_t)S * M * N * sizeof(float), st)) return r;
-    }
-    return launch_prefill(x, w, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, S, st);
-  }
   return launch_qgemm_generic(x, w, bias, y, M, N, K, qt, dtype, st);
 }
 
@@ -450,10 +462,11 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
   const void* wgu[2] = {w_gate, w_up};
   // more than two tokens: RMSNorm, then gate/up with the SiLU(gate) * up epilogue and down on the
   // tensor-core kernels (three launches; the decode kernel is built for batch 1-2)
-  const bool small = M >= 3 && weight_tile_supported(qt, M, inter, hidden, dtype, x, w_gate) &&
-                     weight_tile_supported(qt, M, inter, hidden, dtype, x, w_up) &&
-                     weight_tile_supported(qt, M, hidden, inter, dtype, x, w_down) &&
-                     (2 * inter + 127) / 128 <= kSyncWords - 16;
+  TcPath path = kTcNone;
+  WidePlan wide;
+  DensePlan dense;
+  if (M >= 3) if (int r = tc_path(qt, M, inter, hidden, dtype, x, w_gate, w_up, &wide, &dense, &path)) return r;
+  const bool small = path != kTcNone && (path != kTcSmall || (2 * inter + 127) / 128 <= kSyncWords - 16);
   const bool decode = !small && decode_supported(qt, M, hidden, wgu, 2) && decode_supported(qt, M, inter, &w_down, 1);
   if (int r = get_workspace(st, decode ? kDecodeScratchBytes : kDecodeScratchBytes + n_bytes + 2 * i_bytes, &ws, 0,
                             decode ? decode_tagged_bytes(M, inter, dtype) : 0))
@@ -481,7 +494,7 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
     n = nbuf;
   }
   if (small) {
-    if (int r = run_weight_tile(n, w_gate, w_up, nullptr, gbuf, M, inter, hidden, qt, dtype, st)) return r;
+    if (int r = run_tc(path, wide, dense, n, w_gate, w_up, nullptr, gbuf, M, inter, hidden, qt, dtype, st)) return r;
     if (!y_f32) return run_linear(gbuf, w_down, nullptr, y, M, hidden, inter, qt, dtype, st);
     if (int r = run_linear(gbuf, w_down, nullptr, nbuf, M, hidden, inter, qt, dtype, st)) return r;
     return launch_cast_to_f32(nbuf, (float*)y, (size_t)M * hidden, dtype, st);
@@ -704,6 +717,7 @@ int mlxr_release_workspaces(void) {
     cudaError_t e;
     if (ws.buf && (e = cudaFree(ws.buf)) != cudaSuccess && first == cudaSuccess) first = e;
     if (ws.stage && (e = cudaFree(ws.stage)) != cudaSuccess && first == cudaSuccess) first = e;
+    if (ws.w16 && (e = cudaFree(ws.w16)) != cudaSuccess && first == cudaSuccess) first = e;
     if (ws.part && (e = cudaFree(ws.part)) != cudaSuccess && first == cudaSuccess) first = e;
     if (ws.tagged && (e = cudaFree(ws.tagged)) != cudaSuccess && first == cudaSuccess) first = e;
     if (ws.sync && (e = cudaFree(ws.sync)) != cudaSuccess && first == cudaSuccess) first = e;

@@ -138,10 +138,15 @@ int widem_plan(int M, int rows, int K, WidePlan* out);     // rows = weight rows
 int launch_widem(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K, int qt, int dtype,
                  int* status, float* partials, uint32_t* counters, const WidePlan& plan, cudaStream_t st);
 
-// ---- tensor-core GEMM for batch >= 9 on Q4_K with 16-bit activations (prefill.cu) -------------
-bool prefill_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w, const void* y);
-int prefill_slices(int M, int N, int K);     // K-slices (grid z); S > 1 needs S*M*N floats of scratch
-int launch_prefill(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, int qt, int dtype,
-                   int* status, float* partials, uint32_t* counters, int S, cudaStream_t st);
+// ---- many tokens (dense.cu): 16-bit weights once, then a dense GEMM; Q4_K, Q4_0, Q8_0, NF4, fp16 / bf16 ---
+struct DensePlan {
+  int nt, slice;           // weight rows per tile; rows of the 16-bit buffer filled at a time
+  size_t bytes;            // scratch for the 16-bit weights
+  double cost_us;
+};
+bool dense_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w);
+int dense_plan(int M, int rows, int K, DensePlan* out);
+int launch_dense(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K, int qt, int dtype,
+                 int* status, void* buf, const DensePlan& plan, cudaStream_t st);
 
 }  // namespace mlxr

@@ -254,40 +254,38 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
         const int sb = (int)((sb_first + i) % P.nsb);
         row += (136 * sb + ((local & 1) ? P.odd_shift : 0)) & 8;
       }
-      const Hdr h = load_header<QT, BF, MODE>(row);
       bool ok = true;
-      auto step = [&](auto SC) {
-        constexpr int s = decltype(SC)::value, q = s % kSlots;        // step of the unit, slot
-        const uint32_t u = use * (kSteps / kSlots) + s / kSlots;      // how often the slot has been filled before
-        ok = ok && __all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty_a[g][q]), (u & 1u) ^ 1u, dead));
-        if (!ok) return;
-        tc_fence_after();
-        uint32_t a[16], b[16];
-        const uint32_t col = a_col + q * 2 * kBlockCols;
-        if constexpr (MODE != kSplit) {
-          convert32<QT, BF, MODE, 4 * s>(row, h, sh->nf4, a, b);
-          tmem_st16(col, a);
-          convert32<QT, BF, MODE, 4 * s + 1>(row, h, sh->nf4, a, b);
-          tmem_st16(col + 16, a);
-          convert32<QT, BF, MODE, 4 * s + 2>(row, h, sh->nf4, a, b);
-          tmem_st16(col + 32, a);
-          convert32<QT, BF, MODE, 4 * s + 3>(row, h, sh->nf4, a, b);
-          tmem_st16(col + 48, a);
-        } else {
-          convert32<QT, BF, MODE, 2 * s>(row, h, sh->nf4, a, b);
-          tmem_st16(col, a);
-          tmem_st16(col + kBlockCols, b);
-          convert32<QT, BF, MODE, 2 * s + 1>(row, h, sh->nf4, a, b);
-          tmem_st16(col + 16, a);
-          tmem_st16(col + kBlockCols + 16, b);
+      // k-block kb: half of slot kb / 2, or for kSplit (leading part and residual) all of slot kb & 1
+      auto step = [&](auto KB) {
+        const int kb = block_of(KB);
+        const int st = MODE == kSplit ? kb : kb >> 1, q = st & 1;
+        if (MODE == kSplit || (kb & 1) == 0) {
+          const uint32_t u = use * (kSteps / kSlots) + st / kSlots;     // how often the slot has been filled before
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty_a[g][q]), (u & 1u) ^ 1u, dead));
+          if (!ok) return;
+          tc_fence_after();
         }
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sh->full_a[g][q][use & 1u]));
+        const uint32_t col = a_col + (MODE == kSplit ? q * 2 * kBlockCols : kb * kBlockCols);
+        convert64<QT, BF, MODE>(row, KB, sh->nf4, [&](auto H, const uint32_t (&a)[16], const uint32_t (&b)[16]) {
+          tmem_st16(col + 16 * decltype(H)::value, a);
+          if constexpr (MODE == kSplit) tmem_st16(col + kBlockCols + 16 * decltype(H)::value, b);
+        });
+        if (MODE == kSplit || (kb & 1) == 1) {
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sh->full_a[g][q][use & 1u]));
+        }
       };
-      step(Int<0>{}); step(Int<1>{});
-      if constexpr (kSteps == 4) { step(Int<2>{}); step(Int<3>{}); }
+      if constexpr (MODE == kSplit) {
+#pragma unroll 1
+        for (int kb = 0; kb < 4 && ok; kb++) step(kb);
+      } else {
+        step(Int<0>{});
+        if (ok) step(Int<1>{});
+        if (ok) step(Int<2>{});
+        if (ok) step(Int<3>{});
+      }
       if (!ok) break;
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sh->raw_empty[r]));

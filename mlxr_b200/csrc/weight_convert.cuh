@@ -2,7 +2,7 @@
 // that hold the weight tile in tensor memory.
 //
 // One thread owns one weight row.  A work unit is 256 consecutive weights of a row ("super-block"
-// whatever the format), staged by TMA; convert32 turns 32 of them into 16 registers of packed pairs,
+// whatever the format), staged by TMA; convert64 turns 64 of them into 2 x 16 registers of packed pairs,
 // element order = K order, ready for tcgen05.st (a 32-bit tensor-memory column holds two
 // consecutive K elements of the row that is its lane).
 #pragma once
@@ -31,39 +31,6 @@ template <int QT> struct Geo {
   static constexpr int kStage = QT == MLXR_NF4 ? 144 : kUnit;
 };
 
-template <int ALIGN> struct Vec;
-template <> struct Vec<16> { using T = uint4; };
-template <> struct Vec<8> { using T = uint2; };
-
-// The 32-bit words covering bytes [OFF, OFF + LEN) of a row, fetched with ALIGN-byte shared-memory
-// loads; word(k) is the (possibly half-word shifted) word at byte OFF + 4 k.
-template <int OFF, int LEN, int ALIGN> struct Span {
-  static constexpr int kFirst = OFF / ALIGN, kCount = (OFF + LEN + ALIGN - 1) / ALIGN - kFirst;
-  uint32_t w[kCount * (ALIGN / 4)];
-  __device__ __forceinline__ explicit Span(const uint8_t* row) {
-#pragma unroll
-    for (int i = 0; i < kCount; i++) {
-      const typename Vec<ALIGN>::T v = *reinterpret_cast<const typename Vec<ALIGN>::T*>(row + (kFirst + i) * ALIGN);
-      if constexpr (ALIGN == 16) { w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w; }
-      else { w[2 * i] = v.x; w[2 * i + 1] = v.y; }
-    }
-  }
-  template <int BYTE> __device__ __forceinline__ uint32_t word() const {   // BYTE is even
-    constexpr int rel = BYTE - kFirst * ALIGN, i = rel / 4;
-    if constexpr (rel % 4 == 0) return w[i];
-    else return __funnelshift_r(w[i], w[i + 1], 16);
-  }
-  template <int BYTE> __device__ __forceinline__ __half half() const {
-    constexpr int rel = BYTE - kFirst * ALIGN;
-    return __ushort_as_half((unsigned short)((rel & 2) ? (w[rel / 4] >> 16) : (w[rel / 4] & 0xFFFFu)));
-  }
-};
-
-// Per-row constants of a unit, decoded once for its 256 weights: scale and min of the four (scale,
-// min) pairs of a Q4_K super-block in the form the conversion wants, or the packed header of a
-// canonical ggml super-block.
-struct Hdr { uint32_t s[4], m[4]; };
-
 __device__ __forceinline__ uint32_t dup_bf16(float f) {
   const __nv_bfloat162 v = __float2bfloat162_rn(f);
   return *reinterpret_cast<const uint32_t*>(&v);
@@ -71,34 +38,6 @@ __device__ __forceinline__ uint32_t dup_bf16(float f) {
 __device__ __forceinline__ uint32_t dup_f16(__half h) {
   const __half2 v = __half2half2(h);
   return *reinterpret_cast<const uint32_t*>(&v);
-}
-
-template <int QT, int BF, int MODE>
-__device__ __forceinline__ Hdr load_header(const uint8_t* row) {
-  Hdr h = {};
-  if constexpr (QT == MLXR_Q4_K) {
-    // d, dmin (fp16), scales[12] of which the shader reads six bytes: eight consecutive 6-bit fields,
-    // scale and min of pairs 0 .. 3 (q_gemm_dequant.metal:222-242); sub-block scale = rn16(sc * d),
-    // sub-block min = rn16(m * dmin)
-    const uint4 q = *reinterpret_cast<const uint4*>(row);
-    const __half d = __ushort_as_half((unsigned short)(q.x & 0xFFFFu)), dmin = __ushort_as_half((unsigned short)(q.x >> 16));
-    const uint32_t f[4] = {q.y, q.y >> 12, __funnelshift_r(q.y, q.z, 24), q.z >> 4};
-#pragma unroll
-    for (int p = 0; p < 4; p++) {
-      // 1024 + n as fp16 is 0x6400 | n: the exact half of a 6-bit field without a conversion instruction
-      const __half k1024 = __ushort_as_half((unsigned short)0x6400);
-      const __half sc = __hsub(__ushort_as_half((unsigned short)(0x6400u | (f[p] & 63u))), k1024);
-      const __half mn = __hsub(__ushort_as_half((unsigned short)(0x6400u | ((f[p] >> 6) & 63u))), k1024);
-      const __half ss = __hmul_rn(sc, d), sm = __hmul_rn(mn, dmin);
-      if constexpr (BF == 0) { h.s[p] = dup_f16(ss); h.m[p] = dup_f16(sm); }
-      else if constexpr (MODE == kFast) { h.s[p] = dup_bf16(__half2float(ss)); h.m[p] = dup_bf16(__half2float(sm)); }
-      else { const float s = __half2float(ss); h.s[p] = __float_as_uint(s); h.m[p] = __float_as_uint(fmaf(-136.0f, s, __half2float(sm))); }
-    }
-  } else if constexpr (QT == MLXR_GGML_Q4_K) {
-    const uint4 q = *reinterpret_cast<const uint4*>(row);
-    h.s[0] = q.x; h.s[1] = q.y; h.s[2] = q.z; h.s[3] = q.w;
-  }
-  return h;
 }
 
 // Nibbles 2 j and 2 j + 1 of word v (consecutive weights) as a pair of 16-bit floats n0 - 8, n1 - 8:
@@ -165,93 +104,172 @@ __device__ __forceinline__ void emit(float a, float b, uint32_t& hi, uint32_t& l
   }
 }
 
-// Weights 32 S .. 32 S + 31 of the unit at `row` (shared memory) -> hi[16] (and lo[16] for kSplit).
-// nf4: the 16 codebook levels in shared memory (one word per bank: lookups never conflict).
-template <int QT, int BF, int MODE, int S>
-__device__ __forceinline__ void convert32(const uint8_t* row, const Hdr& h, const float* nf4, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
+// N consecutive words of a row in shared memory from byte PER * kb (rounded down to a word).  A run-time kb takes
+// word loads; a compile-time one (tc::Int) the widest loads that the row's alignment of ALIGN bytes allows, and
+// the bytes around the words go unused.
+template <int PER, int ALIGN, int N> __device__ __forceinline__ void lds_words(const uint8_t* row, int kb, uint32_t (&w)[N]) {
+  const uint32_t* p = reinterpret_cast<const uint32_t*>(row + ((PER * kb) & ~3));
+#pragma unroll
+  for (int i = 0; i < N; i++) w[i] = p[i];
+}
+template <int PER, int ALIGN, int N, int KB> __device__ __forceinline__ void lds_words(const uint8_t* row, tc::Int<KB>, uint32_t (&w)[N]) {
+  constexpr int at = (PER * KB) & ~3, first = at / ALIGN, count = (at + 4 * N + ALIGN - 1) / ALIGN - first, skip = (at - first * ALIGN) / 4, per = ALIGN / 4;
+  uint32_t v[count * per];
+#pragma unroll
+  for (int i = 0; i < count; i++) {
+    if constexpr (ALIGN == 16) {
+      const uint4 q = *reinterpret_cast<const uint4*>(row + (first + i) * 16);
+      v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
+    } else {
+      const uint2 q = *reinterpret_cast<const uint2*>(row + (first + i) * 8);
+      v[2 * i] = q.x; v[2 * i + 1] = q.y;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < N; i++) w[i] = v[skip + i];
+}
+template <int KB> __device__ __forceinline__ constexpr int block_of(tc::Int<KB>) { return KB; }
+__device__ __forceinline__ int block_of(int kb) { return kb; }
+__device__ __forceinline__ __half low_half(uint32_t v) { return __ushort_as_half((unsigned short)(v & 0xFFFFu)); }
+__device__ __forceinline__ __half high_half(uint32_t v) { return __ushort_as_half((unsigned short)(v >> 16)); }
+// 1024 + n as fp16 is 0x6400 | n: the exact half of a 6-bit field without a conversion instruction
+__device__ __forceinline__ __half half_of6(uint32_t n) {
+  return __hsub(__ushort_as_half((unsigned short)(0x6400u | n)), __ushort_as_half((unsigned short)0x6400));
+}
+
+// Eight weights q ss + sm of one word of nibbles (q = n - 8), in the form MODE asks for
+template <int BF, int MODE> struct Scale { uint32_t s, m; };      // packed pair, or float32 bits
+template <int BF, int MODE> __device__ __forceinline__ Scale<BF, MODE> make_scale(__half ss, __half sm) {
+  if constexpr (BF == 0) return {dup_f16(ss), dup_f16(sm)};
+  else if constexpr (MODE == kFast) return {dup_bf16(__half2float(ss)), dup_bf16(__half2float(sm))};
+  else { const float f = __half2float(ss); return {__float_as_uint(f), __float_as_uint(fmaf(-136.0f, f, __half2float(sm)))}; }
+}
+template <int BF, int MODE> __device__ __forceinline__ void nibbles8(uint32_t v, const Scale<BF, MODE>& c, uint32_t* out) {
+  if constexpr (BF == 0) exact8_f16(v, c.s, c.m, out);
+  else if constexpr (MODE == kFast) fast8_bf16(v, c.s, c.m, out);
+  else put(dequant8_bf16(v, __uint_as_float(c.s), __uint_as_float(c.m)), out);
+}
+
+// Weights 64 kb .. 64 kb + 63 of the unit at `row` (shared memory): out(Int<0>, hi, lo) gets the first 32,
+// out(Int<1>, hi, lo) the others (lo only for kSplit).  nf4: the 16 codebook levels in shared memory (one word per
+// bank: lookups never conflict).  KB is int or tc::Int.  With a run-time kb the body stays at a few hundred
+// instructions that every producer warp shares; unrolled over a unit of the long conversions (kSplit), or
+// specialised per group, the warps of a scheduler fetch more code than its instruction cache holds and
+// wait for it (the largest stall by far: canonical Q4_K [16, 4096] x [37888, 4096]^T 90.9 us unrolled, 52.5
+// us rolled).  The short conversions fit unrolled and are faster so (Q4_K, same size: 27.8 rolled, 24.7).
+template <int QT, int BF, int MODE, typename KB, typename F>
+__device__ __forceinline__ void convert64(const uint8_t* row, KB KBV, const float* nf4, F&& out) {
+  const int kb = block_of(KBV);
+  uint32_t a[16], b[16];
   if constexpr (QT == MLXR_Q4_K) {
-    constexpr int p = S == 1 ? 1 : S == 5 ? 3 : S < 4 ? 0 : 2;     // sub-blocks 0, 2, 3 / 1 / 4, 6, 7 / 5 share a pair
-    const Span<16 + 16 * S, 16, 16> q(row);
+    // d, dmin (fp16), scales[12] of which the shader reads six bytes: (scale, min) pairs 0 .. 3 as eight 6-bit
+    // fields (q_gemm_dequant.metal:222-242); sub-block 2 kb takes the first pair of its half, sub-block
+    // 2 kb + 1 the second one for even kb.  Sub-block scale = rn16(sc * d), min = rn16(m * dmin).
+    const uint4 h = *reinterpret_cast<const uint4*>(row);
+    const uint4 q0 = *reinterpret_cast<const uint4*>(row + 16 + 32 * kb), q1 = *reinterpret_cast<const uint4*>(row + 32 + 32 * kb);
+    const uint32_t f = (kb & 2) ? __funnelshift_r(h.y, h.z, 24) : h.y, g = (kb & 1) ? f : f >> 12;
+    const __half d = low_half(h.x), dmin = high_half(h.x);
+    const auto c0 = make_scale<BF, MODE>(__hmul_rn(half_of6(f & 63u), d), __hmul_rn(half_of6((f >> 6) & 63u), dmin));
+    const auto c1 = make_scale<BF, MODE>(__hmul_rn(half_of6(g & 63u), d), __hmul_rn(half_of6((g >> 6) & 63u), dmin));
+    const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if constexpr (BF == 0) exact8_f16(q.w[i], h.s[p], h.m[p], hi + 4 * i);
-      else if constexpr (MODE == kFast) fast8_bf16(q.w[i], h.s[p], h.m[p], hi + 4 * i);
-      else put(dequant8_bf16(q.w[i], __uint_as_float(h.s[p]), __uint_as_float(h.m[p])), hi + 4 * i);
-    }
-  } else if constexpr (QT == MLXR_Q4_0) {       // 18-byte blocks: fp16 d, 16 bytes of nibbles (q_gemm_dequant.metal:142-161)
-    const Span<18 * S, 18, 16> q(row);
-    const __half d = q.template half<18 * S>();
-    const uint32_t w[4] = {q.template word<18 * S + 2>(), q.template word<18 * S + 6>(), q.template word<18 * S + 10>(), q.template word<18 * S + 14>()};
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[i], c0, a + 4 * i);
+    out(tc::Int<0>{}, a, b);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if constexpr (BF == 0) exact8_f16(w[i], dup_f16(d), 0u, hi + 4 * i);
-      else if constexpr (MODE == kFast) fast8_bf16(w[i], dup_bf16(__half2float(d)), 0u, hi + 4 * i);
-      else { const float s = __half2float(d); put(dequant8_bf16(w[i], s, -136.0f * s), hi + 4 * i); }
-    }
-  } else if constexpr (QT == MLXR_Q8_0) {       // 34-byte blocks: fp16 d, 32 int8 (q_gemm_dequant.metal:190-201)
-    const Span<34 * S, 34, 16> q(row);
-    const __half d = q.template half<34 * S>();
-    const float df = __half2float(d);
-    const uint32_t w[8] = {q.template word<34 * S + 2>(),  q.template word<34 * S + 6>(),  q.template word<34 * S + 10>(), q.template word<34 * S + 14>(),
-                           q.template word<34 * S + 18>(), q.template word<34 * S + 22>(), q.template word<34 * S + 26>(), q.template word<34 * S + 30>()};
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[4 + i], c1, a + 4 * i);
+    out(tc::Int<1>{}, a, b);
+  } else if constexpr (QT == MLXR_Q4_0) {       // two 18-byte blocks: fp16 d, 16 bytes of nibbles (q_gemm_dequant.metal:142-161)
+    uint32_t w[9];
+    lds_words<36, 16>(row, KBV, w);
+    const __half zero = __ushort_as_half((unsigned short)0);
+    const auto c0 = make_scale<BF, MODE>(low_half(w[0]), zero), c1 = make_scale<BF, MODE>(high_half(w[4]), zero);
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const uint32_t u = w[i] ^ 0x80808080u;    // bytes q + 128
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(__funnelshift_r(w[i], w[i + 1], 16), c0, a + 4 * i);
+    out(tc::Int<0>{}, a, b);
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        if constexpr (BF == 0 && MODE != kSplit) {
-          // 1024 + (q + 128) as fp16 is 0x6400 | byte; minus 1152 is q exactly; one rounding of q * d
-          const uint32_t bits = __byte_perm(u, 0x64646464u, j == 0 ? 0x4140 : 0x4342);
-          const __half2 r = __hmul2_rn(__hsub2(*reinterpret_cast<const __half2*>(&bits), __half2half2(__ushort_as_half((unsigned short)0x6480))), __half2half2(d));
-          hi[2 * i + j] = *reinterpret_cast<const uint32_t*>(&r);
-        } else {
-          // byte b one byte up in 0x4300'0000 is the fp32 number 128 + b / 256:
-          // (128 + b / 256) * 256 d - (32768 + 128) d = (b - 128) d
-          const float fe = __uint_as_float(__byte_perm(u, 0x00004300u, 0x5606u | ((uint32_t)(2 * j) << 4)));
-          const float fo = __uint_as_float(__byte_perm(u, 0x00004300u, 0x5606u | ((uint32_t)(2 * j + 1) << 4)));
-          const float s256 = 256.0f * df, c = -32896.0f * df;
-          emit<BF, MODE>(fmaf(fe, s256, c), fmaf(fo, s256, c), hi[2 * i + j], lo[2 * i + j]);
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[5 + i], c1, a + 4 * i);
+    out(tc::Int<1>{}, a, b);
+  } else if constexpr (QT == MLXR_Q8_0) {       // two 34-byte blocks: fp16 d, 32 int8 (q_gemm_dequant.metal:190-201)
+    uint32_t w[17];
+    lds_words<68, 16>(row, KBV, w);
+    auto block = [&](auto S) {
+      constexpr int s = decltype(S)::value;
+      const __half d = s ? high_half(w[8]) : low_half(w[0]);
+      const float df = __half2float(d), s256 = 256.0f * df, c = -32896.0f * df;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const uint32_t u = (s ? w[9 + i] : __funnelshift_r(w[i], w[i + 1], 16)) ^ 0x80808080u;    // bytes q + 128
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          if constexpr (BF == 0 && MODE != kSplit) {
+            // 1024 + (q + 128) as fp16 is 0x6400 | byte; minus 1152 is q exactly; one rounding of q * d
+            const uint32_t bits = __byte_perm(u, 0x64646464u, j == 0 ? 0x4140 : 0x4342);
+            const __half2 r = __hmul2_rn(__hsub2(as_half2(bits), __half2half2(__ushort_as_half((unsigned short)0x6480))), __half2half2(d));
+            a[2 * i + j] = *reinterpret_cast<const uint32_t*>(&r);
+          } else {
+            // byte b one byte up in 0x4300'0000 is the fp32 number 128 + b / 256:
+            // (128 + b / 256) * 256 d - (32768 + 128) d = (b - 128) d
+            const float fe = __uint_as_float(__byte_perm(u, 0x00004300u, 0x5606u | ((uint32_t)(2 * j) << 4)));
+            const float fo = __uint_as_float(__byte_perm(u, 0x00004300u, 0x5606u | ((uint32_t)(2 * j + 1) << 4)));
+            emit<BF, MODE>(fmaf(fe, s256, c), fmaf(fo, s256, c), a[2 * i + j], b[2 * i + j]);
+          }
         }
       }
-    }
-  } else if constexpr (QT == MLXR_NF4) {        // 34-byte blocks of 64: fp16 absmax, 32 bytes of codes
-    constexpr int B = 34 * (S / 2), Q = B + 2 + 16 * (S & 1);
-    const Span<B, 34, 8> q(row);
-    const float a = __half2float(q.template half<B>());
-    const uint32_t w[4] = {q.template word<Q>(), q.template word<Q + 4>(), q.template word<Q + 8>(), q.template word<Q + 12>()};
+      out(S, a, b);
+    };
+    block(tc::Int<0>{});
+    block(tc::Int<1>{});
+  } else if constexpr (QT == MLXR_NF4) {        // one 34-byte block: fp16 absmax, 32 bytes of codes; odd blocks start 2 bytes off a word
+    uint32_t w[9];
+    lds_words<34, 8>(row, KBV, w);
+    const uint32_t sh = (kb & 1) ? 16 : 0;
+    const float am = __half2float((kb & 1) ? high_half(w[0]) : low_half(w[0]));
+    // codes from byte 2 of the block: shifted by 16 bits for even blocks, whole words for odd ones
+    auto block = [&](auto S) {
+      constexpr int s = decltype(S)::value;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+      for (int i = 0; i < 4; i++) {
+        const uint32_t v = sh ? w[4 * s + i + 1] : __funnelshift_r(w[4 * s + i], w[4 * s + i + 1], 16);
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float e = nf4[(w[i] >> (8 * j)) & 15u], o = nf4[(w[i] >> (8 * j + 4)) & 15u];
-        emit<BF, MODE>(e * a, o * a, hi[4 * i + j], lo[4 * i + j]);
+        for (int j = 0; j < 4; j++) {
+          const float e = nf4[(v >> (8 * j)) & 15u], o = nf4[(v >> (8 * j + 4)) & 15u];
+          emit<BF, MODE>(e * am, o * am, a[4 * i + j], b[4 * i + j]);
+        }
       }
+      out(S, a, b);
+    };
+    block(tc::Int<0>{});
+    block(tc::Int<1>{});
   } else if constexpr (QT == MLXR_GGML_Q4_K) {
-    // sub-block S of 64-element chunk S / 2: low (S even) or high nibbles of its 32 bytes; eight
-    // 6-bit (scale, min) pairs; w = (d sc) q - dmin m in float32 (both products are exact)
-    const Span<16 + 32 * (S / 2), 32, 16> q(row);
-    uint32_t sc, mn;
-    if constexpr (S < 4) { sc = (h.s[1] >> (8 * S)) & 63u; mn = (h.s[2] >> (8 * S)) & 63u; }
-    else {
-      constexpr int t = 8 * (S - 4);
-      sc = ((h.s[3] >> t) & 15u) | (((h.s[1] >> (t + 6)) & 3u) << 4);
-      mn = ((h.s[3] >> (t + 4)) & 15u) | (((h.s[2] >> (t + 6)) & 3u) << 4);
-    }
-    const float d = __half2float(__ushort_as_half((unsigned short)(h.s[0] & 0xFFFFu))), dmin = __half2float(__ushort_as_half((unsigned short)(h.s[0] >> 16)));
-    const float ds = d * (float)sc, dm = dmin * (float)mn;
+    // chunk kb: low nibbles of its 32 bytes are sub-block 2 kb, high nibbles sub-block 2 kb + 1; eight 6-bit
+    // (scale, min) pairs, unpacked here four at a time; w = (d sc) q - dmin m in float32 (both products are exact)
+    const uint4 h = *reinterpret_cast<const uint4*>(row);
+    const uint4 q0 = *reinterpret_cast<const uint4*>(row + 16 + 32 * kb), q1 = *reinterpret_cast<const uint4*>(row + 32 + 32 * kb);
+    const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    const uint32_t sc4 = (kb & 2) ? (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu;
+    const uint32_t mn4 = (kb & 2) ? ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu;
+    const float d = __half2float(low_half(h.x)), dmin = __half2float(high_half(h.x));
+    auto block = [&](auto S) {
+      constexpr int s = decltype(S)::value;
+      const int at = 16 * (kb & 1) + 8 * s;
+      const float ds = d * (float)((sc4 >> at) & 0xFFu), dm = dmin * (float)((mn4 >> at) & 0xFFu);
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const uint32_t n = (S & 1) ? (q.w[i] >> 4) & 0x0F0F0F0Fu : q.w[i] & 0x0F0F0F0Fu;
-      float v[4];
+      for (int i = 0; i < 8; i++) {
+        const uint32_t n = (w[i] >> (4 * s)) & 0x0F0F0F0Fu;
+        float v[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        // byte n in the low byte of 0x4B00'0000 is the fp32 number 2^23 + n: exact difference
-        const float f = __uint_as_float(__byte_perm(n, 0x4B000000u, 0x7440u | (uint32_t)j)) - 8388608.0f;
-        v[j] = __fsub_rn(__fmul_rn(ds, f), dm);
+        for (int j = 0; j < 4; j++) {
+          // byte n in the low byte of 0x4B00'0000 is the fp32 number 2^23 + n: exact difference
+          const float f = __uint_as_float(__byte_perm(n, 0x4B000000u, 0x7440u | (uint32_t)j)) - 8388608.0f;
+          v[j] = __fsub_rn(__fmul_rn(ds, f), dm);
+        }
+        emit<BF, MODE>(v[0], v[1], a[2 * i], b[2 * i]);
+        emit<BF, MODE>(v[2], v[3], a[2 * i + 1], b[2 * i + 1]);
       }
-      emit<BF, MODE>(v[0], v[1], hi[2 * i], lo[2 * i]);
-      emit<BF, MODE>(v[2], v[3], hi[2 * i + 1], lo[2 * i + 1]);
-    }
+      out(S, a, b);
+    };
+    block(tc::Int<0>{});
+    block(tc::Int<1>{});
   }
 }
 

@@ -72,4 +72,9 @@ int activation_map(const void* x, int M, int K, int dtype, int rows, CUtensorMap
                    CU_TENSOR_MAP_SWIZZLE_128B, out);
 }
 
+int result_map(void* y, int M, int N, int dtype, int box_cols, int box_rows, CUtensorMap* out) {
+  return encode_2d(dtype == MLXR_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, y, N, M, (size_t)N * 2, box_cols, box_rows,
+                   box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE, out);
+}
+
 }  // namespace mlxr

@@ -13,6 +13,8 @@ namespace mlxr {
 int weight_maps(int qt, const void* w, int N, int K, int tile_rows, CUtensorMap* out, int* odd_shift);
 // X [M, K] of a 16-bit type, boxes of 64 x `rows` with the 128-byte swizzle; rows past M read as zero
 int activation_map(const void* x, int M, int K, int dtype, int rows, CUtensorMap* out);
+// Y [M, N] of a 16-bit type for stores, boxes of box_cols (16: plain, 32: 64-byte swizzle) x box_rows
+int result_map(void* y, int M, int N, int dtype, int box_cols, int box_rows, CUtensorMap* out);
 int device_sms(int* out);
 
 }  // namespace mlxr

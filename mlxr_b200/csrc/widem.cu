@@ -203,32 +203,25 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     const int row_off = (kSplitRows ? mat_off + (local & 1) * (mrows / 2) + (local >> 1) : mat_off + local) * Geo<QT>::kStage;
     const uint32_t col = tmem + R::kA0 + (uint32_t)(g * kSlots * kSlotCols) + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t full[2] = {cluster_map(smem_u32(&sh->full[g * kSlots]), 0), cluster_map(smem_u32(&sh->full[g * kSlots + 1]), 0)};
-    auto loop = [&](auto GC) {
-      constexpr int kb = decltype(GC)::value;
-      int r = 0, sb = sb_first;
-      uint32_t rpar = 0;
-      for (int i = 0; i < nunits; i++) {
-        const int q = i & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->raw_full[r]), rpar, dead))) break;   // warp-uniform
-        const uint8_t* row = rawring + (size_t)r * kRawBytes + row_off;
-        if constexpr (kSplitRows) row += (136 * sb + ((local & 1) ? P.odd_shift : 0)) & 8;
-        const Hdr h = load_header<QT, BF, kRound>(row);
-        uint32_t a[16], b[16];
-        convert32<QT, BF, kRound, 2 * kb>(row, h, sh->nf4, a, b);
-        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty[g * kSlots + q]), (uint32_t)((i >> 1) & 1) ^ 1u, dead))) break;
-        tc_fence_after();
-        tmem_st16(col + q * kSlotCols, a);
-        convert32<QT, BF, kRound, 2 * kb + 1>(row, h, sh->nf4, a, b);
-        tmem_st16(col + q * kSlotCols + 16, a);
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) { mbar_arrive_cluster(full[q]); mbar_arrive(smem_u32(&sh->raw_empty[r])); }
-        if (++r == kRawStages) { r = 0; rpar ^= 1u; }
-        if (++sb == P.nsb) sb = 0;
-      }
-    };
-    if (g == 0) loop(Int<0>{}); else if (g == 1) loop(Int<1>{}); else if (g == 2) loop(Int<2>{}); else loop(Int<3>{});
+    int r = 0, sb = sb_first;
+    uint32_t rpar = 0;
+    for (int i = 0; i < nunits; i++) {
+      const int q = i & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->raw_full[r]), rpar, dead))) break;   // warp-uniform
+      const uint8_t* row = rawring + (size_t)r * kRawBytes + row_off;
+      if constexpr (kSplitRows) row += (136 * sb + ((local & 1) ? P.odd_shift : 0)) & 8;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty[g * kSlots + q]), (uint32_t)((i >> 1) & 1) ^ 1u, dead))) break;
+      tc_fence_after();
+      convert64<QT, BF, kRound>(row, g, sh->nf4, [&](auto H, const uint32_t (&a)[16], const uint32_t (&)[16]) {
+        tmem_st16(col + q * kSlotCols + 16 * decltype(H)::value, a);
+      });
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) { mbar_arrive_cluster(full[q]); mbar_arrive(smem_u32(&sh->raw_empty[r])); }
+      if (++r == kRawStages) { r = 0; rpar ^= 1u; }
+      if (++sb == P.nsb) sb = 0;
+    }
   } else if (warp == kWarpMma) {
    if (rank == 0) {
     // ===== MMA issuer of the pair: the whole warp walks the loop, one elected lane issues =====
@@ -476,10 +469,10 @@ bool widem_supported(int qt, int M, int N, int K, int dtype, const void* x, cons
   return ((((uintptr_t)x) | ((uintptr_t)w)) & 15u) == 0;
 }
 
-// Token tile, grid and dealing of the units.  Time of a unit: 16 MMAs of nt / 2 cycles each, or the
-// conversion of its 32768 weights (about 1300 cycles beside everything else), whichever is longer; a
-// shared tile costs its parts' trip through L2 at the end of the kernel (about 2500 cycles plus 20 per
-// token); a whole tile per CTA needs none of that but leaves SMs idle in the last wave.
+// Token tile, grid and dealing of the units.  Fitted to measurements (65 to 2048 tokens, 14336 x 4096 and 4096 x
+// 14336): a unit takes about 2000 cycles (the conversion of its 65536 weights and the turn-around of a stage)
+// plus 4.3 per token of the tile, a launch 14000 before and after its units; a shared tile costs its parts'
+// trip through L2 at the end; a whole tile per pair needs none of that but leaves SMs idle in the last wave.
 int widem_plan(int M, int rows, int K, WidePlan* out) {
   int sms = 0;
   if (int r = device_sms(&sms)) return r;
@@ -489,13 +482,13 @@ int widem_plan(int M, int rows, int K, WidePlan* out) {
     const int nt = ((M + ntt - 1) / ntt + 15) / 16 * 16;
     if (nt < 16 || nt > 256) continue;
     const long long ntiles = (long long)wtiles * ((M + nt - 1) / nt), U = ntiles * nsb;
-    const double unit = std::max(8.0 * nt, 1300.0), drain = nt > 128 ? 1200.0 + 8.0 * nt : 600.0;
+    const double unit = 2000.0 + 4.3 * nt, drain = nt > 128 ? 1200.0 + 8.0 * nt : 600.0;
     for (int whole = 0; whole < 2; whole++) {
       if (!whole && 2 * ntiles > kSyncWords - 16) continue;        // two counters per tile
       const int G = (int)std::min<long long>(pairs, whole ? ntiles : U);
       double c;
       if (whole) { const double tiles = (double)((ntiles + G - 1) / G); c = tiles * (nsb * unit + drain); }
-      else { const double units = (double)((U + G - 1) / G); c = units * unit + units / nsb * drain + 2500.0 + 20.0 * nt; }
+      else { const double units = (double)((U + G - 1) / G); c = units * unit + units / nsb * drain + 2500.0 + 20.0 * nt + 1200.0 * (double)((nsb + units - 1) / units); }
       if (c < best) {
         best = c;
         out->nt = nt; out->ntt = (M + nt - 1) / nt; out->ntiles = (int)ntiles; out->grid = 2 * G; out->whole = whole;
@@ -503,7 +496,7 @@ int widem_plan(int M, int rows, int K, WidePlan* out) {
       }
     }
   }
-  out->cost_us = best / 1850.0;
+  out->cost_us = (14000.0 + best) / 1750.0;
   return MLXR_OK;
 }
 

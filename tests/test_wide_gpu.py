@@ -1,0 +1,90 @@
+"""Linears of more than 64 tokens (csrc/widem.cu: weights converted beside the MMAs; csrc/dense.cu: converted to
+16 bits in a pass of their own) through the C ABI.
+
+Sizes are the edges of the kernels' tiles: one token more and less than a token tile, weight rows that end inside a
+tile of 128 or 256 and, odd, inside a 16-byte store, an odd number of super-blocks (NF4 rows then start 8 bytes
+off), few and many units per CTA, tiles shared by CTAs, and K that is no multiple of 256 or of 64.
+
+Bound: the products are exact and accumulate in float32; the weight is rounded once to the activation dtype, at
+most 2^-9 (bf16) or 2^-12 (fp16; Q4_K's scale and min round in half precision in both sides) of itself, the result
+once more: the 2-norm of the sum of the two is below 2^-8 and 2^-11."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import make_acts, make_weights
+
+pytestmark = pytest.mark.gpu
+DT = {"f16": torch.float16, "bf16": torch.bfloat16}
+BOUND = {"f16": 2.0 ** -11, "bf16": 2.0 ** -8}
+
+
+def _status():
+    import mlxr_b200 as mx
+    st = torch.zeros(1, dtype=torch.int32)
+    mx._capi.check(mx._capi.lib.mlxr_stream_status(torch.cuda.current_stream().cuda_stream, st.data_ptr()))
+    return int(st[0])
+
+
+def _dense(oracle, packed, N, K, qt):
+    """The weights as float64: the shader's half values for Q4_K, the float32 products otherwise."""
+    f, h = oracle.dequantize(packed, N, K, qt)
+    w = h.view(np.float16) if qt == 3 else f
+    return torch.from_numpy(w.astype(np.float64).reshape(N, K)).cuda()
+
+
+def _check(oracle, qt, dt, M, N, K, bias=True, offset=0):
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    packed = quantize(make_weights(N, K, 7 + M), qt)
+    xt, _ = make_acts(M, K, 8 + M, DT[dt])
+    b = make_acts(1, N, 9, DT[dt])[0][0].contiguous().cuda() if bias else None
+    x = xt.cuda()
+    buf = torch.empty(packed.size + offset, dtype=torch.uint8, device="cuda")
+    w = buf[offset:]
+    w.copy_(torch.from_numpy(packed))
+    args = (x, w, M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt), b)
+    y = mx.q_gemm_dequant(*args)
+    assert torch.equal(y, mx.q_gemm_dequant(*args))     # nothing depends on the order of arrival
+    assert _status() == 0
+    want = x.double() @ _dense(oracle, packed, N, K, qt).T + (b.double() if bias else 0)
+    assert float((y.double() - want).norm() / want.norm()) <= BOUND[dt]
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3, 16])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("M,N,K", [(65, 2, 256), (128, 257, 768), (129, 1000, 1280), (257, 385, 512), (333, 2304, 2816)])
+def test_beside_the_mmas(oracle, qt, dt, M, N, K):
+    _check(oracle, qt, dt, M, N, K)
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3, 16])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("M,N,K", [(2048, 255, 512), (2049, 520, 256), (4095, 1001, 768)])
+def test_in_a_pass_of_its_own(oracle, qt, dt, M, N, K):
+    _check(oracle, qt, dt, M, N, K, bias=(N == 520))
+
+
+@pytest.mark.parametrize("qt,M,N,K,offset", [(0, 9, 33, 96, 0), (2, 130, 300, 320, 0), (16, 70, 129, 448, 0), (0, 100, 256, 512, 2), (2, 20, 64, 256, 2)])
+def test_ragged_k_and_rows_off_16_bytes(oracle, qt, M, N, K, offset):
+    _check(oracle, qt, "f16", M, N, K, offset=offset)
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3, 16])
+@pytest.mark.parametrize("M,H,I", [(100, 768, 1280), (2100, 256, 768)])
+def test_gate_up(oracle, qt, M, H, I):
+    """The SiLU(gate) * up forms of both kernels inside the block, against the block built from this package's own
+    single operators in float64: n and h are rounded to bf16 on both sides (2^-9 each where they differ by an ulp),
+    weights and result once: 1e-2 covers the four."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    g, u, d = (quantize(make_weights(n, k, s), qt) for n, k, s in ((I, H, 1), (I, H, 2), (H, I, 3)))
+    x = make_acts(M, H, 4, torch.bfloat16)[0].cuda()
+    nw = make_acts(1, H, 5, torch.bfloat16)[0][0].contiguous().cuda()
+    y = mx.mlp_block(x, nw, *(torch.from_numpy(w).cuda() for w in (g, u, d)), I, mx.QuantType(qt), 1e-5)
+    assert _status() == 0
+    n = mx.rmsnorm_fused(x, nw, 1e-5).double()
+    gate, up = (n @ _dense(oracle, w, I, H, qt).T for w in (g, u))
+    h = (torch.nn.functional.silu(gate.bfloat16().double()) * up.bfloat16().double()).bfloat16().double()
+    want = h @ _dense(oracle, d, H, I, qt).T
+    assert float((y.double() - want).norm() / want.norm()) <= 1e-2
