@@ -175,15 +175,17 @@ static int run_tc(TcPath path, const WidePlan& wide, const DensePlan& dense, con
 // split-K partial sums; intermediates of the fused entry points start after them.
 static int run_linear(const void* x, const void* w, const void* bias, void* y, int M, int N, int K,
                       int qt, int dtype, cudaStream_t st) {
-  if (M > 0 && N > 0 && stream_gemv_supported(qt, M, K, &w, 1) && !tune_env("MLXR_NO_STREAM")) {
+  if (M > 0 && N > 0 && gemv_supported(qt, M, K, N, dtype, &w, 1)) {
     Workspace* ws = nullptr;
     if (int r = get_workspace(st, 0, &ws)) return r;
     DecodeLinear L;
     memset(&L, 0, sizeof(L));
     L.w[0] = w; L.rows[0] = N; L.nmat = 1; L.K = K; L.x = x; L.y[0] = y; L.bias[0] = bias;
-    return launch_stream_gemv(L, M, dtype, ws->status, st);
+    return launch_gemv(L, M, qt, dtype, ws->status, st);
   }
-  if (M >= 3 && N > 0) {
+  // canonical Q4_K, and NF4 rows that do not start on 16 bytes, have no kernel of their own for one or two tokens
+  const bool small_only = qt == MLXR_GGML_Q4_K || (qt == MLXR_NF4 && !gemv_rows_supported(qt, M, K, x, w));
+  if ((M >= 3 || (M > 0 && small_only)) && N > 0) {
     TcPath path;
     WidePlan wide;
     DensePlan dense;
@@ -465,9 +467,13 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
   TcPath path = kTcNone;
   WidePlan wide;
   DensePlan dense;
-  if (M >= 3) if (int r = tc_path(qt, M, inter, hidden, dtype, x, w_gate, w_up, &wide, &dense, &path)) return r;
+  // (NF4 has no fused form of its own below three tokens)
+  if (M >= 3 || qt == MLXR_NF4) if (int r = tc_path(qt, M, inter, hidden, dtype, x, w_gate, w_up, &wide, &dense, &path)) return r;
   const bool small = path != kTcNone && (path != kTcSmall || (2 * inter + 127) / 128 <= kSyncWords - 16);
-  const bool decode = !small && decode_supported(qt, M, hidden, wgu, 2) && decode_supported(qt, M, inter, &w_down, 1);
+  // one or two tokens: [RMSNorm ->] gate/up with the SiLU(gate) * up epilogue, then down: two launches, the second
+  // one's weights on their way before the first has ended
+  const bool gemv = gemv_supported(qt, M, hidden, 2 * inter, dtype, wgu, 2) && gemv_supported(qt, M, inter, hidden, dtype, &w_down, 1);
+  const bool decode = !small && !gemv && decode_supported(qt, M, hidden, wgu, 2) && decode_supported(qt, M, inter, &w_down, 1);
   if (int r = get_workspace(st, decode ? kDecodeScratchBytes : kDecodeScratchBytes + n_bytes + 2 * i_bytes, &ws, 0,
                             decode ? decode_tagged_bytes(M, inter, dtype) : 0))
     return r;
@@ -487,6 +493,17 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
   }
   void* nbuf = base;
   void* gbuf = base + n_bytes;
+  if (gemv) {
+    DecodeLinear L;
+    memset(&L, 0, sizeof(L));
+    L.w[0] = w_gate; L.w[1] = w_up; L.rows[0] = L.rows[1] = inter; L.nmat = 2;
+    L.interleave = 1; L.K = hidden; L.x = x; L.gamma = norm_weight; L.eps = eps; L.y[0] = gbuf;
+    if (int r = launch_gemv(L, M, qt, dtype, ws->status, st)) return r;
+    memset(&L, 0, sizeof(L));
+    L.w[0] = w_down; L.rows[0] = hidden; L.nmat = 1; L.K = inter; L.x = gbuf; L.y[0] = y;
+    if (y_f32) L.epi[0] = 3;
+    return launch_gemv(L, M, qt, dtype, ws->status, st);
+  }
   void* ubuf = base + n_bytes + i_bytes;
   const void* n = x;
   if (norm_weight) {
@@ -600,7 +617,7 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
   Workspace* ws = nullptr;
   if (int r = get_workspace(st, kDecodeScratchBytes + align_up((size_t)M * hidden * es, 256), &ws)) return r;
   const void* wqkv[3] = {wq, wk, wv};
-  if (stream_gemv_supported(qt, M, hidden, wqkv, 3) && !tune_env("MLXR_NO_STREAM")) {
+  if (gemv_supported(qt, M, hidden, (q_heads + 2 * kv_heads) * head_dim, dtype, wqkv, 3) && q_heads * head_dim % 4 == 0 && kv_heads * head_dim % 4 == 0) {
     DecodeLinear L;
     memset(&L, 0, sizeof(L));
     L.w[0] = wq; L.w[1] = wk; L.w[2] = wv;
@@ -610,7 +627,7 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
     L.epi[0] = L.epi[1] = 2;
     L.cos_t = cos_f16; L.sin_t = sin_f16; L.positions = positions;
     L.head_dim = head_dim; L.max_seq = max_seq_len; L.pos_offset = position_offset;
-    return launch_stream_gemv(L, M, dtype, ws->status, st);
+    return launch_gemv(L, M, qt, dtype, ws->status, st);
   }
   if (decode_supported(qt, M, hidden, wqkv, 3)) {
     // one launch: [RMSNorm ->] q, k, v stacked along N, RoPE in the epilogue of q and k rows

@@ -76,7 +76,7 @@ template <int QT> __device__ __forceinline__ Word8<QT> load8w(const uint8_t* row
 }
 
 template <int QT, int BF> __device__ __forceinline__ uint4 convert8w(const Word8<QT>& o, int w, const float* nf4) {
-  uint32_t r[4], lo = 0;
+  uint32_t r[4] = {}, lo = 0;
   if constexpr (QT == MLXR_Q4_K) {
     // sub-blocks 0, 2, 3 / 1 / 4, 6, 7 / 5 share (scale, min) pairs 0 / 1 / 2 / 3: 6-bit fields from bit 12 p
     const int s = (w >> 2) & 7, p = (s >> 2) * 2 + ((s & 3) == 1 ? 1 : 0);

@@ -1,0 +1,689 @@
+// Linears for one or two tokens (Q4_K, Q4_0, Q8_0), single, stacked along N (q / k / v) or gate / up.
+//
+// Roofline: HBM.  Two things kept the earlier kernels at 0.4 of it: the time between a launch's end and the next
+// one's first product, because each filled its SM and nothing of the next launch could be there, and a
+// meeting of all warps for every 16 rows.  Here
+//   * a CTA (one per SM) takes at most half of the SM's shared memory, registers and threads, so that under
+//     programmatic stream serialization the next launch's CTA sits beside it, its ring full of weights, and
+//     only waits for its activations;
+//   * a CTA owns a contiguous range of rows (in granules of four: 14336 rows are 24 or 25 granules each on 148
+//     SMs); its work units, (16-row tile, stage of K), are dealt to the eight warps in contiguous ranges, every
+//     warp keeps its own sums, and the warps meet once, at the end, when all partial sums lie in shared
+//     memory and are added in warp order (deterministic);
+//   * every warp fills its own ring with 2-D tensor TMA (four boxes of 4 rows per stage) and drains it, so
+//     nothing inside the stream waits on another warp.
+//
+// Arithmetic, 4-bit formats: activations as 16-bit fixed point per 256 elements, split in a high and a low
+// signed byte; raw nibbles multiplied as unsigned bytes by mma.sync.m16n8k32 (the 16 MMA rows are weight
+// rows); scales and the offset term in float32.  Q8_0: q is exact in fp16, so are the activations (bf16 ones
+// times a power of two per segment), mma.sync.m16n8k16 with float32 accumulation, the block's scale on the sum.  In both the MMA's columns
+// keep apart what has a scale of its own: a thread's part of the K range is one block (or (scale, min) pair)
+// and its B fragment is zero outside that block's columns, so each thread ends up with the sums of the block
+// whose scale it holds and no shuffles are needed before the end.
+#include <atomic>
+#include <cstring>
+#include <mutex>
+
+#include "decode_kernel.cuh"
+#include "kernels.h"
+#include "weight_maps.h"
+
+namespace mlxr {
+namespace gemv {
+
+using decode::bounded_wait;
+using decode::imma16832;
+using decode::load8;
+using decode::mbar_arrive_expect_tx;
+using decode::mbar_init;
+using decode::mbar_wait;
+using decode::smem_u32;
+using decode::tma_load_2d;
+
+constexpr int kWarps = 16, kThreads = kWarps * 32;
+constexpr int kMaxStages = 4;
+constexpr int kSmemMax = 227 * 1024;
+
+// Bytes of 256 weights of a row, 256-element segments per stage, and sums of the activations kept per segment
+template <int QT> struct Geo {
+  static constexpr int kSeg = QT == MLXR_Q8_0 ? 272 : 144;
+  static constexpr int kSegs = QT == MLXR_Q8_0 ? 1 : 2;
+  static constexpr int kPitch = kSeg * kSegs;
+  static constexpr int kBox = (4 * kPitch + 127) & ~127;     // four rows; TMA wants 128-byte aligned places in shared memory
+  static constexpr int kStage = 4 * kBox;
+  static constexpr int kAux = QT == MLXR_Q4_K ? 4 : QT == MLXR_Q4_0 ? 8 : 0;
+};
+
+struct Params {
+  alignas(64) CUtensorMap map[3];
+  int rows[3];
+  int nmat, interleave;      // interleave: map[0] gate, map[1] up; y[0] = h [M, rows[0]]
+  int n_total, granules;     // rows (h elements) and granules of four of them
+  int K, nseg, nst;          // nst: stages per row
+  int M;
+  const void* x;
+  const void* gamma;
+  float eps;
+  void* y[3];
+  const void* bias[3];
+  int epi[3];                // decode::Epilogue
+  const __half* cos_t;
+  const __half* sin_t;
+  const int32_t* positions;
+  int head_dim, max_seq, pos_offset;
+  int* status;
+  unsigned long long wait_ns;
+  int stages, x_stride;
+  int off_x, off_aux, off_delta, off_sums, off_head, off_misc;
+};
+struct Misc {
+  unsigned long long full[kWarps][kMaxStages];
+  float red[kWarps * 2];
+  float rinv[2];             // 1 / rms of the batch rows
+  int dead;
+};
+
+// Fixed-point conversion of one (batch row, segment): v holds this lane's eight activations.  x ~ delta * xi with
+// |xi| <= 32000, xi = 256 hi + lo as two signed-byte rows in MMA k order, and the exact integer sums of xi that
+// the offset / min terms need.  1.5 * 2^23 added in the multiply leaves xi, rounded to nearest, in the low bits.
+template <int QT>
+__device__ __forceinline__ void emit_fixed(uint8_t* smem, const Params& P, int m, int sg, int lane, const float (&v)[8]) {
+  float amax = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
+  // non-negative floats order like their bit patterns (NaN and Inf sort above every finite value)
+  amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+  float dl = 1.0f, inv = 0.0f;
+  if (!(amax <= 3.0e38f)) { dl = __int_as_float(0x7fc00000); }   // a non-finite block poisons its outputs
+  else if (amax > 0.0f) { dl = amax * (1.0f / 32000.0f); inv = __fdividef(32000.0f, amax); }
+  uint32_t t[8], sum = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) { t[i] = __float_as_uint(fmaf(v[i], inv, 12582912.0f)); sum += t[i]; }
+  const int ssum = (int)(sum - 8u * 0x4B400000u);
+  // bytes of an 8-group are stored as (e0,e2,e4,e6 | e1,e3,e5,e7): the MMA k order
+  uint8_t* row = smem + P.off_x + (size_t)(2 * m) * P.x_stride + sg * 256 + lane * 8;
+  const uint32_t lo_e = __byte_perm(__byte_perm(t[0], t[2], 0x0040), __byte_perm(t[4], t[6], 0x0040), 0x5410);
+  const uint32_t lo_o = __byte_perm(__byte_perm(t[1], t[3], 0x0040), __byte_perm(t[5], t[7], 0x0040), 0x5410);
+#pragma unroll
+  for (int i = 0; i < 8; i++) t[i] += 128u;                       // q = 256 h + l, both in [-128, 127]
+  const uint32_t hi_e = __byte_perm(__byte_perm(t[0], t[2], 0x0051), __byte_perm(t[4], t[6], 0x0051), 0x5410);
+  const uint32_t hi_o = __byte_perm(__byte_perm(t[1], t[3], 0x0051), __byte_perm(t[5], t[7], 0x0051), 0x5410);
+  *reinterpret_cast<uint2*>(row) = make_uint2(hi_e, hi_o);
+  *reinterpret_cast<uint2*>(row + P.x_stride) = make_uint2(lo_e, lo_o);
+  float* aux = reinterpret_cast<float*>(smem + P.off_aux) + ((size_t)m * P.nseg + sg) * Geo<QT>::kAux;
+  if (lane == 0) reinterpret_cast<float*>(smem + P.off_delta)[m * P.nseg + sg] = dl;
+  // sums per sub-block of 32 (four lanes)
+  int s4 = ssum;
+  s4 += __shfl_xor_sync(0xffffffffu, s4, 1);
+  s4 += __shfl_xor_sync(0xffffffffu, s4, 2);
+  if constexpr (QT == MLXR_Q4_0) {
+    if ((lane & 3) == 0) aux[lane >> 2] = (float)s4;
+  } else {
+    // per (scale, min) pair: sub-blocks {0,2,3}, {1}, {4,6,7}, {5} (q_gemm_dequant.metal:222-242)
+    const int base = lane & 16;
+    const int a = __shfl_sync(0xffffffffu, s4, base), b = __shfl_sync(0xffffffffu, s4, base + 4);
+    const int c = __shfl_sync(0xffffffffu, s4, base + 8), d = __shfl_sync(0xffffffffu, s4, base + 12);
+    if ((lane & 15) == 0) *reinterpret_cast<float2*>(aux + (lane >> 3)) = make_float2((float)(a + c + d), (float)b);
+  }
+}
+
+// Per-thread constants of the MMA mapping: lane = 4 g + c
+struct Lane {
+  int g, c, rg;              // MMA rows g and g + 8 are tile rows rg and rg + 8 (rows two apart lie 16 banks apart)
+  bool keep0, keep1;         // this thread's B fragment belongs to its column (first / second half of the segment)
+  int sh1, sh2;
+};
+__device__ __forceinline__ Lane make_lane(int lane, int qt) {
+  Lane L;
+  L.g = lane >> 2;
+  L.c = lane & 3;
+  L.rg = (L.g & 4) | ((L.g & 1) << 1) | ((L.g >> 1) & 1);
+  if (qt == MLXR_Q4_K) {
+    // sub-block s belongs to pair {0,1,0,0,2,3,2,2}[s]; MMA column g stands for pair g >> 1
+    L.keep0 = (int)((0x22320010u >> (4 * L.c)) & 7u) == (L.g >> 1);
+    L.keep1 = (int)((0x22320010u >> (4 * (L.c + 4))) & 7u) == (L.g >> 1);
+  } else {
+    L.keep0 = L.keep1 = (L.g >> 1) == L.c;    // columns 2 c and 2 c + 1 stand for thread c's own block
+  }
+  L.sh1 = L.c < 2 ? 12 * L.c : 24;
+  L.sh2 = L.c == 3 ? 12 : 0;
+  return L;
+}
+
+// One segment (256 weights) of 16 rows.  rl / rh: rows rg and rg + 8 in the stage at the segment; sg: segment of K.
+// tot[j][h] gets this thread's part of batch row j, tile row rg + 8 h.
+//
+// Q4_K: thread c feeds the words of sub-block c, then 4 + c; columns 2 p + part stand for (scale, min) pair p, and
+// the thread ends up with pair c's sums.  High nibbles stay in place (w & 0xf0f0f0f0 = 16 x nibble) and
+// accumulate apart: two logic operations per word and two independent MMA chains.
+template <int NT>
+__device__ __forceinline__ void seg_q4k(const uint8_t* rl, const uint8_t* rh, const uint8_t* smem, const Params& P, int sg, const Lane& L, float (&tot)[NT][2]) {
+  const uint4 hl = *reinterpret_cast<const uint4*>(rl), hh = *reinterpret_cast<const uint4*>(rh);
+  int lo[NT][4] = {}, hi[NT][4] = {};
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const bool keep = h ? L.keep1 : L.keep0;
+    const uint4 wl = *reinterpret_cast<const uint4*>(rl + 16 + 64 * h + 16 * L.c), wh = *reinterpret_cast<const uint4*>(rh + 16 + 64 * h + 16 * L.c);
+    uint4 xa[NT], xb[NT];
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+      xa[j] = xb[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (keep) {
+        const uint8_t* xr = smem + P.off_x + (size_t)(2 * j + (L.g & 1)) * P.x_stride + sg * 256 + 128 * h + 32 * L.c;
+        xa[j] = *reinterpret_cast<const uint4*>(xr);
+        xb[j] = *reinterpret_cast<const uint4*>(xr + 16);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const uint32_t wa = i == 0 ? wl.x : wl.z, wb = i == 0 ? wl.y : wl.w, va = i == 0 ? wh.x : wh.z, vb = i == 0 ? wh.y : wh.w;
+#pragma unroll
+      for (int j = 0; j < NT; j++) {
+        const uint4 xv = i == 0 ? xa[j] : xb[j];
+        imma16832(lo[j], wa & 0x0f0f0f0fu, va & 0x0f0f0f0fu, wb & 0x0f0f0f0fu, vb & 0x0f0f0f0fu, xv.x, xv.z);
+        imma16832(hi[j], wa & 0xf0f0f0f0u, va & 0xf0f0f0f0u, wb & 0xf0f0f0f0u, vb & 0xf0f0f0f0u, xv.y, xv.w);
+      }
+    }
+  }
+  // pair c of both rows: 6-bit fields at bit 12 c (scale) and 12 c + 6 (min) of scales[0..5]; sub-block scale =
+  // rn16(sc * d), min = rn16(m * dmin); w = (q - 8) ss + sm = q ss + (sm - 8 ss)
+  const uint32_t ul = __funnelshift_r(hl.y, hl.z, L.sh1) >> L.sh2, uh = __funnelshift_r(hh.y, hh.z, L.sh1) >> L.sh2;
+  const __half2 dl2 = *reinterpret_cast<const __half2*>(&hl.x), dh2 = *reinterpret_cast<const __half2*>(&hh.x);
+  const float ss_l = __half2float(__hmul(__int2half_rn((int)(ul & 63u)), __low2half(dl2)));
+  const float ss_h = __half2float(__hmul(__int2half_rn((int)(uh & 63u)), __low2half(dh2)));
+  const float sm_l = __half2float(__hmul(__int2half_rn((int)((ul >> 6) & 63u)), __high2half(dl2)));
+  const float sm_h = __half2float(__hmul(__int2half_rn((int)((uh >> 6) & 63u)), __high2half(dh2)));
+  const float of_l = fmaf(-8.0f, ss_l, sm_l), of_h = fmaf(-8.0f, ss_h, sm_h);
+#pragma unroll
+  for (int j = 0; j < NT; j++) {
+    const float sx = reinterpret_cast<const float*>(smem + P.off_aux)[((size_t)j * P.nseg + sg) * 4 + L.c];
+    const float dl = reinterpret_cast<const float*>(smem + P.off_delta)[j * P.nseg + sg];
+    // the high-nibble sums are exact multiples of 16
+    const float v0 = (float)((lo[j][0] + (hi[j][0] >> 4)) * 256 + (lo[j][1] + (hi[j][1] >> 4)));
+    const float v1 = (float)((lo[j][2] + (hi[j][2] >> 4)) * 256 + (lo[j][3] + (hi[j][3] >> 4)));
+    tot[j][0] = fmaf(dl, fmaf(ss_l, v0, of_l * sx), tot[j][0]);
+    tot[j][1] = fmaf(dl, fmaf(ss_h, v1, of_h * sx), tot[j][1]);
+  }
+}
+
+// N words from a 2-byte aligned place whose first word also holds the 16 bits before them: odd = the scale is the
+// high half of the first word and the words follow whole, else it is the low half and they are 16 bits off
+template <int N> __device__ __forceinline__ void words_after_scale(const uint8_t* p, bool odd, __half& d, uint32_t (&v)[N]) {
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(p - (odd ? 2 : 0));
+  uint32_t w[N + 1];
+#pragma unroll
+  for (int i = 0; i <= N; i++) w[i] = q[i];
+  d = __ushort_as_half((unsigned short)(odd ? w[0] >> 16 : w[0] & 0xFFFFu));
+#pragma unroll
+  for (int i = 0; i < N; i++) v[i] = __funnelshift_rc(w[i], w[i + 1], odd ? 32 : 16);
+}
+
+// Q4_0: thread c feeds block 4 i + c (18 bytes), columns 2 c and 2 c + 1 stand for the high and low bytes of its x
+template <int NT>
+__device__ __forceinline__ void seg_q40(const uint8_t* rl, const uint8_t* rh, const uint8_t* smem, const Params& P, int sg, const Lane& L, float (&tot)[NT][2]) {
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int at = 72 * i + 18 * L.c;
+    __half dl, dh;
+    uint32_t wl[4], wh[4];
+    words_after_scale<4>(rl + at, L.c & 1, dl, wl);
+    words_after_scale<4>(rh + at, L.c & 1, dh, wh);
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+      uint4 xa = make_uint4(0u, 0u, 0u, 0u), xb = xa;
+      if (L.keep0) {
+        const uint8_t* xr = smem + P.off_x + (size_t)(2 * j + (L.g & 1)) * P.x_stride + sg * 256 + 128 * i + 32 * L.c;
+        xa = *reinterpret_cast<const uint4*>(xr);
+        xb = *reinterpret_cast<const uint4*>(xr + 16);
+      }
+      int lo[4] = {}, hi[4] = {};
+      imma16832(lo, wl[0] & 0x0f0f0f0fu, wh[0] & 0x0f0f0f0fu, wl[1] & 0x0f0f0f0fu, wh[1] & 0x0f0f0f0fu, xa.x, xa.z);
+      imma16832(hi, wl[0] & 0xf0f0f0f0u, wh[0] & 0xf0f0f0f0u, wl[1] & 0xf0f0f0f0u, wh[1] & 0xf0f0f0f0u, xa.y, xa.w);
+      imma16832(lo, wl[2] & 0x0f0f0f0fu, wh[2] & 0x0f0f0f0fu, wl[3] & 0x0f0f0f0fu, wh[3] & 0x0f0f0f0fu, xb.x, xb.z);
+      imma16832(hi, wl[2] & 0xf0f0f0f0u, wh[2] & 0xf0f0f0f0u, wl[3] & 0xf0f0f0f0u, wh[3] & 0xf0f0f0f0u, xb.y, xb.w);
+      const float sx = reinterpret_cast<const float*>(smem + P.off_aux)[((size_t)j * P.nseg + sg) * 8 + 4 * i + L.c];
+      const float dx = reinterpret_cast<const float*>(smem + P.off_delta)[j * P.nseg + sg];
+      const float v0 = (float)((lo[0] + (hi[0] >> 4)) * 256 + (lo[1] + (hi[1] >> 4)));
+      const float v1 = (float)((lo[2] + (hi[2] >> 4)) * 256 + (lo[3] + (hi[3] >> 4)));
+      tot[j][0] = fmaf(dx * __half2float(dl), fmaf(-8.0f, sx, v0), tot[j][0]);
+      tot[j][1] = fmaf(dx * __half2float(dh), fmaf(-8.0f, sx, v1), tot[j][1]);
+    }
+  }
+}
+
+__device__ __forceinline__ void hmma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Bytes 2 J and 2 J + 1 of four signed bytes, plus 128 each, as a pair of fp16 numbers, exactly: 1024 + b is 0x6400 | b
+template <int J> __device__ __forceinline__ uint32_t pair_of_bytes(uint32_t u) {
+  const uint32_t b = __byte_perm(u, 0x64646464u, J == 0 ? 0x4140u : 0x4342u), k = 0x64806480u;
+  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&b), *reinterpret_cast<const __half2*>(&k));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// Q8_0: thread c feeds block 4 i + c (34 bytes); columns 2 c and 2 c + 1 stand for its two batch rows
+template <bool SCALED, int NT>
+__device__ __forceinline__ void seg_q80(const uint8_t* rl, const uint8_t* rh, const uint8_t* smem, const Params& P, int sg, const Lane& L, float (&tot)[NT][2]) {
+  const bool keep = L.keep0 && (L.g & 1) < NT;
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int at = 136 * i + 34 * L.c;
+    __half dl, dh;
+    uint32_t wl[8], wh[8];
+    words_after_scale<8>(rl + at, L.c & 1, dl, wl);
+    words_after_scale<8>(rh + at, L.c & 1, dh, wh);
+    float acc[2][4] = {};
+    const uint8_t* xr = smem + P.off_x + (size_t)(L.g & 1) * P.x_stride + (sg * 256 + 128 * i + 32 * L.c) * 2;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      uint4 xv = make_uint4(0u, 0u, 0u, 0u);
+      if (keep) xv = *reinterpret_cast<const uint4*>(xr + 16 * q);
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const uint32_t ul = wl[2 * q + k] ^ 0x80808080u, uh = wh[2 * q + k] ^ 0x80808080u;
+        hmma16816(acc[k], pair_of_bytes<0>(ul), pair_of_bytes<0>(uh), pair_of_bytes<1>(ul), pair_of_bytes<1>(uh), k ? xv.z : xv.x, k ? xv.w : xv.y);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+      const float dx = SCALED ? reinterpret_cast<const float*>(smem + P.off_delta)[j * P.nseg + sg] : 1.0f;
+      tot[j][0] = fmaf(__half2float(dl) * dx, acc[0][j] + acc[1][j], tot[j][0]);
+      tot[j][1] = fmaf(__half2float(dh) * dx, acc[0][2 + j] + acc[1][2 + j], tot[j][1]);
+    }
+  }
+}
+
+template <int QT, typename T, int NT>
+__global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant__ Params P) {
+  using G_ = Geo<QT>;
+  extern __shared__ __align__(128) uint8_t smem[];
+  Misc* misc = reinterpret_cast<Misc*>(smem + P.off_misc);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int D = P.stages, S = P.nst;
+
+  // this CTA's granules, its tiles, and this warp's units [ub, ue): unit u = (tile u / S, stage u % S)
+  const int g0 = (int)(((long long)P.granules * blockIdx.x) / gridDim.x), g1 = (int)(((long long)P.granules * (blockIdx.x + 1)) / gridDim.x);
+  const int gpt = P.interleave ? 2 : 4, ntiles = (g1 - g0 + gpt - 1) / gpt, units = ntiles * S;
+  const int ub = (units * warp) / kWarps, ue = (units * (warp + 1)) / kWarps;
+
+  // The activations' and the norm weight's lines and pages are asked for first, into L2 only: the data itself is
+  // read after griddepcontrol.wait.
+  {
+    const int xl = (int)(((size_t)NT * P.K * sizeof(T) + 127) >> 7), gl = P.gamma ? (int)(((size_t)P.K * sizeof(T) + 127) >> 7) : 0;
+    for (int i = tid; i < xl + gl; i += kThreads)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(i < xl ? (const char*)P.x + (size_t)i * 128 : (const char*)P.gamma + (size_t)(i - xl) * 128));
+  }
+  // ---- this warp's copy stream; weights are constants of the model, so it starts before the activations are there ----
+  const uint32_t ring = smem_u32(smem) + warp * D * G_::kStage;
+  int i_tile = ub / S, i_st = ub - i_tile * S, i_slot = 0, i_left = ue - ub;
+  auto issue = [&]() {
+    if (i_left <= 0) return;
+    i_left--;
+    const int first = g0 + i_tile * gpt, have = min(gpt, g1 - first);
+    const uint32_t bar = smem_u32(&misc->full[warp][i_slot]);
+    if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)(P.interleave ? 2 * have : have) * (4 * G_::kPitch));
+    __syncwarp();
+    if (lane < 4) {
+      const int k = P.interleave ? (lane & 1) : lane;
+      if (k < have) {
+        int m = 0, row = 4 * (first + k);
+        if (P.interleave) m = lane >> 1;
+        else if (P.nmat > 1 && row >= P.rows[0]) { row -= P.rows[0]; m = 1; if (P.nmat > 2 && row >= P.rows[1]) { row -= P.rows[1]; m = 2; } }
+        tma_load_2d(ring + i_slot * G_::kStage + lane * G_::kBox, &P.map[m], i_st * (G_::kPitch / 8), row, bar);
+      }
+    }
+    if (++i_slot == D) i_slot = 0;
+    if (++i_st == S) { i_st = 0; i_tile++; }
+  };
+  if (lane == 0) {
+    for (int s = 0; s < D; s++) mbar_init(smem_u32(&misc->full[warp][s]), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (warp == 0) misc->dead = 0;
+  }
+  __syncwarp();
+  // Half of the ring now, the rest once the activations' loads are on their way: requested behind a full ring
+  // of every SM (22 MB), they came 3 us after the previous kernel's end instead of 1.5.
+  for (int i = 0; i < D / 2; i++) issue();
+  int held = D - D / 2;
+  auto issue_held = [&]() { for (; held > 0; held--) issue(); };
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  // ---- activations: a warp per segment of 256 ----
+  const T* xg = reinterpret_cast<const T*>(P.x);
+  const T* gam = reinterpret_cast<const T*>(P.gamma);
+  // up to four segments (v) of batch row m from s0 on, kWarps apart
+  auto load_x = [&](int m, int s0, float (&v)[4][8]) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) if (s0 + u * kWarps < P.nseg) load8(xg + (size_t)m * P.K + (s0 + u * kWarps) * 256 + lane * 8, v[u]);
+  };
+  if constexpr (QT == MLXR_Q8_0) {
+    // fp16 as they are; bf16 times a power of two per segment that brings its largest value to 2^14 .. 2^15, as fp16:
+    // exact for every value above 2^-31 of the largest, so the products are those of the bf16 values and the
+    // weights need only the cheaper conversion to fp16.  With RMSNorm the norm is rounded to T first, so the
+    // row's sum of squares comes before.
+    float rinv[NT];
+#pragma unroll
+    for (int m = 0; m < NT; m++) {
+      rinv[m] = 1.0f;
+      if (gam) {
+        float ss = 0.0f;
+        for (int s0 = warp; s0 < P.nseg; s0 += 4 * kWarps) {
+          float v[4][8];
+          load_x(m, s0, v);
+          issue_held();
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (s0 + u * kWarps < P.nseg)
+#pragma unroll
+              for (int i = 0; i < 8; i++) ss = fmaf(v[u][i], v[u][i], ss);
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) misc->red[warp * NT + m] = ss;
+      }
+    }
+    if (gam) {
+      __syncthreads();
+#pragma unroll
+      for (int m = 0; m < NT; m++) {
+        float tot = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) tot += misc->red[w * NT + m];
+        rinv[m] = 1.0f / sqrtf(tot / (float)P.K + P.eps);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < NT; m++)
+      for (int s0 = warp; s0 < P.nseg; s0 += 4 * kWarps) {
+        float v[4][8];
+        load_x(m, s0, v);
+        issue_held();
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int sg = s0 + u * kWarps;
+          if (sg >= P.nseg) break;
+          if (gam) {
+            float gv[8];
+            load8(gam + sg * 256 + lane * 8, gv);
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[u][i] = Act<T>::to_f(Act<T>::from_f(__fmul_rn(__fmul_rn(v[u][i], rinv[m]), gv[i])));
+          }
+          float scale = 1.0f;
+          if constexpr (Act<T>::kDtype == MLXR_BF16) {
+            float amax = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[u][i]));
+            const int e = (int)(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)) >> 23);     // biased exponent
+            const int se = e == 0 || e == 255 ? 127 : min(254, 268 - e);                            // 2^14 / 2^(e - 127)
+            scale = __int_as_float(se << 23);
+            if (lane == 0) reinterpret_cast<float*>(smem + P.off_delta)[m * P.nseg + sg] = 1.0f / scale;
+          }
+          __half o[8];
+#pragma unroll
+          for (int i = 0; i < 8; i++) o[i] = __float2half_rn(v[u][i] * scale);
+          *reinterpret_cast<uint4*>(smem + P.off_x + (size_t)m * P.x_stride + (sg * 256 + lane * 8) * 2) = *reinterpret_cast<const uint4*>(o);
+        }
+      }
+  } else {
+    // fixed point; the block scaling is independent of a factor common to the row, so 1 / rms multiplies the sums at
+    // the end and the conversion does not wait for the sum of squares
+#pragma unroll
+    for (int m = 0; m < NT; m++) {
+      float ss = 0.0f;
+      for (int s0 = warp; s0 < P.nseg; s0 += 4 * kWarps) {
+        float v[4][8];
+        load_x(m, s0, v);
+        if (!gam) issue_held();
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int sg = s0 + u * kWarps;
+          if (sg >= P.nseg) break;
+          if (gam) {
+            float gv[8];
+            load8(gam + sg * 256 + lane * 8, gv);
+            issue_held();
+#pragma unroll
+            for (int i = 0; i < 8; i++) { ss = fmaf(v[u][i], v[u][i], ss); v[u][i] *= gv[i]; }
+          }
+          emit_fixed<QT>(smem, P, m, sg, lane, v[u]);
+        }
+      }
+      if (gam) {
+        ss = warp_sum(ss);
+        if (lane == 0) misc->red[warp * NT + m] = ss;
+      }
+    }
+  }
+  issue_held();
+  __syncthreads();
+  if (QT != MLXR_Q8_0 && gam && tid >= kThreads - NT) {
+    const int m = kThreads - 1 - tid;
+    float tot = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) tot += misc->red[w * NT + m];
+    misc->rinv[m] = 1.0f / sqrtf(tot / (float)P.K + P.eps);
+  }
+
+  // ---- the stream ----
+  const Lane L = make_lane(lane, QT);
+  float* sums = reinterpret_cast<float*>(smem + P.off_sums);            // [ntiles][16][NT]: the part that begins a tile
+  float* head = reinterpret_cast<float*>(smem + P.off_head) + warp * 16 * NT;   // this warp's later part of its first tile
+  float tot[NT][2] = {};
+  int tile = ub / S, st = ub - tile * S, slot = 0;
+  bool own = st == 0;                                                   // this warp holds the tile's first stage
+  uint32_t par = 0;
+  for (int u = ub; u < ue; u++) {
+    const uint8_t* stage = smem + (size_t)(warp * D + slot) * G_::kStage;
+    mbar_wait(smem_u32(&misc->full[warp][slot]), par, &misc->dead, P.wait_ns);
+    const uint8_t *rl = stage + (L.rg >> 2) * G_::kBox + (L.rg & 3) * G_::kPitch, *rh = rl + 2 * G_::kBox;
+    const int sg = st * G_::kSegs;
+    if constexpr (QT == MLXR_Q8_0) {
+      seg_q80<Act<T>::kDtype == MLXR_BF16, NT>(rl, rh, smem, P, sg, L, tot);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        if (k && sg + 1 >= P.nseg) break;
+        if constexpr (QT == MLXR_Q4_K) seg_q4k<NT>(rl + k * 144, rh + k * 144, smem, P, sg + k, L, tot);
+        else seg_q40<NT>(rl + k * 144, rh + k * 144, smem, P, sg + k, L, tot);
+      }
+    }
+    if (++slot == D) { slot = 0; par ^= 1u; }
+    __syncwarp();
+    issue();      // refill the stage that was just drained
+    if (++st == S || u + 1 == ue) {
+      // the quad's four parts of (row, batch), then the tile's row sums go to shared memory
+      float* dst = own ? sums + tile * 16 * NT : head;
+#pragma unroll
+      for (int j = 0; j < NT; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          float v = tot[j][h];
+          v += __shfl_xor_sync(0xffffffffu, v, 1);
+          v += __shfl_xor_sync(0xffffffffu, v, 2);
+          if (L.c == 0) dst[(L.rg + 8 * h) * NT + j] = v;
+          tot[j][h] = 0.0f;
+        }
+      st = 0;
+      tile++;
+      own = true;
+    }
+  }
+  __syncthreads();
+
+  // ---- rows of this CTA: a thread per row and batch row adds the parts in warp order ----
+  for (int e = tid; e < ntiles * 16 * NT; e += kThreads) {
+    const int t = e / (16 * NT), r = e - t * 16 * NT;
+    float v = sums[e];
+    // the warps after the one that holds the tile's first stage, as long as their ranges begin inside the tile
+    for (int w = ((t * S + 1) * kWarps - 1) / units + 1; w < kWarps && (units * w) / kWarps < (t + 1) * S; w++)
+      if ((units * (w + 1)) / kWarps > (units * w) / kWarps) v += reinterpret_cast<const float*>(smem + P.off_head)[w * 16 * NT + r];
+    sums[e] = QT != MLXR_Q8_0 && P.gamma ? v * misc->rinv[r % NT] : v;
+  }
+  __syncthreads();
+  // ---- epilogue: a thread per pair of adjacent rows and batch row ----
+  auto row_sum = [&](int t, int r, int m) { return sums[(t * 16 + r) * NT + m]; };
+  const int npair = 2 * (g1 - g0);                     // pairs of rows (or of h elements)
+  for (int e = tid; e < npair * NT; e += kThreads) {
+    const int pr = e % npair, m = e / npair;
+    if (P.interleave) {
+      const int col = 4 * g0 + 2 * pr, t = pr >> 2, r = (2 * pr) & 7;
+      T h[2];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const float gv = Act<T>::to_f(Act<T>::from_f(row_sum(t, r + k, m))), uv = Act<T>::to_f(Act<T>::from_f(row_sum(t, r + 8 + k, m)));
+        h[k] = Act<T>::from_f(swish_f(gv) * uv);
+      }
+      T* out = reinterpret_cast<T*>(P.y[0]) + (size_t)m * P.n_total + col;
+      if (col < P.n_total) out[0] = h[0];
+      if (col + 1 < P.n_total) out[1] = h[1];
+      continue;
+    }
+    int R = 4 * g0 + 2 * pr;
+    if (R >= P.n_total) continue;
+    float ve = row_sum(pr >> 3, (2 * pr) & 15, m), vo = row_sum(pr >> 3, ((2 * pr) & 15) + 1, m);
+    int mat = 0;
+    if (P.nmat > 1 && R >= P.rows[0]) { R -= P.rows[0]; mat = 1; if (P.nmat > 2 && R >= P.rows[1]) { R -= P.rows[1]; mat = 2; } }
+    const bool odd = R + 1 < P.rows[mat];
+    const T* bias = reinterpret_cast<const T*>(P.bias[mat]);
+    if (bias) { ve += Act<T>::to_f(bias[R]); if (odd) vo += Act<T>::to_f(bias[R + 1]); }
+    if (P.epi[mat] == decode::kEpiF32) {
+      float* of = reinterpret_cast<float*>(P.y[mat]) + (size_t)m * P.rows[mat] + R;
+      of[0] = ve;
+      if (odd) of[1] = vo;
+      continue;
+    }
+    T* out = reinterpret_cast<T*>(P.y[mat]) + (size_t)m * P.rows[mat] + R;
+    if (P.epi[mat] == decode::kEpiRope) {
+      const float qe = Act<T>::to_f(Act<T>::from_f(ve)), qo = Act<T>::to_f(Act<T>::from_f(vo));
+      const long long pos = (long long)P.positions[m] + P.pos_offset;
+      if (pos < 0 || pos >= P.max_seq) { atomicExch(P.status, MLXR_ERR_SHAPE); continue; }
+      const int pairs = P.head_dim >> 1, pi = (R % P.head_dim) >> 1;
+      const float cs = __half2float(P.cos_t[(size_t)pos * pairs + pi]), sn = __half2float(P.sin_t[(size_t)pos * pairs + pi]);
+      out[0] = Act<T>::from_f(__fsub_rn(__fmul_rn(qe, cs), __fmul_rn(qo, sn)));
+      out[1] = Act<T>::from_f(__fadd_rn(__fmul_rn(qo, cs), __fmul_rn(qe, sn)));
+    } else {
+      out[0] = Act<T>::from_f(ve);
+      if (odd) out[1] = Act<T>::from_f(vo);
+    }
+  }
+  if (tid == 0 && misc->dead) atomicExch(P.status, MLXR_ERR_TIMEOUT);
+}
+
+}  // namespace gemv
+
+using namespace gemv;
+
+static size_t unit_bytes(int qt) { return qt == MLXR_Q8_0 ? 272 : 144; }
+
+// Shared-memory layout for a launch; the total, or 0 if it does not fit an SM
+template <int QT> static size_t layout(Params* P, int M, int grid) {
+  using G = Geo<QT>;
+  const int per = P->interleave ? 2 : 4, most = (P->granules + grid - 1) / grid, tiles = (most + per - 1) / per;
+  P->x_stride = (QT == MLXR_Q8_0 ? 2 * P->K : P->K) + 16;
+  for (P->stages = kMaxStages; P->stages >= 2; P->stages--) {
+    size_t o = (size_t)kWarps * P->stages * G::kStage;
+    auto take = [&](size_t n) { const size_t at = o; o += (n + 15) & ~(size_t)15; return (int)at; };
+    P->off_x = take((size_t)(QT == MLXR_Q8_0 ? M : 2 * M) * P->x_stride);
+    P->off_aux = take((size_t)M * P->nseg * G::kAux * 4);
+    P->off_delta = take((size_t)M * P->nseg * 4);
+    P->off_sums = take((size_t)tiles * 16 * M * 4);
+    P->off_head = take((size_t)kWarps * 16 * M * 4);
+    P->off_misc = take(sizeof(Misc));
+    if (o <= (size_t)kSmemMax) return o;
+  }
+  return 0;
+}
+
+bool gemv_supported(int qt, int M, int K, int rows, int dtype, const void* const* w, int nmat) {
+  if (qt != MLXR_Q4_K && qt != MLXR_Q4_0 && !(qt == MLXR_Q8_0 && dtype != MLXR_F32)) return false;
+  // shared memory: two 16-row stages per warp (74 KB), the activations, 4 bytes per row, token and SM
+  if (M < 1 || M > 2 || K < 256 || K % 256 != 0 || K > 32768 || rows > (1 << 19)) return false;
+  for (int i = 0; i < nmat; i++)
+    if (((uintptr_t)w[i]) & 15u) return false;
+  return true;
+}
+
+template <int QT, typename T, int NT>
+static int launch_gemv_inst(Params& P, int grid, cudaStream_t st) {
+  auto kern = gemv_kernel<QT, T, NT>;
+  const size_t smem = layout<QT>(&P, NT, grid);
+  if (!smem) { set_error("gemv: K = %d does not fit shared memory", P.K); return MLXR_ERR_UNSUPPORTED; }
+  static std::atomic<bool> attr_done[64] = {};
+  int dev = 0;
+  MLXR_CUDA_TRY(cudaGetDevice(&dev));
+  if (!attr_done[dev & 63].load(std::memory_order_acquire)) {
+    MLXR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+    attr_done[dev & 63].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P));
+  count_launch();
+  return MLXR_OK;
+}
+
+// L: see DecodeLinear (no tagged hand-over: chained linears are separate launches)
+int launch_gemv(const DecodeLinear& L, int M, int qt, int dtype, int* status, cudaStream_t st) {
+  int sms = 0;
+  if (int r = device_sms(&sms)) return r;
+  Params P;
+  memset(&P, 0, sizeof(P));
+  int total = 0;
+  for (int j = 0; j < L.nmat; j++) {
+    P.rows[j] = L.rows[j];
+    total += L.rows[j];
+    if (L.nmat > 1 && !L.interleave && L.rows[j] % 4 != 0) {
+      set_error("gemv: stacked matrices need row counts that are multiples of 4");
+      return MLXR_ERR_UNSUPPORTED;
+    }
+    const size_t rb = (size_t)(L.K / 256) * unit_bytes(qt);
+    if (int r = rows_map(L.w[j], L.rows[j], rb, (int)(qt == MLXR_Q8_0 ? Geo<MLXR_Q8_0>::kPitch : Geo<MLXR_Q4_K>::kPitch), 4, &P.map[j])) return r;
+  }
+  for (int j = 0; j < 3; j++) { P.y[j] = L.y[j]; P.bias[j] = L.bias[j]; P.epi[j] = L.epi[j]; }
+  P.nmat = L.nmat;
+  P.interleave = L.interleave;
+  P.n_total = L.interleave ? L.rows[0] : total;
+  P.granules = (P.n_total + 3) / 4;
+  P.K = L.K;
+  P.nseg = L.K / 256;
+  P.nst = qt == MLXR_Q8_0 ? P.nseg : (P.nseg + 1) / 2;
+  P.M = M;
+  P.x = L.x;
+  P.gamma = L.gamma;
+  P.eps = L.eps;
+  P.cos_t = (const __half*)L.cos_t;
+  P.sin_t = (const __half*)L.sin_t;
+  P.positions = L.positions;
+  P.head_dim = L.head_dim;
+  P.max_seq = L.max_seq;
+  P.pos_offset = L.pos_offset;
+  P.status = status;
+  P.wait_ns = wait_limit_ns();
+  if (P.granules < 1) return MLXR_OK;
+  const int grid = P.granules < sms ? P.granules : sms;
+#define MLXR_GEMV_T(QTV, T) return M == 1 ? launch_gemv_inst<QTV, T, 1>(P, grid, st) : launch_gemv_inst<QTV, T, 2>(P, grid, st)
+#define MLXR_GEMV_4(QTV)                                                       \
+  do {                                                                         \
+    if (dtype == MLXR_F16) MLXR_GEMV_T(QTV, __half);                           \
+    if (dtype == MLXR_BF16) MLXR_GEMV_T(QTV, __nv_bfloat16);                   \
+    MLXR_GEMV_T(QTV, float);                                                   \
+  } while (0)
+  if (qt == MLXR_Q4_K) MLXR_GEMV_4(MLXR_Q4_K);
+  if (qt == MLXR_Q4_0) MLXR_GEMV_4(MLXR_Q4_0);
+  if (qt == MLXR_Q8_0) { if (dtype == MLXR_F16) MLXR_GEMV_T(MLXR_Q8_0, __half); MLXR_GEMV_T(MLXR_Q8_0, __nv_bfloat16); }
+#undef MLXR_GEMV_4
+#undef MLXR_GEMV_T
+  set_error("gemv: no code for %s", mlxr_quant_type_name(qt));
+  return MLXR_ERR_UNSUPPORTED;
+}
+
+}  // namespace mlxr

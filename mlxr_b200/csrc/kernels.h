@@ -105,16 +105,11 @@ int mlp_block_tp_fused(const void* x, const void* norm_weight, const void* w_gat
                        int M, int hidden, int inter_local, int qt, float eps, int dtype, const DecodeTp* tp,
                        cudaStream_t st);
 
-// ---- streaming decode linear for Q4_K at batch 1 and 2 (stream_gemv.cu) ------------------------
-// One launch per linear (or per stacked / interleaved group of linears): many small CTAs, weights
-// straight from global memory into tensor-core fragments, bulk L2 prefetch, programmatic stream
-// serialization between consecutive launches.  Takes the DecodeLinear description (no tagged
-// hand-over: chained linears are separate launches).
-bool stream_gemv_supported(int qt, int M, int K, const void* const* w, int nmat);
-// next_w / next_bytes (optional): packed weights of the launch the caller issues next on the stream; the
-// tail of this launch requests them into L2.
-int launch_stream_gemv(const DecodeLinear& L, int M, int dtype, int* status, cudaStream_t st,
-                       const void* next_w = nullptr, size_t next_bytes = 0);
+// ---- linears for one or two tokens (gemv.cu): Q4_K, Q4_0, and Q8_0 with 16-bit activations ------------------
+// One launch per linear (or per stacked / interleaved group of linears); takes the DecodeLinear description
+// (no tagged hand-over: chained linears are separate launches).  rows: weight rows in all.
+bool gemv_supported(int qt, int M, int K, int rows, int dtype, const void* const* w, int nmat);
+int launch_gemv(const DecodeLinear& L, int M, int qt, int dtype, int* status, cudaStream_t st);
 
 // ---- small-batch tensor-core linear (smallm.cu): Q4_K, Q4_0, Q8_0, NF4, canonical Q4_K; 1 <= M <= 64, fp16 / bf16 ----
 bool smallm_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w);

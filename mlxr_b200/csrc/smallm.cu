@@ -408,7 +408,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     }
   } else {
     // ===== epilogue: warp quarter q owns TMEM lanes 32 q .. 32 q + 31 = weight rows of the tile =====
-    const int quarter = warp & 3, et = tid - kWarpEpi0 * 32;
+    const int quarter = warp & 3;
     const int rt = quarter * 32 + lane;      // row within the tile
     const T* bias = reinterpret_cast<const T*>(P.bias);
     int t = t_first, sb = sb_first, g = 0, fix_bar = 2;

@@ -67,6 +67,10 @@ int weight_maps(int qt, const void* w, int N, int K, int tile_rows, CUtensorMap*
   return encode_2d(CU_TENSOR_MAP_DATA_TYPE_UINT64, (const char*)w + rb - sh, (rb + sh) / 8, N / 2, 2 * rb, 18, tile_rows / 2, CU_TENSOR_MAP_SWIZZLE_NONE, out + 1);
 }
 
+int rows_map(const void* w, int rows, size_t row_bytes, int box_bytes, int box_rows, CUtensorMap* out) {
+  return encode_2d(CU_TENSOR_MAP_DATA_TYPE_UINT64, w, row_bytes / 8, rows, row_bytes, box_bytes / 8, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE, out);
+}
+
 int activation_map(const void* x, int M, int K, int dtype, int rows, CUtensorMap* out) {
   return encode_2d(dtype == MLXR_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, K, M, (size_t)K * 2, 64, rows,
                    CU_TENSOR_MAP_SWIZZLE_128B, out);

@@ -11,6 +11,8 @@ namespace mlxr {
 // twice the row stride, the odd one starting at the 16-byte boundary at or below row 1 (*odd_shift bytes
 // before it).  Rows past the end read as zero.
 int weight_maps(int qt, const void* w, int N, int K, int tile_rows, CUtensorMap* out, int* odd_shift);
+// Packed rows of `row_bytes`, boxes of box_bytes x box_rows; rows past the end and bytes past a row's read as zero
+int rows_map(const void* w, int rows, size_t row_bytes, int box_bytes, int box_rows, CUtensorMap* out);
 // X [M, K] of a 16-bit type, boxes of 64 x `rows` with the 128-byte swizzle; rows past M read as zero
 int activation_map(const void* x, int M, int K, int dtype, int rows, CUtensorMap* out);
 // Y [M, N] of a 16-bit type for stores, boxes of box_cols (16: plain, 32: 64-byte swizzle) x box_rows

@@ -1,0 +1,100 @@
+"""Linears of one or two tokens (csrc/gemv.cu) through the C ABI, against float64 products of the dequantized weights.
+
+Sizes: fewer rows than SMs, row counts that are no multiple of the granule of four, more warps than work units, an
+odd number of 256-weight segments, segments that go round the sixteen warps more than once, long K.
+
+Bounds (2-norm, relative).  Result: rounded once to p significant bits, at most 2^-p of each value: 2^-8 (bf16, p = 8)
+and 2^-11 (fp16, p = 11).  Q4_K and Q4_0 hold the
+activations as 16-bit fixed point per segment: an error of at most amax / 64000 per element, uniform, that is
+3.6e-5 of the root mean square for N(0, 1) (amax about 4).  Q4_K's reference is the shader's half arithmetic, two
+roundings of at most 2^-11 per weight that this kernel does not make: 2^-10.  Q8_0 is exact up to float32 sums."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import make_acts, make_weights
+
+pytestmark = pytest.mark.gpu
+DT = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}
+RESULT = {"f16": 2.0 ** -11, "bf16": 2.0 ** -8, "f32": 2e-6}
+WEIGHT = {0: 5e-5, 2: 1e-6, 3: 2.0 ** -10}
+
+
+def _status():
+    import mlxr_b200 as mx
+    st = torch.zeros(1, dtype=torch.int32)
+    mx._capi.check(mx._capi.lib.mlxr_stream_status(torch.cuda.current_stream().cuda_stream, st.data_ptr()))
+    return int(st[0])
+
+
+def _dense(oracle, packed, N, K, qt):
+    f, h = oracle.dequantize(packed, N, K, qt)
+    return torch.from_numpy((h.view(np.float16) if qt == 3 else f).astype(np.float64).reshape(N, K)).cuda()
+
+
+@pytest.mark.parametrize("qt,dt", [(3, "bf16"), (3, "f16"), (3, "f32"), (0, "bf16"), (0, "f16"), (0, "f32"), (2, "bf16"), (2, "f16")])
+@pytest.mark.parametrize("M,N,K", [(1, 4, 256), (2, 5, 256), (1, 67, 768), (2, 593, 512), (1, 1000, 1280), (2, 2369, 4352), (1, 130, 16640)])
+def test_linear(oracle, qt, dt, M, N, K):
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    packed = quantize(make_weights(N, K, 7 + N), qt)
+    x = make_acts(M, K, 8 + N, DT[dt])[0].cuda()
+    b = make_acts(1, N, 9, DT[dt])[0][0].contiguous().cuda() if N % 2 else None
+    args = (x, torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt), b)
+    y = mx.q_gemm_dequant(*args)
+    assert torch.equal(y, mx.q_gemm_dequant(*args))
+    assert _status() == 0
+    want = x.double() @ _dense(oracle, packed, N, K, qt).T + (b.double() if b is not None else 0)
+    assert float((y.double() - want).norm() / want.norm()) <= RESULT[dt] + WEIGHT[qt]
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3])
+@pytest.mark.parametrize("scale", [1e-30, 1.0, 1e30])
+def test_range_of_bf16(oracle, qt, scale):
+    """Activations of any magnitude: the segments' scales carry it, nothing over- or underflows inside."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    N, K = 64, 1024
+    packed = quantize(make_weights(N, K, 1), qt)
+    x = (make_acts(1, K, 2, torch.float32)[0] * scale).to(torch.bfloat16).cuda()
+    x[0, 512:] *= 2.0 ** -12
+    y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), 1, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt))
+    want = x.double() @ _dense(oracle, packed, N, K, qt).T
+    assert float((y.double() - want).norm() / want.norm()) <= RESULT["bf16"] + WEIGHT[qt]
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3])
+@pytest.mark.parametrize("M,H,I", [(1, 512, 1280), (2, 768, 2304)])
+def test_block(oracle, qt, M, H, I):
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    g, u, d = (quantize(make_weights(n, k, s), qt) for n, k, s in ((I, H, 1), (I, H, 2), (H, I, 3)))
+    xt, xf = make_acts(M, H, 4, torch.bfloat16)
+    nt, nf = make_acts(1, H, 5, torch.bfloat16)
+    y = mx.mlp_block(xt.cuda(), nt[0].contiguous().cuda(), *(torch.from_numpy(w).cuda() for w in (g, u, d)), I, mx.QuantType(qt), 1e-5)
+    assert _status() == 0
+    assert oracle.rel_l2(y.float().cpu().numpy(), oracle.mlp_block(xf, nf[0], g, u, d, I, qt, 1e-5, oracle.BF16)) <= 1e-2
+
+
+@pytest.mark.parametrize("qt,M", [(33, 1), (33, 2), (16, 1)])
+def test_formats_of_the_small_batch_kernel(oracle, qt, M):
+    """Canonical Q4_K, and NF4 with an odd number of segments, at one and two tokens: the weights keep 16 bits."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    N, K = 300, 1280
+    if qt == 33:
+        import gguf
+        import gguf.quants as gq
+        rng = np.random.Generator(np.random.PCG64(3))
+        raw = rng.integers(0, 256, size=(N * (K // 256), 144), dtype=np.uint8)
+        raw[:, 0:4] = (rng.random((raw.shape[0], 2)) * 0.002 + 0.0005).astype(np.float16).view(np.uint8)
+        packed = raw.reshape(-1)
+        w = torch.from_numpy(gq.dequantize(packed.reshape(N, -1), gguf.GGMLQuantizationType.Q4_K).astype(np.float64)).cuda()
+    else:
+        packed = quantize(make_weights(N, K, 1), qt)
+        w = _dense(oracle, packed, N, K, qt)
+    x = make_acts(M, K, 2, torch.bfloat16)[0].cuda()
+    y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt))
+    assert _status() == 0
+    want = x.double() @ w.T
+    assert float((y.double() - want).norm() / want.norm()) <= RESULT["bf16"] + 2.0 ** -16

@@ -5,9 +5,10 @@ Sizes are the edges of the kernels' tiles: one token more and less than a token 
 tile of 128 or 256 and, odd, inside a 16-byte store, an odd number of super-blocks (NF4 rows then start 8 bytes
 off), few and many units per CTA, tiles shared by CTAs, and K that is no multiple of 256 or of 64.
 
-Bound: the products are exact and accumulate in float32; the weight is rounded once to the activation dtype, at
-most 2^-9 (bf16) or 2^-12 (fp16; Q4_K's scale and min round in half precision in both sides) of itself, the result
-once more: the 2-norm of the sum of the two is below 2^-8 and 2^-11."""
+Bound: the products are exact and accumulate in float32; the weight is rounded once to the activation dtype and the
+result once more, each by at most 2^-8 (bf16, eight significant bits) or 2^-11 (fp16) of itself and about 0.4 of
+that in the root mean square (Q4_K's scale and min round in half precision in both sides), so the 2-norm of the
+two together is below 2^-8 and 2^-11."""
 import numpy as np
 import pytest
 import torch
