@@ -17,7 +17,8 @@ _OPS = ("compute_quantized_weight_size", "compute_rope_tables", "dequantize", "m
 def __getattr__(name):
     if name in _OPS:
         from . import ops
-        return getattr(ops, name)
+        globals()[name] = fn = getattr(ops, name)     # found at once from now on
+        return fn
     if name in ("ops", "_capi", "quantize", "build", "build_cpp", "tp", "gguf_layout"):
         import importlib
         return importlib.import_module(f".{name}", __name__)

@@ -124,7 +124,7 @@ int launch_smallm(const void* x, const void* w, const void* w2, const void* bias
 // ---- the same form for more tokens (widem.cu): Q4_K, Q4_0, Q8_0, NF4, fp16 / bf16 ---------------------
 struct WidePlan {
   int nt, ntt, ntiles;     // tokens per tile, token tiles, tiles in all
-  int grid, whole;         // CTAs; 1: whole tiles per CTA, 0: equal ranges of work units
+  int grid, whole;         // CTAs; 1: whole tiles per pair, 0: ranges of work units
   size_t partial_bytes;    // fp32 partial sums needed
   double cost_us;          // the plan's own estimate
 };

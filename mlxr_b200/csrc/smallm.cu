@@ -41,6 +41,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 
@@ -484,25 +485,20 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     tmem_dealloc(tmem, R::kCols);
   }
   if (tid == 0 && sh->dead) atomicExch(P.status, MLXR_ERR_TIMEOUT);
-  // ===== shared tiles of which this CTA delivered the last part: all warps, one batch row each at a
-  // time, four weight rows per lane, up to four parts in flight, added in CTA order =====
+  // ===== shared tiles of which this CTA delivered the last part: all warps, four weight rows per lane, parts
+  // added in CTA order.  Bound by L2 latency: sixteen 16-byte loads in flight per lane, as four batch rows of
+  // four parts or, up to one batch row per warp, one of sixteen (with four, a matrix of 2368 rows, shared by
+  // eight CTAs a tile, took 4 us longer at batch 64) =====
   const int ntodo = sh->dead ? 0 : sh->ntodo;
+  constexpr int kW = kThreads / 32;
   for (int k = 0; k < ntodo; k++) {
     const int t = sh->todo_tile[k], nc = sh->todo_parts[k];
     const T* bias = reinterpret_cast<const T*>(P.bias);
     T* y = reinterpret_cast<T*>(P.y);
     const int n = SWIGLU ? 64 * t + 16 * (lane >> 3) + 4 * (lane & 3) : t * kRows + 4 * lane;
     const bool writer = !SWIGLU || (lane & 4) == 0;
-    for (int m = warp; m < P.M; m += kThreads / 32) {
-      const float4* src = reinterpret_cast<const float4*>(P.partials + ((size_t)t * P.maxc * NPAD + m) * kRows) + lane;
-      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      for (int z = 0; z < nc; z += 4) {
-        float4 a[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) a[e] = z + e < nc ? __ldcg(src + (size_t)(z + e) * NPAD * (kRows / 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-        for (int e = 0; e < 4; e++) { v[0] += a[e].x; v[1] += a[e].y; v[2] += a[e].z; v[3] += a[e].w; }
-      }
+    const float4* parts = reinterpret_cast<const float4*>(P.partials + (size_t)t * P.maxc * NPAD * kRows) + lane;
+    auto store = [&](int m, const float (&v)[4]) {
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         T o;
@@ -514,7 +510,28 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
         }
         if (writer && n + e < P.N) y[(size_t)m * P.N + n + e] = o;
       }
-    }
+    };
+    auto sum = [&](auto RC, int m0) {
+      constexpr int R = decltype(RC)::value, Z = 16 / R;               // batch rows m0, m0 + kW, .. and parts at a time
+      float v[R][4] = {};
+      for (int z = 0; z < nc; z += Z) {
+        float4 a[R][Z];
+#pragma unroll
+        for (int q = 0; q < R; q++)
+#pragma unroll
+          for (int e = 0; e < Z; e++)
+            a[q][e] = z + e < nc && m0 + q * kW < P.M ? __ldcg(parts + ((size_t)(z + e) * NPAD + m0 + q * kW) * (kRows / 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int q = 0; q < R; q++)
+#pragma unroll
+          for (int e = 0; e < Z; e++) { v[q][0] += a[q][e].x; v[q][1] += a[q][e].y; v[q][2] += a[q][e].z; v[q][3] += a[q][e].w; }
+      }
+#pragma unroll
+      for (int q = 0; q < R; q++)
+        if (m0 + q * kW < P.M) store(m0 + q * kW, v[q]);
+    };
+    if (P.M <= kW) { if (warp < P.M) sum(Int<1>{}, warp); }
+    else if (warp < P.M) sum(Int<4>{}, warp);
   }
 }
 
@@ -545,15 +562,18 @@ int smallm_plan(int M, int rows, int K, int* grid, int* maxc, size_t* partial_by
   if (int r = device_sms(&sms)) return r;
   const int nsb = K / 256, ntiles = (N + smallm::kRows - 1) / smallm::kRows;
   const long long U = (long long)ntiles * nsb;
+  // Either all SMs get equal ranges, which cross tiles, or every tile gets c CTAs of its own (the same formula with
+  // c * ntiles CTAs).  Measured at K = 4096, widths 16 and 64 of the padded batch: a unit takes 0.58 / 0.90 us, a
+  // shared tile 1.6 / 2.0 us plus 0.16 / 0.77 per part (parked, counted, read by the CTA that adds them), and
+  // a range that crosses tiles 1.5 more, because its CTA parks two parts (2368 rows, batch 16: 8.4 us with equal
+  // ranges on 148 SMs, 6.7 with four CTAs for each of the 19 tiles; 4096 rows, batch 64: 11.8 and 10.0).
+  const double w = smallm_npad(M), unit = 0.47 + 0.0067 * w, shared = 1.5 + 0.0085 * w, part = 0.012 * w;
   int G = (int)std::min<long long>(sms, U);
-  // Equal ranges make most tiles shared, and a shared tile costs its CTAs an epilogue whose length
-  // grows with the padded batch width (partial sums stored, counted, re-read by the last arriver:
-  // measured about 3 us at width 16 and 7 to 15 us at width 64).  When there is at most one tile
-  // per SM, one whole tile per CTA needs no fix-up at all and only lengthens the loop from U / G
-  // units to K / 256: taken when that difference (about 1 us per unit) is below 0.13 us per
-  // column of the padded width (measured at N = 14336, K = 4096: batch 32 23.1 -> 19.4 us,
-  // batch 64 29.4 -> 21.5 us; at width 16 the equal ranges stay ahead, 19.1 us).
-  if (ntiles <= sms && (double)nsb - (double)U / G < 0.13 * smallm_npad(M)) G = ntiles;
+  double best = std::ceil((double)U / G) * unit + (U % G == 0 && U / G % nsb == 0 ? 0.0 : shared + 1.5 + part * ((double)nsb * G / U + 1.0));
+  for (int c = 1; c <= nsb && (long long)c * ntiles <= sms; c++) {
+    const double cost = (nsb + c - 1) / c * unit + (c > 1 ? shared + part * c : 0.0);
+    if (cost < best) { best = cost; G = c * ntiles; }
+  }
   int mc = 1;
   for (int t = 0; t < ntiles; t++)
     mc = std::max(mc, smallm::unit_owner(U, G, (long long)(t + 1) * nsb - 1) - smallm::unit_owner(U, G, (long long)t * nsb) + 1);

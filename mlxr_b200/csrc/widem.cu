@@ -483,16 +483,22 @@ int widem_plan(int M, int rows, int K, WidePlan* out) {
     if (nt < 16 || nt > 256) continue;
     const long long ntiles = (long long)wtiles * ((M + nt - 1) / nt), U = ntiles * nsb;
     const double unit = 2000.0 + 4.3 * nt, drain = nt > 128 ? 1200.0 + 8.0 * nt : 600.0;
-    for (int whole = 0; whole < 2; whole++) {
-      if (!whole && 2 * ntiles > kSyncWords - 16) continue;        // two counters per tile
-      const int G = (int)std::min<long long>(pairs, whole ? ntiles : U);
+    // split 0: equal ranges of units for all pairs; else so many pairs for each tile (1: whole tiles, any number of them)
+    for (int split = 0; split == 0 || split == 1 || (split <= nsb && split * ntiles <= pairs); split++) {
+      if (split != 1 && 2 * ntiles > kSyncWords - 16) continue;        // two counters per tile
+      const int G = (int)(split == 0 ? std::min<long long>(pairs, U) : split == 1 ? std::min<long long>(pairs, ntiles) : split * ntiles);
       double c;
-      if (whole) { const double tiles = (double)((ntiles + G - 1) / G); c = tiles * (nsb * unit + drain); }
-      else { const double units = (double)((U + G - 1) / G); c = units * unit + units / nsb * drain + 2500.0 + 20.0 * nt + 1200.0 * (double)((nsb + units - 1) / units); }
+      if (split == 0) {
+        const double units = (double)((U + G - 1) / G);
+        c = units * unit + units / nsb * drain + 2500.0 + 20.0 * nt + 1200.0 * (double)((nsb + units - 1) / units) + 2500.0;
+      } else {
+        const double tiles = (double)((ntiles + G - 1) / G);
+        c = tiles * ((nsb + split - 1) / split * unit + drain) + (split > 1 ? 2500.0 + 20.0 * nt + 1200.0 * split : 0.0);
+      }
       if (c < best) {
         best = c;
-        out->nt = nt; out->ntt = (M + nt - 1) / nt; out->ntiles = (int)ntiles; out->grid = 2 * G; out->whole = whole;
-        out->partial_bytes = whole ? 0 : (size_t)2 * G * 2 * nt * widem::kRows * sizeof(float);
+        out->nt = nt; out->ntt = (M + nt - 1) / nt; out->ntiles = (int)ntiles; out->grid = 2 * G; out->whole = split == 1;
+        out->partial_bytes = split == 1 ? 0 : (size_t)2 * G * 2 * nt * widem::kRows * sizeof(float);
       }
     }
   }
