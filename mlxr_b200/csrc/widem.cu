@@ -412,7 +412,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
   }
   if (tid == 0 && sh->dead) atomicExch(P.status, MLXR_ERR_TIMEOUT);
   // ===== shared tiles of which this CTA delivered the last part: all warps, four tokens each at a time,
-  // four weight rows per lane, added in CTA order =====
+  // four weight rows per lane, two parts in flight, added in CTA order =====
   const int ntodo = sh->dead ? 0 : sh->ntodo;
   constexpr int kW = kThreads / 32;
   for (int k = 0; k < ntodo; k++) {
@@ -422,22 +422,27 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     const T* bias = reinterpret_cast<const T*>(P.bias);
     const int n = SWIGLU ? 64 * wt + 16 * (lane >> 3) + 4 * (lane & 3) : wt * kRows + 4 * lane;
     const bool writer = !SWIGLU || (lane & 4) == 0;
-    // part of pair c: its first tile's (0) unless the tile starts inside its range (1)
-    auto part_of = [&](int z) {
-      const int c = c0 + z, at = (int)(unit_begin(U, G, c) / P.nsb) == t ? 0 : 1;
-      return reinterpret_cast<const float4*>(P.partials + (size_t)(2 * (2 * c + rank) + at) * P.nt * kRows) + lane;
-    };
+    // parts of the tile: the first pair's is its first tile's (0) if its range begins with this tile, else its last
+    // tile's (1); the others' ranges begin inside the tile
+    const size_t slab = (size_t)P.nt * (kRows / 4);
+    const float4* first = reinterpret_cast<const float4*>(P.partials) + (size_t)(2 * (2 * c0 + rank) + (unit_begin(U, G, c0) < (long long)t * P.nsb ? 1 : 0)) * slab + lane;
+    const float4* later = reinterpret_cast<const float4*>(P.partials) + (size_t)(2 * (2 * c0 + rank)) * slab + lane;
     for (int m0 = warp; m0 < ntok; m0 += 4 * kW) {
       float v[4][4];
 #pragma unroll
       for (int q = 0; q < 4; q++) v[q][0] = v[q][1] = v[q][2] = v[q][3] = 0.0f;
-      for (int z = 0; z < nc; z++) {
-        const float4* src = part_of(z);
-        float4 a[4];
+      for (int z = 0; z < nc; z += 2) {
+        float4 a[2][4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) a[q] = m0 + q * kW < ntok ? __ldcg(src + (size_t)(m0 + q * kW) * (kRows / 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int e = 0; e < 2; e++) {
+          const float4* src = z + e == 0 ? first : later + (size_t)(4 * (z + e)) * slab;
 #pragma unroll
-        for (int q = 0; q < 4; q++) { v[q][0] += a[q].x; v[q][1] += a[q].y; v[q][2] += a[q].z; v[q][3] += a[q].w; }
+          for (int q = 0; q < 4; q++) a[e][q] = z + e < nc && m0 + q * kW < ntok ? __ldcg(src + (size_t)(m0 + q * kW) * (kRows / 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+#pragma unroll
+          for (int q = 0; q < 4; q++) { v[q][0] += a[e][q].x; v[q][1] += a[e][q].y; v[q][2] += a[e][q].z; v[q][3] += a[e][q].w; }
       }
 #pragma unroll
       for (int q = 0; q < 4; q++) {
