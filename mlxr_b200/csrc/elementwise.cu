@@ -296,19 +296,30 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x,
 
 // The same for 16-bit types and heads of a multiple of 8 elements: one thread per four pairs, 128-bit
 // accesses to x and y, 64-bit to the tables; the token's position is checked once per thread.
+//
+// Two tensors that share the positions (q and k of a layer) can go in one launch: vectors from `total` on are z's,
+// up to total_z.
 template <typename T>
 __global__ void __launch_bounds__(256) rope_vec_kernel(const T* __restrict__ x, const __half* __restrict__ cos_t, const __half* __restrict__ sin_t,
                                                        const int32_t* __restrict__ positions, T* __restrict__ y, size_t total, int vec_per_token,
+                                                       T* __restrict__ z, size_t total_z, int vec_per_token_z,
                                                        int vec_per_head, int max_seq, int linear, float scale, int offset, int* status) {
-  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t)gridDim.x * 256) {
-    const size_t tok = i / vec_per_token;
-    const int c = (int)(i - tok * vec_per_token) % vec_per_head;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (size_t j = (size_t)blockIdx.x * 256 + threadIdx.x; j < total + total_z; j += (size_t)gridDim.x * 256) {
+    const bool first = j < total;
+    const size_t i = first ? j : j - total;
+    const int per = first ? vec_per_token : vec_per_token_z;
+    const T* src = first ? x : z;
+    T* dst = first ? y : z;
+    const size_t tok = i / per;
+    const int c = (int)(i - tok * per) % vec_per_head;
     const long long pos = (long long)positions[tok] + offset;
     if (pos < 0 || pos >= max_seq) {
       if (status) atomicExch_system(status, 1);
       continue;
     }
-    const uint4 xv = *reinterpret_cast<const uint4*>(x + i * 8);
+    const uint4 xv = *reinterpret_cast<const uint4*>(src + i * 8);
     const uint2 cv = __ldg(reinterpret_cast<const uint2*>(cos_t + (size_t)pos * vec_per_head * 4) + c);
     const uint2 sv = __ldg(reinterpret_cast<const uint2*>(sin_t + (size_t)pos * vec_per_head * 4) + c);
     const T* h = reinterpret_cast<const T*>(&xv);
@@ -321,8 +332,39 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(const T* __restrict__ x, 
       o[2 * p + 1] = __fadd_rn(__fmul_rn(xo, cs), __fmul_rn(xe, sn));
       if (linear) { o[2 * p] *= scale; o[2 * p + 1] *= scale; }
     }
-    store8v(y + i * 8, o);
+    store8v(dst + i * 8, o);
   }
+}
+
+template <typename T>
+static int launch_rope_vec(const void* x, const uint16_t* cos_t, const uint16_t* sin_t, const int32_t* positions, void* y, size_t tokens, int heads,
+                           void* z, int heads_z, int head_dim, int max_seq, int linear, float scale, int offset, int* status, cudaStream_t st) {
+  const int vh = head_dim / 8;
+  const size_t total = tokens * heads * vh, total_z = tokens * heads_z * vh;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min<size_t>((total + total_z + 255) / 256, 148 * 8 * 4));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rope_vec_kernel<T>, (const T*)x, (const __half*)cos_t, (const __half*)sin_t, positions, (T*)y, total, heads * vh,
+                                   (T*)z, total_z, heads_z * vh, vh, max_seq, linear, scale, offset, status));
+  count_launch();
+  return MLXR_OK;
+}
+static bool rope_vec_ok(const void* x, const void* y, const uint16_t* cos_t, const uint16_t* sin_t, int head_dim, int dtype) {
+  return dtype != MLXR_F32 && head_dim % 8 == 0 && aligned16(x, y) && (((uintptr_t)cos_t | (uintptr_t)sin_t) & 7u) == 0;
+}
+bool rope_qk_supported(const void* q, const void* k, const uint16_t* cos_t, const uint16_t* sin_t, int head_dim, int dtype) {
+  return rope_vec_ok(q, k, cos_t, sin_t, head_dim, dtype);
+}
+int launch_rope_qk(void* q, void* k, const uint16_t* cos_t, const uint16_t* sin_t, const int32_t* positions, size_t tokens, int q_heads, int kv_heads,
+                   int head_dim, int max_seq, int offset, int dtype, int* status, cudaStream_t st) {
+  return dtype == MLXR_F16 ? launch_rope_vec<__half>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, st)
+                           : launch_rope_vec<__nv_bfloat16>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, st);
 }
 
 int launch_rope(const void* x, const uint16_t* cos_t, const uint16_t* sin_t,
@@ -331,16 +373,9 @@ int launch_rope(const void* x, const uint16_t* cos_t, const uint16_t* sin_t,
                 cudaStream_t st) {
   const size_t total = tokens * heads * (head_dim / 2);
   if (total == 0) return MLXR_OK;
-  if (dtype != MLXR_F32 && head_dim % 8 == 0 && aligned16(x, y) && (((uintptr_t)cos_t | (uintptr_t)sin_t) & 7u) == 0) {
-    const size_t nvec = tokens * heads * (head_dim / 8);
-    const int vb = (int)std::min<size_t>((nvec + 255) / 256, 148 * 8 * 4);
-#define MLXR_ROPE(T) rope_vec_kernel<T><<<vb, 256, 0, st>>>((const T*)x, (const __half*)cos_t, (const __half*)sin_t, positions, (T*)y, nvec, heads * (head_dim / 8), \
-                                                           head_dim / 8, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status)
-    if (dtype == MLXR_F16) MLXR_ROPE(__half); else MLXR_ROPE(__nv_bfloat16);
-#undef MLXR_ROPE
-    MLXR_LAUNCH_CHECK("rope_vec_kernel");
-    return MLXR_OK;
-  }
+  if (rope_vec_ok(x, y, cos_t, sin_t, head_dim, dtype))
+    return dtype == MLXR_F16 ? launch_rope_vec<__half>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, st)
+                             : launch_rope_vec<__nv_bfloat16>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, st);
   size_t blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   MLXR_DISPATCH_DTYPE(dtype, T, {

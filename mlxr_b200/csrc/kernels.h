@@ -32,6 +32,10 @@ int launch_rope(const void* x, const uint16_t* cos_t, const uint16_t* sin_t,
                 int max_seq, int mode, float scale, int offset, int dtype, int* status,
                 cudaStream_t st);
 
+// rope_apply on q and k [tokens, heads, head_dim] in place, one launch; false if their layout needs launch_rope
+bool rope_qk_supported(const void* q, const void* k, const uint16_t* cos_t, const uint16_t* sin_t, int head_dim, int dtype);
+int launch_rope_qk(void* q, void* k, const uint16_t* cos_t, const uint16_t* sin_t, const int32_t* positions, size_t tokens, int q_heads, int kv_heads,
+                   int head_dim, int max_seq, int offset, int dtype, int* status, cudaStream_t st);
 int launch_rope_split_half(const void* x, const float* cos_t, const float* sin_t, void* y, size_t batch, int seq,
                            int heads, int head_dim, int offset, int dtype, cudaStream_t st);
 
@@ -117,8 +121,8 @@ void smallm_partition(long long units, int ctas, int cta, long long unit, long l
 // grid size, the most CTAs that share one output tile, and the bytes of fp32 partial sums needed;
 // rows = weight rows streamed (N, or 2 N for the gate/up form)
 int smallm_plan(int M, int rows, int K, int* grid, int* maxc, size_t* partial_bytes);
-// w2 == nullptr: Y = X W^T (+ bias); otherwise Y = SiLU(X w^T) * (X w2^T) (gate, up; no bias)
-int launch_smallm(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K, int qt, int dtype,
+// nmat stacked matrices y[i] [M, rows[i]] = X w[i]^T (+ bias, one matrix only), or swiglu: w[0] = gate, w[1] = up
+int launch_smallm(const void* x, const void* const* w, const int* rows, int nmat, bool swiglu, const void* bias, void* const* y, int M, int K, int qt, int dtype,
                   int* status, float* partials, uint32_t* counters, int grid, int maxc, cudaStream_t st);
 
 // ---- the same form for more tokens (widem.cu): Q4_K, Q4_0, Q8_0, NF4, fp16 / bf16 ---------------------

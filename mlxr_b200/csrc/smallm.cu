@@ -72,8 +72,10 @@ constexpr int kSmemMax = 227 * 1024;
 
 struct Params {
   const void* bias;
-  void* y;
-  int M, N, K;
+  int M, K;
+  // matrices stacked along the tiles (q / k / v; one otherwise): rows of each, the tile after its last, its Y
+  int rows[3], end[3];
+  void* y[3];
   int nsb;             // super-blocks per row = K / 256
   int ntiles;          // ceil(rows / 128)
   int maxc;            // most CTAs that share one tile
@@ -84,9 +86,21 @@ struct Params {
   uint32_t* counters;  // one per tile, self-clearing
 };
 
-// Tensor maps of the packed weights: [0] W or gate, [1] up; NF4 (rows only 8-byte aligned): even
-// and odd rows of each, [0] [1] W or gate, [2] [3] up.
-struct Maps { CUtensorMap x, w[4]; };
+// Tensor maps of the packed weights: one per stacked matrix, or [0] gate, [1] up; NF4 (rows only 8-byte
+// aligned): two of each, for its even and its odd rows.
+struct Maps { CUtensorMap x, w[6]; };
+
+// One matrix, gate and up with SiLU(gate) * up, or matrices stacked along the tiles.  (A kernel for all three, which
+// finds every tile's matrix, took 1.1 us longer on one: 8.9 us instead of 7.8 at 16 x 4096 x 4096.)
+enum Form { kPlain, kSwiglu, kStacked };
+
+// the matrix of tile t and the tile's number in it
+struct Place { int mat, tile; };
+template <int FORM>
+__device__ __forceinline__ Place place_of(const Params& P, int t) {
+  if (FORM != kStacked || t < P.end[0]) return {0, t};
+  return t < P.end[1] ? Place{1, t - P.end[0]} : Place{2, t - P.end[1]};
+}
 
 struct Shared {
   // The group's four warps have written the slot.  Consecutive units of a group belong to different
@@ -147,16 +161,18 @@ template <int QT, int NPAD> struct Rings {
 // SWIGLU: the tile's rows are 16 gate rows and 16 up rows per TMEM lane quarter (from two weight
 // matrices), Y = SiLU(gate) * up with gate and up rounded to T first, N = the number of gate rows; a
 // tile then covers 64 output columns.
-template <int QT, typename T, int NPAD, int MODE, bool SWIGLU>
+template <int QT, typename T, int NPAD, int MODE, int FORM>
 __global__ void __launch_bounds__(kThreads, 1)
 qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
+  constexpr bool SWIGLU = FORM == kSwiglu;
   extern __shared__ uint8_t smem_raw[];
   constexpr int BF = Fmt<T>::v;
   constexpr bool kSplitRows = QT == MLXR_NF4;                 // even and odd rows come through maps of their own
   // the TMA unit fetches a tensor map on first use: ask for them before anything else
-  if (threadIdx.x < 5) {
-    const CUtensorMap* m = threadIdx.x == 4 ? &maps.x : &maps.w[threadIdx.x];
-    if (threadIdx.x == 4 || threadIdx.x < (SWIGLU ? 2 : 1) * (kSplitRows ? 2 : 1))
+  if (threadIdx.x < 7) {
+    const CUtensorMap* m = threadIdx.x == 6 ? &maps.x : &maps.w[threadIdx.x];
+    constexpr int mats = FORM == kPlain ? 1 : FORM == kSwiglu ? 2 : 3;
+    if (threadIdx.x == 6 || threadIdx.x < mats * (kSplitRows ? 2 : 1))
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
   }
   using R = Rings<QT, NPAD>;
@@ -182,12 +198,13 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     constexpr int nbox = (SWIGLU ? 2 : 1) * (kSplitRows ? 2 : 1);
     const uint32_t bar = smem_u32(&sh->raw_full[r]);
     mbar_expect_tx(bar, kRawBytes);
-    const int row0 = (SWIGLU ? 64 : kRows) * t;
+    const Place at = place_of<FORM>(P, t);
+    const int row0 = (SWIGLU ? 64 : kRows) * at.tile;
 #pragma unroll
     for (int b = 0; b < nbox; b++) {
       int x = Geo<QT>::kUnit / 8 * sb, y = row0;
       if constexpr (kSplitRows) { x = ((136 * sb + ((b & 1) ? P.odd_shift : 0)) & ~15) >> 3; y = row0 >> 1; }
-      tma_load_2d(smem_u32(rawring + (size_t)r * kRawBytes + (size_t)b * (kRawBytes / nbox)), &maps.w[b], x, y, bar);
+      tma_load_2d(smem_u32(rawring + (size_t)r * kRawBytes + (size_t)b * (kRawBytes / nbox)), &maps.w[at.mat * nbox + b], x, y, bar);
     }
   };
   int raw_t = t_first, raw_sb = sb_first, raw_issued = 0;     // copy warp: the next unit to request
@@ -427,8 +444,10 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
       tc_fence_after();
       const bool whole = cnt == P.nsb;       // this CTA summed the tile's whole K: store Y directly
       // output column of this lane: its weight row, or for SWIGLU the gate row that lanes l and l + 16 share
-      const int n = SWIGLU ? 64 * t + 16 * quarter + (lane & 15) : t * kRows + rt;
-      const bool writer = (!SWIGLU || lane < 16) && n < P.N;
+      const Place at = place_of<FORM>(P, t);
+      const int N = P.rows[at.mat], n = SWIGLU ? 64 * at.tile + 16 * quarter + (lane & 15) : at.tile * kRows + rt;
+      const bool writer = (!SWIGLU || lane < 16) && n < N;
+      T* y = reinterpret_cast<T*>(P.y[at.mat]);
       // sums of one batch row -> Y: plain (+ bias), or SiLU(gate) * up across the lane pair
       auto finish = [&](float v, float bv) -> T {
         if constexpr (SWIGLU) {
@@ -441,7 +460,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
       };
       const int slot = whole ? 0 : cta - unit_owner(P.U, G, (long long)t * P.nsb);
       float* part = P.partials + (((size_t)t * P.maxc + slot) * NPAD) * kRows + rt;
-      const float bv = (!SWIGLU && bias && n < P.N) ? Act<T>::to_f(bias[n]) : 0.0f;
+      const float bv = (!SWIGLU && bias && n < N) ? Act<T>::to_f(bias[n]) : 0.0f;
 #pragma unroll 1
       for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) {
         uint32_t r[16];
@@ -460,7 +479,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
           for (int c = 0; c < 16; c++) {
             if (c0 + c < P.M) {             // uniform: every lane takes part in the exchange
               const T o = finish(__uint_as_float(r[c]), bv);
-              if (writer) reinterpret_cast<T*>(P.y)[(size_t)(c0 + c) * P.N + n] = o;
+              if (writer) y[(size_t)(c0 + c) * N + n] = o;
             }
           }
         } else {
@@ -494,8 +513,10 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
   for (int k = 0; k < ntodo; k++) {
     const int t = sh->todo_tile[k], nc = sh->todo_parts[k];
     const T* bias = reinterpret_cast<const T*>(P.bias);
-    T* y = reinterpret_cast<T*>(P.y);
-    const int n = SWIGLU ? 64 * t + 16 * (lane >> 3) + 4 * (lane & 3) : t * kRows + 4 * lane;
+    const Place at = place_of<FORM>(P, t);
+    const int N = P.rows[at.mat];
+    T* y = reinterpret_cast<T*>(P.y[at.mat]);
+    const int n = SWIGLU ? 64 * at.tile + 16 * (lane >> 3) + 4 * (lane & 3) : at.tile * kRows + 4 * lane;
     const bool writer = !SWIGLU || (lane & 4) == 0;
     const float4* parts = reinterpret_cast<const float4*>(P.partials + (size_t)t * P.maxc * NPAD * kRows) + lane;
     auto store = [&](int m, const float (&v)[4]) {
@@ -506,9 +527,9 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
           const float up = __shfl_xor_sync(0xffffffffu, v[e], 4);      // lanes 0-3 of eight: gate, lanes 4-7: up
           o = Act<T>::from_f(swish_fast(Act<T>::to_f(Act<T>::from_f(v[e]))) * Act<T>::to_f(Act<T>::from_f(up)));
         } else {
-          o = Act<T>::from_f(v[e] + (bias && n + e < P.N ? Act<T>::to_f(bias[n + e]) : 0.0f));
+          o = Act<T>::from_f(v[e] + (bias && n + e < N ? Act<T>::to_f(bias[n + e]) : 0.0f));
         }
-        if (writer && n + e < P.N) y[(size_t)m * P.N + n + e] = o;
+        if (writer && n + e < N) y[(size_t)m * N + n + e] = o;
       }
     };
     auto sum = [&](auto RC, int m0) {
@@ -583,10 +604,10 @@ int smallm_plan(int M, int rows, int K, int* grid, int* maxc, size_t* partial_by
   return MLXR_OK;
 }
 
-template <int QT, typename T, int NPAD, int MODE, bool SWIGLU>
+template <int QT, typename T, int NPAD, int MODE, int FORM>
 static int launch_inst(const smallm::Maps& maps, const smallm::Params& P, int grid, cudaStream_t st) {
   using namespace smallm;
-  auto kern = qgemm_smallm_kernel<QT, T, NPAD, MODE, SWIGLU>;
+  auto kern = qgemm_smallm_kernel<QT, T, NPAD, MODE, FORM>;
   constexpr size_t smem = Rings<QT, NPAD>::kBytes + sizeof(Shared) + 1024;
   static_assert(smem <= (size_t)kSmemMax, "shared memory");
   static std::atomic<bool> attr_done[64] = {};
@@ -611,26 +632,31 @@ static int launch_inst(const smallm::Maps& maps, const smallm::Params& P, int gr
   return MLXR_OK;
 }
 
-// w2 == nullptr: Y[M, N] = X W^T (+ bias).  Otherwise w = gate, w2 = up (both [N, K]) and
-// Y[M, N] = SiLU(X gate^T) * (X up^T), the two products rounded to the activation dtype first.
-int launch_smallm(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K, int qt, int dtype,
+// One matrix, or three [rows[i], K] stacked: y[i] [M, rows[i]] = X w[i]^T (+ bias, one matrix only).  Or swiglu: w[0] = gate,
+// w[1] = up (both [rows[0], K]) and y[0] = SiLU(X gate^T) * (X up^T), the two products rounded to the
+// activation dtype first.
+int launch_smallm(const void* x, const void* const* w, const int* rows, int nmat, bool swiglu, const void* bias, void* const* y, int M, int K, int qt, int dtype,
                   int* status, float* partials, uint32_t* counters, int grid, int maxc, cudaStream_t st) {
-  const int npad = smallm_npad(M);
-  const bool swiglu = w2 != nullptr;
+  const int npad = smallm_npad(M), form = swiglu ? smallm::kSwiglu : nmat == 1 ? smallm::kPlain : smallm::kStacked;
   smallm::Maps maps;
   smallm::Params P;
   memset(&maps, 0, sizeof(maps));
   memset(&P, 0, sizeof(P));
   if (int r = activation_map(x, M, K, dtype, npad, &maps.x)) return r;
-  const int tile_rows = swiglu ? 64 : smallm::kRows;
-  if (int r = weight_maps(qt, w, N, K, tile_rows, maps.w, &P.odd_shift)) return r;
-  if (swiglu)
-    if (int r = weight_maps(qt, w2, N, K, tile_rows, maps.w + (qt == MLXR_NF4 ? 2 : 1), &P.odd_shift)) return r;
+  const int tile_rows = swiglu ? 64 : smallm::kRows, per = qt == MLXR_NF4 ? 2 : 1;
+  for (int i = 0; i < nmat; i++)
+    if (int r = weight_maps(qt, w[i], rows[swiglu ? 0 : i], K, tile_rows, maps.w + per * i, &P.odd_shift)) return r;
+  for (int i = 0; i < 3; i++) {
+    if (i < (swiglu ? 1 : nmat)) {
+      P.rows[i] = rows[i];
+      P.y[i] = y[i];
+      P.ntiles += (rows[i] + tile_rows - 1) / tile_rows;
+    }
+    P.end[i] = P.ntiles;
+  }
   P.bias = bias;
-  P.y = y;
-  P.M = M; P.N = N; P.K = K;
+  P.M = M; P.K = K;
   P.nsb = K / 256;
-  P.ntiles = ((swiglu ? 2 * N : N) + smallm::kRows - 1) / smallm::kRows;
   P.maxc = maxc;
   P.U = (long long)P.ntiles * P.nsb;
   P.status = status;
@@ -650,16 +676,23 @@ int launch_smallm(const void* x, const void* w, const void* w2, const void* bias
   } while (0)
 #define MLXR_SMALLM(QTV, MODE)                                                           \
   do {                                                                                   \
-    if (swiglu) MLXR_SMALLM_BY_DTYPE(QTV, MODE, true);                                   \
-    else MLXR_SMALLM_BY_DTYPE(QTV, MODE, false);                                         \
+    if (form == smallm::kSwiglu) MLXR_SMALLM_BY_DTYPE(QTV, MODE, smallm::kSwiglu);       \
+    else if (form == smallm::kPlain) MLXR_SMALLM_BY_DTYPE(QTV, MODE, smallm::kPlain);    \
+    else MLXR_SMALLM_BY_DTYPE(QTV, MODE, smallm::kStacked);                              \
   } while (0)
   // Q8_0 and NF4 at batch <= 8 and canonical Q4_K at any keep the precision of the float32 weights
   // (wconv::kSplit)
+#define MLXR_SMALLM_SPLIT_BY_DTYPE(QTV, FORM)                                            \
+  do {                                                                                   \
+    if (dtype == MLXR_F16) rc = launch_inst<QTV, __half, 16, wconv::kSplit, FORM>(maps, P, grid, st);    \
+    else rc = launch_inst<QTV, __nv_bfloat16, 16, wconv::kSplit, FORM>(maps, P, grid, st);               \
+  } while (0)
 #define MLXR_SMALLM_SPLIT(QTV)                                                           \
   do {                                                                                   \
     if (M > 8) MLXR_SMALLM(QTV, wconv::kRound);                                          \
-    else if (swiglu) { if (dtype == MLXR_F16) rc = launch_inst<QTV, __half, 16, wconv::kSplit, true>(maps, P, grid, st); else rc = launch_inst<QTV, __nv_bfloat16, 16, wconv::kSplit, true>(maps, P, grid, st); } \
-    else { if (dtype == MLXR_F16) rc = launch_inst<QTV, __half, 16, wconv::kSplit, false>(maps, P, grid, st); else rc = launch_inst<QTV, __nv_bfloat16, 16, wconv::kSplit, false>(maps, P, grid, st); }            \
+    else if (form == smallm::kSwiglu) MLXR_SMALLM_SPLIT_BY_DTYPE(QTV, smallm::kSwiglu);  \
+    else if (form == smallm::kPlain) MLXR_SMALLM_SPLIT_BY_DTYPE(QTV, smallm::kPlain);    \
+    else MLXR_SMALLM_SPLIT_BY_DTYPE(QTV, smallm::kStacked);                              \
   } while (0)
   switch (qt) {
     case MLXR_Q4_K: MLXR_SMALLM(MLXR_Q4_K, wconv::kFast); break;
@@ -670,6 +703,7 @@ int launch_smallm(const void* x, const void* w, const void* w2, const void* bias
     default: set_error("small-batch kernel: no producer for %s", mlxr_quant_type_name(qt)); break;
   }
 #undef MLXR_SMALLM_SPLIT
+#undef MLXR_SMALLM_SPLIT_BY_DTYPE
 #undef MLXR_SMALLM
 #undef MLXR_SMALLM_BY_DTYPE
 #undef MLXR_SMALLM_BY_NPAD

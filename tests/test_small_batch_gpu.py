@@ -162,3 +162,27 @@ def test_gate_up_other_formats(oracle, qt, M, H, I):
     y = mx.mlp_block(xt.cuda(), nt[0].contiguous().cuda(), *(torch.from_numpy(w).cuda() for w in (g, u, d)), I, mx.QuantType(qt), 1e-5)
     assert _status() == 0
     assert oracle.rel_l2(y.float().cpu().numpy(), oracle.mlp_block(xf, nf[0], g, u, d, I, qt, 1e-5, oracle.BF16)) <= TIGHT["bf16"]
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3, 16])
+@pytest.mark.parametrize("M,H,QH,KH,D", [(3, 768, 5, 1, 64), (20, 512, 4, 2, 128), (64, 1280, 3, 3, 32)])
+def test_stacked_projections_with_rope(oracle, qt, M, H, QH, KH, D):
+    """q, k and v as one launch (row counts that do not fill their last tile, odd numbers of super-blocks), then
+    q and k rotated in one: against this package's own linear (bit-equal is not required: the tiles are
+    shared by other CTAs, which adds the float32 sums in another order) and rope_apply on its result."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    ws = [torch.from_numpy(quantize(make_weights(n * D, H, 9 + i), qt)).cuda() for i, n in enumerate((QH, KH, KH))]
+    x = make_acts(M, H, 4, torch.float16)[0].cuda()
+    nw = make_acts(1, H, 5, torch.float16)[0][0].contiguous().cuda()
+    cos, sin = mx.compute_rope_tables(512, D, 10000.0, device=torch.device("cuda"))
+    pos = torch.from_numpy(np.random.Generator(np.random.PCG64(1)).integers(0, 512, M).astype(np.int32)).cuda()
+    out = mx.qkv_rope(x, nw, *ws, cos, sin, pos, QH, KH, D, mx.QuantType(qt), 1e-5)
+    assert _status() == 0
+    n = mx.rmsnorm_fused(x, nw, 1e-5)
+    gs = mx._capi.lib.mlxr_default_group_size(qt)
+    for i, (got, heads) in enumerate(zip(out, (QH, KH, KH))):
+        y = mx.q_gemm_dequant(n, ws[i], M, heads * D, H, mx.QuantType(qt), gs).reshape(M, heads, D)
+        want = mx.rope_apply(y, cos, sin, pos) if i < 2 else y
+        # one ulp of the linear's result at most, 2^-10, where the two sums round to different sides
+        assert float((got.double() - want.double()).norm() / want.double().norm()) <= 2.0 ** -11
