@@ -42,9 +42,9 @@ import numpy as np  # noqa: E402
 
 H, I = 4096, 14336            # Llama-3-8B MLP (the default workload)
 SIZES = {"hidden": H, "inter": I}
-# DRAM bytes (read + write) of one decode_kernel launch from an ncu capture of this workload,
+# DRAM bytes (read + write) of one step from an ncu capture of this workload's launches,
 # keyed by (hidden, inter, batch); see profiles/
-TRAFFIC = {(4096, 14336, 1): 105265152}
+TRAFFIC = {}
 QT_Q4_K = 3
 EPS = 1e-5
 SEED = 1234
@@ -574,8 +574,9 @@ def run_mine(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "traffic": TRAFFIC.get((H, I, M)) if world == 1 else None, "peak_source": which,
                          "algorithmic_bytes_per_step": ab, "per": "GPU",
-                         "kernel": "decode_kernel (one persistent launch per step: RMSNorm + gate/up + SwiGLU + down)"
-                                   + ("" if world == 1 else " + exchange of the ranks' sums"),
+                         "kernel": "gemv_kernel (two launches per step: RMSNorm + gate/up + SwiGLU, down)" if world == 1 and M <= 2
+                                   else "decode_kernel (one launch per step) + exchange of the ranks' sums" if world > 1
+                                   else "RMSNorm, gate/up + SwiGLU and down on the tensor-core kernels",
                          "timing": "CUDA events around " + (f"each of {repeats} CUDA-graph replays of the K steps (median)" if use_graph else "K plain launches")},
             "cpu_baseline": cb,
             "cpu_baseline_all_cores": cb_all,
@@ -662,7 +663,7 @@ def run_prefill(args):
         "gpu_launches": int(launches), "clocks": clocks,
         "roofline": {"bound": "tensor", "achieved": achieved, "peak": tf, "unit": "TFLOP/s", "frac": achieved / tf,
                      "traffic": None, "peak_source": which + " (burst bf16 figure)", "flops_per_step": flops,
-                     "kernel": "qgemm_tc_kernel", "timing": "CUDA events around K plain launches"},
+                     "kernel": "qgemm_widem_kernel or weights16_kernel + gemm16_kernel, by the estimated time", "timing": "CUDA events around K plain launches"},
         "cpu_baseline": None,
     }
     print(json.dumps(line))

@@ -137,7 +137,7 @@ MLXR_API int mlxr_dequantize(const void* weights, void* out, int N, int K, int q
  * group_size must be the format's block size, or 32 for Q4_K (the shader's sub-block
  * addressing, q_gemm_dequant.metal:397-430).  K must be a whole number of
  * blocks (the reference overruns the row otherwise).  The kernel is chosen by shape:
- * streaming decode kernel for small M, tcgen05 tensor-core kernel for large M.
+ * a streaming GEMV for one and two tokens, tcgen05 tensor-core kernels for more.
  * Uses the per-(device, stream) workspace of this library, created at the first call. */
 MLXR_API int mlxr_q_gemm_dequant(const void* x, const void* weights, const void* bias,
                                  void* y, int M, int N, int K, int quant_type,
@@ -208,10 +208,8 @@ MLXR_API int mlxr_repack_ggml_q4_0(const void* ggml_blocks, void* mlxr_blocks, i
  * plan/MetalKernelsPlan.md:109-117 intends.  x, y: [M, hidden]; w_gate, w_up:
  * packed [inter, hidden]; w_down: packed [hidden, inter]; all three in `quant_type`.
  * n and h = SiLU(g)*u are rounded to `dtype` where the composition materialises them;
- * h lives only in this library's workspace (L2-resident at decode sizes).  At decode batches
- * the block is ONE launch: the gate/up CTAs publish h as 8-byte words that carry the launch's
- * sequence number, and the down-projection CTAs poll those words instead of meeting at a grid
- * barrier. */
+ * h lives only in this library's workspace (L2-resident at decode sizes).  One and
+ * two tokens take two launches (RMSNorm and SiLU(gate) * up inside the first), more take three. */
 MLXR_API int mlxr_mlp_block(const void* x, const void* norm_weight, const void* w_gate,
                             const void* w_up, const void* w_down, void* y, int M,
                             int hidden, int inter, int quant_type, float eps, int dtype,

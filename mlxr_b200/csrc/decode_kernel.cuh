@@ -1,4 +1,5 @@
-// Persistent decode kernel for quantized linears at small batch (M <= 8), Q4_K and Q4_0.
+// Persistent decode kernel for quantized linears at small batch (M <= 8), Q4_K and Q4_0: float32 activations, the
+// tensor-parallel block in one launch, the entry with static scratch, and shapes that gemv.cu does not take.
 //
 // Roofline: HBM.  One CTA per SM, NG groups of eight warps.  Every compute warp owns a private ring of shared-memory stages that it fills
 // itself with 2-D tensor TMA copies (cp.async.bulk.tensor.2d, one box of 8 rows x 288 bytes
@@ -232,19 +233,6 @@ __device__ __forceinline__ int slice_seg0(const Phase& ph, int ks) {
   return ks * ph.segs_base + (ks < ph.segs_extra ? ks : ph.segs_extra);
 }
 
-// Pointer to the packed row r (0..15) of tile t.
-__device__ __forceinline__ const uint8_t* tile_row(const Phase& ph, int t, int r) {
-  if (ph.interleave) {
-    int row = 8 * t + (r & 7);
-    if (row >= ph.n_total) row = ph.n_total - 1;
-    return ph.w[r >> 3] + (size_t)row * ph.row_bytes;
-  }
-  int R = kTileRows * t + r;
-  if (R >= ph.n_total) R = ph.n_total - 1;
-  int m = 0;
-  if (ph.nmat > 1 && R >= ph.rows[0]) { R -= ph.rows[0]; m = 1; if (ph.nmat > 2 && R >= ph.rows[1]) { R -= ph.rows[1]; m = 2; } }
-  return ph.w[m] + (size_t)R * ph.row_bytes;
-}
 
 // Tiles of one (CTA, group) in a phase: t = first + i * step, i = 0 .. count-1.  The CTA
 // works on K-slice cta % S; the gridDim.x / S CTAs of a slice, times NG groups, share the tiles.

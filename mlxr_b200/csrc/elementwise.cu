@@ -1,6 +1,5 @@
-// RMSNorm, SwiGLU and RoPE as standalone kernels (the fused decode kernels carry their
-// own copies of this arithmetic; these serve the primitives called on their own and the
-// prefill path, where the GEMM dominates and the elementwise work is one HBM pass).
+// RMSNorm, SwiGLU and RoPE as standalone kernels: the primitives called on their own, and RMSNorm and RoPE
+// around the linears of three and more tokens (the kernels for fewer carry their own copies of this arithmetic).
 #include <algorithm>
 
 #include "common.cuh"

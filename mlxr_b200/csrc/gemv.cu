@@ -1,17 +1,20 @@
 // Linears for one or two tokens (Q4_K, Q4_0, Q8_0), single, stacked along N (q / k / v) or gate / up.
 //
-// Roofline: HBM.  Two things kept the earlier kernels at 0.4 of it: the time between a launch's end and the next
-// one's first product, because each filled its SM and nothing of the next launch could be there, and a
-// meeting of all warps for every 16 rows.  Here
-//   * a CTA (one per SM) takes at most half of the SM's shared memory, registers and threads, so that under
-//     programmatic stream serialization the next launch's CTA sits beside it, its ring full of weights, and
-//     only waits for its activations;
-//   * a CTA owns a contiguous range of rows (in granules of four: 14336 rows are 24 or 25 granules each on 148
-//     SMs); its work units, (16-row tile, stage of K), are dealt to the eight warps in contiguous ranges, every
-//     warp keeps its own sums, and the warps meet once, at the end, when all partial sums lie in shared
-//     memory and are added in warp order (deterministic);
+// Roofline: HBM.  What kept the earlier kernels at 0.4 of it was a meeting of all warps for every 16 rows and
+// unequal numbers of tiles per CTA.  Here
+//   * a CTA (one per SM) owns a contiguous range of rows (in granules of four: 14336 rows are 24 or 25
+//     granules each on 148 SMs); its work units, (16-row tile, stage of K), are dealt to the sixteen warps in
+//     contiguous ranges, every warp keeps its own sums, and the warps meet once, at the end, when all
+//     partial sums lie in shared memory and are added in warp order (deterministic);
 //   * every warp fills its own ring with 2-D tensor TMA (four boxes of 4 rows per stage) and drains it, so
-//     nothing inside the stream waits on another warp.
+//     nothing inside the stream waits on another warp;
+//   * under programmatic stream serialization the launch's CTAs fill their rings while the previous launch's
+//     last CTAs finish, and only the activations wait for its end.
+// 8B-shaped block of one token (two launches): 34.9 us with the persistent kernel of decode.cu, 24.7 here.
+// The stream runs at HBM's rate; a launch's boundary, the loading and conversion of its activations and its
+// epilogue (about 5 us of each launch) do not overlap with it.  Eight warps in half an SM's resources,
+// so that the next launch's CTA could sit beside, took 36.8 us: two CTAs of the next launch
+// came to lie on one SM.
 //
 // Arithmetic, 4-bit formats: activations as 16-bit fixed point per 256 elements, split in a high and a low
 // signed byte; raw nibbles multiplied as unsigned bytes by mma.sync.m16n8k32 (the 16 MMA rows are weight

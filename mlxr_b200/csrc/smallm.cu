@@ -64,7 +64,7 @@ constexpr int kSlots = 2;                  // slots of converted weights per gro
                                            // the leading parts and the residuals of one)
 constexpr int kBlockCols = kBK / 2;        // tensor-memory columns of a k-block: two 16-bit elements each
 // Warp roles: single-warp roles first, four epilogue warps (warp % 4 = TMEM lane quarter), producers
-constexpr int kWarpMma = 0, kWarpRaw = 2, kWarpX = 3, kWarpEpi0 = 4, kWarpProd0 = 8;   // two issuer warps: 0 and 1
+[[maybe_unused]] constexpr int kWarpMma = 0, kWarpRaw = 2, kWarpX = 3, kWarpEpi0 = 4, kWarpProd0 = 8;   // two issuer warps: 0 and 1
 constexpr int kWarpFix = kWarpProd0 + 4 * kGroups;                                     // counts shared tiles
 constexpr int kThreads = (kWarpFix + 1) * 32;
 constexpr int kMaxXStages = 4, kMaxRawStages = 2 * kGroups;

@@ -69,13 +69,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// the same with the A operand in tensor memory: lane = row, one 32-bit column per two K elements
+// A operand in tensor memory: lane = row, one 32-bit column per two K elements
 __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -201,25 +195,6 @@ template <typename T> struct Fmt;
 template <> struct Fmt<__half> { static constexpr int v = 0; };
 template <> struct Fmt<__nv_bfloat16> { static constexpr int v = 1; };
 
-// Eight consecutive weights of a Q4_K sub-block (one 32-bit word of nibbles, element order =
-// nibble order) -> four packed pairs of the activation dtype.
-//
-// fp16 activations: the shader's arithmetic exactly (q_gemm_dequant.metal:244-256).  1024 + n as
-// fp16 is 0x6400 | n; subtracting 1032 gives n - 8 exactly; then rn16(rn16((n - 8) * ss) + sm).
-__device__ __forceinline__ uint4 dequant8_f16(uint32_t v, __half2 ss, __half2 sm) {
-  const uint32_t lo = v & 0x0F0F0F0Fu, hi = (v >> 4) & 0x0F0F0F0Fu;
-  const __half2 off = __half2half2(__ushort_as_half((unsigned short)0x6408));   // 1032
-  uint32_t out[4];
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const uint32_t sel = (uint32_t)j | ((uint32_t)j << 4) | ((uint32_t)(4 + j) << 8) | ((uint32_t)(4 + j) << 12);
-    uint32_t bits = (__byte_perm(lo, hi, sel) & 0x00FF00FFu) | 0x64006400u;
-    const __half2 q = __hsub2(*reinterpret_cast<__half2*>(&bits), off);
-    const __half2 r = __hadd2_rn(__hmul2_rn(q, ss), sm);
-    out[j] = *reinterpret_cast<const uint32_t*>(&r);
-  }
-  return make_uint4(out[0], out[1], out[2], out[3]);
-}
 // bf16 activations: the weight is rounded to bf16 for the MMA anyway (2^-9 relative), so the two
 // fp16 roundings of the shader are not reproduced; one fp32 multiply-add per weight from the
 // exact fp16 scale and min, then one rounding to bf16.  The nibble becomes the fp32 number

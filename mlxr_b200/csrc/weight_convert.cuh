@@ -195,7 +195,8 @@ __device__ __forceinline__ void convert64(const uint8_t* row, KB KBV, const floa
     auto block = [&](auto S) {
       constexpr int s = decltype(S)::value;
       const __half d = s ? high_half(w[8]) : low_half(w[0]);
-      const float df = __half2float(d), s256 = 256.0f * df, c = -32896.0f * df;
+      const float df = __half2float(d);
+      [[maybe_unused]] const float s256 = 256.0f * df, c = -32896.0f * df;
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         const uint32_t u = (s ? w[9 + i] : __funnelshift_r(w[i], w[i + 1], 16)) ^ 0x80808080u;    // bytes q + 128

@@ -47,7 +47,7 @@ constexpr int kGroups = 4;                 // producer groups of four warps; gro
 constexpr int kSlots = 2;                  // converted k-blocks per group
 constexpr int kStages = kGroups * kSlots;  // k-blocks in flight: stage g * kSlots + (unit & 1) holds k-block g's weights and X tile
 constexpr int kSlotCols = kBK / 2;         // tensor-memory columns of one: two 16-bit elements each
-constexpr int kWarpMma = 0, kWarpRaw = 1, kWarpX = 2, kWarpFix = 3, kWarpEpi0 = 4, kWarpProd0 = 8;
+[[maybe_unused]] constexpr int kWarpMma = 0, kWarpRaw = 1, kWarpX = 2, kWarpFix = 3, kWarpEpi0 = 4, kWarpProd0 = 8;
 constexpr int kThreads = (kWarpProd0 + 4 * kGroups) * 32;
 constexpr int kTileGroup = 8;              // token tiles that share a sweep over the weights
 constexpr int kSmemMax = 227 * 1024;
