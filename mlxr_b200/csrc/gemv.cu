@@ -584,7 +584,7 @@ template <int QT> static size_t layout(Params* P, int M, int grid) {
   using G = Geo<QT>;
   const int per = P->interleave ? 2 : 4, most = (P->granules + grid - 1) / grid, tiles = (most + per - 1) / per;
   P->x_stride = (QT == MLXR_Q8_0 ? 2 * P->K : P->K) + 16;
-  for (P->stages = kMaxStages; P->stages >= 2; P->stages--) {
+  for (P->stages = kMaxStages; P->stages >= 1; P->stages--) {
     size_t o = (size_t)kWarps * P->stages * G::kStage;
     auto take = [&](size_t n) { const size_t at = o; o += (n + 15) & ~(size_t)15; return (int)at; };
     P->off_x = take((size_t)(QT == MLXR_Q8_0 ? M : 2 * M) * P->x_stride);
@@ -600,8 +600,20 @@ template <int QT> static size_t layout(Params* P, int M, int grid) {
 
 bool gemv_supported(int qt, int M, int K, int rows, int dtype, const void* const* w, int nmat) {
   if (qt != MLXR_Q4_K && qt != MLXR_Q4_0 && !(qt == MLXR_Q8_0 && dtype != MLXR_F32)) return false;
-  // shared memory: two 16-row stages per warp (74 KB), the activations, 4 bytes per row, token and SM
-  if (M < 1 || M > 2 || K < 256 || K % 256 != 0 || K > 32768 || rows > (1 << 19)) return false;
+  if (M < 1 || M > 2 || K < 256 || K % 256 != 0 || K > 32768 || rows < 1 || rows > (1 << 19)) return false;
+  // Shared memory: the ring (74 KB per stage of all warps), the activations, the sums of a CTA's rows.  Two tokens of more
+  // than about 20000 elements leave room for one stage.  As single or stacked rows and as gate / up.
+  int sms = 0;
+  if (device_sms(&sms)) return false;
+  Params P;
+  memset(&P, 0, sizeof(P));
+  P.K = K;
+  P.nseg = K / 256;
+  for (P.interleave = 0; P.interleave < 2; P.interleave++) {
+    P.granules = (rows / (P.interleave + 1) + 3) / 4;
+    const int grid = std::max(1, std::min(sms, P.granules));
+    if (!(qt == MLXR_Q4_K ? layout<MLXR_Q4_K>(&P, M, grid) : qt == MLXR_Q4_0 ? layout<MLXR_Q4_0>(&P, M, grid) : layout<MLXR_Q8_0>(&P, M, grid))) return false;
+  }
   for (int i = 0; i < nmat; i++)
     if (((uintptr_t)w[i]) & 15u) return false;
   return true;

@@ -33,7 +33,7 @@ def _dense(oracle, packed, N, K, qt):
 
 
 @pytest.mark.parametrize("qt,dt", [(3, "bf16"), (3, "f16"), (3, "f32"), (0, "bf16"), (0, "f16"), (0, "f32"), (2, "bf16"), (2, "f16")])
-@pytest.mark.parametrize("M,N,K", [(1, 4, 256), (2, 5, 256), (1, 67, 768), (2, 593, 512), (1, 1000, 1280), (2, 2369, 4352), (1, 130, 16640)])
+@pytest.mark.parametrize("M,N,K", [(1, 4, 256), (2, 5, 256), (1, 67, 768), (2, 593, 512), (1, 1000, 1280), (2, 2369, 4352), (1, 130, 16640), (2, 70, 20992), (1, 33, 32768), (2, 33, 32768)])
 def test_linear(oracle, qt, dt, M, N, K):
     import mlxr_b200 as mx
     from mlxr_b200.quantize import quantize
@@ -64,7 +64,7 @@ def test_range_of_bf16(oracle, qt, scale):
 
 
 @pytest.mark.parametrize("qt", [0, 2, 3])
-@pytest.mark.parametrize("M,H,I", [(1, 512, 1280), (2, 768, 2304)])
+@pytest.mark.parametrize("M,H,I", [(1, 512, 1280), (2, 768, 2304), (2, 256, 24320)])
 def test_block(oracle, qt, M, H, I):
     import mlxr_b200 as mx
     from mlxr_b200.quantize import quantize
