@@ -186,8 +186,12 @@ static int run_linear(const void* x, const void* w, const void* bias, void* y, i
     L.w[0] = w; L.rows[0] = N; L.nmat = 1; L.K = K; L.x = x; L.y[0] = y; L.bias[0] = bias;
     return launch_gemv(L, M, qt, dtype, ws->status, st);
   }
-  // canonical Q4_K, and NF4 rows that do not start on 16 bytes, have no kernel of their own for one or two tokens
-  const bool small_only = qt == MLXR_GGML_Q4_K || (qt == MLXR_NF4 && !gemv_rows_supported(qt, M, K, x, w));
+  // Canonical Q4_K, and NF4 rows that do not start on 16 bytes, have no kernel of their own for one or two tokens.  The
+  // one NF4 has looks every weight up once per token; from 2^24 weights on the small-batch kernel, which converts
+  // once, is the faster one for two (4096 x 4096: 14.5 us there, 11.6 here; 14336 x 4096: 34.4, 27.9; 4096 x 14336:
+  // 40.5, 26.7; 4096 x 2048: 7.6, 8.5).
+  const bool small_only = qt == MLXR_GGML_Q4_K ||
+                          (qt == MLXR_NF4 && (!gemv_rows_supported(qt, M, K, x, w) || (M == 2 && (long long)N * K >= (1 << 24))));
   if ((M >= 3 || (M > 0 && small_only)) && N > 0) {
     TcPath path;
     WidePlan wide;

@@ -186,3 +186,19 @@ def test_stacked_projections_with_rope(oracle, qt, M, H, QH, KH, D):
         want = mx.rope_apply(y, cos, sin, pos) if i < 2 else y
         # one ulp of the linear's result at most, 2^-10, where the two sums round to different sides
         assert float((got.double() - want.double()).norm() / want.double().norm()) <= 2.0 ** -11
+
+
+@pytest.mark.parametrize("N", [4095, 4096, 4097])
+def test_two_tokens_nf4_at_the_border(oracle, N):
+    """Two tokens change kernels at 2^24 weights; bias, and a last tile of one row above it.  Bound as for
+    three tokens in test_other_formats: 2^-9 of the bf16 result."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    K, M = 4096, 2
+    packed = quantize(make_weights(N, K, 5), 16)
+    xt, xf = make_acts(M, K, 6, torch.bfloat16)
+    bt, bf = make_acts(1, N, 7, torch.bfloat16)
+    want = xf.astype(np.float64) @ oracle.dequantize(packed, N, K, 16)[0].astype(np.float64).reshape(N, K).T + bf[0]
+    y = mx.q_gemm_dequant(xt.cuda(), torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(16), 64, bt[0].contiguous().cuda())
+    assert _status() == 0
+    assert oracle.rel_l2(y.float().cpu().numpy(), want) <= 2.0 ** -9
