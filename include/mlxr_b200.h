@@ -309,6 +309,8 @@ MLXR_API int mlxr_debug_smallm_partition(long long units, int ctas, int cta, lon
 /* Attention input projections with RoPE on q and k: n = rmsnorm(x) (norm_weight may be
  * NULL), q = n Wq^T, k = n Wk^T, v = n Wv^T, then rope_apply on q and k
  * (Attention::forward, core/graph/layers.cpp:266-278, with the rope_apply primitive).
+ * n is rounded to `dtype` as RMSNorm materialises it, except for Q4_K at one and two tokens,
+ * where the kernel multiplies the float32 n.
  * wq: packed [q_heads*head_dim, hidden]; wk, wv: packed [kv_heads*head_dim, hidden].
  * q_out [M, q_heads, head_dim]; k_out, v_out [M, kv_heads, head_dim]; positions int32 [M]. */
 MLXR_API int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq,

@@ -504,7 +504,7 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
     DecodeLinear L;
     memset(&L, 0, sizeof(L));
     L.w[0] = w_gate; L.w[1] = w_up; L.rows[0] = L.rows[1] = inter; L.nmat = 2;
-    L.interleave = 1; L.K = hidden; L.x = x; L.gamma = norm_weight; L.eps = eps; L.y[0] = gbuf;
+    L.interleave = 1; L.K = hidden; L.x = x; L.gamma = norm_weight; L.eps = eps; L.round_n = 1; L.y[0] = gbuf;
     if (int r = launch_gemv(L, M, qt, dtype, ws->status, st)) return r;
     memset(&L, 0, sizeof(L));
     L.w[0] = w_down; L.rows[0] = hidden; L.nmat = 1; L.K = inter; L.x = gbuf; L.y[0] = y;
@@ -630,6 +630,7 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
     L.w[0] = wq; L.w[1] = wk; L.w[2] = wv;
     L.rows[0] = q_heads * head_dim; L.rows[1] = L.rows[2] = kv_heads * head_dim; L.nmat = 3;
     L.K = hidden; L.x = x; L.gamma = norm_weight; L.eps = eps;
+    L.round_n = qt == MLXR_Q4_0;     // Q4_K multiplies the unrounded n (see the header)
     L.y[0] = q_out; L.y[1] = k_out; L.y[2] = v_out;
     L.epi[0] = L.epi[1] = 2;
     L.cos_t = cos_f16; L.sin_t = sin_f16; L.positions = positions;

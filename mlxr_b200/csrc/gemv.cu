@@ -67,6 +67,7 @@ struct Params {
   const void* x;
   const void* gamma;
   float eps;
+  int round_n;               // see DecodeLinear
   void* y[3];
   const void* bias[3];
   int epi[3];                // decode::Epilogue
@@ -428,6 +429,57 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
           *reinterpret_cast<uint4*>(smem + P.off_x + (size_t)m * P.x_stride + (sg * 256 + lane * 8) * 2) = *reinterpret_cast<const uint4*>(o);
         }
       }
+  } else if (gam && P.round_n) {
+    // n rounded to T before its conversion, so the row's sum of squares comes first.  A warp's first four
+    // segments wait for it in registers: up to K = 16384 nothing is read twice.
+    float v[NT][4][8], gv[4][8];
+    auto load_g = [&](int s0) {
+#pragma unroll
+      for (int u = 0; u < 4; u++) if (s0 + u * kWarps < P.nseg) load8(gam + (s0 + u * kWarps) * 256 + lane * 8, gv[u]);
+    };
+#pragma unroll
+    for (int m = 0; m < NT; m++) load_x(m, warp, v[m]);
+    if constexpr (NT == 1) load_g(warp);
+    issue_held();
+#pragma unroll
+    for (int m = 0; m < NT; m++) {
+      float ss = 0.0f;
+      auto add = [&](int s0, const float (&a)[4][8]) {
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          if (s0 + u * kWarps < P.nseg)
+#pragma unroll
+            for (int i = 0; i < 8; i++) ss = fmaf(a[u][i], a[u][i], ss);
+      };
+      add(warp, v[m]);
+      for (int s0 = warp + 4 * kWarps; s0 < P.nseg; s0 += 4 * kWarps) {
+        float a[4][8];
+        load_x(m, s0, a);
+        add(s0, a);
+      }
+      ss = warp_sum(ss);
+      if (lane == 0) misc->red[warp * NT + m] = ss;
+    }
+    __syncthreads();
+    for (int s0 = warp; s0 < P.nseg; s0 += 4 * kWarps) {
+      if (NT > 1 || s0 != warp) load_g(s0);
+#pragma unroll
+      for (int m = 0; m < NT; m++) {
+        if (s0 != warp) load_x(m, s0, v[m]);
+        float tot = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) tot += misc->red[w * NT + m];
+        const float rinv = 1.0f / sqrtf(tot / (float)P.K + P.eps);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int sg = s0 + u * kWarps;
+          if (sg >= P.nseg) break;
+#pragma unroll
+          for (int i = 0; i < 8; i++) v[m][u][i] = Act<T>::to_f(Act<T>::from_f(__fmul_rn(__fmul_rn(v[m][u][i], rinv), gv[u][i])));
+          emit_fixed<QT>(smem, P, m, sg, lane, v[m][u]);
+        }
+      }
+    }
   } else {
     // fixed point; the block scaling is independent of a factor common to the row, so 1 / rms multiplies the sums at
     // the end and the conversion does not wait for the sum of squares
@@ -460,7 +512,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
   }
   issue_held();
   __syncthreads();
-  if (QT != MLXR_Q8_0 && gam && tid >= kThreads - NT) {
+  const bool scale_sums = QT != MLXR_Q8_0 && gam && !P.round_n;     // 1 / rms still to be applied
+  if (scale_sums && tid >= kThreads - NT) {
     const int m = kThreads - 1 - tid;
     float tot = 0.0f;
 #pragma unroll
@@ -521,7 +574,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
     // the warps after the one that holds the tile's first stage, as long as their ranges begin inside the tile
     for (int w = ((t * S + 1) * kWarps - 1) / units + 1; w < kWarps && (units * w) / kWarps < (t + 1) * S; w++)
       if ((units * (w + 1)) / kWarps > (units * w) / kWarps) v += reinterpret_cast<const float*>(smem + P.off_head)[w * 16 * NT + r];
-    sums[e] = QT != MLXR_Q8_0 && P.gamma ? v * misc->rinv[r % NT] : v;
+    sums[e] = scale_sums ? v * misc->rinv[r % NT] : v;
   }
   __syncthreads();
   // ---- epilogue: a thread per pair of adjacent rows and batch row ----
@@ -675,6 +728,7 @@ int launch_gemv(const DecodeLinear& L, int M, int qt, int dtype, int* status, cu
   P.x = L.x;
   P.gamma = L.gamma;
   P.eps = L.eps;
+  P.round_n = L.round_n;
   P.cos_t = (const __half*)L.cos_t;
   P.sin_t = (const __half*)L.sin_t;
   P.positions = L.positions;

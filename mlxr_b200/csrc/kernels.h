@@ -68,6 +68,9 @@ struct DecodeLinear {
   const void* x;           // [M, K]
   const void* gamma;       // RMSNorm weight or null
   float eps;
+  // launch_gemv, 4-bit formats: the normalised activations are rounded to the activation type before they are
+  // multiplied, as the composition of RMSNorm and a linear rounds them (Q8_0 and launch_decode always round)
+  int round_n;
   void* y[3];
   const void* bias[3];
   int epi[3];              // 0 plain, 2 RoPE, 3 plain fp32 store (y is float*)

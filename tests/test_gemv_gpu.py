@@ -98,3 +98,26 @@ def test_formats_of_the_small_batch_kernel(oracle, qt, M):
     assert _status() == 0
     want = x.double() @ w.T
     assert float((y.double() - want).norm() / want.norm()) <= RESULT["bf16"] + 2.0 ** -16
+
+
+@pytest.mark.parametrize("qt", [0, 3])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("M,H,I", [(1, 1024, 2816), (2, 1280, 768), (1, 17408, 512), (2, 17408, 512)])
+def test_block_rounds_the_normalised_input(qt, dt, M, H, I):
+    """n = rmsnorm(x) enters the products rounded to the activation type, as RMSNorm called by itself returns it (rows of
+    more than 16384 elements are read a second time for that).  Against the block made of this package's own operators: g,
+    u, h and y are rounded on both sides.  Before that the two sides differ by the step of the fixed point at most, where a
+    segment's largest value fell to another neighbour and with it the scale: d = sqrt(2) 3.6e-5 of the result.  A rounding
+    to p bits turns a difference d into sqrt(d 2^(1 - p)) in the 2-norm (a share d 2^(p - 1) of the values moves by an
+    ulp): 6.3e-4 for bf16, 2.2e-4 for fp16, and d itself.  An unrounded n comes out at 4.6e-3 and 6e-4."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    g, u, d = (torch.from_numpy(quantize(make_weights(n, k, s), qt)).cuda() for n, k, s in ((I, H, 1), (I, H, 2), (H, I, 3)))
+    x, nw = make_acts(M, H, 4, DT[dt])[0].cuda(), make_acts(1, H, 5, DT[dt])[0][0].contiguous().cuda()
+    q, gs = mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt)
+    y = mx.mlp_block(x, nw, g, u, d, I, q, 1e-5)
+    assert _status() == 0
+    n = mx.rmsnorm_fused(x, nw, 1e-5)
+    h = mx.swiglu(mx.q_gemm_dequant(n, g, M, I, H, q, gs), mx.q_gemm_dequant(n, u, M, I, H, q, gs))
+    want = mx.q_gemm_dequant(h, d, M, H, I, q, gs).double()
+    assert float((y.double() - want).norm() / want.norm()) <= {"bf16": 7e-4, "f16": 2.8e-4}[dt]
