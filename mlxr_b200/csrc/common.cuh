@@ -94,11 +94,11 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// SiLU with the sign-split sigmoid of swiglu_mlp_fused.metal:92-99.
+// SiLU with the sign-split sigmoid of swiglu_mlp_fused.metal:92-99: x / (1 + e^-x) for x >= 0, x e^x / (1 + e^x)
+// below, as one exponential and one division (the same operations, without the branch).
 __device__ __forceinline__ float swish_f(float x) {
-  if (x >= 0.0f) return x / (1.0f + expf(-x));
-  float e = expf(x);
-  return x * e / (1.0f + e);
+  const float e = expf(-fabsf(x));
+  return (x >= 0.0f ? x : x * e) / (1.0f + e);
 }
 
 // The 6-bit (scale, min) pair the reference shader uses for sub-block s of a Q4_K

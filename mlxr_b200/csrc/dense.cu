@@ -157,11 +157,6 @@ struct Shared {
 constexpr size_t kSmem = (size_t)kStages * kStageBytes + 4 * 2 * kOutBytes + sizeof(Shared) + 1024;
 static_assert(kSmem <= 227 * 1024, "shared memory");
 
-__device__ __forceinline__ float swish_fast(float x) {
-  const float e = __expf(-fabsf(x));
-  const float s = __fdividef(1.0f, 1.0f + e);
-  return x * (x >= 0.0f ? s : e * s);
-}
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -289,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
             const int j = 2 * e + k;
             if constexpr (SWIGLU) {
               const float g = Act<T>::to_f(Act<T>::from_f(__uint_as_float(r[j]))), u = Act<T>::to_f(Act<T>::from_f(__uint_as_float(r[16 + j])));
-              v[k] = Act<T>::from_f(swish_fast(g) * u);
+              v[k] = Act<T>::from_f(swish_f(g) * u);
             } else {
               v[k] = Act<T>::from_f(__uint_as_float(r[j]) + (bias && n0 + j < P.N ? Act<T>::to_f(bias[n0 + j]) : 0.0f));
             }

@@ -178,14 +178,8 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const T* __restrict__ g,
 }
 
 // The same for 16-bit types, 128-bit accesses, two vectors in flight per thread and operand.  Bound by HBM (three
-// streams) once the exponential and the division are the fast ones (relative error about 1e-6 before the
-// rounding to 16 bits); with expf, an IEEE division and 2-byte accesses [1111, 14336] fp16 took 41 us
-// where the bytes need 14.6.
-__device__ __forceinline__ float swish16(float x) {
-  const float e = __expf(-fabsf(x));
-  const float s = __fdividef(1.0f, 1.0f + e);      // sigmoid(|x|)
-  return x * (x >= 0.0f ? s : e * s);
-}
+// streams) and, close behind, by the exponential and the division; with 2-byte accesses [1111, 14336] fp16 took
+// 41 us where the bytes need 14.6.
 template <typename T, bool UP>
 __global__ void __launch_bounds__(256) swiglu_vec_kernel(const T* __restrict__ g, const T* __restrict__ u, T* __restrict__ o, size_t nvec) {
   const size_t step = (size_t)gridDim.x * 256;
@@ -202,7 +196,7 @@ __global__ void __launch_bounds__(256) swiglu_vec_kernel(const T* __restrict__ g
     for (int k = 0; k < 2; k++) {
       if (k && !two) break;
 #pragma unroll
-      for (int e = 0; e < 8; e++) a[k][e] = UP ? swish16(a[k][e]) * b[k][e] : swish16(a[k][e]);
+      for (int e = 0; e < 8; e++) a[k][e] = UP ? swish_f(a[k][e]) * b[k][e] : swish_f(a[k][e]);
       store8v(o + (i + k * step) * 8, a[k]);
     }
   }

@@ -169,3 +169,16 @@ def test_swiglu_mlp_dense_matches_composition():
     assert float((y - want).norm() / want.norm()) < 1e-5
     with pytest.raises(ValueError):
         mx.swiglu_mlp(x.cuda(), wg.cuda(), wu.cuda()[:, :8].contiguous(), wd.cuda())
+
+
+def test_swiglu_is_rounded_from_float32():
+    """16-bit swiglu is a float32 result rounded once, also where the exponential is small: an error of k float32 ulp
+    before the rounding moves 2 k / 2^16 of all bf16 results to the other neighbour.  expf (1 ulp by its
+    documented bound), 1 + e, the division and two products (half an ulp each) make k at most 3.5 and the share at most
+    1.1e-4; an exponential whose error grows with the argument (2 + 1.17 |x| ulp, 58 on average here) moves 1.8e-3."""
+    import mlxr_b200 as mx
+    g = torch.Generator().manual_seed(1)
+    gate = (-80 + 60 * torch.rand(1 << 21, generator=g)).to(torch.bfloat16).cuda()
+    up = (1e20 * (1 + torch.rand(1 << 21, generator=g))).to(torch.bfloat16).cuda()
+    want = (torch.nn.functional.silu(gate.double()) * up.double()).to(torch.bfloat16)
+    assert float((mx.swiglu(gate, up) != want).float().mean()) <= 2e-4
