@@ -19,8 +19,8 @@ using tc::dequant8_bf16;
 //            the product); everything else as kRound
 //   kRound   the exact value rounded once (fp16 Q4_K / Q4_1: the reference shader's half arithmetic)
 //   kSplit   a leading and a residual 16-bit part, both multiplied: the weight keeps 16 (bf16) or 22
-//            (fp16) significant bits.  For the formats whose small-batch products have always used
-//            the float32 value of the weight
+//            (fp16) significant bits.  For the products that use the float32 value of the weight: Q8_0 and
+//            NF4 up to 8 tokens, canonical Q4_K, and the q / k / v projections of 4-bit formats up to 8 tokens
 enum Mode { kFast = 0, kRound = 1, kSplit = 2 };
 
 // Bytes that 256 weights of a row occupy, and the bytes staged for them.  NF4's 136 bytes are not a
@@ -140,12 +140,23 @@ __device__ __forceinline__ __half half_of6(uint32_t n) {
 // Eight weights q ss + sm of one word of nibbles (q = n - 8), in the form MODE asks for
 template <int BF, int MODE> struct Scale { uint32_t s, m; };      // packed pair, or float32 bits
 template <int BF, int MODE> __device__ __forceinline__ Scale<BF, MODE> make_scale(__half ss, __half sm) {
-  if constexpr (BF == 0) return {dup_f16(ss), dup_f16(sm)};
+  if constexpr (MODE == kSplit) return {__float_as_uint(__half2float(ss)), __float_as_uint(__half2float(sm))};
+  else if constexpr (BF == 0) return {dup_f16(ss), dup_f16(sm)};
   else if constexpr (MODE == kFast) return {dup_bf16(__half2float(ss)), dup_bf16(__half2float(sm))};
   else { const float f = __half2float(ss); return {__float_as_uint(f), __float_as_uint(fmaf(-136.0f, f, __half2float(sm)))}; }
 }
-template <int BF, int MODE> __device__ __forceinline__ void nibbles8(uint32_t v, const Scale<BF, MODE>& c, uint32_t* out) {
-  if constexpr (BF == 0) exact8_f16(v, c.s, c.m, out);
+template <int BF, int MODE> __device__ __forceinline__ void nibbles8(uint32_t v, const Scale<BF, MODE>& c, uint32_t* out, uint32_t* res) {
+  if constexpr (MODE == kSplit) {
+    const uint32_t lo = v & 0x0F0F0F0Fu, hi = (v >> 4) & 0x0F0F0F0Fu;
+    const float s = __uint_as_float(c.s), m = __uint_as_float(c.m);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      // byte n in the low byte of 0x4B00'0000 is the fp32 number 2^23 + n: n - 8 exactly, one rounding of the sum
+      const float fe = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7440u | (uint32_t)j)) - 8388616.0f;
+      const float fo = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7440u | (uint32_t)j)) - 8388616.0f;
+      emit<BF, MODE>(fmaf(fe, s, m), fmaf(fo, s, m), out[j], res[j]);
+    }
+  } else if constexpr (BF == 0) exact8_f16(v, c.s, c.m, out);
   else if constexpr (MODE == kFast) fast8_bf16(v, c.s, c.m, out);
   else put(dequant8_bf16(v, __uint_as_float(c.s), __uint_as_float(c.m)), out);
 }
@@ -173,10 +184,10 @@ __device__ __forceinline__ void convert64(const uint8_t* row, KB KBV, const floa
     const auto c1 = make_scale<BF, MODE>(__hmul_rn(half_of6(g & 63u), d), __hmul_rn(half_of6((g >> 6) & 63u), dmin));
     const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
-    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[i], c0, a + 4 * i);
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[i], c0, a + 4 * i, b + 4 * i);
     out(tc::Int<0>{}, a, b);
 #pragma unroll
-    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[4 + i], c1, a + 4 * i);
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[4 + i], c1, a + 4 * i, b + 4 * i);
     out(tc::Int<1>{}, a, b);
   } else if constexpr (QT == MLXR_Q4_0) {       // two 18-byte blocks: fp16 d, 16 bytes of nibbles (q_gemm_dequant.metal:142-161)
     uint32_t w[9];
@@ -184,10 +195,10 @@ __device__ __forceinline__ void convert64(const uint8_t* row, KB KBV, const floa
     const __half zero = __ushort_as_half((unsigned short)0);
     const auto c0 = make_scale<BF, MODE>(low_half(w[0]), zero), c1 = make_scale<BF, MODE>(high_half(w[4]), zero);
 #pragma unroll
-    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(__funnelshift_r(w[i], w[i + 1], 16), c0, a + 4 * i);
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(__funnelshift_r(w[i], w[i + 1], 16), c0, a + 4 * i, b + 4 * i);
     out(tc::Int<0>{}, a, b);
 #pragma unroll
-    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[5 + i], c1, a + 4 * i);
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[5 + i], c1, a + 4 * i, b + 4 * i);
     out(tc::Int<1>{}, a, b);
   } else if constexpr (QT == MLXR_Q8_0) {       // two 34-byte blocks: fp16 d, 32 int8 (q_gemm_dequant.metal:190-201)
     uint32_t w[17];

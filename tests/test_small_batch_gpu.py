@@ -202,3 +202,24 @@ def test_two_tokens_nf4_at_the_border(oracle, N):
     y = mx.q_gemm_dequant(xt.cuda(), torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(16), 64, bt[0].contiguous().cuda())
     assert _status() == 0
     assert oracle.rel_l2(y.float().cpu().numpy(), want) <= 2.0 ** -9
+
+
+@pytest.mark.parametrize("qt", [0, 3])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("M,H,QH,KH,D", [(3, 768, 5, 1, 64), (8, 1280, 3, 3, 32), (8, 4096, 32, 8, 128)])
+def test_few_tokens_of_stacked_4_bit_weights_are_not_rounded(oracle, qt, dt, M, H, QH, KH, D):
+    """v of q / k / v up to 8 tokens: products with the float32 weights, as for the formats above, so 2^-9 (bf16) and 2^-11
+    (fp16) for the result's rounding.  Q4_K's reference is the shader's half arithmetic, two roundings of at most 2^-11
+    per weight that the kernel does not make.  Weights with scale and min rounded to bf16 come out at 3.4e-3."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    packed = [quantize(make_weights(n * D, H, 9 + i), qt) for i, n in enumerate((QH, KH, KH))]
+    x = make_acts(M, H, 4, DT[dt])[0].cuda()
+    cos, sin = mx.compute_rope_tables(16, D, 10000.0, device=torch.device("cuda"))
+    pos = torch.arange(M, dtype=torch.int32, device="cuda")
+    v = mx.qkv_rope(x, None, *(torch.from_numpy(w).cuda() for w in packed), cos, sin, pos, QH, KH, D, mx.QuantType(qt), 1e-5)[2]
+    assert _status() == 0
+    f, h = oracle.dequantize(packed[2], KH * D, H, qt)
+    w = torch.from_numpy((h.view(np.float16) if qt == 3 else f).astype(np.float64).reshape(KH * D, H)).cuda()
+    want = (x.double() @ w.T).reshape(M, KH, D)
+    assert float((v.double() - want).norm() / want.norm()) <= {"bf16": 2.0 ** -9, "f16": 2.0 ** -11}[dt] + (2.0 ** -11 if qt == 3 else 0)
