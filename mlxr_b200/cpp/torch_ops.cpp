@@ -9,8 +9,12 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <climits>
+
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/mlxr_b200.h"
@@ -28,12 +32,16 @@ decltype(&mlxr_swiglu) p_swiglu;
 
 struct Bad {};   // not plainly valid: leave it to the interpreted wrapper
 
+// A plain tensor with memory on the current device.  Subclasses (whose type the wrapper's results keep) and the
+// wrappers of vmap, torch.func.grad and fake tensors (which have no memory to point at) are not plain.
 const at::Tensor& tensor(PyObject* o) {
-  if (!THPVariable_Check(o)) throw Bad();
+  if (!THPVariable_CheckExact(o)) throw Bad();
   const at::Tensor& t = THPVariable_Unpack(o);
-  if (!t.is_cuda() || t.layout() != at::kStrided || !t.is_contiguous()) throw Bad();
+  if (!t.is_cuda() || t.layout() != at::kStrided || !t.has_storage() || !t.is_contiguous() || t.get_device() != c10::cuda::current_device()) throw Bad();
   return t;
 }
+const at::Tensor* optional(PyObject* o) { return o == Py_None ? nullptr : &tensor(o); }
+const void* data(const at::Tensor* t) { return t ? t->const_data_ptr() : nullptr; }
 int dtype_code(const at::Tensor& t) {
   switch (t.scalar_type()) {
     case at::kHalf: return MLXR_F16;
@@ -57,22 +65,24 @@ size_t bytes(const at::Tensor& t) { return (size_t)t.numel() * t.element_size();
 void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
 void want(bool ok) { if (!ok) throw Bad(); }
 
+// Pointers are taken before: nothing that can throw runs without the interpreter lock.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
 template <typename F> int without_gil(F&& f) {
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = f();
-  Py_END_ALLOW_THREADS
-  return rc;
+  NoGil released;
+  return f();
 }
+// torch's own translation of C++ exceptions (an allocation that fails stays a torch.OutOfMemoryError)
 template <typename F> PyObject* guarded(F&& f) {
+  HANDLE_TH_ERRORS
   try {
     return f();
   } catch (const Bad&) {
     Py_RETURN_NONE;
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
   }
+  END_HANDLE_TH_ERRORS
 }
 PyObject* result(int rc, const at::Tensor& y) { return rc == MLXR_OK ? THPVariable_Wrap(y) : PyLong_FromLong(rc); }
 
@@ -84,18 +94,16 @@ PyObject* mlp_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int inter = integer(a[5]), qt = integer(a[6]), dt = dtype_code(x);
     want(x.dim() == 2);
     const int M = (int)x.size(0), hidden = (int)x.size(1);
-    const void* nw = nullptr;
-    if (a[1] != Py_None) {
-      const at::Tensor& t = tensor(a[1]);
-      want(t.dim() == 1 && t.numel() == hidden && t.scalar_type() == x.scalar_type());
-      nw = t.data_ptr();
-    }
+    const at::Tensor* norm = optional(a[1]);
+    if (norm) want(norm->dim() == 1 && norm->numel() == hidden && norm->scalar_type() == x.scalar_type());
     const size_t gu = p_weight_size(inter, hidden, qt), dn = p_weight_size(hidden, inter, qt);
     want(gu && dn && bytes(wg) == gu && bytes(wu) == gu && bytes(wd) == dn);
     const float eps = real(a[7]);
     const at::Tensor y = at::empty(x.sizes(), x.options());
     void* st = stream();
-    return result(without_gil([&] { return p_mlp_block(x.data_ptr(), nw, wg.data_ptr(), wu.data_ptr(), wd.data_ptr(), y.data_ptr(), M, hidden, inter, qt, eps, dt, st); }), y);
+    const void *xp = data(&x), *np = data(norm), *gp = data(&wg), *up = data(&wu), *dp = data(&wd);
+    void* yp = y.data_ptr();
+    return result(without_gil([&] { return p_mlp_block(xp, np, gp, up, dp, yp, M, hidden, inter, qt, eps, dt, st); }), y);
   });
 }
 
@@ -106,17 +114,15 @@ PyObject* q_gemm_dequant(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor &x = tensor(a[0]), &w = tensor(a[1]);
     const int M = integer(a[2]), N = integer(a[3]), K = integer(a[4]), qt = integer(a[5]), gs = integer(a[6]), dt = dtype_code(x);
     want(x.dim() == 2 && x.size(0) == M && x.size(1) == K);
-    const void* b = nullptr;
-    if (a[7] != Py_None) {
-      const at::Tensor& t = tensor(a[7]);
-      want(t.dim() == 1 && t.size(0) == N && t.scalar_type() == x.scalar_type());
-      b = t.data_ptr();
-    }
+    const at::Tensor* bias = optional(a[7]);
+    if (bias) want(bias->dim() == 1 && bias->size(0) == N && bias->scalar_type() == x.scalar_type());
     const size_t need = p_weight_size(N, K, qt);
     want(need && bytes(w) >= need);
     const at::Tensor y = at::empty({M, N}, x.options());
     void* st = stream();
-    return result(without_gil([&] { return p_q_gemm(x.data_ptr(), w.data_ptr(), b, y.data_ptr(), M, N, K, qt, gs, dt, st); }), y);
+    const void *xp = data(&x), *wp = data(&w), *bp = data(bias);
+    void* yp = y.data_ptr();
+    return result(without_gil([&] { return p_q_gemm(xp, wp, bp, yp, M, N, K, qt, gs, dt, st); }), y);
   });
 }
 
@@ -128,14 +134,21 @@ PyObject* qkv_rope(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int qh = integer(a[8]), kh = integer(a[9]), hd = integer(a[10]), qt = integer(a[11]), off = integer(a[13]), dt = dtype_code(x);
     want(x.dim() == 2 && qh > 0 && kh > 0 && hd > 0 && cs.dim() == 2 && pos.scalar_type() == at::kInt && pos.numel() == x.size(0));
     const int M = (int)x.size(0), hidden = (int)x.size(1);
-    const void* nw = a[1] == Py_None ? nullptr : tensor(a[1]).data_ptr();
+    const at::Tensor* norm = optional(a[1]);
+    if (norm) want(norm->numel() >= hidden && norm->scalar_type() == x.scalar_type());
+    want(hd % 2 == 0 && (long long)qh * hd <= INT_MAX && (long long)kh * hd <= INT_MAX);
+    for (const at::Tensor* t : {&cs, &sn}) want(t->dim() == 2 && t->size(1) == hd / 2 && t->size(0) >= cs.size(0) && t->scalar_type() == at::kHalf);
+    const size_t nq = p_weight_size(qh * hd, hidden, qt), nkv = p_weight_size(kh * hd, hidden, qt);
+    want(nq && nkv && bytes(wq) >= nq && bytes(wk) >= nkv && bytes(wv) >= nkv);
     const float eps = real(a[12]);
     const at::Tensor q = at::empty({M, qh, hd}, x.options()), k = at::empty({M, kh, hd}, x.options()), v = at::empty({M, kh, hd}, x.options());
     void* st = stream();
-    const int rc = without_gil([&] {
-      return p_qkv_rope(x.data_ptr(), nw, wq.data_ptr(), wk.data_ptr(), wv.data_ptr(), (const uint16_t*)cs.data_ptr(), (const uint16_t*)sn.data_ptr(),
-                        (const int32_t*)pos.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), M, hidden, qh, kh, hd, (int)cs.size(0), qt, eps, off, dt, st);
-    });
+    const void *xp = data(&x), *np = data(norm), *qw = data(&wq), *kw = data(&wk), *vw = data(&wv);
+    const uint16_t *cp = (const uint16_t*)data(&cs), *sp = (const uint16_t*)data(&sn);
+    const int32_t* pp = (const int32_t*)data(&pos);
+    void *qp = q.data_ptr(), *kp = k.data_ptr(), *vp = v.data_ptr();
+    const int max_seq = (int)cs.size(0);
+    const int rc = without_gil([&] { return p_qkv_rope(xp, np, qw, kw, vw, cp, sp, pp, qp, kp, vp, M, hidden, qh, kh, hd, max_seq, qt, eps, off, dt, st); });
     if (rc != MLXR_OK) return PyLong_FromLong(rc);
     PyObject* t = PyTuple_New(3);
     if (!t) return nullptr;
@@ -153,12 +166,15 @@ PyObject* rmsnorm_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor &x = tensor(a[0]), &w = tensor(a[1]);
     const int dt = dtype_code(x);
     want(x.dim() >= 1 && w.dim() == 1 && x.size(-1) == w.numel() && w.numel() > 0 && w.scalar_type() == x.scalar_type());
-    const void* r = a[3] == Py_None ? nullptr : tensor(a[3]).data_ptr();
+    const at::Tensor* res = optional(a[3]);
+    if (res) want(res->numel() >= x.numel() && res->scalar_type() == x.scalar_type());
     const float eps = real(a[2]);
     const int hidden = (int)w.numel(), rows = (int)(x.numel() / hidden);
     const at::Tensor y = at::empty(x.sizes(), x.options());
     void* st = stream();
-    return result(without_gil([&] { return p_rmsnorm(x.data_ptr(), w.data_ptr(), r, y.data_ptr(), rows, hidden, eps, dt, st); }), y);
+    const void *xp = data(&x), *wp = data(&w), *rp = data(res);
+    void* yp = y.data_ptr();
+    return result(without_gil([&] { return p_rmsnorm(xp, wp, rp, yp, rows, hidden, eps, dt, st); }), y);
   });
 }
 
@@ -171,7 +187,10 @@ PyObject* swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
     want(g.sizes() == u.sizes() && g.scalar_type() == u.scalar_type());
     const at::Tensor y = at::empty(g.sizes(), g.options());
     void* st = stream();
-    return result(without_gil([&] { return p_swiglu(g.data_ptr(), u.data_ptr(), y.data_ptr(), (size_t)g.numel(), dt, st); }), y);
+    const void *gp = data(&g), *up = data(&u);
+    void* yp = y.data_ptr();
+    const size_t count = (size_t)g.numel();
+    return result(without_gil([&] { return p_swiglu(gp, up, yp, count, dt, st); }), y);
   });
 }
 
@@ -187,16 +206,18 @@ PyObject* rope_apply(PyObject*, PyObject* const* a, Py_ssize_t n) {
     want(x.dim() == 3 || x.dim() == 4);
     const int batch = (int)x.size(0), seq = x.dim() == 4 ? (int)x.size(1) : 1, heads = (int)x.size(-2), hd = (int)x.size(-1);
     want(hd > 0 && hd % 2 == 0);
-    for (const at::Tensor* t : {&cs, &sn}) want(t->dim() == 2 && t->size(1) == hd / 2 && t->scalar_type() == at::kHalf);
+    for (const at::Tensor* t : {&cs, &sn}) want(t->dim() == 2 && t->size(1) == hd / 2 && t->size(0) >= cs.size(0) && t->scalar_type() == at::kHalf);
     if (seq == 1) want(pos.dim() == 1 && pos.size(0) == batch);
     else want(pos.dim() == 2 && pos.size(0) == batch && pos.size(1) == seq);
     want(pos.scalar_type() == at::kInt);
     const at::Tensor y = inplace ? x : at::empty(x.sizes(), x.options());
     void* st = stream();
-    return result(without_gil([&] {
-                    return p_rope(x.data_ptr(), (const uint16_t*)cs.data_ptr(), (const uint16_t*)sn.data_ptr(), (const int32_t*)pos.data_ptr(), y.data_ptr(), batch, seq,
-                                  heads, hd, (int)cs.size(0), mode, scale, off, dt, check ? 1 : 0, st);
-                  }), y);
+    void* yp = y.data_ptr();           // in place: before x's, since it may give a lazily copied tensor memory of its own
+    const void* xp = data(&x);
+    const uint16_t *cp = (const uint16_t*)data(&cs), *sp = (const uint16_t*)data(&sn);
+    const int32_t* pp = (const int32_t*)data(&pos);
+    const int max_seq = (int)cs.size(0);
+    return result(without_gil([&] { return p_rope(xp, cp, sp, pp, yp, batch, seq, heads, hd, max_seq, mode, scale, off, dt, check ? 1 : 0, st); }), y);
   });
 }
 

@@ -35,6 +35,8 @@ def _dev(t: Optional[torch.Tensor], name: str) -> Optional[int]:
         raise _capi.MlxrError(_capi.ERR_CUDA, f"{name} must be a CUDA tensor: there is no CPU path")
     if not t.is_contiguous():
         raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, f"{name} must be contiguous")
+    if t.device.index != torch.cuda.current_device():      # the kernels run on the current device's stream
+        raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, f"{name} is on {t.device}, the current device is cuda:{torch.cuda.current_device()}")
     return t.data_ptr()
 
 
@@ -140,6 +142,8 @@ def rmsnorm_fused(input: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
     x = input.contiguous()
     w = weight.contiguous()
     r = residual.contiguous() if residual is not None else None
+    if r is not None and (r.numel() < x.numel() or r.dtype != x.dtype):
+        raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, "RMSNorm residual must have the input's size and dtype")
     out = torch.empty_like(x)
     rows = x.numel() // hidden if hidden else 0
     check(lib.mlxr_rmsnorm(_dev(x, "input"), _dev(w, "weight"), _dev(r, "residual"), out.data_ptr(),
@@ -217,6 +221,8 @@ def rope_apply(input: torch.Tensor, cos_table: torch.Tensor, sin_table: torch.Te
             raise _capi.MlxrError(_capi.ERR_SHAPE, f"{name} must have shape [max_seq_len, head_dim/2]")
         if t.dtype != torch.float16:
             raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, f"{name} must be float16")
+    if sin_table.shape[0] < cos_table.shape[0]:
+        raise _capi.MlxrError(_capi.ERR_SHAPE, "sin_table must have as many rows as cos_table")
     if seq == 1:
         if positions.dim() != 1 or positions.shape[0] != batch:
             raise _capi.MlxrError(_capi.ERR_SHAPE, "For flattened input, positions must have shape [tokens]")
@@ -350,6 +356,17 @@ def qkv_rope(x: torch.Tensor, norm_weight: Optional[torch.Tensor], wq: torch.Ten
     v = torch.empty((M, kv_heads, head_dim), dtype=x.dtype, device=x.device)
     if positions.dtype != torch.int32 or positions.numel() != M:
         raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, "positions must be int32 [M]")
+    for name, t, heads in (("wq", wq, q_heads), ("wk", wk, kv_heads), ("wv", wv, kv_heads)):
+        need = lib.mlxr_quantized_weight_size(heads * head_dim, hidden, int(quant_type))
+        if t.numel() * t.element_size() < need:
+            raise _capi.MlxrError(_capi.ERR_SHAPE, f"{name} holds {t.numel() * t.element_size()} bytes, {need} needed")
+    for name, t in (("cos_table", cos_table), ("sin_table", sin_table)):
+        if t.dim() != 2 or (head_dim % 2 == 0 and t.shape[1] != head_dim // 2) or t.shape[0] < cos_table.shape[0]:
+            raise _capi.MlxrError(_capi.ERR_SHAPE, f"{name} must have shape [max_seq_len, head_dim/2]")
+        if t.dtype != torch.float16:
+            raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, f"{name} must be float16")
+    if norm_weight is not None and (norm_weight.numel() < hidden or norm_weight.dtype != x.dtype):
+        raise _capi.MlxrInvalidArgument(_capi.ERR_INVALID_ARGUMENT, "RMSNorm weight size must match input's last dimension")
     check(lib.mlxr_qkv_rope(_dev(x, "x"), _dev(norm_weight, "norm_weight"), _dev(wq, "wq"), _dev(wk, "wk"),
                             _dev(wv, "wv"), _dev(cos_table, "cos_table"), _dev(sin_table, "sin_table"),
                             _dev(positions, "positions"), q.data_ptr(), k.data_ptr(), v.data_ptr(), M,
