@@ -121,3 +121,18 @@ def test_block_rounds_the_normalised_input(qt, dt, M, H, I):
     h = mx.swiglu(mx.q_gemm_dequant(n, g, M, I, H, q, gs), mx.q_gemm_dequant(n, u, M, I, H, q, gs))
     want = mx.q_gemm_dequant(h, d, M, H, I, q, gs).double()
     assert float((y.double() - want).norm() / want.norm()) <= {"bf16": 7e-4, "f16": 2.8e-4}[dt]
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3])
+@pytest.mark.parametrize("scale", [2.0 ** -120, 2.0 ** -102, 2.0 ** 126])
+def test_ends_of_the_range_of_bf16(oracle, qt, scale):
+    """Segments whose largest value lies near either end of the type's range, up to 2.9e38.  The scale of a 4-bit segment
+    is 1 / 32000 of its largest value: at 2^-120 a float32 of 13 bits or more (denormal), 2^-13 of the result."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    N, K = 64, 1024
+    packed = quantize(make_weights(N, K, 1, std=0.005), qt)
+    x = (make_acts(1, K, 2, torch.float32)[0] * scale).clamp(-2.9e38, 2.9e38).to(torch.bfloat16).cuda()
+    y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), 1, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt))
+    want = x.double() @ _dense(oracle, packed, N, K, qt).T
+    assert float((y.double() - want).norm() / want.norm()) <= RESULT["bf16"] + WEIGHT[qt] + 2.0 ** -13
