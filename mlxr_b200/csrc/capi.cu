@@ -81,7 +81,7 @@ int get_workspace(cudaStream_t st, size_t need, Workspace** out, size_t need_sta
     MLXR_CUDA_TRY(cudaMalloc(&ws.status, 64));
     MLXR_CUDA_TRY(cudaMemset(ws.status, 0, 64));
     MLXR_CUDA_TRY(cudaMallocHost(&ws.status_host, 64));
-    memset(ws.status_host, 0, 64);
+    ws.status_host[0] = 0;
   }
   if (int r = grow(&ws.buf, &ws.bytes, need, st)) return r;
   if (int r = grow(&ws.stage, &ws.stage_bytes, need_stage, st)) return r;
@@ -95,6 +95,34 @@ int stream_status_word(cudaStream_t st, int** status) {
   if (int r = get_workspace(st, 0, &ws)) return r;
   *status = ws->status;
   return MLXR_OK;
+}
+
+// Words of pinned host memory that the kernels of checked rope_apply calls report into, one per call in flight: callers
+// that share a stream never see one another's.  As many as were ever in flight at once, rounded up to a page;
+// freed by mlxr_release_workspaces().
+static std::mutex g_check_mu;
+static std::vector<int*> g_check_free, g_check_pages;
+constexpr size_t kCheckPage = 4096 / sizeof(int);
+static int take_check_word(int** out) {
+  std::lock_guard<std::mutex> lk(g_check_mu);
+  if (g_check_free.empty()) {
+    int* page = nullptr;
+    MLXR_CUDA_TRY(cudaHostAlloc(&page, kCheckPage * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    memset(page, 0, kCheckPage * sizeof(int));
+    g_check_pages.push_back(page);
+    for (size_t i = 0; i < kCheckPage; i++) g_check_free.push_back(page + i);
+  }
+  *out = g_check_free.back();
+  g_check_free.pop_back();
+  return MLXR_OK;
+}
+// the word's value; the word must not be in use by a kernel any more
+static int give_check_word(int* w) {
+  const int v = *reinterpret_cast<volatile int*>(w);
+  *reinterpret_cast<volatile int*>(w) = 0;
+  std::lock_guard<std::mutex> lk(g_check_mu);
+  g_check_free.push_back(w);
+  return v;
 }
 
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -388,16 +416,17 @@ int mlxr_rope_apply(const void* x, const uint16_t* cos_f16, const uint16_t* sin_
   Workspace* ws = nullptr;
   if (int r = get_workspace(st, 0, &ws)) return r;
   // With `check` the kernel records a violation straight in pinned host memory (under unified addressing the
-  // host address is the device address), which saves a copy and a memset per call; the word is only
-  // read and cleared while the stream is idle.
-  int* const violation = ws->status_host + 8;
+  // host address is the device address), which saves a copy and a memset per call.
+  int* word = ws->status;
+  if (check) if (int r = take_check_word(&word)) return r;
   if (int r = launch_rope(x, cos_f16, sin_f16, positions, y, tokens, heads, head_dim, max_seq_len, mode,
-                          scale_factor, position_offset, dtype, check ? violation : ws->status, st))
+                          scale_factor, position_offset, dtype, word, st)) {
+    if (check) give_check_word(word);       // nothing was launched
     return r;
+  }
   if (check) {
-    MLXR_CUDA_TRY(cudaStreamSynchronize(st));
-    if (*reinterpret_cast<volatile int*>(violation) != 0) {
-      *reinterpret_cast<volatile int*>(violation) = 0;
+    MLXR_CUDA_TRY(cudaStreamSynchronize(st));     // on failure the kernel may still run: the word is not reused
+    if (give_check_word(word) != 0) {
       set_error("rope_apply: a position (+offset) lies outside [0, max_seq_len)");
       return MLXR_ERR_SHAPE;
     }
@@ -771,6 +800,14 @@ int mlxr_release_workspaces(void) {
     if (ws.status_host) cudaFreeHost(ws.status_host);
   }
   g_ws.clear();
+  {
+    std::lock_guard<std::mutex> check_lk(g_check_mu);
+    if (g_check_free.size() == g_check_pages.size() * kCheckPage) {      // no call in flight
+      for (int* page : g_check_pages) cudaFreeHost(page);
+      g_check_pages.clear();
+      g_check_free.clear();
+    }
+  }
   if (first != cudaSuccess) return cuda_fail(first, "mlxr_release_workspaces");
   return MLXR_OK;
 }

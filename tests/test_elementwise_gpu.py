@@ -182,3 +182,29 @@ def test_swiglu_is_rounded_from_float32():
     up = (1e20 * (1 + torch.rand(1 << 21, generator=g))).to(torch.bfloat16).cuda()
     want = (torch.nn.functional.silu(gate.double()) * up.double()).to(torch.bfloat16)
     assert float((mx.swiglu(gate, up) != want).float().mean()) <= 2e-4
+
+
+def test_position_check_of_two_threads_on_one_stream():
+    """The call that has the bad position gets the error, and only that one: the calls of both threads go to the same
+    stream and overlap, since a call releases the interpreter lock while it waits."""
+    import threading
+    import mlxr_b200 as mx
+    cos, sin = mx.compute_rope_tables(64, 64, 10000.0, device=torch.device("cuda"))
+    x = torch.randn(64, 8, 64, device="cuda").half()
+    good = torch.arange(64, dtype=torch.int32, device="cuda")
+    bad = good + 1
+    seen = {"good": 0, "bad": 0}
+
+    def run(name, pos):
+        for _ in range(400):
+            try:
+                mx.rope_apply(x, cos, sin, pos)
+            except mx._capi.MlxrError:
+                seen[name] += 1
+
+    threads = [threading.Thread(target=run, args=a) for a in (("good", good), ("bad", bad), ("good", good))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert seen == {"good": 0, "bad": 400}
