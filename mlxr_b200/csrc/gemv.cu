@@ -92,13 +92,12 @@ struct Misc {
 // the offset / min terms need.  1.5 * 2^23 added in the multiply leaves xi, rounded to nearest, in the low bits.
 template <int QT>
 __device__ __forceinline__ void emit_fixed(uint8_t* smem, const Params& P, int m, int sg, int lane, const float (&x)[8]) {
-  float v[8], amax = 0.0f;
+  float v[8];
+  uint32_t bits = 0;
+  // non-negative floats order like their bit patterns, NaN and Inf above every finite value (fmaxf would drop a NaN)
 #pragma unroll
-  for (int i = 0; i < 8; i++) v[i] = x[i];
-#pragma unroll
-  for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
-  // non-negative floats order like their bit patterns (NaN and Inf sort above every finite value)
-  amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+  for (int i = 0; i < 8; i++) { v[i] = x[i]; bits = max(bits, __float_as_uint(x[i]) & 0x7FFFFFFFu); }
+  float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, bits));
   float dl = 1.0f, inv = 0.0f;
   if (!(amax <= 3.0e38f)) { dl = __int_as_float(0x7fc00000); }   // a non-finite block poisons its outputs
   else if (amax > 0.0f) {

@@ -136,3 +136,25 @@ def test_ends_of_the_range_of_bf16(oracle, qt, scale):
     y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), 1, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt))
     want = x.double() @ _dense(oracle, packed, N, K, qt).T
     assert float((y.double() - want).norm() / want.norm()) <= RESULT["bf16"] + WEIGHT[qt] + 2.0 ** -13
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("norm", [False, True])
+def test_nan_reaches_its_row_only(qt, dt, norm):
+    """A NaN among finite values makes all of its token's outputs NaN and leaves the other token's alone; one that the
+    conversion to fixed point lost came out as finite numbers."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    N, K, M = 96, 768, 2
+    w = torch.from_numpy(quantize(make_weights(N, K, 3), qt)).cuda()
+    x = make_acts(M, K, 4, DT[dt])[0].cuda()
+    x[1, 300] = float("nan")
+    q, gs = mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt)
+    if norm:
+        d = torch.from_numpy(quantize(make_weights(K, 768, 5), qt)).cuda()
+        g = torch.from_numpy(quantize(make_weights(768, K, 6), qt)).cuda()
+        y = mx.mlp_block(x, torch.ones(K, device="cuda", dtype=DT[dt]), g, g, d, 768, q, 1e-5)
+    else:
+        y = mx.q_gemm_dequant(x, w, M, N, K, q, gs)
+    assert torch.isnan(y[1]).all() and torch.isfinite(y[0]).all()
