@@ -377,7 +377,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
   if constexpr (QT == MLXR_Q8_0) {
     // fp16 as they are; bf16 times a power of two per segment that brings its largest value to 2^14 .. 2^15, as fp16:
     // exact for every value above 2^-31 of the largest, so the products are those of the bf16 values and the
-    // weights need only the cheaper conversion to fp16.  With RMSNorm the norm is rounded to T first, so the
+    // weights need only the cheaper conversion to fp16.  An infinity or a NaN stays what it is and does not set the scale,
+    // or the finite values beside it would leave fp16's range.  With RMSNorm the norm is rounded to T first, so the
     // row's sum of squares comes before.
     float rinv[NT];
 #pragma unroll
@@ -429,9 +430,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
           if constexpr (Act<T>::kDtype == MLXR_BF16) {
             float amax = 0.0f;
 #pragma unroll
-            for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[u][i]));
+            for (int i = 0; i < 8; i++) amax = fabsf(v[u][i]) <= 3.4e38f ? fmaxf(amax, fabsf(v[u][i])) : amax;
             const int e = (int)(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)) >> 23);     // biased exponent
-            const int se = e == 0 || e == 255 ? 127 : min(254, 268 - e);                            // 2^14 / 2^(e - 127)
+            const int se = e == 0 ? 127 : min(254, 268 - e);                                        // 2^14 / 2^(e - 127)
             scale = __int_as_float(se << 23);
             if (lane == 0) reinterpret_cast<float*>(smem + P.off_delta)[m * P.nseg + sg] = 1.0f / scale;
           }

@@ -158,3 +158,19 @@ def test_nan_reaches_its_row_only(qt, dt, norm):
     else:
         y = mx.q_gemm_dequant(x, w, M, N, K, q, gs)
     assert torch.isnan(y[1]).all() and torch.isfinite(y[0]).all()
+
+
+def test_infinity_beside_large_values_q8_0():
+    """bf16, one infinity per token and, in the same segment, a value outside fp16's range: the outputs are infinities with
+    the sign of their weight, as the float32 products give them, not NaN."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    N, K, M = 64, 512, 2
+    wf = make_weights(N, K, 3)
+    wf[:, 40] = np.where(np.arange(N) % 2 == 0, 0.05, -0.05)
+    wf[:, 41] = -wf[:, 40]
+    x = make_acts(M, K, 4, torch.bfloat16)[0].cuda()
+    x[:, 40] = float("inf")
+    x[:, 41] = 1e6
+    y = mx.q_gemm_dequant(x, torch.from_numpy(quantize(wf, 2)).cuda(), M, N, K, mx.QuantType.Q8_0, 32).float().cpu().numpy()
+    assert np.array_equal(y, np.tile(np.where(np.arange(N) % 2 == 0, np.inf, -np.inf).astype(np.float32), (M, 1)))
