@@ -544,7 +544,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
   uint32_t par = 0;
   for (int u = ub; u < ue; u++) {
     const uint8_t* stage = smem + (size_t)(warp * D + slot) * G_::kStage;
-    mbar_wait(smem_u32(&misc->full[warp][slot]), par, &misc->dead, P.wait_ns);
+    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc->full[warp][slot]), par, &misc->dead, P.wait_ns))) {
+      // a give-up: the copies in flight must land before the CTA may exit (bounded)
+      if (lane == 0)
+        for (int i = u - ub; i < ue - ub - i_left; i++)
+          bounded_wait([&] { return decode::mbar_try_wait(smem_u32(&misc->full[warp][i % D]), (uint32_t)(i / D) & 1u); }, 1000000000ull);
+      __syncwarp();
+      break;
+    }
     const uint8_t *rl = stage + (L.rg >> 2) * G_::kBox + (L.rg & 3) * G_::kPitch, *rh = rl + 2 * G_::kBox;
     const int sg = st * G_::kSegs;
     if constexpr (QT == MLXR_Q8_0) {
@@ -579,6 +586,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
     }
   }
   __syncthreads();
+  if (misc->dead) {       // some sums are missing: nothing is stored
+    if (tid == 0) atomicExch(P.status, MLXR_ERR_TIMEOUT);
+    return;
+  }
 
   // ---- rows of this CTA: a thread per row and batch row adds the parts in warp order ----
   for (int e = tid; e < ntiles * 16 * NT; e += kThreads) {
@@ -636,7 +647,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
       if (odd) out[1] = Act<T>::from_f(vo);
     }
   }
-  if (tid == 0 && misc->dead) atomicExch(P.status, MLXR_ERR_TIMEOUT);
 }
 
 }  // namespace gemv
