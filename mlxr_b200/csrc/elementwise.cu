@@ -11,10 +11,10 @@ namespace mlxr {
 // rounding at the store (rmsnorm.metal:105-156, :165-217).  The row is read once from
 // HBM and kept in registers for the second pass (the reference reads it twice).
 template <typename T, int THREADS, int PER_THREAD>
-__global__ void __launch_bounds__(THREADS) rmsnorm_kernel(const T* __restrict__ x,
+__global__ void __launch_bounds__(THREADS) rmsnorm_kernel(const T* x,
                                                           const T* __restrict__ w,
-                                                          const T* __restrict__ res,
-                                                          T* __restrict__ y, int hidden,
+                                                          const T* res,
+                                                          T* y, int hidden,
                                                           float eps) {
   __shared__ float red[THREADS / 32];
   // A kernel launched behind this one with programmatic stream serialization (the linears of the
@@ -59,12 +59,18 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_kernel(const T* __restrict__ 
   }
 }
 
-// Eight 16-bit values, one 128-bit access
-template <typename T> __device__ __forceinline__ void load8v(const T* p, float (&v)[8]) {
-  const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+template <typename T> __device__ __forceinline__ void unpack8(const uint4& u, float (&v)[8]) {
   const T* h = reinterpret_cast<const T*>(&u);
 #pragma unroll
   for (int i = 0; i < 8; i++) v[i] = Act<T>::to_f(h[i]);
+}
+// Eight 16-bit values, one 128-bit access.  From L2, coherently: a kernel that starts under the one before it (programmatic
+// stream serialization) may find x still being written when it begins, and in place x is written by the kernel
+// itself; the read-only path (and const __restrict__, which lets the compiler take it) is defined only for data that
+// nobody writes while the kernel runs.  That holds for the norm weight and the tables: __ldg there.
+template <typename T, bool CONST = false> __device__ __forceinline__ void load8v(const T* p, float (&v)[8]) {
+  const uint4 u = CONST ? __ldg(reinterpret_cast<const uint4*>(p)) : __ldcg(reinterpret_cast<const uint4*>(p));
+  unpack8<T>(u, v);
 }
 template <typename T> __device__ __forceinline__ void store8v(T* p, const float (&v)[8]) {
   uint4 u;
@@ -82,17 +88,18 @@ static bool aligned16(const void* a, const void* b, const void* c = nullptr, con
 // of this and [1111, 4096] fp16 took 14 us where the bytes need 4.2.  Launched with programmatic stream
 // serialization: the CTAs are in place when the previous kernel of the stream ends.
 template <typename T, int THREADS, int PER>
-__global__ void __launch_bounds__(THREADS) rmsnorm_vec_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ res,
-                                                              T* __restrict__ y, int nvec, float eps) {
+__global__ void __launch_bounds__(THREADS) rmsnorm_vec_kernel(const T* x, const T* __restrict__ w, const T* res, T* y, int nvec, float eps) {
   __shared__ float red[THREADS / 32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const size_t row = (size_t)blockIdx.x * nvec * 8;
   float v[PER][8], ss = 0.0f;
+  uint4 rv[PER];
 #pragma unroll
   for (int i = 0; i < PER; i++) {
     const int c = threadIdx.x + i * THREADS;
     if (c < nvec) {
+      if (res) rv[i] = __ldcg(reinterpret_cast<const uint4*>(res + row + c * 8));      // before any store: y may be res
       load8v(x + row + c * 8, v[i]);
 #pragma unroll
       for (int e = 0; e < 8; e++) ss = fmaf(v[i][e], v[i][e], ss);
@@ -110,11 +117,11 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_vec_kernel(const T* __restric
     const int c = threadIdx.x + i * THREADS;
     if (c < nvec) {
       float g[8], o[8];
-      load8v(w + c * 8, g);
+      load8v<T, true>(w + c * 8, g);
 #pragma unroll
       for (int e = 0; e < 8; e++) o[e] = (v[i][e] * rms) * g[e];
       if (res) {
-        load8v(res + row + c * 8, g);
+        unpack8<T>(rv[i], g);
 #pragma unroll
         for (int e = 0; e < 8; e++) o[e] += g[e];
       }
@@ -166,8 +173,8 @@ int launch_rmsnorm(const void* x, const void* w, const void* res, void* y, int r
 
 // ---- swish / swiglu --------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_kernel(const T* __restrict__ g,
-                                                     const T* __restrict__ u, T* __restrict__ o,
+__global__ void __launch_bounds__(256) swiglu_kernel(const T* g,
+                                                     const T* u, T* o,
                                                      size_t n) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
@@ -181,7 +188,7 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const T* __restrict__ g,
 // streams) and, close behind, by the exponential and the division; with 2-byte accesses [1111, 14336] fp16 took
 // 41 us where the bytes need 14.6.
 template <typename T, bool UP>
-__global__ void __launch_bounds__(256) swiglu_vec_kernel(const T* __restrict__ g, const T* __restrict__ u, T* __restrict__ o, size_t nvec) {
+__global__ void __launch_bounds__(256) swiglu_vec_kernel(const T* g, const T* u, T* o, size_t nvec) {
   const size_t step = (size_t)gridDim.x * 256;
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < nvec; i += 2 * step) {
     const bool two = i + step < nvec;
@@ -257,11 +264,11 @@ int launch_cast_to_f32(const void* x, float* y, size_t n, int dtype, cudaStream_
 // math, one rounding at the store (rope_apply.metal:103-172).  A token whose position
 // falls outside the table is left untouched and flagged in *status.
 template <typename T>
-__global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x,
+__global__ void __launch_bounds__(256) rope_kernel(const T* x,
                                                    const __half* __restrict__ cos_t,
                                                    const __half* __restrict__ sin_t,
                                                    const int32_t* __restrict__ positions,
-                                                   T* __restrict__ y, size_t tokens, int heads,
+                                                   T* y, size_t tokens, int heads,
                                                    int pairs, int max_seq, int linear,
                                                    float scale, int offset, int* status) {
   const size_t total = tokens * heads * pairs;
@@ -293,9 +300,8 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* __restrict__ x,
 // Two tensors that share the positions (q and k of a layer) can go in one launch: vectors from `total` on are z's,
 // up to total_z.
 template <typename T>
-__global__ void __launch_bounds__(256) rope_vec_kernel(const T* __restrict__ x, const __half* __restrict__ cos_t, const __half* __restrict__ sin_t,
-                                                       const int32_t* __restrict__ positions, T* __restrict__ y, size_t total, int vec_per_token,
-                                                       T* __restrict__ z, size_t total_z, int vec_per_token_z,
+__global__ void __launch_bounds__(256) rope_vec_kernel(const T* x, const __half* __restrict__ cos_t, const __half* __restrict__ sin_t,
+                                                       const int32_t* positions, T* y, size_t total, int vec_per_token, T* z, size_t total_z, int vec_per_token_z,
                                                        int vec_per_head, int max_seq, int linear, float scale, int offset, int* status) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -307,12 +313,12 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(const T* __restrict__ x, 
     T* dst = first ? y : z;
     const size_t tok = i / per;
     const int c = (int)(i - tok * per) % vec_per_head;
-    const long long pos = (long long)positions[tok] + offset;
+    const long long pos = (long long)__ldcg(positions + tok) + offset;
     if (pos < 0 || pos >= max_seq) {
       if (status) atomicExch_system(status, 1);
       continue;
     }
-    const uint4 xv = *reinterpret_cast<const uint4*>(src + i * 8);
+    const uint4 xv = __ldcg(reinterpret_cast<const uint4*>(src + i * 8));
     const uint2 cv = __ldg(reinterpret_cast<const uint2*>(cos_t + (size_t)pos * vec_per_head * 4) + c);
     const uint2 sv = __ldg(reinterpret_cast<const uint2*>(sin_t + (size_t)pos * vec_per_head * 4) + c);
     const T* h = reinterpret_cast<const T*>(&xv);

@@ -208,3 +208,41 @@ def test_position_check_of_two_threads_on_one_stream():
     for t in threads:
         t.join()
     assert seen == {"good": 0, "bad": 400}
+
+
+def test_in_place_and_behind_a_kernel_that_still_runs():
+    """Every operator may write over what it reads, and may follow the kernel that writes its input without a pause
+    between them: the results are those of a call on a copy, alone on the device."""
+    import mlxr_b200 as mx
+    from mlxr_b200._capi import check, lib
+    st = torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(3)
+    H, N = 4096, 2048
+    for M in (1, 64):
+        x = torch.randn(M, H, device="cuda", generator=g).half()
+        r = torch.randn(M, N, device="cuda", generator=g).half()
+        w = torch.randn(N, device="cuda", generator=g).half()
+        blocks = torch.randint(0, 256, (N * H // 32, 18), dtype=torch.uint8, device="cuda", generator=g)
+        blocks[:, :2] = torch.tensor([0, 0x18], dtype=torch.uint8, device="cuda")       # scale 2^-9
+        lin = lambda: mx.q_gemm_dequant(x, blocks, M, N, H, mx.QuantType.Q4_0, 32)
+        cos, sin = mx.compute_rope_tables(M, 64, 10000.0, device=torch.device("cuda"))
+        pos = torch.arange(M, dtype=torch.int32, device="cuda")
+        y = lin()
+        torch.cuda.synchronize()
+        want = [mx.rmsnorm_fused(y, w, 1e-5, r), mx.swiglu(y, r), mx.rope_apply(y.reshape(M, -1, 64), cos, sin, pos).reshape(M, N)]
+        torch.cuda.synchronize()
+        for _ in range(50):
+            a, b, c, d, e = (lin() for _ in range(5))
+            res, gate = r.clone(), r.clone()
+            a = lin()
+            check(lib.mlxr_rmsnorm(a.data_ptr(), w.data_ptr(), r.data_ptr(), a.data_ptr(), M, N, 1e-5, 0, st))       # over x
+            b = lin()
+            check(lib.mlxr_rmsnorm(b.data_ptr(), w.data_ptr(), res.data_ptr(), res.data_ptr(), M, N, 1e-5, 0, st))   # over the residual
+            c = lin()
+            check(lib.mlxr_swiglu(c.data_ptr(), r.data_ptr(), c.data_ptr(), M * N, 0, st))
+            d = lin()
+            check(lib.mlxr_swiglu(d.data_ptr(), gate.data_ptr(), gate.data_ptr(), M * N, 0, st))
+            e = lin().reshape(M, -1, 64)
+            mx.rope_apply(e, cos, sin, pos, inplace=True, check_positions=False)
+            for got, ref in ((a, want[0]), (res, want[0]), (c, want[1]), (gate, want[1]), (e.reshape(M, N), want[2])):
+                assert torch.equal(got, ref)
