@@ -677,6 +677,9 @@ template <int QT> static size_t layout(Params* P, int M, int grid) {
 bool gemv_supported(int qt, int M, int K, int rows, int dtype, const void* const* w, int nmat) {
   if (qt != MLXR_Q4_K && qt != MLXR_Q4_0 && !(qt == MLXR_Q8_0 && dtype != MLXR_F32)) return false;
   if (M < 1 || M > 2 || K < 256 || K % 256 != 0 || K > 32768 || rows < 1 || rows > (1 << 19)) return false;
+  // Q4_0 rows of one segment are gemv_rows_kernel's, which multiplies the float32 activations (K = 256, float32: 8e-8 of
+  // the result there, 2.6e-5 with 16-bit fixed point)
+  if (qt == MLXR_Q4_0 && K < 512) return false;
   // Shared memory: the ring (74 KB per stage of all warps), the activations, the sums of a CTA's rows.  Two tokens of more
   // than about 20000 elements leave room for one stage.  As single or stacked rows and as gate / up.
   int sms = 0;

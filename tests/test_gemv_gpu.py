@@ -174,3 +174,16 @@ def test_infinity_beside_large_values_q8_0():
     x[:, 41] = 1e6
     y = mx.q_gemm_dequant(x, torch.from_numpy(quantize(wf, 2)).cuda(), M, N, K, mx.QuantType.Q8_0, 32).float().cpu().numpy()
     assert np.array_equal(y, np.tile(np.where(np.arange(N) % 2 == 0, np.inf, -np.inf).astype(np.float32), (M, 1)))
+
+
+@pytest.mark.parametrize("M", [1, 2])
+def test_float32_activations_of_one_segment(oracle, M):
+    """Q4_0 rows of 256 weights: float32 products and sums, no fixed point (2.6e-5)."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    N, K = 500, 256
+    packed = quantize(make_weights(N, K, 1), 0)
+    x = make_acts(M, K, 2, torch.float32)[0].cuda()
+    y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType.Q4_0, 32)
+    want = x.double() @ _dense(oracle, packed, N, K, 0).T
+    assert float((y.double() - want).norm() / want.norm()) <= RESULT["f32"]

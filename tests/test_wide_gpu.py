@@ -89,3 +89,19 @@ def test_gate_up(oracle, qt, M, H, I):
     h = (torch.nn.functional.silu(gate.bfloat16().double()) * up.bfloat16().double()).bfloat16().double()
     want = h @ _dense(oracle, d, H, I, qt).T
     assert float((y.double() - want).norm() / want.norm()) <= 1e-2
+
+
+@pytest.mark.parametrize("qt", [0, 2])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("M,K", [(9, 96), (70, 1056)])
+def test_weights_are_not_rounded_at_32_mod_64(oracle, qt, dt, M, K):
+    """Rows of an odd number of 32-weight blocks multiply the float32 weights: the result's own rounding is left, at most 2^-8
+    (2^-11) of each value and about 0.42 of that in the 2-norm; with rounded weights it is 0.6 of it."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    N = 300
+    packed = quantize(make_weights(N, K, 7), qt)
+    x = make_acts(M, K, 8, DT[dt])[0].cuda()
+    y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(qt), 32)
+    want = x.double() @ _dense(oracle, packed, N, K, qt).T
+    assert float((y.double() - want).norm() / want.norm()) <= BOUND[dt] / 2
