@@ -313,12 +313,12 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(const T* x, const __half*
     T* dst = first ? y : z;
     const size_t tok = i / per;
     const int c = (int)(i - tok * per) % vec_per_head;
+    const uint4 xv = __ldcg(reinterpret_cast<const uint4*>(src + i * 8));
     const long long pos = (long long)__ldcg(positions + tok) + offset;
     if (pos < 0 || pos >= max_seq) {
       if (status) atomicExch_system(status, 1);
       continue;
     }
-    const uint4 xv = __ldcg(reinterpret_cast<const uint4*>(src + i * 8));
     const uint2 cv = __ldg(reinterpret_cast<const uint2*>(cos_t + (size_t)pos * vec_per_head * 4) + c);
     const uint2 sv = __ldg(reinterpret_cast<const uint2*>(sin_t + (size_t)pos * vec_per_head * 4) + c);
     const T* h = reinterpret_cast<const T*>(&xv);
