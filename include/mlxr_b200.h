@@ -236,7 +236,9 @@ MLXR_API int mlxr_mlp_block_dense(const void* x, const void* w_gate, const void*
 /* Synchronise `stream`, then report and clear the device status word of its workspace:
  * MLXR_OK, MLXR_ERR_TIMEOUT (a bounded wait inside a persistent kernel gave up; results of
  * that call are invalid) or MLXR_ERR_SHAPE (a RoPE position outside its table in a fused
- * call).  The return value is the status of this call itself. */
+ * call).  After an error the counters that a kernel which gave up may have left behind are zeroed too, so that the
+ * next call on the stream starts clean; until then results on this stream are not to be used.  The return value is the
+ * status of this call itself. */
 MLXR_API int mlxr_stream_status(void* stream, int* status_out);
 
 /* Limit of every device-side wait of this library (copy barriers, hand-over words between the
@@ -305,6 +307,11 @@ MLXR_API int mlxr_debug_set_trace_buffer(void* dev_ptr);
  * 0 <= unit < units. */
 MLXR_API int mlxr_debug_smallm_partition(long long units, int ctas, int cta, long long unit,
                                          long long* begin, long long* end, int* owner);
+
+/* Device addresses of the words a (device, stream) workspace keeps between launches: the counters of parts of shared
+ * output tiles (32-bit, zero between calls) and the status word that mlxr_stream_status reports.  For tests; any
+ * pointer may be NULL. */
+MLXR_API int mlxr_debug_stream_words(void* stream, void** tile_counters, int* n_counters, void** status_word);
 
 /* Attention input projections with RoPE on q and k: n = rmsnorm(x) (norm_weight may be
  * NULL), q = n Wq^T, k = n Wk^T, v = n Wv^T, then rope_apply on q and k

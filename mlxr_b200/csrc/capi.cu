@@ -195,9 +195,9 @@ static int run_tc(TcPath path, const WidePlan& wide, const DensePlan& dense, con
   }
   if (path == kTcSmall) {
     const void* ws2[2] = {w, w2};
-    return launch_smallm(x, ws2, &N, w2 ? 2 : 1, w2 != nullptr, bias, &y, M, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, grid, maxc, st);
+    return launch_smallm(x, ws2, &N, w2 ? 2 : 1, w2 != nullptr, bias, &y, M, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + kTileCounters, grid, maxc, st);
   }
-  if (path == kTcWide) return launch_widem(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, wide, st);
+  if (path == kTcWide) return launch_widem(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, (float*)ws->part, ws->sync + kTileCounters, wide, st);
   return launch_dense(x, w, w2, bias, y, M, N, K, qt, dtype, ws->status, ws->w16, dense, st);
 }
 
@@ -505,7 +505,7 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
   DensePlan dense;
   // (NF4 has no fused form of its own below three tokens)
   if (M >= 3 || qt == MLXR_NF4) if (int r = tc_path(qt, M, inter, hidden, dtype, x, w_gate, w_up, &wide, &dense, &path)) return r;
-  const bool small = path != kTcNone && (path != kTcSmall || (2 * inter + 127) / 128 <= kSyncWords - 16);
+  const bool small = path != kTcNone && (path != kTcSmall || (2 * inter + 127) / 128 <= kSyncWords - kTileCounters);
   // one or two tokens: [RMSNorm ->] gate/up with the SiLU(gate) * up epilogue, then down: two launches, the second
   // one's weights on their way before the first has ended
   const bool gemv = gemv_supported(qt, M, hidden, 2 * inter, dtype, wgu, 2) && gemv_supported(qt, M, inter, hidden, dtype, &w_down, 1);
@@ -617,6 +617,15 @@ int mlxr_debug_smallm_partition(long long units, int ctas, int cta, long long un
   return MLXR_OK;
 }
 
+int mlxr_debug_stream_words(void* stream, void** tile_counters, int* n_counters, void** status_word) {
+  Workspace* ws = nullptr;
+  if (int r = get_workspace((cudaStream_t)stream, 0, &ws)) return r;
+  if (tile_counters) *tile_counters = ws->sync + kTileCounters;
+  if (n_counters) *n_counters = kSyncWords - kTileCounters;
+  if (status_word) *status_word = ws->status;
+  return MLXR_OK;
+}
+
 int mlxr_debug_set_trace_buffer(void* dev_ptr) {
   set_decode_trace(dev_ptr);
   return MLXR_OK;
@@ -629,6 +638,12 @@ int mlxr_stream_status(void* stream, int* status_out) {
   MLXR_CUDA_TRY(cudaMemcpyAsync(ws->status_host, ws->status, sizeof(int), cudaMemcpyDeviceToHost, st));
   MLXR_CUDA_TRY(cudaMemsetAsync(ws->status, 0, sizeof(int), st));
   MLXR_CUDA_TRY(cudaStreamSynchronize(st));
+  // A CTA that gave up has not counted its parts of shared tiles, and the counters clear themselves only when a tile is
+  // complete: after any error they start from zero again.
+  if (ws->status_host[0] != MLXR_OK) {
+    MLXR_CUDA_TRY(cudaMemsetAsync(ws->sync + kTileCounters, 0, (kSyncWords - kTileCounters) * sizeof(uint32_t), st));
+    MLXR_CUDA_TRY(cudaStreamSynchronize(st));
+  }
   if (status_out) *status_out = ws->status_host[0];
   if (ws->status_host[0] == MLXR_ERR_TIMEOUT) set_error("a bounded device-side wait expired in an earlier kernel on this stream");
   else if (ws->status_host[0] == MLXR_ERR_SHAPE) set_error("a RoPE position (+offset) was outside [0, max_seq_len)");
@@ -689,7 +704,7 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
   const int rows[3] = {q_heads * head_dim, kv_heads * head_dim, kv_heads * head_dim};
   void* const outs[3] = {q_out, k_out, v_out};
   const int tiles = (rows[0] + 127) / 128 + 2 * ((rows[1] + 127) / 128);
-  bool stack = (M >= 3 || qt == MLXR_NF4) && tiles <= kSyncWords - 16;
+  bool stack = (M >= 3 || qt == MLXR_NF4) && tiles <= kSyncWords - kTileCounters;
   for (int i = 0; i < 3; i++) stack = stack && smallm_supported(qt, M, rows[i], hidden, dtype, n, wqkv[i]);
   if (stack) {
     // Up to 64 tokens: the three projections in one launch of the small-batch kernel, which fills the SMs better than
@@ -702,7 +717,7 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
       std::lock_guard<std::mutex> lk(g_ws_mu);
       if (int r = grow(&ws->part, &ws->part_bytes, part, st)) return r;
     }
-    if (int r = launch_smallm(n, wqkv, rows, 3, false, nullptr, outs, M, hidden, qt, dtype, ws->status, (float*)ws->part, ws->sync + 16, grid, maxc, st)) return r;
+    if (int r = launch_smallm(n, wqkv, rows, 3, false, nullptr, outs, M, hidden, qt, dtype, ws->status, (float*)ws->part, ws->sync + kTileCounters, grid, maxc, st)) return r;
   } else {
     for (int i = 0; i < 3; i++)
       if (int r = run_linear(n, wqkv[i], nullptr, outs[i], M, rows[i], hidden, qt, dtype, st)) return r;

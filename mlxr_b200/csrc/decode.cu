@@ -237,7 +237,7 @@ static int launch_decode_impl(const DecodeLinear* lin, int nphases, int M, int q
   const int max_x = x_budget(NG);
   int max_slice_segs = 0;
   size_t scratch_off = 0;
-  int counter_off = 16;
+  int counter_off = kTileCounters;
   for (int i = 0; i < nphases; i++) {
     const DecodeLinear& L = lin[i];
     Phase& ph = P.ph[i];

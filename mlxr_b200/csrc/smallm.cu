@@ -573,7 +573,7 @@ bool smallm_supported(int qt, int M, int N, int K, int dtype, const void* x, con
   if (dtype != MLXR_F16 && dtype != MLXR_BF16) return false;
   if (M < 1 || M > 64 || N < 2 || K < 256 || K % 256 != 0) return false;
   if ((((uintptr_t)x) | ((uintptr_t)w)) & 15u) return false;
-  if ((N + smallm::kRows - 1) / smallm::kRows > kSyncWords - 16) return false;   // one counter per tile
+  if ((N + smallm::kRows - 1) / smallm::kRows > kSyncWords - kTileCounters) return false;   // one counter per tile
   return true;
 }
 

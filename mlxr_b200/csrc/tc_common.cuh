@@ -42,13 +42,20 @@ __device__ __forceinline__ bool mbar_try_park(uint32_t bar, uint32_t parity, uin
   return ok != 0;
 }
 // Bounded wait; false when it gave up or another role already did.  kParkPolls polls of up to
-// kParkNs each bound it to about a quarter of a second.
+// kParkNs each bound it to about a quarter of a second.  Under programmatic stream serialization what it waits for may
+// itself wait for the previous kernel of the stream, however long that takes: so when the polls run out it waits
+// for that kernel's end, and the limit starts anew from there (if that kernel has ended the wait is one of two limits).
 constexpr uint32_t kParkNs = 2000, kParkPolls = 1u << 17;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* dead) {
   if (mbar_try(bar, parity)) return true;
-  for (uint32_t i = 0; i < kParkPolls; i++) {
-    if (mbar_try_park(bar, parity, kParkNs)) return true;
-    if ((i & 7u) == 7u && *dead) return false;
+#pragma unroll 1
+  for (int behind = 0; behind < 2; behind++) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < kParkPolls; i++) {
+      if (mbar_try_park(bar, parity, kParkNs)) return true;
+      if ((i & 7u) == 7u && *dead) return false;
+    }
+    if (behind == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   }
   *dead = 1;
   return false;

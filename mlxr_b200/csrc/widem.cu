@@ -491,7 +491,7 @@ int widem_plan(int M, int rows, int K, WidePlan* out) {
     const double unit = 2000.0 + 4.3 * nt, drain = nt > 128 ? 1200.0 + 8.0 * nt : 600.0;
     // split 0: equal ranges of units for all pairs; else so many pairs for each tile (1: whole tiles, any number of them)
     for (int split = 0; split == 0 || split == 1 || (split <= nsb && split * ntiles <= pairs); split++) {
-      if (split != 1 && 2 * ntiles > kSyncWords - 16) continue;        // two counters per tile
+      if (split != 1 && 2 * ntiles > kSyncWords - kTileCounters) continue;        // two counters per tile
       const int G = (int)(split == 0 ? std::min<long long>(pairs, U) : split == 1 ? std::min<long long>(pairs, ntiles) : split * ntiles);
       double c;
       if (split == 0) {

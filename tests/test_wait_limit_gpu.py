@@ -95,3 +95,64 @@ def test_decode_block_is_clean_under_a_short_limit(oracle):
 def test_wait_limit_rejects_zero():
     from mlxr_b200._capi import ERR_INVALID_ARGUMENT, lib
     assert lib.mlxr_set_wait_limit_ns(0) == ERR_INVALID_ARGUMENT
+
+
+def _linears():
+    """Tiles shared by CTAs in the small-batch and in the wide kernel: (call, result of a call on an idle device)."""
+    import mlxr_b200 as mx
+    g = torch.Generator(device="cuda").manual_seed(1)
+    out = []
+    for M, N, K in ((32, 640, 2048), (8, 1536, 4096), (100, 2304, 2816)):
+        w = torch.randint(0, 256, (N * K // 32, 18), dtype=torch.uint8, device="cuda", generator=g)
+        w[:, :2] = torch.tensor([0, 0x18], dtype=torch.uint8, device="cuda")       # scale 2^-9
+        x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+        fn = lambda x=x, w=w, M=M, N=N, K=K: mx.q_gemm_dequant(x, w, M, N, K, mx.QuantType.Q4_0, 32)
+        out.append((fn, fn()))
+    torch.cuda.synchronize()
+    return out
+
+
+def _take_status(st):
+    from mlxr_b200._capi import check, lib
+    status = ctypes.c_int(-1)
+    check(lib.mlxr_stream_status(st, ctypes.byref(status)))
+    return status.value
+
+
+def test_counters_start_from_zero_after_a_time_out():
+    """A kernel that gave up leaves the counters of shared tiles somewhere between; here the host leaves them so.  Once the
+    time-out has been reported the next calls are right."""
+    from cuda.bindings import runtime
+    from mlxr_b200._capi import ERR_TIMEOUT, check, lib
+    calls = _linears()
+    st = torch.cuda.current_stream().cuda_stream
+    words, n, word = ctypes.c_void_p(), ctypes.c_int(), ctypes.c_void_p()
+    check(lib.mlxr_debug_stream_words(st, ctypes.byref(words), ctypes.byref(n), ctypes.byref(word)))
+    left, code = np.ones(n.value, dtype=np.uint32), np.array([ERR_TIMEOUT], dtype=np.int32)
+    for dst, src in ((words.value, left), (word.value, code)):
+        err, = runtime.cudaMemcpy(dst, src.ctypes.data, src.nbytes, runtime.cudaMemcpyKind.cudaMemcpyHostToDevice)
+        assert err == runtime.cudaError_t.cudaSuccess
+    assert _take_status(st) == ERR_TIMEOUT
+    for _ in range(2):
+        for fn, first in calls:
+            assert torch.equal(fn(), first)
+    assert _take_status(st) == 0
+
+
+def test_limit_of_a_kernel_behind_a_long_one():
+    """The tensor-core kernels start under the kernel before them and wait for its end before they read X: that may take
+    longer than the limit of their own waits."""
+    import mlxr_b200 as mx
+    calls = _linears()
+    n = 1 << 29
+    x, w = torch.ones(1, n, device="cuda"), torch.ones(n, device="cuda")      # one row: one CTA, half a second
+    st = torch.cuda.current_stream().cuda_stream
+    for fn, first in calls:
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        mx.rmsnorm_fused(x, w)
+        y = fn()
+        b.record()
+        assert _take_status(st) == 0
+        assert torch.equal(y, first)
+        assert a.elapsed_time(b) > 300, "the row is too short for what this test is about"
