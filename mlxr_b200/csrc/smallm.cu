@@ -84,6 +84,10 @@ struct Params {
   int* status;
   float* partials;     // [ntiles][maxc][NPAD][128] fp32
   uint32_t* counters;  // one per tile, self-clearing
+  // kSplit: X and the packed matrices (gate, up for kSwiglu), for the rows that the two-part products cannot give
+  const void* x;
+  const uint8_t* w[3];
+  size_t row_bytes;
 };
 
 // Tensor maps of the packed weights: one per stacked matrix, or [0] gate, [1] up; NF4 (rows only 8-byte
@@ -136,6 +140,30 @@ __device__ __forceinline__ float swish_fast(float x) {
   const float e = __expf(-fabsf(x));
   const float s = __fdividef(1.0f, 1.0f + e);      // sigmoid(|x|)
   return x * (x >= 0.0f ? s : e * s);
+}
+
+// kSplit: a leading part beyond fp16's range is infinite and its residual the opposite infinity, and an infinite activation
+// meets residuals of the other sign: their sum is NaN where the float32 product is finite or an infinity.  Sums that
+// are not finite are computed again from the float32 weights, a warp per sum; such values are rare, and a
+// row of them takes about as long as the generic kernel's.
+template <int QT, typename T> __device__ __noinline__ float exact_sum(const uint8_t* row, const T* x, int K, int lane) {
+  float acc = 0.0f;
+  for (int u = lane; u < K / 32; u += 32) {
+    float w[32];
+    dequant_unit<QT>(row, u, w);
+#pragma unroll
+    for (int i = 0; i < 32; i++) acc = fmaf(Act<T>::to_f(x[32 * u + i]), w[i], acc);
+  }
+  return warp_sum(acc);
+}
+// v: this lane's sum of row n of matrix mat (n < 0: none) and batch row m, the same for the whole warp
+template <int QT, typename T> __device__ __forceinline__ float repaired(float v, const Params& P, int mat, int n, int m, int lane) {
+  for (unsigned bad = __ballot_sync(0xffffffffu, n >= 0 && !(fabsf(v) <= 3.402823466e38f)); bad; bad &= bad - 1) {
+    const int l = __ffs(bad) - 1, row = __shfl_sync(0xffffffffu, n, l), at = __shfl_sync(0xffffffffu, mat, l);
+    const float s = exact_sum<QT, T>(P.w[at] + (size_t)row * P.row_bytes, reinterpret_cast<const T*>(P.x) + (size_t)m * P.K, P.K, lane);
+    if (lane == l) v = s;
+  }
+  return v;
 }
 
 __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
@@ -478,7 +506,9 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
 #pragma unroll
           for (int c = 0; c < 16; c++) {
             if (c0 + c < P.M) {             // uniform: every lane takes part in the exchange
-              const T o = finish(__uint_as_float(r[c]), bv);
+              float v = __uint_as_float(r[c]);
+              if constexpr (MODE == kSplit) v = repaired<QT, T>(v, P, SWIGLU ? lane >> 4 : at.mat, n < N ? n : -1, c0 + c, lane);
+              const T o = finish(v, bv);
               if (writer) y[(size_t)(c0 + c) * N + n] = o;
             }
           }
@@ -519,10 +549,11 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     const int n = SWIGLU ? 64 * at.tile + 16 * (lane >> 3) + 4 * (lane & 3) : at.tile * kRows + 4 * lane;
     const bool writer = !SWIGLU || (lane & 4) == 0;
     const float4* parts = reinterpret_cast<const float4*>(P.partials + (size_t)t * P.maxc * NPAD * kRows) + lane;
-    auto store = [&](int m, const float (&v)[4]) {
+    auto store = [&](int m, float (&v)[4]) {
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         T o;
+        if constexpr (MODE == kSplit) v[e] = repaired<QT, T>(v[e], P, SWIGLU ? (lane >> 2) & 1 : at.mat, n + e < N ? n + e : -1, m, lane);
         if constexpr (SWIGLU) {
           const float up = __shfl_xor_sync(0xffffffffu, v[e], 4);      // lanes 0-3 of eight: gate, lanes 4-7: up
           o = Act<T>::from_f(swish_fast(Act<T>::to_f(Act<T>::from_f(v[e]))) * Act<T>::to_f(Act<T>::from_f(up)));
@@ -662,6 +693,9 @@ int launch_smallm(const void* x, const void* const* w, const int* rows, int nmat
   P.status = status;
   P.partials = partials;
   P.counters = counters;
+  P.x = x;
+  for (int i = 0; i < nmat; i++) P.w[i] = (const uint8_t*)w[i];
+  P.row_bytes = (size_t)(K / block_elems(qt)) * block_bytes(qt);
   int rc = MLXR_ERR_UNSUPPORTED;
 #define MLXR_SMALLM_BY_NPAD(QTV, T, MODE, SW)                                            \
   do {                                                                                   \

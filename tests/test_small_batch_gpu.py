@@ -223,3 +223,75 @@ def test_few_tokens_of_stacked_4_bit_weights_are_not_rounded(oracle, qt, dt, M, 
     w = torch.from_numpy((h.view(np.float16) if qt == 3 else f).astype(np.float64).reshape(KH * D, H)).cuda()
     want = (x.double() @ w.T).reshape(M, KH, D)
     assert float((v.double() - want).norm() / want.norm()) <= {"bf16": 2.0 ** -9, "f16": 2.0 ** -11}[dt] + (2.0 ** -11 if qt == 3 else 0)
+
+
+def _with_large_blocks(packed, rows, block, d):
+    """Every third row's first block gets the scale d."""
+    p = packed.reshape(rows, -1).copy()
+    p[::3, 0:2] = np.frombuffer(np.float16(d).tobytes(), np.uint8)
+    return p.reshape(-1)
+
+
+@pytest.mark.parametrize("qt,M", [(2, 3), (2, 8), (33, 5), (33, 40)])
+@pytest.mark.parametrize("N,K", [(200, 768), (385, 4096)])
+def test_weights_beyond_the_range_of_fp16(oracle, qt, M, N, K):
+    """fp16 activations and weights up to 2.5e5: the float32 products are finite and so is the result.  Bound as in
+    test_other_formats (22 significant bits of the weights): the result's rounding, 2^-11."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    if qt == 33:
+        import gguf
+        import gguf.quants as gq
+        rng = np.random.Generator(np.random.PCG64(1))
+        raw = rng.integers(0, 256, size=(N * (K // 256), 144), dtype=np.uint8)
+        raw[:, 0:4] = (rng.random((raw.shape[0], 2)) * 0.002 + 0.0005).astype(np.float16).view(np.uint8)
+        packed = _with_large_blocks(raw.reshape(-1), N, 256, 200.0)
+        w = gq.dequantize(packed.reshape(N, -1), gguf.GGMLQuantizationType.Q4_K).astype(np.float64)
+    else:
+        packed = _with_large_blocks(quantize(make_weights(N, K, 3), qt), N, 32, 2000.0)
+        w = oracle.dequantize(packed, N, K, qt)[0].astype(np.float64).reshape(N, K)
+    assert np.abs(w).max() > 65504
+    x = (make_acts(M, K, 4, torch.float32)[0] * 1e-3).half()
+    want = x.double().numpy() @ w.T
+    y = mx.q_gemm_dequant(x.cuda(), torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt))
+    assert _status() == 0
+    assert oracle.rel_l2(y.float().cpu().numpy(), want) <= 2.0 ** -11
+
+
+def test_weights_beyond_the_range_of_fp16_in_the_other_forms(oracle):
+    """The same in the gate / up form (Q8_0) and in the stacked one (Q4_0).  Block: g, u, h and y are rounded to fp16 on both
+    sides, 2e-3 as everywhere for fp16."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    M, H, I = 5, 512, 768
+    g, u, d = (quantize(make_weights(n, k, s), 2) for n, k, s in ((I, H, 1), (I, H, 2), (H, I, 3)))
+    g, u = _with_large_blocks(g, I, 32, 2000.0), _with_large_blocks(u, I, 32, 1500.0)
+    xt = (make_acts(M, H, 4, torch.float32)[0] * 1e-4).half()
+    deq = lambda w, n, k: torch.from_numpy(oracle.dequantize(w, n, k, 2)[0].astype(np.float64).reshape(n, k))
+    half = lambda t: t.half().double()
+    h = half(torch.nn.functional.silu(half(xt.double() @ deq(g, I, H).T)) * half(xt.double() @ deq(u, I, H).T))
+    y = mx.mlp_block(xt.cuda(), None, *(torch.from_numpy(w).cuda() for w in (g, u, d)), I, mx.QuantType.Q8_0)
+    assert oracle.rel_l2(y.float().cpu().numpy(), (h @ deq(d, H, I).T).numpy()) <= 2e-3
+    QH, KH, D = 3, 1, 64
+    packed = [_with_large_blocks(quantize(make_weights(n * D, H, 9 + i), 0), n * D, 32, 20000.0) for i, n in enumerate((QH, KH, KH))]
+    cos, sin = mx.compute_rope_tables(16, D, 10000.0, device=torch.device("cuda"))
+    v = mx.qkv_rope(xt.cuda(), None, *(torch.from_numpy(w).cuda() for w in packed), cos, sin, torch.arange(M, dtype=torch.int32, device="cuda"), QH, KH, D, mx.QuantType.Q4_0)[2]
+    want = xt.double() @ torch.from_numpy(oracle.dequantize(packed[2], KH * D, H, 0)[0].astype(np.float64).reshape(KH * D, H)).T
+    assert oracle.rel_l2(v.float().cpu().numpy().reshape(M, -1), want.numpy()) <= 2.0 ** -11
+    assert _status() == 0
+
+
+@pytest.mark.parametrize("qt", [2, 16])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+def test_infinite_activation_in_two_parts(qt, dt):
+    """One infinity in a token: infinities with the sign of its weights, as float32 products give them, in that token only."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    N, K, M = 300, 512, 4
+    wf = make_weights(N, K, 3)
+    wf[:, 40] = np.where(np.arange(N) % 2 == 0, 0.047, -0.047)
+    x = make_acts(M, K, 4, DT[dt])[0].cuda()
+    x[2, 40] = float("inf")
+    y = mx.q_gemm_dequant(x, torch.from_numpy(quantize(wf, qt)).cuda(), M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt)).float().cpu()
+    assert np.array_equal(y[2].numpy(), np.where(np.arange(N) % 2 == 0, np.inf, -np.inf).astype(np.float32))
+    assert torch.isfinite(y[[0, 1, 3]]).all()
