@@ -269,6 +269,31 @@ __device__ __forceinline__ void load8(const T* p, float (&v)[8]) {
   for (int i = 0; i < 8; i++) v[i] = Act<T>::to_f(__ldcg(p + i));
 }
 
+// Scale of one segment's fixed point (gemv.cu, stream_gemv.cu): v holds this lane's eight of the warp's 256 activations;
+// x ~ dl * xi with xi = v * inv, |xi| <= 32000.
+__device__ __forceinline__ void fixed_scale(float (&v)[8], float& dl, float& inv) {
+  float amax = 0.0f;
+  // max.NaN keeps a NaN, which fmaxf would drop
+#pragma unroll
+  for (int i = 0; i < 8; i++) asm("max.NaN.f32 %0, %0, %1;" : "+f"(amax) : "f"(fabsf(v[i])));
+  // non-negative floats order like their bit patterns, NaN and Inf above every finite value
+  amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+  dl = amax * (1.0f / 32000.0f);
+  inv = __fdividef(32000.0f, amax);
+  if (__builtin_expect(!(amax >= 0x1p-100f && amax <= 0x1p100f), 0)) {
+    if (!(amax <= 3.0e38f)) { dl = __int_as_float(0x7fc00000); inv = 0.0f; }   // a non-finite block poisons its outputs
+    else if (amax == 0.0f) { dl = 1.0f; inv = 0.0f; }
+    else {
+      // The fast division returns 0 for divisors above 2^126 and overflows below 2^-113: near the ends of the range the
+      // segment is multiplied by a power of two first (exact; an IEEE division took 0.2 us more of the launch).
+      const float f = amax < 1.0f ? 0x1p100f : 0x1p-100f;
+#pragma unroll
+      for (int i = 0; i < 8; i++) v[i] *= f;
+      inv = __fdividef(32000.0f, amax * f);
+    }
+  }
+}
+
 // ---- x prologue --------------------------------------------------------------------------
 // The CTA's K-slice of x -> [RMSNorm, round to T] -> 16-bit fixed point per 256-element
 // segment, stored as hi / lo signed bytes in MMA k order, plus the per-segment scale and the

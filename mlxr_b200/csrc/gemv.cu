@@ -87,31 +87,12 @@ struct Misc {
   int dead;
 };
 
-// Fixed-point conversion of one (batch row, segment): v holds this lane's eight activations.  x ~ delta * xi with
+// Fixed-point words of one (batch row, segment): v holds this lane's eight activations.  x ~ dl * xi with xi = v * inv,
 // |xi| <= 32000, xi = 256 hi + lo as two signed-byte rows in MMA k order, and the exact integer sums of xi that
 // the offset / min terms need.  1.5 * 2^23 added in the multiply leaves xi, rounded to nearest, in the low bits.
+// Returns the lane's sum of xi.
 template <int QT>
-__device__ __forceinline__ void emit_fixed(uint8_t* smem, const Params& P, int m, int sg, int lane, const float (&x)[8]) {
-  float v[8];
-  uint32_t bits = 0;
-  // non-negative floats order like their bit patterns, NaN and Inf above every finite value (fmaxf would drop a NaN)
-#pragma unroll
-  for (int i = 0; i < 8; i++) { v[i] = x[i]; bits = max(bits, __float_as_uint(x[i]) & 0x7FFFFFFFu); }
-  float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, bits));
-  float dl = 1.0f, inv = 0.0f;
-  if (!(amax <= 3.0e38f)) { dl = __int_as_float(0x7fc00000); }   // a non-finite block poisons its outputs
-  else if (amax > 0.0f) {
-    // The fast division returns 0 for divisors above 2^126 and overflows below 2^-113: near the ends of the range the
-    // segment is multiplied by a power of two first (exact; an IEEE division took 0.2 us more of the launch).
-    dl = amax * (1.0f / 32000.0f);
-    if (!(amax >= 0x1p-100f && amax <= 0x1p100f)) {
-      const float f = amax < 1.0f ? 0x1p100f : 0x1p-100f;
-#pragma unroll
-      for (int i = 0; i < 8; i++) v[i] *= f;
-      amax *= f;
-    }
-    inv = __fdividef(32000.0f, amax);
-  }
+__device__ __forceinline__ int emit_words(uint8_t* smem, const Params& P, int m, int sg, int lane, const float (&v)[8], float dl, float inv) {
   uint32_t t[8], sum = 0;
 #pragma unroll
   for (int i = 0; i < 8; i++) { t[i] = __float_as_uint(fmaf(v[i], inv, 12582912.0f)); sum += t[i]; }
@@ -141,7 +122,42 @@ __device__ __forceinline__ void emit_fixed(uint8_t* smem, const Params& P, int m
     const int c = __shfl_sync(0xffffffffu, s4, base + 8), d = __shfl_sync(0xffffffffu, s4, base + 12);
     if ((lane & 15) == 0) *reinterpret_cast<float2*>(aux + (lane >> 3)) = make_float2((float)(a + c + d), (float)b);
   }
+  return ssum;
 }
+// The conversion as it nearly always is, in few instructions (every launch fetches them anew: with the rare cases in
+// line 4096 x 14336 took 1.5 us more).  True if the segment has to be done again by emit_any: a largest value
+// outside the range of the fast division (it returns 0 for divisors above 2^126 and overflows below 2^-113), or
+// an infinity or a NaN, whose "words" put the sum far outside +- 8 * 32000 however many there are.
+template <int QT>
+__device__ __forceinline__ bool emit_fixed(uint8_t* smem, const Params& P, int m, int sg, int lane, const float (&v)[8]) {
+  float amax = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
+  amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));     // non-negative floats order like their bit patterns
+  const int ssum = emit_words<QT>(smem, P, m, sg, lane, v, amax * (1.0f / 32000.0f), amax > 0.0f ? __fdividef(32000.0f, amax) : 0.0f);
+  return (uint32_t)(ssum + 8 * 32000) > 16u * 32000u || amax > 0x1p100f || (amax < 0x1p-100f && amax > 0.0f);
+}
+template <int QT>
+__device__ __forceinline__ void emit_any(uint8_t* smem, const Params& P, int m, int sg, int lane, float (&v)[8]) {
+  float dl, inv;
+  decode::fixed_scale(v, dl, inv);
+  emit_words<QT>(smem, P, m, sg, lane, v, dl, inv);
+}
+
+// Eight activations as they lie in memory (16-bit types: four registers)
+template <typename T> struct Raw8 {
+  uint4 q[sizeof(T) / 2];
+  __device__ __forceinline__ void load(const T* p) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+#pragma unroll
+      for (int i = 0; i < (int)(sizeof(T) / 2); i++) q[i] = __ldcg(reinterpret_cast<const uint4*>(p) + i);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; i++) reinterpret_cast<T*>(q)[i] = __ldcg(p + i);
+    }
+  }
+  __device__ __forceinline__ float f(int i) const { return Act<T>::to_f(reinterpret_cast<const T*>(q)[i]); }
+};
 
 // Per-thread constants of the MMA mapping: lane = 4 g + c
 struct Lane {
@@ -374,13 +390,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
 #pragma unroll
     for (int u = 0; u < 4; u++) if (s0 + u * kWarps < P.nseg) load8(xg + (size_t)m * P.K + (s0 + u * kWarps) * 256 + lane * 8, v[u]);
   };
+  float rinv[NT];
+  bool rare = false;                                                    // see emit_fixed
   if constexpr (QT == MLXR_Q8_0) {
     // fp16 as they are; bf16 times a power of two per segment that brings its largest value to 2^14 .. 2^15, as fp16:
     // exact for every value above 2^-31 of the largest, so the products are those of the bf16 values and the
     // weights need only the cheaper conversion to fp16.  An infinity or a NaN stays what it is and does not set the scale,
     // or the finite values beside it would leave fp16's range.  With RMSNorm the norm is rounded to T first, so the
     // row's sum of squares comes before.
-    float rinv[NT];
 #pragma unroll
     for (int m = 0; m < NT; m++) {
       rinv[m] = 1.0f;
@@ -443,53 +460,57 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
         }
       }
   } else if (gam && P.round_n) {
-    // n rounded to T before its conversion, so the row's sum of squares comes first.  A warp's first four
-    // segments wait for it in registers: up to K = 16384 nothing is read twice.
-    float v[NT][4][8], gv[4][8];
-    auto load_g = [&](int s0) {
+    // n rounded to T before its conversion, so the row's sum of squares comes first.  A warp's first four segments
+    // and their norm weights wait for it in registers: up to K = 16384 nothing is read twice.
+    Raw8<T> v[NT][4], gv[4];
+    auto load_raw = [&](const T* row, int s0, Raw8<T> (&r)[4]) {
 #pragma unroll
-      for (int u = 0; u < 4; u++) if (s0 + u * kWarps < P.nseg) load8(gam + (s0 + u * kWarps) * 256 + lane * 8, gv[u]);
+      for (int u = 0; u < 4; u++) if (s0 + u * kWarps < P.nseg) r[u].load(row + (s0 + u * kWarps) * 256 + lane * 8);
     };
 #pragma unroll
-    for (int m = 0; m < NT; m++) load_x(m, warp, v[m]);
-    if constexpr (NT == 1) load_g(warp);
+    for (int m = 0; m < NT; m++) load_raw(xg + (size_t)m * P.K, warp, v[m]);
+    load_raw(gam, warp, gv);
     issue_held();
 #pragma unroll
     for (int m = 0; m < NT; m++) {
       float ss = 0.0f;
-      auto add = [&](int s0, const float (&a)[4][8]) {
+      auto add = [&](int s0, const Raw8<T> (&a)[4]) {
 #pragma unroll
         for (int u = 0; u < 4; u++)
           if (s0 + u * kWarps < P.nseg)
 #pragma unroll
-            for (int i = 0; i < 8; i++) ss = fmaf(a[u][i], a[u][i], ss);
+            for (int i = 0; i < 8; i++) ss = fmaf(a[u].f(i), a[u].f(i), ss);
       };
       add(warp, v[m]);
       for (int s0 = warp + 4 * kWarps; s0 < P.nseg; s0 += 4 * kWarps) {
-        float a[4][8];
-        load_x(m, s0, a);
+        Raw8<T> a[4];
+        load_raw(xg + (size_t)m * P.K, s0, a);
         add(s0, a);
       }
       ss = warp_sum(ss);
       if (lane == 0) misc->red[warp * NT + m] = ss;
     }
     __syncthreads();
+#pragma unroll
+    for (int m = 0; m < NT; m++) {
+      float tot = 0.0f;
+#pragma unroll
+      for (int w = 0; w < kWarps; w++) tot += misc->red[w * NT + m];
+      rinv[m] = 1.0f / sqrtf(tot / (float)P.K + P.eps);
+    }
     for (int s0 = warp; s0 < P.nseg; s0 += 4 * kWarps) {
-      if (NT > 1 || s0 != warp) load_g(s0);
+      if (s0 != warp) load_raw(gam, s0, gv);
 #pragma unroll
       for (int m = 0; m < NT; m++) {
-        if (s0 != warp) load_x(m, s0, v[m]);
-        float tot = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kWarps; w++) tot += misc->red[w * NT + m];
-        const float rinv = 1.0f / sqrtf(tot / (float)P.K + P.eps);
+        if (s0 != warp) load_raw(xg + (size_t)m * P.K, s0, v[m]);
 #pragma unroll
         for (int u = 0; u < 4; u++) {
           const int sg = s0 + u * kWarps;
           if (sg >= P.nseg) break;
+          float n[8];
 #pragma unroll
-          for (int i = 0; i < 8; i++) v[m][u][i] = Act<T>::to_f(Act<T>::from_f(__fmul_rn(__fmul_rn(v[m][u][i], rinv), gv[u][i])));
-          emit_fixed<QT>(smem, P, m, sg, lane, v[m][u]);
+          for (int i = 0; i < 8; i++) n[i] = Act<T>::to_f(Act<T>::from_f(__fmul_rn(__fmul_rn(v[m][u].f(i), rinv[m]), gv[u].f(i))));
+          rare |= emit_fixed<QT>(smem, P, m, sg, lane, n);
         }
       }
     }
@@ -514,7 +535,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
 #pragma unroll
             for (int i = 0; i < 8; i++) { ss = fmaf(v[u][i], v[u][i], ss); v[u][i] *= gv[i]; }
           }
-          emit_fixed<QT>(smem, P, m, sg, lane, v[u]);
+          rare |= emit_fixed<QT>(smem, P, m, sg, lane, v[u]);
         }
       }
       if (gam) {
@@ -524,6 +545,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
     }
   }
   issue_held();
+  if constexpr (QT != MLXR_Q8_0) {
+    if (__builtin_expect(__any_sync(0xffffffffu, rare), 0)) {
+#pragma unroll 1
+      for (int i = 0; i < NT * ((P.nseg - warp + kWarps - 1) / kWarps); i++) {
+        const int m = i % NT, sg = warp + (i / NT) * kWarps;
+        float v[8], gv[8];
+        load8(xg + (size_t)m * P.K + sg * 256 + lane * 8, v);
+        if (gam) load8(gam + sg * 256 + lane * 8, gv);
+        const float r = NT == 1 || m == 0 ? rinv[0] : rinv[NT - 1];
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+          if (gam) v[e] = P.round_n ? Act<T>::to_f(Act<T>::from_f(__fmul_rn(__fmul_rn(v[e], r), gv[e]))) : v[e] * gv[e];
+        emit_any<QT>(smem, P, m, sg, lane, v);
+      }
+    }
+  }
   __syncthreads();
   const bool scale_sums = QT != MLXR_Q8_0 && gam && !P.round_n;     // 1 / rms still to be applied
   if (scale_sums && tid >= kThreads - NT) {
