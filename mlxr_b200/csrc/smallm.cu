@@ -125,6 +125,7 @@ struct Shared {
   int ntodo;                    // shared tiles of which this CTA delivered the last part (the first and the last of its range)
   int todo_tile[2], todo_parts[2];
   int epi_fail;
+  int bad;                      // kSplit: some sum was not finite
   float nf4[16];
 };
 
@@ -146,7 +147,7 @@ __device__ __forceinline__ float swish_fast(float x) {
 // meets residuals of the other sign: their sum is NaN where the float32 product is finite or an infinity.  Sums that
 // are not finite are computed again from the float32 weights, a warp per sum; such values are rare, and a
 // row of them takes about as long as the generic kernel's.
-template <int QT, typename T> __device__ __noinline__ float exact_sum(const uint8_t* row, const T* x, int K, int lane) {
+template <int QT, typename T> __device__ __forceinline__ float exact_sum(const uint8_t* row, const T* x, int K, int lane) {
   float acc = 0.0f;
   for (int u = lane; u < K / 32; u += 32) {
     float w[32];
@@ -156,15 +157,8 @@ template <int QT, typename T> __device__ __noinline__ float exact_sum(const uint
   }
   return warp_sum(acc);
 }
-// v: this lane's sum of row n of matrix mat (n < 0: none) and batch row m, the same for the whole warp
-template <int QT, typename T> __device__ __forceinline__ float repaired(float v, const Params& P, int mat, int n, int m, int lane) {
-  for (unsigned bad = __ballot_sync(0xffffffffu, n >= 0 && !(fabsf(v) <= 3.402823466e38f)); bad; bad &= bad - 1) {
-    const int l = __ffs(bad) - 1, row = __shfl_sync(0xffffffffu, n, l), at = __shfl_sync(0xffffffffu, mat, l);
-    const float s = exact_sum<QT, T>(P.w[at] + (size_t)row * P.row_bytes, reinterpret_cast<const T*>(P.x) + (size_t)m * P.K, P.K, lane);
-    if (lane == l) v = s;
-  }
-  return v;
-}
+// Added to by every sum that is to be stored: stays 0 as long as all are finite
+__device__ __forceinline__ void note_bad(float& t, float v) { t = fmaf(v, 0.0f, t); }
 
 __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
@@ -253,6 +247,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     sh->dead = 0;
     sh->ntodo = 0;
     sh->epi_fail = 0;
+    sh->bad = 0;
     for (int g = 0; g < kGroups; g++)
       for (int s = 0; s < kSlots; s++) {
         mbar_init(smem_u32(&sh->full_a[g][s][0]), 4);
@@ -282,6 +277,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
   // (griddepcontrol.wait).  Without the launch attribute both instructions do nothing.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+  [[maybe_unused]] float bad = 0.0f;    // kSplit, see note_bad
   if (warp >= kWarpProd0 && warp < kWarpFix) {
     // ===== producers =====
     const int g = (warp - kWarpProd0) >> 2, p = (warp & 3) * 32 + lane;       // group, weight row of the tile = TMEM lane
@@ -502,13 +498,15 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
 #pragma unroll
           for (int c = 0; c < 16; c++) r[c] = __float_as_uint(__uint_as_float(r[c]) + __uint_as_float(q[c]));
         }
+        if constexpr (MODE == kSplit) {
+#pragma unroll
+          for (int c = 0; c < 16; c++) note_bad(bad, __uint_as_float(r[c]));
+        }
         if (whole) {
 #pragma unroll
           for (int c = 0; c < 16; c++) {
             if (c0 + c < P.M) {             // uniform: every lane takes part in the exchange
-              float v = __uint_as_float(r[c]);
-              if constexpr (MODE == kSplit) v = repaired<QT, T>(v, P, SWIGLU ? lane >> 4 : at.mat, n < N ? n : -1, c0 + c, lane);
-              const T o = finish(v, bv);
+              const T o = finish(__uint_as_float(r[c]), bv);
               if (writer) y[(size_t)(c0 + c) * N + n] = o;
             }
           }
@@ -549,11 +547,11 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     const int n = SWIGLU ? 64 * at.tile + 16 * (lane >> 3) + 4 * (lane & 3) : at.tile * kRows + 4 * lane;
     const bool writer = !SWIGLU || (lane & 4) == 0;
     const float4* parts = reinterpret_cast<const float4*>(P.partials + (size_t)t * P.maxc * NPAD * kRows) + lane;
-    auto store = [&](int m, float (&v)[4]) {
+    auto store = [&](int m, const float (&v)[4]) {
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         T o;
-        if constexpr (MODE == kSplit) v[e] = repaired<QT, T>(v[e], P, SWIGLU ? (lane >> 2) & 1 : at.mat, n + e < N ? n + e : -1, m, lane);
+        if constexpr (MODE == kSplit) note_bad(bad, v[e]);
         if constexpr (SWIGLU) {
           const float up = __shfl_xor_sync(0xffffffffu, v[e], 4);      // lanes 0-3 of eight: gate, lanes 4-7: up
           o = Act<T>::from_f(swish_fast(Act<T>::to_f(Act<T>::from_f(v[e]))) * Act<T>::to_f(Act<T>::from_f(up)));
@@ -584,6 +582,45 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     };
     if (P.M <= kW) { if (warp < P.M) sum(Int<1>{}, warp); }
     else if (warp < P.M) sum(Int<4>{}, warp);
+  }
+  if constexpr (MODE == kSplit) {
+    // ===== results that are not finite, in the tiles that this CTA stored: again, from the float32 weights (with the
+    // repair beside the stores the kernel took 1.2 us more) =====
+    if (bad != 0.0f) sh->bad = 1;
+    __syncthreads();
+    if (__builtin_expect(*reinterpret_cast<volatile int*>(&sh->bad) && !sh->dead, 0)) {
+      const T* bias = reinterpret_cast<const T*>(P.bias);
+      const T* x = reinterpret_cast<const T*>(P.x);
+#pragma unroll 1
+      for (int i = 0, t = t_first, cnt; i < nunits; i += cnt, t++) {
+        cnt = min(i == 0 ? P.nsb - sb_first : P.nsb, nunits - i);
+        bool mine = cnt == P.nsb;
+        for (int k = 0; k < ntodo; k++) mine = mine || sh->todo_tile[k] == t;
+        if (!mine) continue;
+        const Place at = place_of<FORM>(P, t);
+        constexpr int kCols = SWIGLU ? 64 : kRows;                       // columns of Y in a tile
+        const int N = P.rows[at.mat], n0 = kCols * at.tile;
+        T* y = reinterpret_cast<T*>(P.y[at.mat]);
+#pragma unroll 1
+        for (int e = warp; e < P.M * (kCols / 32); e += kW) {
+          const int m = e / (kCols / 32), n = n0 + 32 * (e % (kCols / 32)) + lane;
+          const bool lost = n < N && !(fabsf(Act<T>::to_f(y[(size_t)m * N + n])) <= 3.402823466e38f);
+#pragma unroll 1
+          for (unsigned left = __ballot_sync(0xffffffffu, lost); left; left &= left - 1) {
+            const int row = n - lane + __ffs(left) - 1;
+            const float g = exact_sum<QT, T>(P.w[at.mat] + (size_t)row * P.row_bytes, x + (size_t)m * P.K, P.K, lane);
+            T o;
+            if constexpr (SWIGLU) {
+              const float u = exact_sum<QT, T>(P.w[1] + (size_t)row * P.row_bytes, x + (size_t)m * P.K, P.K, lane);
+              o = Act<T>::from_f(swish_fast(Act<T>::to_f(Act<T>::from_f(g))) * Act<T>::to_f(Act<T>::from_f(u)));
+            } else {
+              o = Act<T>::from_f(g + (bias ? Act<T>::to_f(bias[row]) : 0.0f));
+            }
+            if (lane == 0) y[(size_t)m * N + row] = o;
+          }
+        }
+      }
+    }
   }
 }
 
