@@ -68,9 +68,8 @@ template <typename T> __device__ __forceinline__ void unpack8(const uint4& u, fl
 // stream serialization) may find x still being written when it begins, and in place x is written by the kernel
 // itself; the read-only path (and const __restrict__, which lets the compiler take it) is defined only for data that
 // nobody writes while the kernel runs.  That holds for the norm weight and the tables: __ldg there.
-template <typename T, bool CONST = false> __device__ __forceinline__ void load8v(const T* p, float (&v)[8]) {
-  const uint4 u = CONST ? __ldg(reinterpret_cast<const uint4*>(p)) : __ldcg(reinterpret_cast<const uint4*>(p));
-  unpack8<T>(u, v);
+template <typename T> __device__ __forceinline__ void load8v(const T* p, float (&v)[8]) {
+  unpack8<T>(__ldcg(reinterpret_cast<const uint4*>(p)), v);
 }
 template <typename T> __device__ __forceinline__ void store8v(T* p, const float (&v)[8]) {
   uint4 u;
@@ -94,13 +93,14 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_vec_kernel(const T* x, const 
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const size_t row = (size_t)blockIdx.x * nvec * 8;
   float v[PER][8], ss = 0.0f;
-  uint4 rv[PER];
+  uint4 wv[PER], rv[PER];
 #pragma unroll
   for (int i = 0; i < PER; i++) {
     const int c = threadIdx.x + i * THREADS;
     if (c < nvec) {
-      if (res) rv[i] = __ldcg(reinterpret_cast<const uint4*>(res + row + c * 8));      // before any store: y may be res
       load8v(x + row + c * 8, v[i]);
+      wv[i] = __ldg(reinterpret_cast<const uint4*>(w) + c);
+      if (res) rv[i] = __ldcg(reinterpret_cast<const uint4*>(res + row) + c);      // before any store: y may be res
 #pragma unroll
       for (int e = 0; e < 8; e++) ss = fmaf(v[i][e], v[i][e], ss);
     }
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_vec_kernel(const T* x, const 
     const int c = threadIdx.x + i * THREADS;
     if (c < nvec) {
       float g[8], o[8];
-      load8v<T, true>(w + c * 8, g);
+      unpack8<T>(wv[i], g);
 #pragma unroll
       for (int e = 0; e < 8; e++) o[e] = (v[i][e] * rms) * g[e];
       if (res) {
@@ -211,7 +211,9 @@ __global__ void __launch_bounds__(256) swiglu_vec_kernel(const T* g, const T* u,
 
 int launch_swiglu(const void* g, const void* u, void* o, size_t n, int dtype, cudaStream_t st) {
   if (n == 0) return MLXR_OK;
-  if (dtype != MLXR_F32 && n % 8 == 0 && aligned16(g, o, u)) {
+  // up to 2^18 elements one element per thread is done sooner than eight one after the other (4096: 2.0 us and 2.8, 2^18: 2.6
+  // and 2.9, 2^21: 7.4 and 4.6)
+  if (dtype != MLXR_F32 && n % 8 == 0 && n > 1 << 18 && aligned16(g, o, u)) {
     const size_t nvec = n / 8;
     const int vb = (int)std::min<size_t>((nvec + 511) / 512, 148 * 8 * 4);
 #define MLXR_SWIGLU(T) do { if (u) swiglu_vec_kernel<T, true><<<vb, 256, 0, st>>>((const T*)g, (const T*)u, (T*)o, nvec); \
