@@ -204,8 +204,29 @@ static int run_tc(TcPath path, const WidePlan& wide, const DensePlan& dense, con
 // Kernel selection for one linear.  Fast kernels need 16-byte aligned rows.
 // The first kDecodeScratchBytes of a workspace's scratch belong to the decode kernel's
 // split-K partial sums; intermediates of the fused entry points start after them.
+// Small matrices of a few tokens: a kernel without copies into shared memory, barriers and partial sums has its result
+// before the others have set themselves up.  bf16, weights from HBM, in us, gemv_rows_kernel / the kernel that larger ones take:
+//   Q8_0  one token 2048 x 2048 5.0 / 5.6, 3000 x 2048 5.8 / 6.0, 4096 x 2048 6.7 / 6.2; two 4096 x 1024 5.2 / 5.9, 2048 x 2048 6.4 / 6.3,
+//         1024 x 4096 7.8 / 7.2; 3, 6 and 8 tokens of 1000 x 1024 4.3, 6.3, 7.2 / 7.2, three of 1024 x 2048 6.2 / 6.3
+//   NF4   3 and 6 tokens of 1000 x 1024 4.6, 6.9 / 7.4; three of 4096 x 1024 6.5 / 7.6, 2048 x 2048 6.7 / 6.8; four of 2048 x 2048 7.5 / 6.9
+static bool rows_kernel_first(int qt, int M, int N, int K, int dtype, const void* x, const void* w) {
+  if (dtype == MLXR_F32 || !gemv_rows_supported(qt, M, K, x, w)) return false;
+  const long long size = (long long)N * K;
+  if (qt == MLXR_Q8_0) return M == 1 ? size <= 3 << 21 : M == 2 ? size <= 1 << 22 && K <= 2048 : M * size <= 6 << 20;
+  return qt == MLXR_NF4 && M >= 3 && (M * size <= 6 << 20 || (M <= 4 && M * K <= 6144 && size <= 1 << 22));
+}
+
 static int run_linear(const void* x, const void* w, const void* bias, void* y, int M, int N, int K,
                       int qt, int dtype, cudaStream_t st) {
+  if (M > 0 && N > 0 && stream_gemv_supported(qt, M, K, N, &w, 1)) {
+    Workspace* ws = nullptr;
+    if (int r = get_workspace(st, 0, &ws)) return r;
+    DecodeLinear L;
+    memset(&L, 0, sizeof(L));
+    L.w[0] = w; L.rows[0] = N; L.nmat = 1; L.K = K; L.x = x; L.y[0] = y; L.bias[0] = bias;
+    return launch_stream_gemv(L, M, dtype, ws->status, st);
+  }
+  if (M > 0 && N > 0 && rows_kernel_first(qt, M, N, K, dtype, x, w)) return launch_gemv_rows(x, w, bias, y, M, N, K, qt, dtype, st);
   if (M > 0 && N > 0 && gemv_supported(qt, M, K, N, dtype, &w, 1)) {
     Workspace* ws = nullptr;
     if (int r = get_workspace(st, 0, &ws)) return r;
@@ -214,11 +235,12 @@ static int run_linear(const void* x, const void* w, const void* bias, void* y, i
     L.w[0] = w; L.rows[0] = N; L.nmat = 1; L.K = K; L.x = x; L.y[0] = y; L.bias[0] = bias;
     return launch_gemv(L, M, qt, dtype, ws->status, st);
   }
-  // Canonical Q4_K, and NF4 rows that do not start on 16 bytes, have no kernel of their own for one or two tokens.  The
+  // Canonical Q4_K, and NF4 rows that do not start on 16 bytes, have no kernel of their own for one or two tokens (one token
+  // of a small canonical matrix is the generic kernel's: 1000 x 1024 5.2 us there, 7.1 here; 1024 x 2048 8.7, 6.6).  The
   // one NF4 has looks every weight up once per token; from 2^24 weights on the small-batch kernel, which converts
   // once, is the faster one for two (4096 x 4096: 14.5 us there, 11.6 here; 14336 x 4096: 34.4, 27.9; 4096 x 14336:
   // 40.5, 26.7; 4096 x 2048: 7.6, 8.5).
-  const bool small_only = qt == MLXR_GGML_Q4_K ||
+  const bool small_only = (qt == MLXR_GGML_Q4_K && (M > 1 || (long long)N * K > 5 << 18)) ||
                           (qt == MLXR_NF4 && (!gemv_rows_supported(qt, M, K, x, w) || (M == 2 && (long long)N * K >= (1 << 24))));
   if ((M >= 3 || (M > 0 && small_only)) && N > 0) {
     TcPath path;
@@ -503,8 +525,11 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
   TcPath path = kTcNone;
   WidePlan wide;
   DensePlan dense;
-  // (NF4 has no fused form of its own below three tokens)
-  if (M >= 3 || qt == MLXR_NF4) if (int r = tc_path(qt, M, inter, hidden, dtype, x, w_gate, w_up, &wide, &dense, &path)) return r;
+  // (NF4 has no fused form of its own below three tokens; one token of a small block is faster as single operators, the
+  // linears on gemv_rows_kernel: 1536 x 4096 21.0 us and 23.2, 2048 x 5632 26.7 and 28.8, 3072 x 8192 45.9 and 41.0)
+  const bool single = qt == MLXR_NF4 && M == 1 && (long long)hidden * inter <= 1 << 24 && gemv_rows_supported(qt, M, hidden, x, w_gate) &&
+                      gemv_rows_supported(qt, M, hidden, x, w_up) && gemv_rows_supported(qt, M, inter, x, w_down);
+  if (M >= 3 || (qt == MLXR_NF4 && !single)) if (int r = tc_path(qt, M, inter, hidden, dtype, x, w_gate, w_up, &wide, &dense, &path)) return r;
   const bool small = path != kTcNone && (path != kTcSmall || (2 * inter + 127) / 128 <= kSyncWords - kTileCounters);
   // one or two tokens: [RMSNorm ->] gate/up with the SiLU(gate) * up epilogue, then down: two launches, the second
   // one's weights on their way before the first has ended
@@ -668,7 +693,8 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
   Workspace* ws = nullptr;
   if (int r = get_workspace(st, kDecodeScratchBytes + align_up((size_t)M * hidden * es, 256), &ws)) return r;
   const void* wqkv[3] = {wq, wk, wv};
-  if (gemv_supported(qt, M, hidden, (q_heads + 2 * kv_heads) * head_dim, dtype, wqkv, 3) && q_heads * head_dim % 4 == 0 && kv_heads * head_dim % 4 == 0) {
+  const bool small_q4k = stream_gemv_supported(qt, M, hidden, (q_heads + 2 * kv_heads) * head_dim, wqkv, 3);
+  if (small_q4k || (gemv_supported(qt, M, hidden, (q_heads + 2 * kv_heads) * head_dim, dtype, wqkv, 3) && q_heads * head_dim % 4 == 0 && kv_heads * head_dim % 4 == 0)) {
     DecodeLinear L;
     memset(&L, 0, sizeof(L));
     L.w[0] = wq; L.w[1] = wk; L.w[2] = wv;
@@ -679,7 +705,7 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
     L.epi[0] = L.epi[1] = 2;
     L.cos_t = cos_f16; L.sin_t = sin_f16; L.positions = positions;
     L.head_dim = head_dim; L.max_seq = max_seq_len; L.pos_offset = position_offset;
-    return launch_gemv(L, M, qt, dtype, ws->status, st);
+    return small_q4k ? launch_stream_gemv(L, M, dtype, ws->status, st) : launch_gemv(L, M, qt, dtype, ws->status, st);
   }
   // 16-bit types of three and more tokens are below: 18.9 us here and 11.7 there at 3 tokens, hidden size 4096
   if ((dtype == MLXR_F32 || M < 3) && decode_supported(qt, M, hidden, wqkv, 3)) {

@@ -119,6 +119,10 @@ int mlp_block_tp_fused(const void* x, const void* norm_weight, const void* w_gat
 bool gemv_supported(int qt, int M, int K, int rows, int dtype, const void* const* w, int nmat);
 int launch_gemv(const DecodeLinear& L, int M, int qt, int dtype, int* status, cudaStream_t st);
 
+// Q4_K, one and two tokens, small matrices (stream_gemv.cu): single or stacked linears
+bool stream_gemv_supported(int qt, int M, int K, int rows, const void* const* w, int nmat);
+int launch_stream_gemv(const DecodeLinear& L, int M, int dtype, int* status, cudaStream_t st);
+
 // ---- small-batch tensor-core linear (smallm.cu): Q4_K, Q4_0, Q8_0, NF4, canonical Q4_K; 1 <= M <= 64, fp16 / bf16 ----
 bool smallm_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w);
 void smallm_partition(long long units, int ctas, int cta, long long unit, long long* begin, long long* end, int* owner);

@@ -187,3 +187,64 @@ def test_float32_activations_of_one_segment(oracle, M):
     y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType.Q4_0, 32)
     want = x.double() @ _dense(oracle, packed, N, K, 0).T
     assert float((y.double() - want).norm() / want.norm()) <= RESULT["f32"]
+
+
+@pytest.mark.parametrize("qt,dt,M,N,K", [(3, "bf16", 1, 4096, 4096), (3, "bf16", 1, 4097, 4096), (3, "f16", 1, 8192, 256), (3, "f16", 1, 8193, 256),
+                                         (3, "bf16", 2, 2048, 4096), (3, "bf16", 2, 2049, 4096), (3, "f32", 2, 77, 4096), (3, "f32", 1, 77, 4352),
+                                         (2, "bf16", 1, 3072, 2048), (2, "bf16", 1, 3073, 2048), (2, "f16", 2, 2048, 2048), (2, "f16", 2, 2049, 2048),
+                                         (2, "bf16", 6, 1024, 1024), (2, "bf16", 6, 1025, 1024), (16, "bf16", 4, 2730, 1536), (16, "bf16", 4, 2731, 1536),
+                                         (16, "f16", 8, 1536, 512), (16, "f16", 8, 1537, 512), (33, "bf16", 1, 1280, 1024), (33, "bf16", 1, 1281, 1024)])
+def test_borders_of_the_small_matrices(oracle, qt, dt, M, N, K):
+    """On both sides of the sizes where a linear of a few tokens changes kernels, with bias.  Bounds as above; NF4 and canonical
+    Q4_K keep 16 significant bits of the weights or all."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    if qt == 33:
+        import gguf
+        import gguf.quants as gq
+        raw = np.random.Generator(np.random.PCG64(3)).integers(0, 256, size=(N * (K // 256), 144), dtype=np.uint8)
+        raw[:, 0:4] = (np.random.Generator(np.random.PCG64(4)).random((raw.shape[0], 2)) * 0.002 + 0.0005).astype(np.float16).view(np.uint8)
+        packed = raw.reshape(-1)
+        w = torch.from_numpy(gq.dequantize(packed.reshape(N, -1), gguf.GGMLQuantizationType.Q4_K).astype(np.float64)).cuda()
+    else:
+        packed = quantize(make_weights(N, K, 7), qt)
+        w = _dense(oracle, packed, N, K, qt)
+    x, b = make_acts(M, K, 8, DT[dt])[0].cuda(), make_acts(1, N, 9, DT[dt])[0][0].contiguous().cuda()
+    args = (x, torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt), b)
+    y = mx.q_gemm_dequant(*args)
+    assert torch.equal(y, mx.q_gemm_dequant(*args))
+    assert _status() == 0
+    want = x.double() @ w.T + b.double()
+    assert float((y.double() - want).norm() / want.norm()) <= RESULT[dt] + WEIGHT.get(qt, 2.0 ** -16)
+
+
+@pytest.mark.parametrize("H,I", [(1024, 1536), (4096, 4096), (4096, 4608)])
+def test_one_token_block_of_nf4_at_the_border(oracle, H, I):
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    g, u, d = (quantize(make_weights(n, k, s), 16) for n, k, s in ((I, H, 1), (I, H, 2), (H, I, 3)))
+    xt, xf = make_acts(1, H, 4, torch.bfloat16)
+    nt, nf = make_acts(1, H, 5, torch.bfloat16)
+    y = mx.mlp_block(xt.cuda(), nt[0].contiguous().cuda(), *(torch.from_numpy(w).cuda() for w in (g, u, d)), I, mx.QuantType.NF4, 1e-5)
+    assert oracle.rel_l2(y.float().cpu().numpy(), oracle.mlp_block(xf, nf[0], g, u, d, I, 16, 1e-5, oracle.BF16)) <= 1e-2
+
+
+@pytest.mark.parametrize("M,H,QH,KH", [(1, 512, 5, 1), (2, 512, 5, 1), (1, 2048, 48, 8), (1, 2048, 50, 8)])
+def test_stacked_projections_of_a_small_hidden_size(M, H, QH, KH):
+    """q / k / v of Q4_K at one and two tokens, on both sides of the border of the kernel for small matrices, against the
+    package's own linears and RoPE on the normalised input.  The kernels multiply the unrounded n: x is a row of equal
+    magnitudes and the norm weight 1, so n is x either way."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    D = 64
+    ws = [torch.from_numpy(quantize(make_weights(n * D, H, 9 + i), 3)).cuda() for i, n in enumerate((QH, KH, KH))]
+    cos, sin = mx.compute_rope_tables(16, D, 10000.0, device=torch.device("cuda"))
+    x = torch.sign(make_acts(M, H, 4, torch.float32)[0]).half().cuda()
+    pos = torch.arange(3, 3 + M, dtype=torch.int32, device="cuda")
+    out = mx.qkv_rope(x, torch.ones(H, device="cuda", dtype=torch.float16), *ws, cos, sin, pos, QH, KH, D, mx.QuantType.Q4_K, 0.0)
+    assert _status() == 0
+    for i, (got, heads) in enumerate(zip(out, (QH, KH, KH))):
+        y = mx.q_gemm_dequant(x, ws[i], M, heads * D, H, mx.QuantType.Q4_K, 256).reshape(M, heads, D)
+        want = mx.rope_apply(y, cos, sin, pos) if i < 2 else y
+        # one ulp of the linear's result at most, 2^-10, where the two sums round to different sides
+        assert float((got.double() - want.double()).norm() / want.double().norm()) <= 2.0 ** -11
