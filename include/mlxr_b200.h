@@ -277,19 +277,22 @@ MLXR_API int mlxr_q_gemm_dequant_static(const void* x, const void* weights, cons
  * reference. */
 MLXR_API int mlxr_static_status(void* stream, int* status_out);
 
-/* How the persistent decode kernel is launched (process-wide; no counterpart in the
+/* How this library's kernels are launched (process-wide; no counterpart in the
  * reference, whose Metal command buffers serialise kernels).
- *   MLXR_DECODE_LAUNCH_OVERLAPPED (default): plain launch with programmatic stream
- *     serialization.  The kernel starts its weight copies while the previous kernel of the
- *     stream drains and waits (griddepcontrol.wait) before it reads activations.  Contract:
- *     weight buffers are model constants - no kernel still in flight on the stream writes
- *     them - and at most one decode launch runs on a device at a time.  The MLP block's
+ *   MLXR_DECODE_LAUNCH_OVERLAPPED (default): with programmatic stream serialization.  A linear,
+ *     a block or q / k / v starts its weight copies while the previous kernel of the stream
+ *     drains and waits (griddepcontrol.wait) before it reads activations; RMSNorm and RoPE take
+ *     their places the same way.  Contract of mlxr_q_gemm_dequant, mlxr_mlp_block, mlxr_qkv_rope
+ *     and their variants: weight buffers are model constants - no kernel still in flight on the
+ *     stream writes them - and at most one launch of the persistent decode kernel runs on a
+ *     device at a time (float32 activations, the tensor-parallel block): its
  *     down-projection CTAs wait for words written by the gate/up CTAs of the same launch; the
- *     library checks once per device that one CTA per SM is resident, but two decode launches
+ *     library checks once per device that one CTA per SM is resident, but two such launches
  *     on concurrent streams could each hold part of the SMs, in which case the bounded wait
  *     reports MLXR_ERR_TIMEOUT through mlxr_stream_status.
- *   MLXR_DECODE_LAUNCH_COOPERATIVE: cooperative launch (the driver guarantees co-residency
- *     or refuses the launch), no overlap with the previous kernel, no contract. */
+ *   MLXR_DECODE_LAUNCH_COOPERATIVE: no kernel overlaps with the previous one of its stream, so a
+ *     kernel before it may have written the weights; the persistent decode kernel is launched
+ *     cooperatively (the driver guarantees co-residency or refuses the launch).  No contract. */
 enum { MLXR_DECODE_LAUNCH_COOPERATIVE = 0, MLXR_DECODE_LAUNCH_OVERLAPPED = 2 };
 MLXR_API int mlxr_set_decode_launch_mode(int mode);
 

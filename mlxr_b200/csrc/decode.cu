@@ -20,6 +20,7 @@ void set_decode_trace(void* p) { g_trace = (unsigned long long*)p; }
 void* get_decode_trace() { return g_trace; }
 static std::atomic<int> g_launch_mode{MLXR_DECODE_LAUNCH_OVERLAPPED};
 void set_decode_launch_mode(int mode) { g_launch_mode.store(mode); }
+bool overlap_launches() { return g_launch_mode.load() == MLXR_DECODE_LAUNCH_OVERLAPPED; }
 static std::atomic<unsigned long long> g_wait_ns{2000000000ull};   // limit of every device-side wait
 void set_wait_limit_ns(unsigned long long ns) { g_wait_ns.store(ns ? ns : 1ull); }
 unsigned long long wait_limit_ns() { return g_wait_ns.load(); }

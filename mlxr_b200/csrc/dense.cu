@@ -385,7 +385,7 @@ static void launch_config(dim3 grid, int threads, size_t smem, int cluster, cuda
   cfg->dynamicSmemBytes = smem;
   cfg->stream = st;
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = cluster;
   at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;

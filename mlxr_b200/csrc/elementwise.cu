@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "kernels.h"
 
 namespace mlxr {
 
@@ -138,7 +139,7 @@ static int launch_rmsnorm_vec(const void* x, const void* w, const void* res, voi
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 1;
 #define MLXR_RMS(TH, PER) do { cfg.blockDim = dim3(TH); MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rmsnorm_vec_kernel<T, TH, PER>, (const T*)x, (const T*)w, (const T*)res, (T*)y, nvec, eps)); } while (0)
@@ -348,7 +349,7 @@ static int launch_rope_vec(const void* x, const uint16_t* cos_t, const uint16_t*
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rope_vec_kernel<T>, (const T*)x, (const __half*)cos_t, (const __half*)sin_t, positions, (T*)y, total, heads * vh,

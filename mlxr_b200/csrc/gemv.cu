@@ -754,7 +754,7 @@ static int launch_gemv_inst(Params& P, int grid, cudaStream_t st) {
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P));

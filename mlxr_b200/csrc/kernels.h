@@ -101,6 +101,7 @@ constexpr size_t kDecodeScratchBytes = (size_t)8 << 20;  // split-K partial sums
 void set_decode_trace(void* dev_ptr);
 void* get_decode_trace();
 void set_decode_launch_mode(int mode);
+bool overlap_launches();                 // launches may start under the previous kernel of the stream (MLXR_DECODE_LAUNCH_OVERLAPPED)
 bool decode_supported(int qt, int M, int K, const void* const* w, int nmat);
 // tp (optional): the last phase must be a single plain linear with epi 3 (float partial sums); its
 // sums then go straight into the peers' exchange buffers and the kernel ends with the reduction.

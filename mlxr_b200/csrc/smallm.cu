@@ -692,7 +692,7 @@ static int launch_inst(const smallm::Maps& maps, const smallm::Params& P, int gr
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, maps, P));

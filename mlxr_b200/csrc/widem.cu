@@ -532,7 +532,7 @@ static int launch_wide_inst(const widem::Maps& maps, const widem::Params& P, int
   cfg.stream = st;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = 2;
   at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
