@@ -105,3 +105,84 @@ def test_weights_are_not_rounded_at_32_mod_64(oracle, qt, dt, M, K):
     y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(qt), 32)
     want = x.double() @ _dense(oracle, packed, N, K, qt).T
     assert float((y.double() - want).norm() / want.norm()) <= BOUND[dt] / 2
+
+
+def _launches(fn):
+    from mlxr_b200._capi import lib
+    before = lib.mlxr_launch_count()
+    y = fn()
+    return y, lib.mlxr_launch_count() - before
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3, 16])
+@pytest.mark.parametrize("M,N,K,launches", [(65, 2, 2816, 1), (128, 257, 2816, 1), (129, 1000, 4096, 1), (257, 385, 2816, 1), (333, 2304, 2816, 1), (65, 4097, 768, 1),
+                                            (512, 8001, 1280, 1), (65, 2, 256, 2), (1100, 2304, 4096, 2), (2048, 255, 512, 2), (2049, 520, 256, 2), (4095, 1001, 768, 2)])
+def test_either_kernel_for_certain(oracle, qt, M, N, K, launches):
+    """Which of the two kernels runs follows from their estimated times: small matrices take the pass and the GEMM (two
+    launches) from 65 tokens on.  The edges of the wide kernel's tiles at sizes that it takes, and both of them told apart."""
+    import mlxr_b200 as mx
+    x = torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
+    w = torch.zeros(mx.compute_quantized_weight_size(N, K, mx.QuantType(qt)), device="cuda", dtype=torch.uint8)
+    assert _launches(lambda: mx.q_gemm_dequant(x, w, M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt)))[1] == launches
+    _check(oracle, qt, "bf16" if M % 2 else "f16", M, N, K)
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3, 16])
+@pytest.mark.parametrize("M,H,I", [(100, 2816, 1280), (200, 2816, 3008)])
+def test_gate_up_beside_the_mmas(oracle, qt, M, H, I):
+    """As test_gate_up, at a hidden size for which gate / up is one launch of the wide kernel (odd numbers of super-blocks, tiles
+    shared by CTAs; 3008 rows do not fill their last tile): 1e-2 as there, for down's K only formats of 32- and 64-blocks."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    if qt == 3 and I % 256:
+        I = 3072
+    g, u, d = (quantize(make_weights(n, k, s), qt) for n, k, s in ((I, H, 1), (I, H, 2), (H, I, 3)))
+    x = make_acts(M, H, 4, torch.bfloat16)[0].cuda()
+    args = [torch.from_numpy(w).cuda() for w in (g, u, d)]
+    down = _launches(lambda: mx.q_gemm_dequant(torch.zeros(M, I, device="cuda", dtype=torch.bfloat16), args[2], M, H, I, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt)))[1]
+    y, launches = _launches(lambda: mx.mlp_block(x, None, *args, I, mx.QuantType(qt)))
+    assert launches == 1 + down and _status() == 0
+    gate, up = (x.double() @ _dense(oracle, w, I, H, qt).T for w in (g, u))
+    h = (torch.nn.functional.silu(gate.bfloat16().double()) * up.bfloat16().double()).bfloat16().double()
+    want = h @ _dense(oracle, d, H, I, qt).T
+    assert float((y.double() - want).norm() / want.norm()) <= 1e-2
+
+
+def _device_blocks(N, K, seed):
+    """Q4_0 blocks with scales around 2^-8, made on the device (large matrices)."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = torch.randint(0, 256, (N * K // 32, 18), dtype=torch.uint8, device="cuda", generator=g)
+    w[:, 1] = 0x1C
+    return w.reshape(-1)
+
+
+def test_slices_of_the_16_bit_weights():
+    """More than 256 MB of 16-bit weights go through the buffer in slices: three of 6912 rows, which the tile of 160 rows does
+    not divide, the last one ragged and the row count odd (K = 64 mod 256 has no other kernel)."""
+    import mlxr_b200 as mx
+    M, N, K = 700, 20001, 16448
+    w = _device_blocks(N, K, 1)
+    x = torch.randn(M, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)).half()
+    b = torch.randn(N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)).half()
+    y, launches = _launches(lambda: mx.q_gemm_dequant(x, w, M, N, K, mx.QuantType.Q4_0, 32, b))
+    assert launches == 2 * 3 and _status() == 0
+    want = x.double() @ mx.dequantize(w, N, K, mx.QuantType.Q4_0, torch.float32).double().T + b.double()
+    assert float((y.double() - want).norm() / want.norm()) <= BOUND["f16"]
+    assert float((y.double() - want).norm(dim=0).max() / want.norm(dim=0).mean()) <= 4 * BOUND["f16"]      # no column is someone else's
+
+
+def test_slices_of_gate_and_up():
+    """The same for gate / up (the slices' rows alternate between the two matrices) and, in two slices, for down."""
+    import mlxr_b200 as mx
+    M, H, I = 700, 16448, 10048
+    g, u, d = _device_blocks(I, H, 1), _device_blocks(I, H, 2), _device_blocks(H, I, 3)
+    x = torch.randn(M, H, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)).half()
+    y, launches = _launches(lambda: mx.mlp_block(x, None, g, u, d, I, mx.QuantType.Q4_0))
+    assert launches == 2 * 3 + 2 * 2 and _status() == 0
+    deq = lambda w, n, k: mx.dequantize(w, n, k, mx.QuantType.Q4_0, torch.float32).double()
+    gate, up = (x.double() @ deq(w, I, H).T for w in (g, u))
+    h = (torch.nn.functional.silu(gate.half().double()) * up.half().double()).half().double()
+    want = h @ deq(d, H, I).T
+    # g, u, h and the result are rounded to fp16 on both sides from sums over weights rounded on one: 2e-3 as everywhere
+    assert float((y.double() - want).norm() / want.norm()) <= 2e-3
+    assert float((y.double() - want).norm(dim=0).max() / want.norm(dim=0).mean()) <= 8e-3
