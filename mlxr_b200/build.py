@@ -59,9 +59,8 @@ def sources() -> list[str]:
 
 
 def _build_ops(force: bool) -> None:
-    """lib/mlxr_torch_ops.so: the Python-to-C-ABI call path of ops.py (g++ against torch's headers)."""
-    if not force and os.path.exists(OPS) and os.path.getmtime(OPS) >= max(os.path.getmtime(OPS_SRC), os.path.getmtime(os.path.join(ROOT, "include", "mlxr_b200.h"))):
-        return
+    """lib/mlxr_torch_ops.so: the Python-to-C-ABI call path of ops.py (g++ against torch's headers).  Rebuilt when a source
+    is newer, or for another command or torch version."""
     import sysconfig
 
     import torch
@@ -70,10 +69,17 @@ def _build_ops(force: bool) -> None:
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            *inc, OPS_SRC, "-o", OPS, f"-L{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    stamp, want = os.path.join(OBJ, "ops.txt"), f"torch {torch.__version__}: {' '.join(cmd)}"
+    current = os.path.exists(stamp) and open(stamp).read() == want
+    newest = max(os.path.getmtime(OPS_SRC), os.path.getmtime(os.path.join(ROOT, "include", "mlxr_b200.h")))
+    if not force and current and os.path.exists(OPS) and os.path.getmtime(OPS) >= newest:
+        return
     p = subprocess.run(cmd, capture_output=True, text=True)
     if p.returncode != 0:
         sys.stderr.write(p.stdout + p.stderr)
         raise RuntimeError("building mlxr_torch_ops.so failed")
+    with open(stamp, "w") as f:
+        f.write(want)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
