@@ -42,9 +42,9 @@ import numpy as np  # noqa: E402
 
 H, I = 4096, 14336            # Llama-3-8B MLP (the default workload)
 SIZES = {"hidden": H, "inter": I}
-# DRAM bytes (read + write) of one step from an ncu capture of this workload's launches,
-# keyed by (hidden, inter, batch); see profiles/
-TRAFFIC = {}
+# DRAM bytes (read + write) of one step from an ncu capture of this workload's two launches,
+# keyed by (hidden, inter, batch); see profiles/tensor_core_and_gemv_kernels.md
+TRAFFIC = {(4096, 14336, 1): 66196224 + 692736 + 33144320}
 QT_Q4_K = 3
 EPS = 1e-5
 SEED = 1234

@@ -163,8 +163,10 @@ static int check_quant(int qt, int K, int group_size, bool check_group) {
 // The tensor-core linears for 16-bit activations: Y = X W^T (+ bias), or SiLU(X w^T) * (X w2^T).
 // Up to 64 tokens the small-batch kernel.  Above that the wide kernel, which converts the weights beside the
 // MMAs once per 256 tokens, or the dense path, which converts them once in a pass of its own: whichever
-// their plans estimate to be faster (for 14336 x 4096 they meet near 1800 tokens).  The dense path also takes what the others
-// do not: K that is not a multiple of 256, rows that do not start on 16 bytes.
+// their plans estimate to be faster: for 14336 x 4096 they meet at 1040 tokens, for 4096 x 14336 at 1790, and
+// matrices of a few super-blocks take the dense path from 65 tokens on.  (The estimates were fitted on the 4-bit formats and
+// serve for all.)  The dense path also takes what the others do not: K that is not a multiple of 256, rows that do
+// not start on 16 bytes.
 enum TcPath { kTcNone = 0, kTcSmall, kTcWide, kTcDense };
 static int tc_path(int qt, int M, int N, int K, int dtype, const void* x, const void* w, const void* w2, WidePlan* wide, DensePlan* dense, TcPath* out) {
   *out = kTcNone;

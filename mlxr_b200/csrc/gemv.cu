@@ -10,7 +10,8 @@
 //     nothing inside the stream waits on another warp;
 //   * under programmatic stream serialization the launch's CTAs fill their rings while the previous launch's
 //     last CTAs finish, and only the activations wait for its end.
-// 8B-shaped block of one token (two launches): 34.9 us with the persistent kernel of decode.cu, 24.7 here.
+// 8B-shaped block of one token (two launches): 34.9 us with the persistent kernel of decode.cu, 25.2 here.  Small Q4_K and
+// Q8_0 matrices, which do not repay the fixed part, are on stream_gemv.cu and gemv_rows_kernel.
 // The stream runs at HBM's rate; a launch's boundary, the loading and conversion of its activations and its
 // epilogue (about 5 us of each launch) do not overlap with it.  Eight warps in half an SM's resources,
 // so that the next launch's CTA could sit beside, took 36.8 us: two CTAs of the next launch

@@ -1,4 +1,4 @@
-// Small-batch quantized linear (3 <= M <= 64 rows of X) on the 5th-generation tensor cores.
+// Small-batch quantized linear (3 <= M <= 64 rows of X; one and two for the formats without a GEMV of their own) on the 5th-generation tensor cores.
 //
 //   Y[M, N] = X[M, K] * dequant(W)[N, K]^T (+ bias),  X, Y fp16 or bf16, W in MLXR's Q4_K, Q4_0 or
 //   Q8_0 layout, NF4 or the canonical ggml Q4_K layout (q_gemm_dequant.metal:142-260 and
@@ -134,8 +134,8 @@ __host__ __device__ inline long long unit_begin(long long U, int G, int c) { ret
 __host__ __device__ inline int unit_owner(long long U, int G, long long u) { return (int)(((u + 1) * G - 1) / U); }
 
 // SiLU with the sign-split sigmoid of swiglu_mlp_fused.metal:92-99, on the fast exponential and
-// reciprocal (relative error about 1e-6, far below the rounding to the activation dtype that
-// follows): the epilogue applies it to every batch row in turn, one thread per output column, and
+// reciprocal (relative error 1e-6 to |x| = 5, 7e-6 at 50: 2 + 1.17 |x| units of 2^-24 for the exponential; the
+// rounding to the activation dtype that follows is 5e-4 or more): the epilogue applies it to every batch row in turn, one thread per output column, and
 // the exact expf and division made that serial chain several times longer than the tile's MMAs.
 __device__ __forceinline__ float swish_fast(float x) {
   const float e = __expf(-fabsf(x));
@@ -652,7 +652,7 @@ int smallm_plan(int M, int rows, int K, int* grid, int* maxc, size_t* partial_by
   const int nsb = K / 256, ntiles = (N + smallm::kRows - 1) / smallm::kRows;
   const long long U = (long long)ntiles * nsb;
   // Either all SMs get equal ranges, which cross tiles, or every tile gets c CTAs of its own (the same formula with
-  // c * ntiles CTAs).  Measured at K = 4096, widths 16 and 64 of the padded batch: a unit takes 0.58 / 0.90 us, a
+  // c * ntiles CTAs).  Measured with Q4_K (a unit of the other formats takes longer, which the plan does not know) at K = 4096, widths 16 and 64 of the padded batch: a unit takes 0.58 / 0.90 us, a
   // shared tile 1.6 / 2.0 us plus 0.16 / 0.77 per part (parked, counted, read by the CTA that adds them), and
   // a range that crosses tiles 1.5 more, because its CTA parks two parts (2368 rows, batch 16: 8.4 us with equal
   // ranges on 148 SMs, 6.7 with four CTAs for each of the 19 tiles; 4096 rows, batch 64: 11.8 and 10.0).

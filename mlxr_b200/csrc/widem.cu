@@ -1,5 +1,5 @@
-// Quantized linear for 65 .. about 1500 tokens on the 5th-generation tensor cores, every weight converted
-// once per 256 tokens:
+// Quantized linear for 65 and more tokens, as long as dense.cu is not faster (14336 x 4096: to 1040), on the 5th-generation
+// tensor cores, every weight converted once per 256 tokens:
 //
 //   Y[M, N] = X[M, K] * dequant(W)[N, K]^T (+ bias),  X, Y fp16 or bf16, W in MLXR's Q4_K, Q4_0 or
 //   Q8_0 layout or NF4 (q_gemm_dequant.metal:142-260 for the formats).
@@ -96,8 +96,8 @@ __device__ inline long long unit_begin(long long U, int G, int c) { return (U * 
 __device__ inline int unit_owner(long long U, int G, long long u) { return (int)(((u + 1) * G - 1) / U); }
 
 // SiLU(gate) * up of two outputs held by a pair of lanes FAR apart: the lower lane has both gates, the upper one both ups.
-// Each of the two computes one output (the upper lane the second): the exact SiLU on one lane for both was 16 us of
-// 138 in the block of 333 tokens, 4096 x 11008.
+// Each of the two computes one output (the upper lane the second): with SiLU on one lane for both the block of 333 tokens,
+// 4096 x 11008, took 138 us, so 127.
 template <typename T> struct Pair { T value; int second; };
 template <typename T, int FAR> __device__ __forceinline__ Pair<T> swiglu_pair(float a, float b, int lane) {
   const bool up = (lane & FAR) != 0;
@@ -475,7 +475,7 @@ bool widem_supported(int qt, int M, int N, int K, int dtype, const void* x, cons
   return ((((uintptr_t)x) | ((uintptr_t)w)) & 15u) == 0;
 }
 
-// Token tile, grid and dealing of the units.  Fitted to measurements (65 to 2048 tokens, 14336 x 4096 and 4096 x
+// Token tile, grid and dealing of the units.  Fitted to measurements (Q4_K, 65 to 2048 tokens, 14336 x 4096 and 4096 x
 // 14336): a unit takes about 2000 cycles (the conversion of its 65536 weights and the turn-around of a stage)
 // plus 4.3 per token of the tile, a launch 14000 before and after its units; a shared tile costs its parts'
 // trip through L2 at the end; a whole tile per pair needs none of that but leaves SMs idle in the last wave.
