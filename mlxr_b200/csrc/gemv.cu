@@ -3,19 +3,24 @@
 // Roofline: HBM.  What kept the earlier kernels at 0.4 of it was a meeting of all warps for every 16 rows and
 // unequal numbers of tiles per CTA.  Here
 //   * a CTA (one per SM) owns a contiguous range of rows (in granules of four: 14336 rows are 24 or 25
-//     granules each on 148 SMs); its work units, (16-row tile, stage of K), are dealt to the sixteen warps in
-//     contiguous ranges, every warp keeps its own sums, and the warps meet once, at the end, when all
-//     partial sums lie in shared memory and are added in warp order (deterministic);
-//   * every warp fills its own ring with 2-D tensor TMA (four boxes of 4 rows per stage) and drains it, so
-//     nothing inside the stream waits on another warp;
+//     granules each on 148 SMs); its work units, (16-row tile, stage of K), go to the sixteen warps in turn, so that
+//     what a CTA has in flight is contiguous (a stream of 400 MB: 6.5 TB/s; 6.0 to 6.25 when every warp has a range of
+//     units of its own).  Every warp keeps its own sums of a tile, and the warps meet once in up to 32 tiles, when
+//     their sums lie in shared memory and are added in the order of K (deterministic);
+//   * every warp fills its own ring of two stages with 2-D tensor TMA (four boxes of 4 rows per stage) and drains it, so
+//     nothing inside the stream waits on another warp (147 KB in flight per SM; with three stages, 221 KB, the same
+//     stream of 400 MB falls to 5.9 TB/s);
 //   * under programmatic stream serialization the launch's CTAs fill their rings while the previous launch's
 //     last CTAs finish, and only the activations wait for its end.
-// 8B-shaped block of one token (two launches): 34.9 us with the persistent kernel of decode.cu, 25.2 here.  Small Q4_K and
-// Q8_0 matrices, which do not repay the fixed part, are on stream_gemv.cu and gemv_rows_kernel.
-// The stream runs at HBM's rate; a launch's boundary, the loading and conversion of its activations and its
-// epilogue (about 5 us of each launch) do not overlap with it.  Eight warps in half an SM's resources,
-// so that the next launch's CTA could sit beside, took 36.8 us: two CTAs of the next launch
-// came to lie on one SM.
+// 8B-shaped block of one token (two launches): 34.9 us with the persistent kernel of decode.cu, 22.9 here (25.2 with the
+// units in ranges, 64-bit divisions before the first copy and a serial addition of the warps' sums); 2048 x 5632 Q4_0
+// 12.7 -> 9.9.  Small Q4_K and Q8_0 matrices, which do not repay the fixed part, are on stream_gemv.cu and gemv_rows_kernel.
+// What is left beside the stream, per launch: its CTAs start when the previous one's leave the SMs, request weights 0.8 us
+// later and learn of its end 1.1 us after it; activations, their conversion and a meeting 2 to 3 us (the ring
+// fills meanwhile), the last sums and the epilogue 0.7 us; the slowest SM ends 1 us after the median one.
+// Eight warps in half an SM's resources, so that the next launch's CTA could sit beside, took 36.8 us: two CTAs of the next
+// launch came to lie on one SM.  Requests into L2 for the weights that the next launch reads first, sent behind the last of
+// gate / up's own, took the block from 24.2 to 25.8 us.
 //
 // Arithmetic, 4-bit formats: activations as 16-bit fixed point per 256 elements, split in a high and a low
 // signed byte; raw nibbles multiplied as unsigned bytes by mma.sync.m16n8k32 (the 16 MMA rows are weight
@@ -27,6 +32,7 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "decode_kernel.cuh"
 #include "kernels.h"
@@ -45,7 +51,8 @@ using decode::smem_u32;
 using decode::tma_load_2d;
 
 constexpr int kWarps = 16, kThreads = kWarps * 32;
-constexpr int kMaxStages = 4;
+constexpr int kMaxStages = 2;
+constexpr int kMaxChunk = 32, kMinChunk = 8;     // tiles between two meetings: as many as shared memory has places for
 constexpr int kSmemMax = 227 * 1024;
 
 // Bytes of 256 weights of a row, 256-element segments per stage, and sums of the activations kept per segment
@@ -62,8 +69,11 @@ struct Params {
   alignas(64) CUtensorMap map[3];
   int rows[3];
   int nmat, interleave;      // interleave: map[0] gate, map[1] up; y[0] = h [M, rows[0]]
-  int n_total, granules;     // rows (h elements) and granules of four of them
+  int n_total;               // rows (h elements)
+  int granules, gbase, gextra;      // granules of four rows: in all, per CTA, and CTAs with one more
   int K, nseg, nst;          // nst: stages per row
+  int step_tiles, step_st;   // kWarps units on: so many tiles and stages
+  int chunk;                 // tiles between two meetings of the warps
   int M;
   const void* x;
   const void* gamma;
@@ -79,7 +89,7 @@ struct Params {
   int* status;
   unsigned long long wait_ns;
   int stages, x_stride;
-  int off_x, off_aux, off_delta, off_sums, off_head, off_misc;
+  int off_x, off_aux, off_delta, off_parts, off_misc;
 };
 struct Misc {
   unsigned long long full[kWarps][kMaxStages];
@@ -90,22 +100,20 @@ struct Misc {
 
 // Fixed-point words of one (batch row, segment): v holds this lane's eight activations.  x ~ dl * xi with xi = v * inv,
 // |xi| <= 32000, xi = 256 hi + lo as two signed-byte rows in MMA k order, and the exact integer sums of xi that
-// the offset / min terms need.  1.5 * 2^23 added in the multiply leaves xi, rounded to nearest, in the low bits.
+// the offset / min terms need.  1.5 * 2^23 + 2^15 added in the multiply leaves xi + 2^15, rounded to nearest, in the low bits.
 // Returns the lane's sum of xi.
 template <int QT>
 __device__ __forceinline__ int emit_words(uint8_t* smem, const Params& P, int m, int sg, int lane, const float (&v)[8], float dl, float inv) {
   uint32_t t[8], sum = 0;
 #pragma unroll
-  for (int i = 0; i < 8; i++) { t[i] = __float_as_uint(fmaf(v[i], inv, 12582912.0f)); sum += t[i]; }
-  const int ssum = (int)(sum - 8u * 0x4B400000u);
-  // bytes of an 8-group are stored as (e0,e2,e4,e6 | e1,e3,e5,e7): the MMA k order
+  for (int i = 0; i < 8; i++) { t[i] = __float_as_uint(fmaf(v[i], inv, 12582912.0f + 32768.0f)); sum += t[i]; }
+  const int ssum = (int)(sum - 8u * 0x4B408000u);
+  // bytes of an 8-group are stored as (e0,e2,e4,e6 | e1,e3,e5,e7): the MMA k order.  xi + 32768 in 16 bits: its low
+  // byte is the low part; plus 128, its high byte is the high part plus 128.
   uint8_t* row = smem + P.off_x + (size_t)(2 * m) * P.x_stride + sg * 256 + lane * 8;
-  const uint32_t lo_e = __byte_perm(__byte_perm(t[0], t[2], 0x0040), __byte_perm(t[4], t[6], 0x0040), 0x5410);
-  const uint32_t lo_o = __byte_perm(__byte_perm(t[1], t[3], 0x0040), __byte_perm(t[5], t[7], 0x0040), 0x5410);
-#pragma unroll
-  for (int i = 0; i < 8; i++) t[i] += 128u;                       // q = 256 h + l, both in [-128, 127]
-  const uint32_t hi_e = __byte_perm(__byte_perm(t[0], t[2], 0x0051), __byte_perm(t[4], t[6], 0x0051), 0x5410);
-  const uint32_t hi_o = __byte_perm(__byte_perm(t[1], t[3], 0x0051), __byte_perm(t[5], t[7], 0x0051), 0x5410);
+  const uint32_t p02 = __byte_perm(t[0], t[2], 0x5410), p46 = __byte_perm(t[4], t[6], 0x5410), p13 = __byte_perm(t[1], t[3], 0x5410), p57 = __byte_perm(t[5], t[7], 0x5410);
+  const uint32_t lo_e = __byte_perm(p02, p46, 0x6420), lo_o = __byte_perm(p13, p57, 0x6420);
+  const uint32_t hi_e = __byte_perm(p02 + 0x00800080u, p46 + 0x00800080u, 0x7531) ^ 0x80808080u, hi_o = __byte_perm(p13 + 0x00800080u, p57 + 0x00800080u, 0x7531) ^ 0x80808080u;
   *reinterpret_cast<uint2*>(row) = make_uint2(hi_e, hi_o);
   *reinterpret_cast<uint2*>(row + P.x_stride) = make_uint2(lo_e, lo_o);
   float* aux = reinterpret_cast<float*>(smem + P.off_aux) + ((size_t)m * P.nseg + sg) * Geo<QT>::kAux;
@@ -170,7 +178,8 @@ __device__ __forceinline__ Lane make_lane(int lane, int qt) {
   Lane L;
   L.g = lane >> 2;
   L.c = lane & 3;
-  L.rg = (L.g & 4) | ((L.g & 1) << 1) | ((L.g >> 1) & 1);
+  // Q8_0: eight threads that read together have rows 16 bytes apart modulo 32
+  L.rg = qt == MLXR_Q8_0 ? L.g : (L.g & 4) | ((L.g & 1) << 1) | ((L.g >> 1) & 1);
   if (qt == MLXR_Q4_K) {
     // sub-block s belongs to pair {0,1,0,0,2,3,2,2}[s]; MMA column g stands for pair g >> 1
     L.keep0 = (int)((0x22320010u >> (4 * L.c)) & 7u) == (L.g >> 1);
@@ -284,6 +293,22 @@ __device__ __forceinline__ void seg_q40(const uint8_t* rl, const uint8_t* rh, co
   }
 }
 
+// Block 4 I + c of a Q8_0 segment: its 34 bytes begin 2 c (+ 8 for I = 1) bytes behind a 16-byte boundary and are read as three
+// 16-byte words.  (Word by word, 36 loads a unit with four-way bank conflicts, they were what bound the
+// stream: 14336 x 4096 16.9 us, 15.0 so.)
+template <int I> __device__ __forceinline__ void block_q80(const uint8_t* r, int c, __half& d, uint32_t (&v)[8]) {
+  const uint4* q = reinterpret_cast<const uint4*>(r + ((136 * I + 34 * c) & ~15));
+  const uint4 a = q[0], b = q[1], e = q[2];
+  const uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, e.x, e.y, e.z, e.w};
+  uint32_t t[9];
+#pragma unroll
+  for (int j = 0; j < 9; j++) t[j] = (c & 2) ? w[2 * I + j + 1] : w[2 * I + j];
+  const bool odd = c & 1;
+  d = __ushort_as_half((unsigned short)(odd ? t[0] >> 16 : t[0] & 0xFFFFu));
+#pragma unroll
+  for (int j = 0; j < 8; j++) v[j] = __funnelshift_rc(t[j], t[j + 1], odd ? 32 : 16);
+}
+
 __device__ __forceinline__ void hmma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -298,13 +323,12 @@ template <int J> __device__ __forceinline__ uint32_t pair_of_bytes(uint32_t u) {
 template <bool SCALED, int NT>
 __device__ __forceinline__ void seg_q80(const uint8_t* rl, const uint8_t* rh, const uint8_t* smem, const Params& P, int sg, const Lane& L, float (&tot)[NT][2]) {
   const bool keep = L.keep0 && (L.g & 1) < NT;
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const int at = 136 * i + 34 * L.c;
+  auto half = [&](auto I) {
+    constexpr int i = decltype(I)::value;
     __half dl, dh;
     uint32_t wl[8], wh[8];
-    words_after_scale<8>(rl + at, L.c & 1, dl, wl);
-    words_after_scale<8>(rh + at, L.c & 1, dh, wh);
+    block_q80<i>(rl, L.c, dl, wl);
+    block_q80<i>(rh, L.c, dh, wh);
     float acc[2][4] = {};
     const uint8_t* xr = smem + P.off_x + (size_t)(L.g & 1) * P.x_stride + (sg * 256 + 128 * i + 32 * L.c) * 2;
 #pragma unroll
@@ -323,7 +347,9 @@ __device__ __forceinline__ void seg_q80(const uint8_t* rl, const uint8_t* rh, co
       tot[j][0] = fmaf(__half2float(dl) * dx, acc[0][j] + acc[1][j], tot[j][0]);
       tot[j][1] = fmaf(__half2float(dh) * dx, acc[0][2 + j] + acc[1][2 + j], tot[j][1]);
     }
-  }
+  };
+  half(std::integral_constant<int, 0>{});
+  half(std::integral_constant<int, 1>{});
 }
 
 template <int QT, typename T, int NT>
@@ -334,21 +360,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = P.stages, S = P.nst;
 
-  // this CTA's granules, its tiles, and this warp's units [ub, ue): unit u = (tile u / S, stage u % S)
-  const int g0 = (int)(((long long)P.granules * blockIdx.x) / gridDim.x), g1 = (int)(((long long)P.granules * (blockIdx.x + 1)) / gridDim.x);
-  const int gpt = P.interleave ? 2 : 4, ntiles = (g1 - g0 + gpt - 1) / gpt, units = ntiles * S;
-  const int ub = (units * warp) / kWarps, ue = (units * (warp + 1)) / kWarps;
+  // This CTA's granules and tiles.  Unit u = (tile u / S, stage u % S); warp w takes units w, w + 16, ..
+  const int cta = blockIdx.x, g0 = cta * P.gbase + min(cta, P.gextra), g1 = g0 + P.gbase + (cta < P.gextra ? 1 : 0);
+  const int gpt = P.interleave ? 2 : 4, ntiles = (g1 - g0 + gpt - 1) >> (P.interleave ? 1 : 2), mine = (ntiles * S - warp + kWarps - 1) / kWarps;
+  int tile0 = 0, st0 = warp;
+  if (S <= warp) { tile0 = warp / S; st0 = warp - tile0 * S; }
+  auto advance = [&](int& tile, int& st) {
+    tile += P.step_tiles;
+    st += P.step_st;
+    if (st >= S) { st -= S; tile++; }
+  };
 
-  // The activations' and the norm weight's lines and pages are asked for first, into L2 only: the data itself is
-  // read after griddepcontrol.wait.
-  {
-    const int xl = (int)(((size_t)NT * P.K * sizeof(T) + 127) >> 7), gl = P.gamma ? (int)(((size_t)P.K * sizeof(T) + 127) >> 7) : 0;
-    for (int i = tid; i < xl + gl; i += kThreads)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(i < xl ? (const char*)P.x + (size_t)i * 128 : (const char*)P.gamma + (size_t)(i - xl) * 128));
-  }
   // ---- this warp's copy stream; weights are constants of the model, so it starts before the activations are there ----
   const uint32_t ring = smem_u32(smem) + warp * D * G_::kStage;
-  int i_tile = ub / S, i_st = ub - i_tile * S, i_slot = 0, i_left = ue - ub;
+  int i_tile = tile0, i_st = st0, i_slot = 0, i_left = mine;
   auto issue = [&]() {
     if (i_left <= 0) return;
     i_left--;
@@ -366,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
       }
     }
     if (++i_slot == D) i_slot = 0;
-    if (++i_st == S) { i_st = 0; i_tile++; }
+    advance(i_tile, i_st);
   };
   if (lane == 0) {
     for (int s = 0; s < D; s++) mbar_init(smem_u32(&misc->full[warp][s]), 1);
@@ -376,10 +401,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
   }
   __syncwarp();
   // Half of the ring now, the rest once the activations' loads are on their way: requested behind a full ring
-  // of every SM (22 MB), they came 3 us after the previous kernel's end instead of 1.5.
-  for (int i = 0; i < D / 2; i++) issue();
-  int held = D - D / 2;
+  // of every SM (22 MB), they came 3 us after the previous kernel's end instead of 1.5.  A CTA whose units all fit the ring
+  // does not have that much to request (2048 x 5632: 10.4 us in halves, 9.8 at once).
+  int held = ntiles * S <= D * kWarps ? 0 : D - D / 2;
+  for (int i = held; i < D; i++) issue();
   auto issue_held = [&]() { for (; held > 0; held--) issue(); };
+  // The activations' and the norm weight's lines and pages are asked for, into L2 only: the data itself is
+  // read after griddepcontrol.wait.
+  {
+    const int xl = (int)(((size_t)NT * P.K * sizeof(T) + 127) >> 7), gl = P.gamma ? (int)(((size_t)P.K * sizeof(T) + 127) >> 7) : 0;
+    for (int i = tid; i < xl + gl; i += kThreads)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(i < xl ? (const char*)P.x + (size_t)i * 128 : (const char*)P.gamma + (size_t)(i - xl) * 128));
+  }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
@@ -390,6 +423,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
   auto load_x = [&](int m, int s0, float (&v)[4][8]) {
 #pragma unroll
     for (int u = 0; u < 4; u++) if (s0 + u * kWarps < P.nseg) load8(xg + (size_t)m * P.K + (s0 + u * kWarps) * 256 + lane * 8, v[u]);
+  };
+  auto load_raw = [&](const T* row, int s0, Raw8<T> (&r)[4]) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) if (s0 + u * kWarps < P.nseg) r[u].load(row + (s0 + u * kWarps) * 256 + lane * 8);
   };
   float rinv[NT];
   bool rare = false;                                                    // see emit_fixed
@@ -464,10 +501,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
     // n rounded to T before its conversion, so the row's sum of squares comes first.  A warp's first four segments
     // and their norm weights wait for it in registers: up to K = 16384 nothing is read twice.
     Raw8<T> v[NT][4], gv[4];
-    auto load_raw = [&](const T* row, int s0, Raw8<T> (&r)[4]) {
-#pragma unroll
-      for (int u = 0; u < 4; u++) if (s0 + u * kWarps < P.nseg) r[u].load(row + (s0 + u * kWarps) * 256 + lane * 8);
-    };
 #pragma unroll
     for (int m = 0; m < NT; m++) load_raw(xg + (size_t)m * P.K, warp, v[m]);
     load_raw(gam, warp, gv);
@@ -521,23 +554,30 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
 #pragma unroll
     for (int m = 0; m < NT; m++) {
       float ss = 0.0f;
+      Raw8<T> cur[4], next[4];
+      load_raw(xg + (size_t)m * P.K, warp, cur);
+#pragma unroll 1
       for (int s0 = warp; s0 < P.nseg; s0 += 4 * kWarps) {
-        float v[4][8];
-        load_x(m, s0, v);
+        load_raw(xg + (size_t)m * P.K, s0 + 4 * kWarps, next);      // on their way while these are converted
         if (!gam) issue_held();
 #pragma unroll
         for (int u = 0; u < 4; u++) {
           const int sg = s0 + u * kWarps;
           if (sg >= P.nseg) break;
+          float v[8];
+#pragma unroll
+          for (int i = 0; i < 8; i++) v[i] = cur[u].f(i);
           if (gam) {
             float gv[8];
             load8(gam + sg * 256 + lane * 8, gv);
             issue_held();
 #pragma unroll
-            for (int i = 0; i < 8; i++) { ss = fmaf(v[u][i], v[u][i], ss); v[u][i] *= gv[i]; }
+            for (int i = 0; i < 8; i++) { ss = fmaf(v[i], v[i], ss); v[i] *= gv[i]; }
           }
-          rare |= emit_fixed<QT>(smem, P, m, sg, lane, v[u]);
+          rare |= emit_fixed<QT>(smem, P, m, sg, lane, v);
         }
+#pragma unroll
+        for (int u = 0; u < 4; u++) cur[u] = next[u];
       }
       if (gam) {
         ss = warp_sum(ss);
@@ -574,116 +614,111 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
 
   // ---- the stream ----
   const Lane L = make_lane(lane, QT);
-  float* sums = reinterpret_cast<float*>(smem + P.off_sums);            // [ntiles][16][NT]: the part that begins a tile
-  float* head = reinterpret_cast<float*>(smem + P.off_head) + warp * 16 * NT;   // this warp's later part of its first tile
+  float* parts = reinterpret_cast<float*>(smem + P.off_parts);          // [tiles of a chunk][warp][16][NT]
   float tot[NT][2] = {};
-  int tile = ub / S, st = ub - tile * S, slot = 0;
-  bool own = st == 0;                                                   // this warp holds the tile's first stage
+  int tile = tile0, st = st0, slot = 0, left = mine;
   uint32_t par = 0;
-  for (int u = ub; u < ue; u++) {
-    const uint8_t* stage = smem + (size_t)(warp * D + slot) * G_::kStage;
-    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc->full[warp][slot]), par, &misc->dead, P.wait_ns))) {
-      // a give-up: the copies in flight must land before the CTA may exit (bounded)
+  const int row_end = min(4 * g1, P.n_total);
+  for (int t0 = 0;; t0 += P.chunk) {
+    const int t1 = min(t0 + P.chunk, ntiles);
+    while (left > 0 && tile < t1) {
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc->full[warp][slot]), par, &misc->dead, P.wait_ns))) break;
+      const uint8_t* stage = smem + (size_t)(warp * D + slot) * G_::kStage;
+      const uint8_t *rl = stage + (L.rg >> 2) * G_::kBox + (L.rg & 3) * G_::kPitch, *rh = rl + 2 * G_::kBox;
+      const int sg = st * G_::kSegs;
+      if constexpr (QT == MLXR_Q8_0) {
+        seg_q80<Act<T>::kDtype == MLXR_BF16, NT>(rl, rh, smem, P, sg, L, tot);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          if (k && sg + 1 >= P.nseg) break;
+          if constexpr (QT == MLXR_Q4_K) seg_q4k<NT>(rl + k * 144, rh + k * 144, smem, P, sg + k, L, tot);
+          else seg_q40<NT>(rl + k * 144, rh + k * 144, smem, P, sg + k, L, tot);
+        }
+      }
+      if (++slot == D) { slot = 0; par ^= 1u; }
+      __syncwarp();
+      issue();      // refill the stage that was just drained
+      left--;
+      const int was = tile;
+      advance(tile, st);
+      if (tile != was || left == 0) {
+        // the quad's four parts of (row, batch) go to shared memory
+        float* dst = parts + ((was - t0) * kWarps + warp) * 16 * NT;
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            float v = tot[j][h];
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if (L.c == 0) dst[(L.rg + 8 * h) * NT + j] = v;
+            tot[j][h] = 0.0f;
+          }
+      }
+    }
+    __syncthreads();
+    if (misc->dead) {       // some sums are missing: nothing is stored; the copies in flight must land before the CTA may exit (bounded)
       if (lane == 0)
-        for (int i = u - ub; i < ue - ub - i_left; i++)
+        for (int i = mine - left; i < mine - i_left; i++)
           bounded_wait([&] { return decode::mbar_try_wait(smem_u32(&misc->full[warp][i % D]), (uint32_t)(i / D) & 1u); }, 1000000000ull);
       __syncwarp();
-      break;
+      if (tid == 0) atomicExch(P.status, MLXR_ERR_TIMEOUT);
+      return;
     }
-    const uint8_t *rl = stage + (L.rg >> 2) * G_::kBox + (L.rg & 3) * G_::kPitch, *rh = rl + 2 * G_::kBox;
-    const int sg = st * G_::kSegs;
-    if constexpr (QT == MLXR_Q8_0) {
-      seg_q80<Act<T>::kDtype == MLXR_BF16, NT>(rl, rh, smem, P, sg, L, tot);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 2; k++) {
-        if (k && sg + 1 >= P.nseg) break;
-        if constexpr (QT == MLXR_Q4_K) seg_q4k<NT>(rl + k * 144, rh + k * 144, smem, P, sg + k, L, tot);
-        else seg_q40<NT>(rl + k * 144, rh + k * 144, smem, P, sg + k, L, tot);
-      }
-    }
-    if (++slot == D) { slot = 0; par ^= 1u; }
-    __syncwarp();
-    issue();      // refill the stage that was just drained
-    if (++st == S || u + 1 == ue) {
-      // the quad's four parts of (row, batch), then the tile's row sums go to shared memory
-      float* dst = own ? sums + tile * 16 * NT : head;
-#pragma unroll
-      for (int j = 0; j < NT; j++)
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          float v = tot[j][h];
-          v += __shfl_xor_sync(0xffffffffu, v, 1);
-          v += __shfl_xor_sync(0xffffffffu, v, 2);
-          if (L.c == 0) dst[(L.rg + 8 * h) * NT + j] = v;
-          tot[j][h] = 0.0f;
-        }
-      st = 0;
-      tile++;
-      own = true;
-    }
-  }
-  __syncthreads();
-  if (misc->dead) {       // some sums are missing: nothing is stored
-    if (tid == 0) atomicExch(P.status, MLXR_ERR_TIMEOUT);
-    return;
-  }
 
-  // ---- rows of this CTA: a thread per row and batch row adds the parts in warp order ----
-  for (int e = tid; e < ntiles * 16 * NT; e += kThreads) {
-    const int t = e / (16 * NT), r = e - t * 16 * NT;
-    float v = sums[e];
-    // the warps after the one that holds the tile's first stage, as long as their ranges begin inside the tile
-    for (int w = ((t * S + 1) * kWarps - 1) / units + 1; w < kWarps && (units * w) / kWarps < (t + 1) * S; w++)
-      if ((units * (w + 1)) / kWarps > (units * w) / kWarps) v += reinterpret_cast<const float*>(smem + P.off_head)[w * 16 * NT + r];
-    sums[e] = scale_sums ? v * misc->rinv[r % NT] : v;
-  }
-  __syncthreads();
-  // ---- epilogue: a thread per pair of adjacent rows and batch row ----
-  auto row_sum = [&](int t, int r, int m) { return sums[(t * 16 + r) * NT + m]; };
-  const int npair = 2 * (g1 - g0);                     // pairs of rows (or of h elements)
-  for (int e = tid; e < npair * NT; e += kThreads) {
-    const int pr = e % npair, m = e / npair;
-    if (P.interleave) {
-      const int col = 4 * g0 + 2 * pr, t = pr >> 2, r = (2 * pr) & 7;
-      T h[2];
+    // ---- rows of these tiles: a thread per row and batch row adds the warps' parts in the order of K; a row's partner (the
+    // up row of a gate row, the other row of a RoPE pair) is a lane of the same warp ----
+    const int n = (t1 - t0) * 16 * NT;
+    for (int e0 = warp * 32; e0 < n; e0 += kThreads) {
+      const int e = e0 + lane, tl = e / (16 * NT), r = (e / NT) & 15, m = e % NT;
+      float v = 0.0f;
+      if (e < n) {
+        const float* p = parts + tl * (kWarps * 16 * NT) + r * NT + m;
+        const int first = (t0 + tl) * S;
+        float a[kWarps];
 #pragma unroll
-      for (int k = 0; k < 2; k++) {
-        const float gv = Act<T>::to_f(Act<T>::from_f(row_sum(t, r + k, m))), uv = Act<T>::to_f(Act<T>::from_f(row_sum(t, r + 8 + k, m)));
-        h[k] = Act<T>::from_f(swish_f(gv) * uv);
+        for (int k = 0; k < kWarps; k++) a[k] = k < S ? p[((first + k) & (kWarps - 1)) * (16 * NT)] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < kWarps; k++) v += a[k];
+        if (scale_sums) v *= misc->rinv[m];
       }
-      T* out = reinterpret_cast<T*>(P.y[0]) + (size_t)m * P.n_total + col;
-      if (col < P.n_total) out[0] = h[0];
-      if (col + 1 < P.n_total) out[1] = h[1];
-      continue;
+      if (P.interleave) {
+        const float up = __shfl_xor_sync(0xffffffffu, v, 8 * NT);
+        const int col = 4 * g0 + 8 * (t0 + tl) + r;
+        if (e < n && r < 8 && col < row_end) {
+          const float gv = Act<T>::to_f(Act<T>::from_f(v)), uv = Act<T>::to_f(Act<T>::from_f(up));
+          reinterpret_cast<T*>(P.y[0])[(size_t)m * P.n_total + col] = Act<T>::from_f(swish_f(gv) * uv);
+        }
+        continue;
+      }
+      int R = 4 * g0 + 16 * (t0 + tl) + r;
+      const bool store = e < n && R < row_end;
+      int mat = 0;
+      if (P.nmat > 1 && R >= P.rows[0]) { R -= P.rows[0]; mat = 1; if (P.nmat > 2 && R >= P.rows[1]) { R -= P.rows[1]; mat = 2; } }
+      const T* bias = reinterpret_cast<const T*>(P.bias[mat]);
+      if (bias && store) v += Act<T>::to_f(bias[R]);
+      const float other = __shfl_xor_sync(0xffffffffu, v, NT);
+      if (!store) continue;
+      const size_t at = (size_t)m * P.rows[mat] + R;
+      if (P.epi[mat] == decode::kEpiF32) {
+        reinterpret_cast<float*>(P.y[mat])[at] = v;
+        continue;
+      }
+      T* out = reinterpret_cast<T*>(P.y[mat]) + at;
+      if (P.epi[mat] == decode::kEpiRope) {
+        const float own = Act<T>::to_f(Act<T>::from_f(v)), oth = Act<T>::to_f(Act<T>::from_f(other));
+        const long long pos = (long long)P.positions[m] + P.pos_offset;
+        if (pos < 0 || pos >= P.max_seq) { atomicExch(P.status, MLXR_ERR_SHAPE); continue; }
+        const int pairs = P.head_dim >> 1, pi = (R % P.head_dim) >> 1;
+        const float cs = __half2float(P.cos_t[(size_t)pos * pairs + pi]), sn = __half2float(P.sin_t[(size_t)pos * pairs + pi]);
+        *out = Act<T>::from_f((R & 1) ? __fadd_rn(__fmul_rn(own, cs), __fmul_rn(oth, sn)) : __fsub_rn(__fmul_rn(own, cs), __fmul_rn(oth, sn)));
+      } else {
+        *out = Act<T>::from_f(v);
+      }
     }
-    int R = 4 * g0 + 2 * pr;
-    if (R >= P.n_total) continue;
-    float ve = row_sum(pr >> 3, (2 * pr) & 15, m), vo = row_sum(pr >> 3, ((2 * pr) & 15) + 1, m);
-    int mat = 0;
-    if (P.nmat > 1 && R >= P.rows[0]) { R -= P.rows[0]; mat = 1; if (P.nmat > 2 && R >= P.rows[1]) { R -= P.rows[1]; mat = 2; } }
-    const bool odd = R + 1 < P.rows[mat];
-    const T* bias = reinterpret_cast<const T*>(P.bias[mat]);
-    if (bias) { ve += Act<T>::to_f(bias[R]); if (odd) vo += Act<T>::to_f(bias[R + 1]); }
-    if (P.epi[mat] == decode::kEpiF32) {
-      float* of = reinterpret_cast<float*>(P.y[mat]) + (size_t)m * P.rows[mat] + R;
-      of[0] = ve;
-      if (odd) of[1] = vo;
-      continue;
-    }
-    T* out = reinterpret_cast<T*>(P.y[mat]) + (size_t)m * P.rows[mat] + R;
-    if (P.epi[mat] == decode::kEpiRope) {
-      const float qe = Act<T>::to_f(Act<T>::from_f(ve)), qo = Act<T>::to_f(Act<T>::from_f(vo));
-      const long long pos = (long long)P.positions[m] + P.pos_offset;
-      if (pos < 0 || pos >= P.max_seq) { atomicExch(P.status, MLXR_ERR_SHAPE); continue; }
-      const int pairs = P.head_dim >> 1, pi = (R % P.head_dim) >> 1;
-      const float cs = __half2float(P.cos_t[(size_t)pos * pairs + pi]), sn = __half2float(P.sin_t[(size_t)pos * pairs + pi]);
-      out[0] = Act<T>::from_f(__fsub_rn(__fmul_rn(qe, cs), __fmul_rn(qo, sn)));
-      out[1] = Act<T>::from_f(__fadd_rn(__fmul_rn(qo, cs), __fmul_rn(qe, sn)));
-    } else {
-      out[0] = Act<T>::from_f(ve);
-      if (odd) out[1] = Act<T>::from_f(vo);
-    }
+    if (t1 == ntiles) break;
+    __syncthreads();        // the parts' places are free again
   }
 }
 
@@ -698,17 +733,17 @@ template <int QT> static size_t layout(Params* P, int M, int grid) {
   using G = Geo<QT>;
   const int per = P->interleave ? 2 : 4, most = (P->granules + grid - 1) / grid, tiles = (most + per - 1) / per;
   P->x_stride = (QT == MLXR_Q8_0 ? 2 * P->K : P->K) + 16;
-  for (P->stages = kMaxStages; P->stages >= 1; P->stages--) {
-    size_t o = (size_t)kWarps * P->stages * G::kStage;
-    auto take = [&](size_t n) { const size_t at = o; o += (n + 15) & ~(size_t)15; return (int)at; };
-    P->off_x = take((size_t)(QT == MLXR_Q8_0 ? M : 2 * M) * P->x_stride);
-    P->off_aux = take((size_t)M * P->nseg * G::kAux * 4);
-    P->off_delta = take((size_t)M * P->nseg * 4);
-    P->off_sums = take((size_t)tiles * 16 * M * 4);
-    P->off_head = take((size_t)kWarps * 16 * M * 4);
-    P->off_misc = take(sizeof(Misc));
-    if (o <= (size_t)kSmemMax) return o;
-  }
+  for (P->stages = kMaxStages; P->stages >= 1; P->stages--)
+    for (P->chunk = kMaxChunk; P->chunk >= kMinChunk; P->chunk /= 2) {
+      size_t o = (size_t)kWarps * P->stages * G::kStage;
+      auto take = [&](size_t n) { const size_t at = o; o += (n + 15) & ~(size_t)15; return (int)at; };
+      P->off_x = take((size_t)(QT == MLXR_Q8_0 ? M : 2 * M) * P->x_stride);
+      P->off_aux = take((size_t)M * P->nseg * G::kAux * 4);
+      P->off_delta = take((size_t)M * P->nseg * 4);
+      P->off_parts = take((size_t)std::min(tiles, P->chunk) * kWarps * 16 * M * 4);
+      P->off_misc = take(sizeof(Misc));
+      if (o <= (size_t)kSmemMax) return o;
+    }
   return 0;
 }
 
@@ -803,6 +838,10 @@ int launch_gemv(const DecodeLinear& L, int M, int qt, int dtype, int* status, cu
   P.wait_ns = wait_limit_ns();
   if (P.granules < 1) return MLXR_OK;
   const int grid = P.granules < sms ? P.granules : sms;
+  P.gbase = P.granules / grid;
+  P.gextra = P.granules % grid;
+  P.step_tiles = kWarps / P.nst;
+  P.step_st = kWarps % P.nst;
 #define MLXR_GEMV_T(QTV, T) return M == 1 ? launch_gemv_inst<QTV, T, 1>(P, grid, st) : launch_gemv_inst<QTV, T, 2>(P, grid, st)
 #define MLXR_GEMV_4(QTV)                                                       \
   do {                                                                         \

@@ -48,6 +48,24 @@ def test_linear(oracle, qt, dt, M, N, K):
     assert float((y.double() - want).norm() / want.norm()) <= RESULT[dt] + WEIGHT[qt]
 
 
+@pytest.mark.parametrize("qt,M,N,K", [(3, 1, 80003, 256), (3, 2, 40961, 1024), (0, 1, 76001, 512), (2, 2, 90001, 256), (2, 1, 5, 16384)])
+def test_warps_meet_more_than_once(oracle, qt, M, N, K):
+    """More rows per CTA than the places for the warps' sums hold (32 tiles of 16 rows, fewer for two tokens), and one tile
+    whose stages go round the warps four times.  Rows are drawn from 4096 quantized ones; every result is compared."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    block = quantize(make_weights(4096, K, 3), qt).reshape(4096, -1)
+    which = np.random.Generator(np.random.PCG64(5)).integers(0, 4096, N)
+    packed = np.ascontiguousarray(block[which]).reshape(-1)
+    x = make_acts(M, K, 4, torch.bfloat16)[0].cuda()
+    y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt))
+    assert _status() == 0
+    want = (x.double() @ _dense(oracle, block.reshape(-1), 4096, K, qt).T)[:, torch.from_numpy(which).cuda()]
+    assert float((y.double() - want).norm() / want.norm()) <= RESULT["bf16"] + WEIGHT[qt]
+    # no row may be wrong by itself: the largest results are below 6 rms, their rounding below 6 * 2^-8
+    assert float((y.double() - want).abs().max() / want.square().mean().sqrt()) <= 6 * (RESULT["bf16"] + WEIGHT[qt])
+
+
 @pytest.mark.parametrize("qt", [0, 2, 3])
 @pytest.mark.parametrize("scale", [1e-30, 1.0, 1e30])
 def test_range_of_bf16(oracle, qt, scale):
