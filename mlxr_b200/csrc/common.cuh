@@ -100,6 +100,16 @@ __device__ __forceinline__ float swish_f(float x) {
   const float e = expf(-fabsf(x));
   return (x >= 0.0f ? x : x * e) / (1.0f + e);
 }
+// The same for results that are rounded to a 16-bit type, in half the instructions: the denominator lies in [1, 2], so the
+// quotient needs no care for its range, and one residual correction of n * (1 / d) leaves it within a unit of the last
+// place of float32 of the exact one (for every 16-bit x the product with `up` rounds as swish_f's does).
+__device__ __forceinline__ float swish_h(float x) {
+  const float e = expf(-fabsf(x)), d = 1.0f + e, n = x >= 0.0f ? x : x * e;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = n * r, rest = fmaf(-q, d, n);
+  return fabsf(rest) > 0.0f ? fmaf(rest, r, q) : q;      // x = +infinity has none, and -0 stays -0
+}
 
 // The 6-bit (scale, min) pair the reference shader uses for sub-block s of a Q4_K
 // super-block (q_gemm_dequant.metal:222-242): only scales[0..5] are read, and offsets 2

@@ -1,6 +1,7 @@
 // RMSNorm, SwiGLU and RoPE as standalone kernels: the primitives called on their own, and RMSNorm and RoPE
 // around the linears of three and more tokens (the kernels for fewer carry their own copies of this arithmetic).
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -83,6 +84,19 @@ static bool aligned16(const void* a, const void* b, const void* c = nullptr, con
   return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d) & 15u) == 0;
 }
 
+// A launch that may start under the previous kernel of the stream (both wait with griddepcontrol before they touch memory)
+static cudaLaunchConfig_t overlapped(int grid, int threads, cudaStream_t st, cudaLaunchAttribute* at) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = st;
+  at->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at->val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
 // The same row for 16-bit types in 128-bit accesses: a row stays in registers between the two passes.
 // Bound by HBM (three streams with a residual); with 2-byte accesses the loads in flight were an eighth
 // of this and [1111, 4096] fp16 took 14 us where the bytes need 4.2.  Launched with programmatic stream
@@ -134,14 +148,8 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_vec_kernel(const T* x, const 
 template <typename T>
 static int launch_rmsnorm_vec(const void* x, const void* w, const void* res, void* y, int rows, int hidden, float eps, cudaStream_t st) {
   const int nvec = hidden / 8;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(rows);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at;
+  cudaLaunchConfig_t cfg = overlapped(rows, 0, st, &at);
 #define MLXR_RMS(TH, PER) do { cfg.blockDim = dim3(TH); MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rmsnorm_vec_kernel<T, TH, PER>, (const T*)x, (const T*)w, (const T*)res, (T*)y, nvec, eps)); } while (0)
   if (nvec <= 128) MLXR_RMS(128, 1);
   else if (nvec <= 256) MLXR_RMS(256, 1);
@@ -185,28 +193,41 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const T* g,
   }
 }
 
-// The same for 16-bit types, 128-bit accesses, two vectors in flight per thread and operand.  Bound by HBM (three
-// streams) and, close behind, by the exponential and the division; with 2-byte accesses [1111, 14336] fp16 took
-// 41 us where the bytes need 14.6.
+// The same for 16-bit types, 128-bit accesses, resident CTAs: a thread has two vectors of each operand in work and the next
+// two on their way.  Bound by HBM (three streams).  With the exact division, in a grid of 3889 short CTAs, it was bound by
+// issue (73 %).  rmsnorm, rope_apply of q and of k, swiglu on 1111 tokens of 4096 x 14336: 55.1 us a pass, 45.5 with this, the
+// rotation's 32-bit quotients and its early answer.
 template <typename T, bool UP>
-__global__ void __launch_bounds__(256) swiglu_vec_kernel(const T* g, const T* u, T* o, size_t nvec) {
+__global__ void __launch_bounds__(256, 4) swiglu_vec_kernel(const T* g, const T* u, T* o, size_t nvec) {
   const size_t step = (size_t)gridDim.x * 256;
-  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < nvec; i += 2 * step) {
-    const bool two = i + step < nvec;
-    float a[2][8], b[2][8];
-    load8v(g + i * 8, a[0]);
-    if (two) load8v(g + (i + step) * 8, a[1]);
-    if constexpr (UP) {
-      load8v(u + i * 8, b[0]);
-      if (two) load8v(u + (i + step) * 8, b[1]);
-    }
+  size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  uint4 a[2], b[2];
+  auto load = [&](size_t at, uint4 (&x)[2], uint4 (&y)[2]) {
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+      if (at + k * step < nvec) {
+        x[k] = __ldcg(reinterpret_cast<const uint4*>(g) + at + k * step);
+        if constexpr (UP) y[k] = __ldcg(reinterpret_cast<const uint4*>(u) + at + k * step);
+      }
+  };
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  load(i, a, b);
+  for (; i < nvec; i += 2 * step) {
+    uint4 na[2], nb[2];
+    load(i + 2 * step, na, nb);
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-      if (k && !two) break;
+      if (i + k * step >= nvec) break;
+      float x[8], y[8];
+      unpack8<T>(a[k], x);
+      if constexpr (UP) unpack8<T>(b[k], y);
 #pragma unroll
-      for (int e = 0; e < 8; e++) a[k][e] = UP ? swish_f(a[k][e]) * b[k][e] : swish_f(a[k][e]);
-      store8v(o + (i + k * step) * 8, a[k]);
+      for (int e = 0; e < 8; e++) x[e] = UP ? swish_h(x[e]) * y[e] : swish_h(x[e]);
+      store8v(o + (i + k * step) * 8, x);
     }
+#pragma unroll
+    for (int k = 0; k < 2; k++) { a[k] = na[k]; if constexpr (UP) b[k] = nb[k]; }
   }
 }
 
@@ -216,12 +237,14 @@ int launch_swiglu(const void* g, const void* u, void* o, size_t n, int dtype, cu
   // and 2.9, 2^21: 7.4 and 4.6)
   if (dtype != MLXR_F32 && n % 8 == 0 && n > 1 << 18 && aligned16(g, o, u)) {
     const size_t nvec = n / 8;
-    const int vb = (int)std::min<size_t>((nvec + 511) / 512, 148 * 8 * 4);
-#define MLXR_SWIGLU(T) do { if (u) swiglu_vec_kernel<T, true><<<vb, 256, 0, st>>>((const T*)g, (const T*)u, (T*)o, nvec); \
-                            else swiglu_vec_kernel<T, false><<<vb, 256, 0, st>>>((const T*)g, (const T*)u, (T*)o, nvec); } while (0)
+    const int vb = (int)std::min<size_t>((nvec + 511) / 512, 148 * 4);
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = overlapped(vb, 256, st, &at);
+#define MLXR_SWIGLU(T) do { if (u) MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, swiglu_vec_kernel<T, true>, (const T*)g, (const T*)u, (T*)o, nvec)); \
+                            else MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, swiglu_vec_kernel<T, false>, (const T*)g, (const T*)u, (T*)o, nvec)); } while (0)
     if (dtype == MLXR_F16) MLXR_SWIGLU(__half); else MLXR_SWIGLU(__nv_bfloat16);
 #undef MLXR_SWIGLU
-    MLXR_LAUNCH_CHECK("swiglu_vec_kernel");
+    count_launch();
     return MLXR_OK;
   }
   size_t blocks = (n + 255) / 256;
@@ -297,63 +320,101 @@ __global__ void __launch_bounds__(256) rope_kernel(const T* x,
   }
 }
 
+// Quotients of n < 2^31 by a divisor known to the host (Granlund and Montgomery, "Division by invariant integers using
+// multiplication", 1994): a 64-bit division of the vector's number took more instructions than its rotation.
+struct Divisor {
+  uint32_t d, mul, shift;
+  explicit Divisor(uint32_t d_) : d(d_), shift(0) {
+    while ((1ull << shift) < d) shift++;
+    mul = (uint32_t)((((1ull << 32) * ((1ull << shift) - d)) / d) + 1);
+  }
+  __device__ __forceinline__ uint32_t quot(uint32_t n) const { return (__umulhi(n, mul) + n) >> shift; }
+};
+
 // The same for 16-bit types and heads of a multiple of 8 elements: one thread per four pairs, 128-bit
 // accesses to x and y, 64-bit to the tables; the token's position is checked once per thread.
 //
 // Two tensors that share the positions (q and k of a layer) can go in one launch: vectors from `total` on are z's,
 // up to total_z.
-template <typename T>
-__global__ void __launch_bounds__(256) rope_vec_kernel(const T* x, const __half* __restrict__ cos_t, const __half* __restrict__ sin_t,
-                                                       const int32_t* positions, T* y, size_t total, int vec_per_token, T* z, size_t total_z, int vec_per_token_z,
-                                                       int vec_per_head, int max_seq, int linear, float scale, int offset, int* status) {
+//
+// early: the word in host memory that a waiting caller reads.  CTA 0 then rotates nothing and checks all positions
+// first, so that the caller knows them valid (1) or not (2) while the rotation still runs.
+struct RopeArgs {
+  const __half *cos_t, *sin_t;
+  const int32_t* positions;
+  size_t total, total_z, tokens;
+  Divisor per, per_z, per_head;          // vectors of a token of x, of z, of a head
+  int max_seq, linear;
+  float scale;
+  int offset;
+  int *status, *early;
+};
+template <typename T, bool WIDE>          // WIDE: 2^31 vectors and more
+__global__ void __launch_bounds__(256) rope_vec_kernel(const T* x, T* y, T* z, const RopeArgs A) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  for (size_t j = (size_t)blockIdx.x * 256 + threadIdx.x; j < total + total_z; j += (size_t)gridDim.x * 256) {
+  auto valid = [&](long long pos) { return pos >= 0 && pos < A.max_seq; };
+  int cta = blockIdx.x, ctas = gridDim.x;
+  if (A.early) {
+    if (cta == 0) {
+      bool ok = true;
+#pragma unroll 8
+      for (size_t t = threadIdx.x; t < A.tokens; t += 256) ok = ok && valid((long long)__ldcg(A.positions + t) + A.offset);
+      ok = __syncthreads_and(ok);
+      if (threadIdx.x == 0) atomicExch_system(A.early, ok ? 1 : 2);
+      return;
+    }
+    cta--;
+    ctas--;
+  }
+  using Index = typename std::conditional<WIDE, size_t, uint32_t>::type;
+  const Index total = (Index)A.total, all = (Index)(A.total + A.total_z);
+  for (size_t j0 = (size_t)cta * 256 + threadIdx.x; j0 < all; j0 += (size_t)ctas * 256) {
+    const Index j = (Index)j0;
     const bool first = j < total;
-    const size_t i = first ? j : j - total;
-    const int per = first ? vec_per_token : vec_per_token_z;
+    const Index i = first ? j : j - total;
+    const Divisor& per = first ? A.per : A.per_z;
     const T* src = first ? x : z;
     T* dst = first ? y : z;
-    const size_t tok = i / per;
-    const int c = (int)(i - tok * per) % vec_per_head;
-    const uint4 xv = __ldcg(reinterpret_cast<const uint4*>(src + i * 8));
-    const long long pos = (long long)__ldcg(positions + tok) + offset;
-    if (pos < 0 || pos >= max_seq) {
-      if (status) atomicExch_system(status, 1);
+    Index tok;
+    uint32_t c, h;
+    if constexpr (WIDE) tok = i / per.d; else tok = per.quot(i);
+    c = (uint32_t)(i - tok * per.d);
+    h = A.per_head.quot(c);
+    c -= h * A.per_head.d;
+    const uint4 xv = __ldcg(reinterpret_cast<const uint4*>(src) + i);
+    const long long pos = (long long)__ldcg(A.positions + tok) + A.offset;
+    if (!valid(pos)) {
+      if (A.status) atomicExch_system(A.status, 1);
       continue;
     }
-    const uint2 cv = __ldg(reinterpret_cast<const uint2*>(cos_t + (size_t)pos * vec_per_head * 4) + c);
-    const uint2 sv = __ldg(reinterpret_cast<const uint2*>(sin_t + (size_t)pos * vec_per_head * 4) + c);
-    const T* h = reinterpret_cast<const T*>(&xv);
+    const uint2 cv = __ldg(reinterpret_cast<const uint2*>(A.cos_t) + (size_t)pos * A.per_head.d + c);
+    const uint2 sv = __ldg(reinterpret_cast<const uint2*>(A.sin_t) + (size_t)pos * A.per_head.d + c);
+    const T* hx = reinterpret_cast<const T*>(&xv);
     const __half *hc = reinterpret_cast<const __half*>(&cv), *hs = reinterpret_cast<const __half*>(&sv);
     float o[8];
 #pragma unroll
     for (int p = 0; p < 4; p++) {
-      const float cs = __half2float(hc[p]), sn = __half2float(hs[p]), xe = Act<T>::to_f(h[2 * p]), xo = Act<T>::to_f(h[2 * p + 1]);
+      const float cs = __half2float(hc[p]), sn = __half2float(hs[p]), xe = Act<T>::to_f(hx[2 * p]), xo = Act<T>::to_f(hx[2 * p + 1]);
       o[2 * p] = __fsub_rn(__fmul_rn(xe, cs), __fmul_rn(xo, sn));
       o[2 * p + 1] = __fadd_rn(__fmul_rn(xo, cs), __fmul_rn(xe, sn));
-      if (linear) { o[2 * p] *= scale; o[2 * p + 1] *= scale; }
+      if (A.linear) { o[2 * p] *= A.scale; o[2 * p + 1] *= A.scale; }
     }
-    store8v(dst + i * 8, o);
+    store8v(dst + (size_t)i * 8, o);
   }
 }
 
 template <typename T>
 static int launch_rope_vec(const void* x, const uint16_t* cos_t, const uint16_t* sin_t, const int32_t* positions, void* y, size_t tokens, int heads,
-                           void* z, int heads_z, int head_dim, int max_seq, int linear, float scale, int offset, int* status, cudaStream_t st) {
+                           void* z, int heads_z, int head_dim, int max_seq, int linear, float scale, int offset, int* status, int* early, cudaStream_t st) {
   const int vh = head_dim / 8;
-  const size_t total = tokens * heads * vh, total_z = tokens * heads_z * vh;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)std::min<size_t>((total + total_z + 255) / 256, 148 * 8 * 4));
-  cfg.blockDim = dim3(256);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rope_vec_kernel<T>, (const T*)x, (const __half*)cos_t, (const __half*)sin_t, positions, (T*)y, total, heads * vh,
-                                   (T*)z, total_z, heads_z * vh, vh, max_seq, linear, scale, offset, status));
+  const RopeArgs A = {(const __half*)cos_t, (const __half*)sin_t, positions, tokens * heads * vh, tokens * heads_z * vh, tokens,
+                      Divisor((uint32_t)heads * vh), Divisor((uint32_t)std::max(1, heads_z * vh)), Divisor((uint32_t)vh), max_seq, linear, scale, offset, early ? nullptr : status, early};
+  const size_t all = A.total + A.total_z;
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = overlapped((int)std::min<size_t>((all + 255) / 256, 148 * 8 * 4) + (early ? 1 : 0), 256, st, &at);
+  if (all >> 31) MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rope_vec_kernel<T, true>, (const T*)x, (T*)y, (T*)z, A));
+  else MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rope_vec_kernel<T, false>, (const T*)x, (T*)y, (T*)z, A));
   count_launch();
   return MLXR_OK;
 }
@@ -365,19 +426,24 @@ bool rope_qk_supported(const void* q, const void* k, const uint16_t* cos_t, cons
 }
 int launch_rope_qk(void* q, void* k, const uint16_t* cos_t, const uint16_t* sin_t, const int32_t* positions, size_t tokens, int q_heads, int kv_heads,
                    int head_dim, int max_seq, int offset, int dtype, int* status, cudaStream_t st) {
-  return dtype == MLXR_F16 ? launch_rope_vec<__half>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, st)
-                           : launch_rope_vec<__nv_bfloat16>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, st);
+  return dtype == MLXR_F16 ? launch_rope_vec<__half>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, nullptr, st)
+                           : launch_rope_vec<__nv_bfloat16>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, nullptr, st);
 }
 
 int launch_rope(const void* x, const uint16_t* cos_t, const uint16_t* sin_t,
                 const int32_t* positions, void* y, size_t tokens, int heads, int head_dim,
-                int max_seq, int mode, float scale, int offset, int dtype, int* status,
+                int max_seq, int mode, float scale, int offset, int dtype, int* status, bool* early,
                 cudaStream_t st) {
+  const bool want_early = early && *early;
+  if (early) *early = false;
   const size_t total = tokens * heads * (head_dim / 2);
   if (total == 0) return MLXR_OK;
-  if (rope_vec_ok(x, y, cos_t, sin_t, head_dim, dtype))
-    return dtype == MLXR_F16 ? launch_rope_vec<__half>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, st)
-                             : launch_rope_vec<__nv_bfloat16>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, st);
+  if (rope_vec_ok(x, y, cos_t, sin_t, head_dim, dtype)) {
+    if (early) *early = want_early;
+    int* word = want_early ? status : nullptr;
+    return dtype == MLXR_F16 ? launch_rope_vec<__half>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, word, st)
+                             : launch_rope_vec<__nv_bfloat16>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, word, st);
+  }
   size_t blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   MLXR_DISPATCH_DTYPE(dtype, T, {

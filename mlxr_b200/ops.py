@@ -234,7 +234,10 @@ def rope_apply(input: torch.Tensor, cos_table: torch.Tensor, sin_table: torch.Te
     check(lib.mlxr_rope_apply(_dev(input, "input"), _dev(cos_table, "cos_table"), _dev(sin_table, "sin_table"),
                               _dev(positions, "positions"), out.data_ptr(), batch, seq, heads, hd,
                               cos_table.shape[0], int(scaling_mode), scale_factor, position_offset,
-                              _dtype_code(input), 1 if check_positions else 0, _stream()))
+                              _dtype_code(input), 2 if check_positions else 0, _stream()))
+    if check_positions:
+        for t in (input, cos_table, sin_table, positions):      # the rotation may still run
+            t.record_stream(torch.cuda.current_stream())
     return out
 
 

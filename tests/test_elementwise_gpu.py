@@ -246,3 +246,58 @@ def test_in_place_and_behind_a_kernel_that_still_runs():
             mx.rope_apply(e, cos, sin, pos, inplace=True, check_positions=False)
             for got, ref in ((a, want[0]), (res, want[0]), (c, want[1]), (gate, want[1]), (e.reshape(M, N), want[2])):
                 assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_swiglu_of_many_elements_is_that_of_few(dtype):
+    """The vector kernel's quotient against the other kernel's IEEE division, every 16-bit gate (infinities and NaN among them):
+    up to 2^18 elements take the one, more take the other."""
+    import mlxr_b200 as mx
+    gate = torch.arange(-32768, 32768, dtype=torch.int32, device="cuda").to(torch.int16).view(dtype)
+    for scale in (1.0, 0.37, 250.0):
+        up = torch.full((65536,), scale, device="cuda").to(dtype)
+        few = mx.swiglu(gate, up)
+        many = mx.swiglu(gate.repeat(5), up.repeat(5)).reshape(5, -1)
+        nan = torch.isnan(few)
+        assert torch.equal(torch.isnan(many), nan.expand(5, -1))
+        assert torch.equal(many.view(torch.int16)[:, ~nan], few.view(torch.int16)[~nan].expand(5, -1))
+
+
+@pytest.mark.parametrize("tokens,heads,dim", [(1, 1, 8), (257, 3, 24), (1001, 5, 64), (3000, 2, 136)])
+def test_rope_of_odd_shapes_and_its_check(tokens, heads, dim):
+    """Quotients of the vector's number by any count of vectors per token and head, bit for bit; the check sees the last of many
+    positions, leaves that token alone and says so, and a call that was told so leaves nothing behind for the next."""
+    import mlxr_b200 as mx
+    cos, sin = mx.compute_rope_tables(512, dim, 10000.0, device=torch.device("cuda"))
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(tokens, heads, dim, device="cuda", generator=g).to(torch.float16)
+    pos = torch.randint(0, 512, (tokens,), device="cuda", generator=g, dtype=torch.int32)
+    c, s = cos[pos.long()].float()[:, None], sin[pos.long()].float()[:, None]
+    e, o = x[..., 0::2].float(), x[..., 1::2].float()
+    want = torch.stack([e * c - o * s, o * c + e * s], -1).reshape(x.shape).half()
+    assert torch.equal(mx.rope_apply(x, cos, sin, pos), want)
+    bad = pos.clone()
+    bad[-1] = 512
+    y = x.clone()
+    with pytest.raises(mx._capi.MlxrError):
+        mx.rope_apply(y, cos, sin, bad, inplace=True)
+    torch.cuda.synchronize()
+    assert torch.equal(y[:-1], want[:-1]) and torch.equal(y[-1], x[-1])
+    assert torch.equal(mx.rope_apply(x, cos, sin, pos), want)
+
+
+def test_checked_rope_behind_a_long_queue():
+    """Positions written by a kernel far back in the stream's queue: the call waits for them however long that takes."""
+    import mlxr_b200 as mx
+    cos, sin = mx.compute_rope_tables(64, 64, 10000.0, device=torch.device("cuda"))
+    x = torch.randn(64, 8, 64, device="cuda").half()
+    pos = torch.full((64,), 99, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)         # about 10 ms
+    pos.copy_(torch.arange(64, dtype=torch.int32, device="cuda"))
+    good = mx.rope_apply(x, cos, sin, pos)
+    assert torch.equal(good, mx.rope_apply(x, cos, sin, torch.arange(64, dtype=torch.int32, device="cuda")))
+    torch.cuda._sleep(20_000_000)
+    pos.fill_(99)
+    with pytest.raises(mx._capi.MlxrError):
+        mx.rope_apply(x, cos, sin, pos)
