@@ -126,7 +126,6 @@ struct Shared {
   int todo_tile[2], todo_parts[2];
   int epi_fail;
   int bad;                      // kSplit: some sum was not finite
-  float nf4[16];
 };
 
 // first unit of CTA c, and the CTA that owns unit u, when U units are dealt to G CTAs
@@ -167,10 +166,11 @@ template <int QT, int NPAD> struct Rings {
   static constexpr int kXTile = NPAD * kBK * 2;                             // one k-block of X
   static constexpr int kXUnit = 4 * kXTile;                                 // the four k-blocks of a unit
   static constexpr int kXStages = NPAD == 64 ? 2 : 4;                // even: see Shared::full_a
-  static constexpr int kFree = kSmemMax - kXStages * kXUnit - (int)sizeof(Shared) - 1024;
+  static constexpr int kTable = QT == MLXR_NF4 ? PairLevels::kBytes : 0;
+  static constexpr int kFree = kSmemMax - kXStages * kXUnit - kTable - (int)sizeof(Shared) - 1024;
   // a multiple of the number of groups, so that a stage's barrier is always waited on by one group
   static constexpr int kRawStages = kFree / kRawBytes >= 2 * kGroups ? 2 * kGroups : kGroups;
-  static constexpr size_t kBytes = (size_t)kXStages * kXUnit + (size_t)kRawStages * kRawBytes;
+  static constexpr size_t kBytes = (size_t)kXStages * kXUnit + (size_t)kRawStages * kRawBytes + kTable;
   // tensor-memory columns: accumulators [buffer][issuer][NPAD], then the converted weights; the widest
   // batch has no room for a second buffer
   static constexpr int kBufs = NPAD == 64 ? 1 : 2;
@@ -205,7 +205,8 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
   uint8_t* smem = smem_raw + pad;
   uint8_t* xring = smem;
   uint8_t* rawring = xring + (size_t)kXStages * kXUnit;
-  Shared* sh = reinterpret_cast<Shared*>(rawring + (size_t)kRawStages * kRawBytes);
+  [[maybe_unused]] uint8_t* table = rawring + (size_t)kRawStages * kRawBytes;      // NF4
+  Shared* sh = reinterpret_cast<Shared*>(table + R::kTable);
   volatile int* dead = &sh->dead;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int G = gridDim.x, cta = blockIdx.x;
@@ -265,7 +266,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (QT == MLXR_NF4 && tid >= 32 && tid < 48) sh->nf4[tid - 32] = kNF4[tid - 32];
+  if constexpr (QT == MLXR_NF4) PairLevels::fill(table, tid, kThreads);
   if (warp == kWarpMma) tmem_alloc(smem_u32(&sh->tmem_base), R::kCols);
   tc_fence_before();
   __syncthreads();
@@ -288,6 +289,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     const int row_off = (kSplitRows ? mat_off + (local & 1) * (mrows / 2) + (local >> 1) : mat_off + local) * Geo<QT>::kStage;
     const uint32_t a_col = tmem + R::kA0 + (uint32_t)(g * kSlots * 2 * kBlockCols) + ((uint32_t)((warp & 3) * 32) << 16);
     int r = g;
+    [[maybe_unused]] const PairLevels levels(table, lane);
     uint32_t rpar = 0, use = 0;         // use: how often this group's slots have been filled
     for (int i = g; i < nunits; i += kGroups) {
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->raw_full[r]), rpar, dead))) break;   // warp-uniform
@@ -308,7 +310,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
           tc_fence_after();
         }
         const uint32_t col = a_col + (MODE == kSplit ? q * 2 * kBlockCols : kb * kBlockCols);
-        convert64<QT, BF, MODE>(row, KB, sh->nf4, [&](auto H, const uint32_t (&a)[16], const uint32_t (&b)[16]) {
+        convert64<QT, BF, MODE>(row, KB, levels, [&](auto H, const uint32_t (&a)[16], const uint32_t (&b)[16]) {
           tmem_st16(col + 16 * decltype(H)::value, a);
           if constexpr (MODE == kSplit) tmem_st16(col + kBlockCols + 16 * decltype(H)::value, b);
         });

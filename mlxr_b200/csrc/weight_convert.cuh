@@ -161,15 +161,39 @@ template <int BF, int MODE> __device__ __forceinline__ void nibbles8(uint32_t v,
   else put(dequant8_bf16(v, __uint_as_float(c.s), __uint_as_float(c.m)), out);
 }
 
+// NF4 levels of the codes in byte J of v, from tables in shared memory.  Levels: the 16 levels, one word per bank, so that lookups
+// never conflict.  PairLevels: the two levels of every byte, once for each thread of a half warp, whose eight bytes lie
+// in banks of their own: half the address arithmetic and loads per weight.
+struct Levels {
+  const float* t;
+  template <int J> __device__ __forceinline__ float2 pair(uint32_t v) const { return make_float2(t[(v >> (8 * J)) & 15u], t[(v >> (8 * J + 4)) & 15u]); }
+};
+struct PairLevels {
+  static constexpr int kBytes = 256 * 16 * 8;
+  uint32_t t;                 // shared address of this thread's copy
+  __device__ __forceinline__ PairLevels(const void* table, int lane) : t(tc::smem_u32(table) + 8u * (uint32_t)(lane & 15)) {}
+  template <int J> __device__ __forceinline__ float2 pair(uint32_t v) const {
+    float2 r;
+    asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "r"(__byte_perm(v, 0u, 0x4440u | J) * 128u + t));
+    return r;
+  }
+  // by all threads of the CTA; a barrier must follow
+  static __device__ __forceinline__ void fill(void* table, int tid, int threads) {
+    for (int i = tid; i < kBytes / 16; i += threads) {
+      const float lo = kNF4[(i >> 3) & 15], hi = kNF4[i >> 7];
+      reinterpret_cast<float4*>(table)[i] = make_float4(lo, hi, lo, hi);
+    }
+  }
+};
+
 // Weights 64 kb .. 64 kb + 63 of the unit at `row` (shared memory): out(Int<0>, hi, lo) gets the first 32,
-// out(Int<1>, hi, lo) the others (lo only for kSplit).  nf4: the 16 codebook levels in shared memory (one word per
-// bank: lookups never conflict).  KB is int or tc::Int.  With a run-time kb the body stays at a few hundred
+// out(Int<1>, hi, lo) the others (lo only for kSplit).  nf4: Levels or PairLevels.  KB is int or tc::Int.  With a run-time kb the body stays at a few hundred
 // instructions that every producer warp shares; unrolled over a unit of the long conversions (kSplit), or
 // specialised per group, the warps of a scheduler fetch more code than its instruction cache holds and
 // wait for it (the largest stall by far: canonical Q4_K [16, 4096] x [37888, 4096]^T 90.9 us unrolled, 52.5
 // us rolled).  The short conversions fit unrolled and are faster so (Q4_K, same size: 27.8 rolled, 24.7).
-template <int QT, int BF, int MODE, typename KB, typename F>
-__device__ __forceinline__ void convert64(const uint8_t* row, KB KBV, const float* nf4, F&& out) {
+template <int QT, int BF, int MODE, typename KB, typename L, typename F>
+__device__ __forceinline__ void convert64(const uint8_t* row, KB KBV, const L& nf4, F&& out) {
   const int kb = block_of(KBV);
   uint32_t a[16], b[16];
   if constexpr (QT == MLXR_Q4_K) {
@@ -242,11 +266,9 @@ __device__ __forceinline__ void convert64(const uint8_t* row, KB KBV, const floa
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const uint32_t v = sh ? w[4 * s + i + 1] : __funnelshift_r(w[4 * s + i], w[4 * s + i + 1], 16);
+        const float2 l[4] = {nf4.template pair<0>(v), nf4.template pair<1>(v), nf4.template pair<2>(v), nf4.template pair<3>(v)};
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const float e = nf4[(v >> (8 * j)) & 15u], o = nf4[(v >> (8 * j + 4)) & 15u];
-          emit<BF, MODE>(e * am, o * am, a[4 * i + j], b[4 * i + j]);
-        }
+        for (int j = 0; j < 4; j++) emit<BF, MODE>(l[j].x * am, l[j].y * am, a[4 * i + j], b[4 * i + j]);
       }
       out(S, a, b);
     };

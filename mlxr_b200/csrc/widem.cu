@@ -216,7 +216,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       if constexpr (kSplitRows) row += (136 * sb + ((local & 1) ? P.odd_shift : 0)) & 8;
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty[g * kSlots + q]), (uint32_t)((i >> 1) & 1) ^ 1u, dead))) break;
       tc_fence_after();
-      convert64<QT, BF, kRound>(row, g, sh->nf4, [&](auto H, const uint32_t (&a)[16], const uint32_t (&)[16]) {
+      convert64<QT, BF, kRound>(row, g, Levels{sh->nf4}, [&](auto H, const uint32_t (&a)[16], const uint32_t (&)[16]) {
         tmem_st16(col + q * kSlotCols + 16 * decltype(H)::value, a);
       });
       tmem_wait_st();
