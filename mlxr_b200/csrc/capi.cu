@@ -210,12 +210,12 @@ static int run_tc(TcPath path, const WidePlan& wide, const DensePlan& dense, con
 // Small matrices of a few tokens: a kernel without copies into shared memory, barriers and partial sums has its result
 // before the others have set themselves up.  bf16, weights from HBM, in us, gemv_rows_kernel / the kernel that larger ones take:
 //   Q8_0  one token 2048 x 2048 5.0 / 5.6, 3000 x 2048 5.8 / 6.0, 4096 x 2048 6.7 / 6.2; two 4096 x 1024 5.2 / 5.9, 2048 x 2048 6.4 / 6.3,
-//         1024 x 4096 7.8 / 7.2; 3, 6 and 8 tokens of 1000 x 1024 4.3, 6.3, 7.2 / 7.2, three of 1024 x 2048 6.2 / 6.3
+//         1024 x 4096 7.8 / 7.2 (three tokens and more are gemv_tokens.cu's: 8 tokens of 1000 x 1024 3.4 there)
 //   NF4   3 and 6 tokens of 1000 x 1024 4.6, 6.9 / 7.4; three of 4096 x 1024 6.5 / 7.6, 2048 x 2048 6.7 / 6.8; four of 2048 x 2048 7.5 / 6.9
 static bool rows_kernel_first(int qt, int M, int N, int K, int dtype, const void* x, const void* w) {
   if (dtype == MLXR_F32 || !gemv_rows_supported(qt, M, K, x, w)) return false;
   const long long size = (long long)N * K;
-  if (qt == MLXR_Q8_0) return M == 1 ? size <= 3 << 21 : M == 2 ? size <= 1 << 22 && K <= 2048 : M * size <= 6 << 20;
+  if (qt == MLXR_Q8_0) return M == 1 ? size <= 3 << 21 : M == 2 && size <= 1 << 22 && K <= 2048;
   return qt == MLXR_NF4 && M >= 3 && (M * size <= 6 << 20 || (M <= 4 && M * K <= 6144 && size <= 1 << 22));
 }
 
@@ -229,6 +229,11 @@ static int run_linear(const void* x, const void* w, const void* bias, void* y, i
     L.w[0] = w; L.rows[0] = N; L.nmat = 1; L.K = K; L.x = x; L.y[0] = y; L.bias[0] = bias;
     return launch_stream_gemv(L, M, dtype, ws->status, st);
   }
+  if (M > 0 && N > 0 && gemv_tokens_supported(qt, M, K, N, kTokensPlain, dtype, x, &w, 1)) {
+    Workspace* ws = nullptr;
+    if (int r = get_workspace(st, 0, &ws)) return r;
+    return launch_gemv_tokens(x, &w, &N, 1, kTokensPlain, bias, &y, M, K, qt, dtype, ws->status, st);
+  }
   if (M > 0 && N > 0 && rows_kernel_first(qt, M, N, K, dtype, x, w)) return launch_gemv_rows(x, w, bias, y, M, N, K, qt, dtype, st);
   if (M > 0 && N > 0 && gemv_supported(qt, M, K, N, dtype, &w, 1)) {
     Workspace* ws = nullptr;
@@ -238,12 +243,11 @@ static int run_linear(const void* x, const void* w, const void* bias, void* y, i
     L.w[0] = w; L.rows[0] = N; L.nmat = 1; L.K = K; L.x = x; L.y[0] = y; L.bias[0] = bias;
     return launch_gemv(L, M, qt, dtype, ws->status, st);
   }
-  // Canonical Q4_K, and NF4 rows that do not start on 16 bytes, have no kernel of their own for one or two tokens (one token
-  // of a small canonical matrix is the generic kernel's: 1000 x 1024 5.2 us there, 7.1 here; 1024 x 2048 8.7, 6.6).  The
-  // one NF4 has looks every weight up once per token; from 2^24 weights on the small-batch kernel, which converts
+  // Canonical Q4_K (with more activations than gemv_tokens.cu takes), and NF4 rows that do not start on 16 bytes, have no other
+  // kernel for one or two tokens.  The one NF4 has looks every weight up once per token; from 2^24 weights on the small-batch kernel, which converts
   // once, is the faster one for two (4096 x 4096: 14.5 us there, 11.6 here; 14336 x 4096: 34.4, 27.9; 4096 x 14336:
   // 40.5, 26.7; 4096 x 2048: 7.6, 8.5).
-  const bool small_only = (qt == MLXR_GGML_Q4_K && (M > 1 || (long long)N * K > 5 << 18)) ||
+  const bool small_only = qt == MLXR_GGML_Q4_K ||
                           (qt == MLXR_NF4 && (!gemv_rows_supported(qt, M, K, x, w) || (M == 2 && (long long)N * K >= (1 << 24))));
   if ((M >= 3 || (M > 0 && small_only)) && N > 0) {
     TcPath path;
@@ -584,8 +588,10 @@ static int mlp_block_impl(const void* x, const void* norm_weight, const void* w_
     if (int r = launch_rmsnorm(x, norm_weight, nullptr, nbuf, M, hidden, eps, dtype, st)) return r;
     n = nbuf;
   }
-  if (small) {
-    if (int r = run_tc(path, wide, dense, n, w_gate, w_up, nullptr, gbuf, M, inter, hidden, qt, dtype, st)) return r;
+  const bool tokens = M >= 3 && gemv_tokens_supported(qt, M, hidden, 2 * inter, kTokensGateUp, dtype, n, wgu, 2);
+  if (tokens || small) {
+    if (tokens) { if (int r = launch_gemv_tokens(n, wgu, &inter, 2, kTokensGateUp, nullptr, &gbuf, M, hidden, qt, dtype, ws->status, st)) return r; }
+    else if (int r = run_tc(path, wide, dense, n, w_gate, w_up, nullptr, gbuf, M, inter, hidden, qt, dtype, st)) return r;
     if (!y_f32) return run_linear(gbuf, w_down, nullptr, y, M, hidden, inter, qt, dtype, st);
     if (int r = run_linear(gbuf, w_down, nullptr, nbuf, M, hidden, inter, qt, dtype, st)) return r;
     return launch_cast_to_f32(nbuf, (float*)y, (size_t)M * hidden, dtype, st);
@@ -745,7 +751,9 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
   const int tiles = (rows[0] + 127) / 128 + 2 * ((rows[1] + 127) / 128);
   bool stack = (M >= 3 || qt == MLXR_NF4) && tiles <= kSyncWords - kTileCounters;
   for (int i = 0; i < 3; i++) stack = stack && smallm_supported(qt, M, rows[i], hidden, dtype, n, wqkv[i]);
-  if (stack) {
+  if (M >= 3 && rows[0] % 4 == 0 && rows[1] % 4 == 0 && gemv_tokens_supported(qt, M, hidden, rows[0] + 2 * rows[1], kTokensStacked, dtype, n, wqkv, 3)) {
+    if (int r = launch_gemv_tokens(n, wqkv, rows, 3, kTokensStacked, nullptr, outs, M, hidden, qt, dtype, ws->status, st)) return r;
+  } else if (stack) {
     // Up to 64 tokens: the three projections in one launch of the small-batch kernel, which fills the SMs better than
     // three and meets once.  With one RoPE launch for q and k three launches in all, not six: hidden size 4096, 8
     // tokens 31 -> 12.6 us; 8192, 64 tokens 49 -> 31; 1280, 36 tokens 27 -> 10.6.

@@ -270,4 +270,16 @@ __device__ __forceinline__ void dequant_unit(const uint8_t* __restrict__ row, in
              return MLXR_ERR_UNSUPPORTED;                                           \
   }
 
+// A row's product with the float32 weights, by a warp: for the results of kernels with other arithmetic that are not finite
+template <int QT, typename T> __device__ __forceinline__ float exact_sum(const uint8_t* row, const T* x, int K, int lane) {
+  float acc = 0.0f;
+  for (int u = lane; u < K / 32; u += 32) {
+    float w[32];
+    dequant_unit<QT>(row, u, w);
+#pragma unroll
+    for (int i = 0; i < 32; i++) acc = fmaf(Act<T>::to_f(x[32 * u + i]), w[i], acc);
+  }
+  return warp_sum(acc);
+}
+
 }  // namespace mlxr

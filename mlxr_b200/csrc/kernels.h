@@ -126,6 +126,13 @@ int launch_gemv(const DecodeLinear& L, int M, int qt, int dtype, int* status, cu
 bool stream_gemv_supported(int qt, int M, int K, int rows, const void* const* w, int nmat);
 int launch_stream_gemv(const DecodeLinear& L, int M, int dtype, int* status, cudaStream_t st);
 
+// ---- up to eight tokens of 16-bit activations (gemv_tokens.cu): canonical Q4_K from one token on, Q8_0, Q4_K, Q4_0 from three ----
+// rows: weight rows in all.  w[0 .. nmat): one matrix, gate and up (y[0] = SiLU(X gate^T) * (X up^T), rows[0] columns), or stacked
+enum TokensForm { kTokensPlain = 0, kTokensGateUp = 1, kTokensStacked = 2 };
+bool gemv_tokens_supported(int qt, int M, int K, int rows, int form, int dtype, const void* x, const void* const* w, int nmat);
+int launch_gemv_tokens(const void* x, const void* const* w, const int* rows, int nmat, int form, const void* bias, void* const* y, int M, int K, int qt, int dtype,
+                       int* status, cudaStream_t st);
+
 // ---- small-batch tensor-core linear (smallm.cu): Q4_K, Q4_0, Q8_0, NF4, canonical Q4_K; 1 <= M <= 64, fp16 / bf16 ----
 bool smallm_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w);
 void smallm_partition(long long units, int ctas, int cta, long long unit, long long* begin, long long* end, int* owner);

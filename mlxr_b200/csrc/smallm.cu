@@ -146,16 +146,6 @@ __device__ __forceinline__ float swish_fast(float x) {
 // meets residuals of the other sign: their sum is NaN where the float32 product is finite or an infinity.  Sums that
 // are not finite are computed again from the float32 weights, a warp per sum; such values are rare, and a
 // row of them takes about as long as the generic kernel's.
-template <int QT, typename T> __device__ __forceinline__ float exact_sum(const uint8_t* row, const T* x, int K, int lane) {
-  float acc = 0.0f;
-  for (int u = lane; u < K / 32; u += 32) {
-    float w[32];
-    dequant_unit<QT>(row, u, w);
-#pragma unroll
-    for (int i = 0; i < 32; i++) acc = fmaf(Act<T>::to_f(x[32 * u + i]), w[i], acc);
-  }
-  return warp_sum(acc);
-}
 // Added to by every sum that is to be stored: stays 0 as long as all are finite
 __device__ __forceinline__ void note_bad(float& t, float v) { t = fmaf(v, 0.0f, t); }
 

@@ -1,0 +1,130 @@
+"""Linears of up to eight tokens (csrc/gemv_tokens.cu) through the C ABI, against float64 products of the dequantized weights.
+
+Sizes: fewer rows than SMs, row counts that are no multiple of the granule of four, more warps than work units, an odd number
+of 256-weight segments, every token count, rows that make the warps meet more than once, one ring stage.
+
+Bounds (2-norm, relative).  Result: rounded once to p significant bits, at most 2^-8 (bf16) and 2^-11 (fp16).  Products and sums
+are float32: 1e-6.  Q4_K's reference is the shader's half arithmetic, two roundings of at most 2^-11 per weight that the kernel does
+not make: 2^-10."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import make_acts, make_weights
+
+pytestmark = pytest.mark.gpu
+DT = {"f16": torch.float16, "bf16": torch.bfloat16}
+RESULT = {"f16": 2.0 ** -11, "bf16": 2.0 ** -8}
+WEIGHT = {0: 1e-6, 2: 1e-6, 3: 2.0 ** -10, 33: 1e-6}
+
+
+def _status():
+    import mlxr_b200 as mx
+    st = torch.zeros(1, dtype=torch.int32)
+    mx._capi.check(mx._capi.lib.mlxr_stream_status(torch.cuda.current_stream().cuda_stream, st.data_ptr()))
+    return int(st[0])
+
+
+def _weights(N, K, qt, seed):
+    """Packed weights on the device: quantized, or for canonical Q4_K random blocks with scales of ordinary size."""
+    from mlxr_b200.quantize import quantize
+    if qt != 33:
+        return torch.from_numpy(quantize(make_weights(N, K, seed), qt)).cuda()
+    rng = np.random.Generator(np.random.PCG64(seed))
+    b = rng.integers(0, 256, (N * K // 256, 144), dtype=np.uint8)
+    b[:, :4] = rng.uniform(1e-4, 3e-4, (N * K // 256, 2)).astype(np.float16).view(np.uint8)
+    return torch.from_numpy(b.reshape(-1)).cuda()
+
+
+def _dense(w, N, K, qt):
+    import mlxr_b200 as mx
+    return mx.dequantize(w, N, K, mx.QuantType(qt), torch.float32).double()
+
+
+def _linear(x, w, N, K, qt, b=None):
+    import mlxr_b200 as mx
+    return mx.q_gemm_dequant(x, w, x.shape[0], N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt), b)
+
+
+def _check(y, want, dt, qt):
+    assert float((y.double() - want).norm() / want.norm()) <= RESULT[dt] + WEIGHT[qt]
+    # no result may be wrong by itself: the largest are below 6 rms
+    assert float((y.double() - want).abs().max() / want.square().mean().sqrt()) <= 6 * (RESULT[dt] + WEIGHT[qt]) + 1e-3
+
+
+@pytest.mark.parametrize("qt,dt", [(33, "f16"), (33, "bf16"), (2, "f16"), (2, "bf16"), (0, "bf16"), (3, "bf16")])
+@pytest.mark.parametrize("M,N,K", [(3, 4, 256), (4, 67, 768), (5, 593, 512), (6, 1000, 1280), (7, 2369, 256), (8, 130, 2048), (3, 40, 16384)])
+def test_linear(qt, dt, M, N, K):
+    w = _weights(N, K, qt, 7 + N)
+    x = make_acts(M, K, 8 + N, DT[dt])[0].cuda()
+    b = make_acts(1, N, 9, DT[dt])[0][0].contiguous().cuda() if N % 2 else None
+    y = _linear(x, w, N, K, qt, b)
+    assert torch.equal(y, _linear(x, w, N, K, qt, b)) and _status() == 0
+    _check(y, x.double() @ _dense(w, N, K, qt).T + (b.double() if b is not None else 0), dt, qt)
+
+
+@pytest.mark.parametrize("qt,M,N,K", [(33, 1, 5, 256), (33, 2, 4097, 1792), (33, 1, 300, 32768), (33, 8, 41001, 256), (2, 3, 45003, 256), (0, 3, 33001, 256), (33, 8, 700, 6144)])
+def test_few_and_many_rows(qt, M, N, K):
+    w = _weights(N, K, qt, 3)
+    x = make_acts(M, K, 4, torch.bfloat16)[0].cuda()
+    y = _linear(x, w, N, K, qt)
+    assert _status() == 0
+    _check(y, x.double() @ _dense(w, N, K, qt).T, "bf16", qt)
+
+
+@pytest.mark.parametrize("qt,dt", [(0, "f16"), (0, "bf16"), (2, "f16"), (2, "bf16"), (3, "f16"), (3, "bf16")])
+@pytest.mark.parametrize("M,H,QH,KH,D", [(3, 512, 3, 1, 64), (8, 1280, 10, 2, 128)])
+def test_stacked_is_the_three_linears(qt, dt, M, H, QH, KH, D):
+    """q, k and v of one launch, without RMSNorm and with positions at zero (a rotation by nothing)."""
+    import mlxr_b200 as mx
+    w = [_weights(n * D, H, qt, i) for i, n in enumerate((QH, KH, KH))]
+    x = make_acts(M, H, 5, DT[dt])[0].cuda()
+    cos, sin = mx.compute_rope_tables(4, D, 10000.0, device=torch.device("cuda"))
+    out = mx.qkv_rope(x, None, *w, cos, sin, torch.zeros(M, dtype=torch.int32, device="cuda"), QH, KH, D, mx.QuantType(qt), 1e-5)
+    assert _status() == 0
+    for y, p, n in zip(out, w, (QH, KH, KH)):
+        _check(y.reshape(M, -1), x.double() @ _dense(p, n * D, H, qt).T, dt, qt)
+
+
+@pytest.mark.parametrize("qt", [0, 2, 3])
+@pytest.mark.parametrize("M,H,I", [(3, 256, 1280), (8, 512, 1024), (5, 768, 2304)])
+def test_gate_up(qt, M, H, I):
+    """The block without a norm weight: h and y are rounded to bf16, h from rounded gate and up."""
+    import mlxr_b200 as mx
+    wg, wu, wd = _weights(I, H, qt, 1), _weights(I, H, qt, 2), _weights(H, I, qt, 3)
+    x = make_acts(M, H, 4, torch.bfloat16)[0].cuda()
+    y = mx.mlp_block(x, None, wg, wu, wd, I, mx.QuantType(qt), 1e-5)
+    assert _status() == 0
+    g, u = (x.double() @ _dense(w, I, H, qt).T for w in (wg, wu))
+    h = torch.nn.functional.silu(g.bfloat16().double()) * u.bfloat16().double()
+    want = h.bfloat16().double() @ _dense(wd, H, I, qt).T
+    # rounding of g, u, h and y: each at most 2^-8, independent
+    assert float((y.double() - want).norm() / want.norm()) <= 2 * RESULT["bf16"] + WEIGHT[qt]
+
+
+@pytest.mark.parametrize("qt", [2, 33])
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+def test_values_that_are_not_finite(qt, dt):
+    """An infinite activation: every result of its token is what the float32 weights give (a canonical weight of code 0 is its
+    offset), the other tokens' are what they are without it.  A NaN reaches its token only."""
+    M, N, K = 4, 300, 512
+    w = _weights(N, K, qt, 1)
+    x = make_acts(M, K, 2, DT[dt])[0].cuda()
+    clean = _linear(x, w, N, K, qt)
+    x[1, 77], x[2, 300] = float("inf"), float("nan")
+    y = _linear(x, w, N, K, qt)
+    d = _dense(w, N, K, qt).float()
+    want = x.float()[1, 77] * d[:, 77]
+    assert torch.equal(torch.isnan(y[1]), torch.isnan(want))
+    assert torch.equal(y[1].float()[~torch.isnan(want)], want[~torch.isnan(want)])
+    assert torch.isnan(y[2]).all() and torch.equal(y[0], clean[0]) and torch.equal(y[3], clean[3])
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -100, 2.0 ** 100])
+def test_range_of_bf16(scale):
+    """Activations of any magnitude, segments of one row apart by 2^12."""
+    N, K = 200, 1024
+    w = _weights(N, K, 33, 1)
+    x = (make_acts(3, K, 2, torch.float32)[0] * scale).to(torch.bfloat16).cuda()
+    x[:, 512:] *= 2.0 ** -12
+    _check(_linear(x, w, N, K, 33), x.double() @ _dense(w, N, K, 33).T, "bf16", 33)
