@@ -209,13 +209,13 @@ static int run_tc(TcPath path, const WidePlan& wide, const DensePlan& dense, con
 // split-K partial sums; intermediates of the fused entry points start after them.
 // Small matrices of a few tokens: a kernel without copies into shared memory, barriers and partial sums has its result
 // before the others have set themselves up.  bf16, weights from HBM, in us, gemv_rows_kernel / the kernel that larger ones take:
-//   Q8_0  one token 2048 x 2048 5.0 / 5.6, 3000 x 2048 5.8 / 6.0, 4096 x 2048 6.7 / 6.2; two 4096 x 1024 5.2 / 5.9, 2048 x 2048 6.4 / 6.3,
-//         1024 x 4096 7.8 / 7.2 (three tokens and more are gemv_tokens.cu's: 8 tokens of 1000 x 1024 3.4 there)
+//   Q8_0  two tokens of 1000 x 1024 4.1 / 4.6, 2048 x 1024 5.1 / 4.6; one token is gemv.cu's (1000 x 1024 4.1 / 3.5, 3000 x 2048 7.1 /
+//         4.4), three and more gemv_tokens.cu's (8 tokens of 1000 x 1024 7.2 / 3.4)
 //   NF4   3 and 6 tokens of 1000 x 1024 4.6, 6.9 / 7.4; three of 4096 x 1024 6.5 / 7.6, 2048 x 2048 6.7 / 6.8; four of 2048 x 2048 7.5 / 6.9
 static bool rows_kernel_first(int qt, int M, int N, int K, int dtype, const void* x, const void* w) {
   if (dtype == MLXR_F32 || !gemv_rows_supported(qt, M, K, x, w)) return false;
   const long long size = (long long)N * K;
-  if (qt == MLXR_Q8_0) return M == 1 ? size <= 3 << 21 : M == 2 && size <= 1 << 22 && K <= 2048;
+  if (qt == MLXR_Q8_0) return M == 2 && size <= 1 << 20;
   return qt == MLXR_NF4 && M >= 3 && (M * size <= 6 << 20 || (M <= 4 && M * K <= 6144 && size <= 1 << 22));
 }
 

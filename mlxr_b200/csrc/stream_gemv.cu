@@ -3,9 +3,8 @@
 //
 // Roofline: HBM, but at these sizes a launch's fixed part decides: nothing is set up (no barriers, no copies into shared
 // memory), a CTA takes half an SM, so the next launch's CTAs are in place and have requested their first
-// weights when this one ends, and a tile's K range is split over the warps.  [1, 1024] x [1000, 1024]^T 2.7 us
-// against 4.1 with the kernel of gemv.cu, 4096 x 2048 3.4 against 4.9, 4096 x 4096 5.1 against 5.6; on larger matrices
-// the meeting of the warps after every 16 rows costs more than that (11008 x 4096: 10.4 against 9.1).
+// weights when this one ends, and a tile's K range is split over the warps.  [1, 1024] x [1000, 1024]^T 2.8 us against 3.3 with
+// the kernel of gemv.cu; on larger matrices the meeting of the warps after every 16 rows costs more than that.
 // The next tiles' rows are requested into L2 ahead (a prefetch per 128-byte line).
 // Arithmetic is that of gemv.cu: activations as 16-bit fixed point per 256 elements, split in a high and a low signed
 // byte; raw nibbles multiplied as unsigned bytes; (scale, min) pairs of the Q4_K super-block in the MMA
@@ -361,13 +360,13 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) stream_gemv_kernel(const
 
 using namespace sgemv;
 
-// Where this kernel is the faster one of the two that take Q4_K (bf16, weights from HBM, this / gemv.cu in us): one
-// token of 4096 x 4096 5.1 / 5.6, 8192 x 1024 4.2 / 4.7, but 16384 x 1024 7.0 / 5.2, 1024 x 8192 7.0 / 6.1; two
-// tokens of 4096 x 2048 4.4 / 6.0, 2048 x 4096 6.6 / 6.6; q / k / v of hidden size 2048 (3072 rows) 4.0 / 5.6 and
-// 3072 (5120 rows) 7.2 / 6.4.
+// Where this kernel is the faster one of the two that take Q4_K (bf16, this / gemv.cu in us): one token of 1000 x 1024 2.8 / 3.3,
+// 2048 x 2048 3.3 / 3.4, 4096 x 2048 3.4 / 3.6, but 8192 x 1024 4.1 / 3.5, 2048 x 4096 4.7 / 3.7, 4096 x 4096 5.0 / 4.4; two tokens of
+// 2048 x 2048 4.2 / 5.0, 4096 x 2048 4.4 / 5.1, 8192 x 1024 4.9 / 5.0, but 2048 x 4096 6.4 / 5.4; q / k / v of hidden size
+// 2048 (3072 rows), one and two tokens 4.2 / 4.3 and 5.4 / 6.1.
 bool stream_gemv_supported(int qt, int M, int K, int rows, const void* const* w, int nmat) {
-  if (qt != MLXR_Q4_K || M < 1 || M > 2 || K < 256 || K % 256 != 0 || K > 4096 || rows < 1 || rows > 8192) return false;
-  if ((long long)rows * K > (M == 1 && nmat == 1 ? 1 << 24 : 1 << 23)) return false;
+  if (qt != MLXR_Q4_K || M < 1 || M > 2 || K < 256 || K % 256 != 0 || K > 2048 || rows < 1 || rows > 4096 * M) return false;
+  if ((long long)rows * K > 1 << 23) return false;
   for (int i = 0; i < nmat; i++)
     if (((uintptr_t)w[i]) & 15u) return false;
   return true;

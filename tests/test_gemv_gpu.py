@@ -207,9 +207,10 @@ def test_float32_activations_of_one_segment(oracle, M):
     assert float((y.double() - want).norm() / want.norm()) <= RESULT["f32"]
 
 
-@pytest.mark.parametrize("qt,dt,M,N,K", [(3, "bf16", 1, 4096, 4096), (3, "bf16", 1, 4097, 4096), (3, "f16", 1, 8192, 256), (3, "f16", 1, 8193, 256),
+@pytest.mark.parametrize("qt,dt,M,N,K", [(3, "bf16", 1, 4096, 2048), (3, "f16", 1, 4097, 2048), (3, "bf16", 1, 300, 2304), (3, "f16", 2, 8192, 1024), (3, "bf16", 2, 8193, 1024), (3, "f32", 2, 4097, 2048),
+                                         (3, "bf16", 1, 4096, 4096), (3, "bf16", 1, 4097, 4096), (3, "f16", 1, 8192, 256), (3, "f16", 1, 8193, 256),
                                          (3, "bf16", 2, 2048, 4096), (3, "bf16", 2, 2049, 4096), (3, "f32", 2, 77, 4096), (3, "f32", 1, 77, 4352),
-                                         (2, "bf16", 1, 3072, 2048), (2, "bf16", 1, 3073, 2048), (2, "f16", 2, 2048, 2048), (2, "f16", 2, 2049, 2048),
+                                         (2, "f16", 1, 1000, 256), (2, "bf16", 2, 1024, 1024), (2, "f16", 2, 1025, 1024), (2, "bf16", 1, 3072, 2048), (2, "bf16", 1, 3073, 2048), (2, "f16", 2, 2048, 2048), (2, "f16", 2, 2049, 2048),
                                          (2, "bf16", 6, 1024, 1024), (2, "bf16", 6, 1025, 1024), (16, "bf16", 4, 2730, 1536), (16, "bf16", 4, 2731, 1536),
                                          (16, "f16", 8, 1536, 512), (16, "f16", 8, 1537, 512), (33, "bf16", 1, 1280, 1024), (33, "bf16", 1, 1281, 1024)])
 def test_borders_of_the_small_matrices(oracle, qt, dt, M, N, K):
