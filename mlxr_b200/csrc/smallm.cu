@@ -525,9 +525,10 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
   }
   if (tid == 0 && sh->dead) atomicExch(P.status, MLXR_ERR_TIMEOUT);
   // ===== shared tiles of which this CTA delivered the last part: all warps, four weight rows per lane, parts
-  // added in CTA order.  Bound by L2 latency: sixteen 16-byte loads in flight per lane, as four batch rows of
-  // four parts or, up to one batch row per warp, one of sixteen (with four, a matrix of 2368 rows, shared by
-  // eight CTAs a tile, took 4 us longer at batch 64) =====
+  // added in CTA order.  Bound by L2 latency and by fetching this code, which runs once: a warp has as many batch rows in
+  // work at a time as the padded batch gives it, with four parts of each in flight (eight of a single row).  With sixteen
+  // loads in flight at any batch, in two forms, 32 tokens of Q8_0, 4096 x 11008, took 47.6 us instead of 45.9; with eight at
+  // batch 64, 4402 x 6144 canonical Q4_K, 18.2 instead of 17.8 =====
   const int ntodo = sh->dead ? 0 : sh->ntodo;
   constexpr int kW = kThreads / 32;
   for (int k = 0; k < ntodo; k++) {
@@ -554,7 +555,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
       }
     };
     auto sum = [&](auto RC, int m0) {
-      constexpr int R = decltype(RC)::value, Z = 16 / R;               // batch rows m0, m0 + kW, .. and parts at a time
+      constexpr int R = decltype(RC)::value, Z = R == 1 ? 8 : 4;       // batch rows m0, m0 + kW, .. and parts at a time
       float v[R][4] = {};
       for (int z = 0; z < nc; z += Z) {
         float4 a[R][Z];
@@ -572,8 +573,8 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
       for (int q = 0; q < R; q++)
         if (m0 + q * kW < P.M) store(m0 + q * kW, v[q]);
     };
-    if (P.M <= kW) { if (warp < P.M) sum(Int<1>{}, warp); }
-    else if (warp < P.M) sum(Int<4>{}, warp);
+    static_assert(kW >= 16 && 2 * kW >= 32 && 4 * kW >= 64, "a round covers the batch");
+    if (warp < P.M) sum(Int<NPAD / 16>{}, warp);
   }
   if constexpr (MODE == kSplit) {
     // ===== results that are not finite, in the tiles that this CTA stored: again, from the float32 weights (with the
