@@ -137,7 +137,7 @@ MLXR_API int mlxr_dequantize(const void* weights, void* out, int N, int K, int q
  * group_size must be the format's block size, or 32 for Q4_K (the shader's sub-block
  * addressing, q_gemm_dequant.metal:397-430).  K must be a whole number of
  * blocks (the reference overruns the row otherwise).  The kernel is chosen by shape:
- * a streaming GEMV for one and two tokens, tcgen05 tensor-core kernels for more.
+ * streaming GEMVs for one to eight tokens, tcgen05 tensor-core kernels for more.
  * Uses the per-(device, stream) workspace of this library, created at the first call. */
 MLXR_API int mlxr_q_gemm_dequant(const void* x, const void* weights, const void* bias,
                                  void* y, int M, int N, int K, int quant_type,

@@ -1,4 +1,4 @@
-// Small-batch quantized linear (3 <= M <= 64 rows of X; one and two for the formats without a GEMV of their own) on the 5th-generation tensor cores.
+// Small-batch quantized linear (M <= 64 rows of X; few of them as far as gemv.cu and gemv_tokens.cu are not faster) on the 5th-generation tensor cores.
 //
 //   Y[M, N] = X[M, K] * dequant(W)[N, K]^T (+ bias),  X, Y fp16 or bf16, W in MLXR's Q4_K, Q4_0 or
 //   Q8_0 layout, NF4 or the canonical ggml Q4_K layout (q_gemm_dequant.metal:142-260 and
