@@ -6,15 +6,17 @@
 // tiles at the end: [5, 4096] x [4096, 4096]^T canonical Q4_K took 11.1 us there for 1.5 us of weights.  Here the weights go from
 // a warp's TMA ring straight into mma.sync fragments as gemv.cu does it (the same CTAs, rows, units and rings), with the
 // eight columns of m16n8k16 for the tokens:
-//   * a code of four bits is a subnormal fp16 number where it lies (w & 0x000f000f = code * 2^-24; w & 0x00f000f0 = 16 times
-//     that), exactly: two logic operations convert four weights, and 2^24 goes into the block's scale; Q8_0's bytes become
-//     fp16 integers as in gemv.cu;
+//   * a code of four bits, less 8, becomes an fp16 integer where it lies: (w & 0x000f000f) | 0x64006400 is 1024 + code,
+//     w & 0x00f000f0 likewise 16 times the code, and one subtraction of pairs is exact; Q8_0's bytes as in gemv.cu.  (Codes left
+//     as the subnormal numbers that they are need no subtraction, but the MMA then aligns its products some seven bits
+//     too high and drops as many bits of the sum: the results of [1, 1536] x [1318, 1536]^T with some activations 1000 times the others
+//     were 7.5e-6 off before their rounding, 4e-7 so.  It takes 5 to 19 % longer: 4 tokens, 7424 x 14336, 24.6 us and 29.2.)
 //   * activations are fp16 as they are, bf16 ones times a power of two per 256 elements (exact: gemv.cu); they are stored so
 //     that a thread's 16 bytes are the B fragments of the eight weights it holds;
 //   * a block's sum over its 32 weights is complete in the accumulators of two MMAs: scale, minimum and the sum of the
 //     block's activations are applied in float32, so the products are those of the float32 weights.
 // Sums of the warps meet in shared memory and are added in the order of K.  A sum that is not finite is computed again from
-// the float32 weights (a code of 0 times an infinite activation is not what the weight's offset makes of it).
+// the float32 weights (a code times an infinite activation is not what the weight's offset makes of it).
 #include <atomic>
 #include <cstring>
 #include <type_traits>
@@ -40,6 +42,7 @@ constexpr int kSmemMax = 227 * 1024;
 template <int QT> struct Geo {
   static constexpr int kSeg = QT == MLXR_Q8_0 ? 272 : 144, kSegs = QT == MLXR_Q8_0 ? 1 : 2, kPitch = kSeg * kSegs;
   static constexpr int kBox = (4 * kPitch + 127) & ~127, kStage = 4 * kBox;
+  static constexpr bool kSums = QT == MLXR_GGML_Q4_K || QT == MLXR_Q4_K;      // formats with an offset per block
 };
 
 struct Params {
@@ -81,9 +84,16 @@ __device__ __forceinline__ float hi_f(uint32_t v) { return __half2float(__ushort
 // a thread's fragments of two MMAs
 template <int QT> constexpr uint32_t kOrder = QT == MLXR_GGML_Q4_K ? 0x75643120u : QT == MLXR_Q8_0 ? 0x76543210u : 0x73516240u;
 
+__device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
+  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// The low nibbles of bytes 0 and 2 less 8; their high nibbles, 16 times that
+__device__ __forceinline__ uint32_t codes_lo(uint32_t w) { return sub2((w & 0x000F000Fu) | 0x64006400u, 0x64086408u); }
+__device__ __forceinline__ uint32_t codes_hi(uint32_t w) { return sub2((w & 0x00F000F0u) | 0x64006400u, 0x64806480u); }
+
 // One segment (256 weights) of 16 rows.  rl / rh: this thread's two rows at the segment; x: its token's row at the segment
 // (+ 16 c bytes); s: sums of the activations per block of 32 of its two tokens, [block][8].  a[2 h + t]: row h, token t.
-constexpr uint32_t kLo = 0x000F000Fu, kHi = 0x00F000F0u;
 template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const uint8_t* rh, const uint8_t* x, const float* s, int c, float (&a)[4]) {
   auto xblock = [&](int b) { return *reinterpret_cast<const uint4*>(x + 64 * b); };
   auto sblock = [&](int b) { return *reinterpret_cast<const float2*>(s + 8 * b); };
@@ -95,9 +105,9 @@ template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const u
     a[3] = fmaf(sh, d[3], fmaf(oh, sm.y, a[3]));
   };
   if constexpr (QT == MLXR_GGML_Q4_K) {
-    // w = (d sc) q - dmin m; chunk j: low nibbles of its 32 bytes are block 2 j, high nibbles block 2 j + 1
+    // w = (d sc) (q - 8) + (8 d sc - dmin m); chunk j: low nibbles of its 32 bytes are block 2 j, high nibbles block 2 j + 1
     const uint4 hl = *reinterpret_cast<const uint4*>(rl), hh = *reinterpret_cast<const uint4*>(rh);
-    const float dl = lo_f(hl.x) * 0x1p24f, ml = -hi_f(hl.x), dh = lo_f(hh.x) * 0x1p24f, mh = -hi_f(hh.x);
+    const float dl = lo_f(hl.x), ml = -hi_f(hl.x), dh = lo_f(hh.x), mh = -hi_f(hh.x);
     auto half = [&](auto H) {
       constexpr int h = decltype(H)::value;
       const uint32_t scl = h ? (hl.w & 0x0F0F0F0Fu) | ((hl.y >> 2) & 0x30303030u) : hl.y & 0x3F3F3F3Fu, mnl = h ? ((hl.w >> 4) & 0x0F0F0F0Fu) | ((hl.z >> 2) & 0x30303030u) : hl.z & 0x3F3F3F3Fu;
@@ -107,12 +117,15 @@ template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const u
         const uint2 wl = *reinterpret_cast<const uint2*>(rl + 16 + 16 * b + 8 * c), wh = *reinterpret_cast<const uint2*>(rh + 16 + 16 * b + 8 * c);
         const uint4 xa = xblock(b), xb = xblock(b + 1);
         float lo[4] = {}, hi[4] = {};
-        hmma(lo, wl.x & kLo, wh.x & kLo, (wl.x >> 8) & kLo, (wh.x >> 8) & kLo, xa.x, xa.y);
-        hmma(hi, wl.x & kHi, wh.x & kHi, (wl.x >> 8) & kHi, (wh.x >> 8) & kHi, xb.x, xb.y);
-        hmma(lo, wl.y & kLo, wh.y & kLo, (wl.y >> 8) & kLo, (wh.y >> 8) & kLo, xa.z, xa.w);
-        hmma(hi, wl.y & kHi, wh.y & kHi, (wl.y >> 8) & kHi, (wh.y >> 8) & kHi, xb.z, xb.w);
-        add(lo, dl * byte_f<2 * j>(scl), dh * byte_f<2 * j>(sch), ml * byte_f<2 * j>(mnl), mh * byte_f<2 * j>(mnh), sblock(b));
-        add(hi, dl * 0x1p-4f * byte_f<2 * j + 1>(scl), dh * 0x1p-4f * byte_f<2 * j + 1>(sch), ml * byte_f<2 * j + 1>(mnl), mh * byte_f<2 * j + 1>(mnh), sblock(b + 1));
+        hmma(lo, codes_lo(wl.x), codes_lo(wh.x), codes_lo(wl.x >> 8), codes_lo(wh.x >> 8), xa.x, xa.y);
+        hmma(hi, codes_hi(wl.x), codes_hi(wh.x), codes_hi(wl.x >> 8), codes_hi(wh.x >> 8), xb.x, xb.y);
+        hmma(lo, codes_lo(wl.y), codes_lo(wh.y), codes_lo(wl.y >> 8), codes_lo(wh.y >> 8), xa.z, xa.w);
+        hmma(hi, codes_hi(wl.y), codes_hi(wh.y), codes_hi(wl.y >> 8), codes_hi(wh.y >> 8), xb.z, xb.w);
+        auto finish = [&](const float (&d)[4], float part, float sl, float sh, float nl, float nh, float2 sm) {
+          add(d, sl * part, sh * part, fmaf(8.0f, sl, ml * nl), fmaf(8.0f, sh, mh * nh), sm);
+        };
+        finish(lo, 1.0f, dl * byte_f<2 * j>(scl), dh * byte_f<2 * j>(sch), byte_f<2 * j>(mnl), byte_f<2 * j>(mnh), sblock(b));
+        finish(hi, 0x1p-4f, dl * byte_f<2 * j + 1>(scl), dh * byte_f<2 * j + 1>(sch), byte_f<2 * j + 1>(mnl), byte_f<2 * j + 1>(mnh), sblock(b + 1));
       };
       chunk(std::integral_constant<int, 0>{});
       chunk(std::integral_constant<int, 1>{});
@@ -121,21 +134,20 @@ template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const u
     half(std::integral_constant<int, 1>{});
   } else if constexpr (QT == MLXR_Q4_K) {
     // (scale, min) pairs of blocks {0, 2, 3}, {1}, {4, 6, 7}, {5} (q_gemm_dequant.metal:222-242); scale rn16(sc d), min
-    // rn16(m dmin); w = q ss + (sm - 8 ss)
+    // rn16(m dmin); w = (q - 8) ss + sm
     const uint4 hl = *reinterpret_cast<const uint4*>(rl), hh = *reinterpret_cast<const uint4*>(rh);
     auto block = [&](int b, float (&d)[4]) {
       const uint32_t wl = *reinterpret_cast<const uint32_t*>(rl + 16 + 16 * b + 4 * c), wh = *reinterpret_cast<const uint32_t*>(rh + 16 + 16 * b + 4 * c);
       const uint4 xv = xblock(b);
-      hmma(d, wl & kLo, wh & kLo, (wl >> 8) & kLo, (wh >> 8) & kLo, xv.x, xv.y);
-      hmma(d, (wl >> 4) & kLo, (wh >> 4) & kLo, (wl >> 12) & kLo, (wh >> 12) & kLo, xv.z, xv.w);
+      hmma(d, codes_lo(wl), codes_lo(wh), codes_lo(wl >> 8), codes_lo(wh >> 8), xv.x, xv.y);
+      hmma(d, codes_lo(wl >> 4), codes_lo(wh >> 4), codes_lo(wl >> 12), codes_lo(wh >> 12), xv.z, xv.w);
     };
     auto finish = [&](int p, const float (&d)[4], float2 sm) {
       auto pair = [&](const uint4& h, float& sc, float& of) {
         const uint32_t f = p == 3 ? h.z >> 4 : p == 2 ? __funnelshift_r(h.y, h.z, 24) : h.y >> (12 * p);
         const __half2 dd = *reinterpret_cast<const __half2*>(&h.x);
-        const float ss = __half2float(__hmul(__int2half_rn((int)(f & 63u)), __low2half(dd)));
-        of = fmaf(-8.0f, ss, __half2float(__hmul(__int2half_rn((int)((f >> 6) & 63u)), __high2half(dd))));
-        sc = ss * 0x1p24f;
+        sc = __half2float(__hmul(__int2half_rn((int)(f & 63u)), __low2half(dd)));
+        of = __half2float(__hmul(__int2half_rn((int)((f >> 6) & 63u)), __high2half(dd)));
       };
       float sl, ol, sh, oh;
       pair(hl, sl, ol);
@@ -167,9 +179,10 @@ template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const u
       }
       const uint4 xv = xblock(b);
       float d[4] = {};
-      hmma(d, w[0] & kLo, w[1] & kLo, (w[0] >> 8) & kLo, (w[1] >> 8) & kLo, xv.x, xv.y);
-      hmma(d, (w[0] >> 4) & kLo, (w[1] >> 4) & kLo, (w[0] >> 12) & kLo, (w[1] >> 12) & kLo, xv.z, xv.w);
-      add(d, d2[0] * 0x1p24f, d2[1] * 0x1p24f, -8.0f * d2[0], -8.0f * d2[1], sblock(b));
+      hmma(d, codes_lo(w[0]), codes_lo(w[1]), codes_lo(w[0] >> 8), codes_lo(w[1] >> 8), xv.x, xv.y);
+      hmma(d, codes_lo(w[0] >> 4), codes_lo(w[1] >> 4), codes_lo(w[0] >> 12), codes_lo(w[1] >> 12), xv.z, xv.w);
+#pragma unroll
+      for (int i = 0; i < 4; i++) a[i] = fmaf(d2[i >> 1], d[i], a[i]);
     }
   } else {
 #pragma unroll
@@ -197,7 +210,7 @@ template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const u
 template <int QT, typename T>
 __global__ void __launch_bounds__(kThreads, 1) gemv_tokens_kernel(const __grid_constant__ Params P) {
   using G_ = Geo<QT>;
-  constexpr bool kScaled = Act<T>::kDtype == MLXR_BF16, kSums = QT != MLXR_Q8_0;
+  constexpr bool kScaled = Act<T>::kDtype == MLXR_BF16, kSums = Geo<QT>::kSums;
   extern __shared__ __align__(128) uint8_t smem[];
   Misc* misc = reinterpret_cast<Misc*>(smem + P.off_misc);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
@@ -434,7 +447,7 @@ template <int QT> static size_t layout(Params* P, int grid) {
       size_t o = (size_t)kWarps * P->stages * G::kStage;
       auto take = [&](size_t n) { const size_t at = o; o += (n + 15) & ~(size_t)15; return (int)at; };
       P->off_x = take((size_t)P->M * P->x_stride);
-      P->off_sum = take(QT == MLXR_Q8_0 ? 0 : (size_t)P->nseg * 8 * kTokens * 4);
+      P->off_sum = take(G::kSums ? (size_t)P->nseg * 8 * kTokens * 4 : 0);
       P->off_delta = take((size_t)P->nseg * kTokens * 4);
       P->off_parts = take((size_t)std::min(tiles, P->chunk) * kWarps * 16 * P->M * 4);
       P->off_misc = take(sizeof(Misc));

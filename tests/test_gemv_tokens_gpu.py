@@ -128,3 +128,25 @@ def test_range_of_bf16(scale):
     x = (make_acts(3, K, 2, torch.float32)[0] * scale).to(torch.bfloat16).cuda()
     x[:, 512:] *= 2.0 ** -12
     _check(_linear(x, w, N, K, 33), x.double() @ _dense(w, N, K, 33).T, "bf16", 33)
+
+
+@pytest.mark.parametrize("qt,dt,M", [(33, "f16", 1), (33, "bf16", 3), (33, "f16", 8), (2, "f16", 3), (2, "bf16", 8), (0, "bf16", 3), (3, "bf16", 5)])
+def test_large_activations_that_cancel(qt, dt, M):
+    """Every block of 32 has activations 256 and -256 on equal weights; the others are at most 2^-5, in steps of 2^-9.  A block's sums of
+    code * x stay below 2^13, so float32 holds them exactly in any order and the large ones leave nothing behind: the
+    bounds are those of the small ones alone.  (Sums of 17 bits leave 1 to 3 % of the results.)"""
+    N, K = 130, 512
+    p = _weights(N, K, qt, 3).cpu().numpy().reshape(-1, {0: 18, 2: 34, 3: 144, 33: 144}[qt])
+    if qt == 33:
+        p[:, 16:].reshape(-1, 4, 32)[..., 20] = p[:, 16:].reshape(-1, 4, 32)[..., 2]      # byte i: element i of two blocks
+    elif qt == 3:
+        p[:, 16:].reshape(-1, 8, 16)[..., 10] = p[:, 16:].reshape(-1, 8, 16)[..., 1]      # byte i: elements 2 i and 2 i + 1
+    else:
+        p[:, 2 + (20 if qt == 2 else 10)] = p[:, 2 + (2 if qt == 2 else 1)]
+    w = torch.from_numpy(p.reshape(-1)).cuda()
+    d = _dense(w, N, K, qt)
+    assert torch.equal(d[:, 2::32], d[:, 20::32])
+    x = torch.randint(-16, 17, (M, K), generator=torch.Generator().manual_seed(5)).double() / 512
+    x[:, 2::32], x[:, 20::32] = 256.0, -256.0
+    x = x.to(DT[dt]).cuda()
+    _check(_linear(x, w, N, K, qt), x.double() @ d.T, dt, qt)
