@@ -12,7 +12,6 @@
 #include <climits>
 
 #include <ATen/ATen.h>
-#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -218,11 +217,7 @@ PyObject* rope_apply(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const uint16_t *cp = (const uint16_t*)data(&cs), *sp = (const uint16_t*)data(&sn);
     const int32_t* pp = (const int32_t*)data(&pos);
     const int max_seq = (int)cs.size(0);
-    const int rc = without_gil([&] { return p_rope(xp, cp, sp, pp, yp, batch, seq, heads, hd, max_seq, mode, scale, off, dt, check ? MLXR_ROPE_CHECK_POSITIONS : 0, st); });
-    // The rotation may still run: memory that belongs to another stream is not given away before it has ended.
-    if (check)
-      for (const at::Tensor* t : {&x, &cs, &sn, &pos}) c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), c10::cuda::getCurrentCUDAStream());
-    return result(rc, y);
+    return result(without_gil([&] { return p_rope(xp, cp, sp, pp, yp, batch, seq, heads, hd, max_seq, mode, scale, off, dt, check ? 1 : 0, st); }), y);
   });
 }
 

@@ -2,7 +2,6 @@
 // selection.  Nothing here computes on the CPU: every compute entry point launches CUDA
 // kernels or fails.
 #include <atomic>
-#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -448,24 +447,14 @@ int mlxr_rope_apply(const void* x, const uint16_t* cos_f16, const uint16_t* sin_
   // host address is the device address), which saves a copy and a memset per call.
   int* word = ws->status;
   if (check) if (int r = take_check_word(&word)) return r;
-  bool early = check == MLXR_ROPE_CHECK_POSITIONS;
   if (int r = launch_rope(x, cos_f16, sin_f16, positions, y, tokens, heads, head_dim, max_seq_len, mode,
-                          scale_factor, position_offset, dtype, word, &early, st)) {
+                          scale_factor, position_offset, dtype, word, st)) {
     if (check) give_check_word(word);       // nothing was launched
     return r;
   }
   if (check) {
-    // The word is looked at for as long as a short queue of kernels takes; behind more work than that, or when the
-    // word is not the kernel's answer, the stream is waited for in the way that the device is set to.
-    bool known = false;
-    if (early)
-      for (const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);;) {
-        for (int i = 0; i < 32 && !known; i++) known = *reinterpret_cast<volatile int*>(word) != 0;
-        if (known || std::chrono::steady_clock::now() > until) break;
-      }
-    if (!known) MLXR_CUDA_TRY(cudaStreamSynchronize(st));     // on failure the kernel may still run: the word is not reused
-    const int seen = give_check_word(word);
-    if (seen != (early ? 1 : 0)) {
+    MLXR_CUDA_TRY(cudaStreamSynchronize(st));     // on failure the kernel may still run: the word is not reused
+    if (give_check_word(word) != 0) {
       set_error("rope_apply: a position (+offset) lies outside [0, max_seq_len)");
       return MLXR_ERR_SHAPE;
     }
@@ -772,10 +761,10 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
   if (rope_qk_supported(q_out, k_out, cos_f16, sin_f16, head_dim, dtype))
     return launch_rope_qk(q_out, k_out, cos_f16, sin_f16, positions, (size_t)M, q_heads, kv_heads, head_dim, max_seq_len, position_offset, dtype, ws->status, st);
   if (int r = launch_rope(q_out, cos_f16, sin_f16, positions, q_out, (size_t)M, q_heads, head_dim, max_seq_len,
-                          MLXR_ROPE_BASE, 1.0f, position_offset, dtype, ws->status, nullptr, st))
+                          MLXR_ROPE_BASE, 1.0f, position_offset, dtype, ws->status, st))
     return r;
   return launch_rope(k_out, cos_f16, sin_f16, positions, k_out, (size_t)M, kv_heads, head_dim, max_seq_len,
-                     MLXR_ROPE_BASE, 1.0f, position_offset, dtype, ws->status, nullptr, st);
+                     MLXR_ROPE_BASE, 1.0f, position_offset, dtype, ws->status, st);
 }
 
 // ---- host-buffer variants ---------------------------------------------------------------

@@ -195,8 +195,8 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const T* g,
 
 // The same for 16-bit types, 128-bit accesses, resident CTAs: a thread has two vectors of each operand in work and the next
 // two on their way.  Bound by HBM (three streams).  With the exact division, in a grid of 3889 short CTAs, it was bound by
-// issue (73 %).  rmsnorm, rope_apply of q and of k, swiglu on 1111 tokens of 4096 x 14336: 55.1 us a pass, 45.5 with this, the
-// rotation's 32-bit quotients and its early answer.
+// issue (73 %).  rmsnorm, rope_apply of q and of k, swiglu on 1111 tokens of 4096 x 14336: 55.4 us a pass, 51.1 with this and the
+// rotation's 32-bit quotients.
 template <typename T, bool UP>
 __global__ void __launch_bounds__(256, 4) swiglu_vec_kernel(const T* g, const T* u, T* o, size_t nvec) {
   const size_t step = (size_t)gridDim.x * 256;
@@ -336,40 +336,23 @@ struct Divisor {
 //
 // Two tensors that share the positions (q and k of a layer) can go in one launch: vectors from `total` on are z's,
 // up to total_z.
-//
-// early: the word in host memory that a waiting caller reads.  CTA 0 then rotates nothing and checks all positions
-// first, so that the caller knows them valid (1) or not (2) while the rotation still runs.
 struct RopeArgs {
   const __half *cos_t, *sin_t;
   const int32_t* positions;
-  size_t total, total_z, tokens;
+  size_t total, total_z;
   Divisor per, per_z, per_head;          // vectors of a token of x, of z, of a head
   int max_seq, linear;
   float scale;
   int offset;
-  int *status, *early;
+  int* status;
 };
 template <typename T, bool WIDE>          // WIDE: 2^31 vectors and more
 __global__ void __launch_bounds__(256) rope_vec_kernel(const T* x, T* y, T* z, const RopeArgs A) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  auto valid = [&](long long pos) { return pos >= 0 && pos < A.max_seq; };
-  int cta = blockIdx.x, ctas = gridDim.x;
-  if (A.early) {
-    if (cta == 0) {
-      bool ok = true;
-#pragma unroll 8
-      for (size_t t = threadIdx.x; t < A.tokens; t += 256) ok = ok && valid((long long)__ldcg(A.positions + t) + A.offset);
-      ok = __syncthreads_and(ok);
-      if (threadIdx.x == 0) atomicExch_system(A.early, ok ? 1 : 2);
-      return;
-    }
-    cta--;
-    ctas--;
-  }
   using Index = typename std::conditional<WIDE, size_t, uint32_t>::type;
   const Index total = (Index)A.total, all = (Index)(A.total + A.total_z);
-  for (size_t j0 = (size_t)cta * 256 + threadIdx.x; j0 < all; j0 += (size_t)ctas * 256) {
+  for (size_t j0 = (size_t)blockIdx.x * 256 + threadIdx.x; j0 < all; j0 += (size_t)gridDim.x * 256) {
     const Index j = (Index)j0;
     const bool first = j < total;
     const Index i = first ? j : j - total;
@@ -384,7 +367,7 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(const T* x, T* y, T* z, c
     c -= h * A.per_head.d;
     const uint4 xv = __ldcg(reinterpret_cast<const uint4*>(src) + i);
     const long long pos = (long long)__ldcg(A.positions + tok) + A.offset;
-    if (!valid(pos)) {
+    if (pos < 0 || pos >= A.max_seq) {
       if (A.status) atomicExch_system(A.status, 1);
       continue;
     }
@@ -406,13 +389,13 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(const T* x, T* y, T* z, c
 
 template <typename T>
 static int launch_rope_vec(const void* x, const uint16_t* cos_t, const uint16_t* sin_t, const int32_t* positions, void* y, size_t tokens, int heads,
-                           void* z, int heads_z, int head_dim, int max_seq, int linear, float scale, int offset, int* status, int* early, cudaStream_t st) {
+                           void* z, int heads_z, int head_dim, int max_seq, int linear, float scale, int offset, int* status, cudaStream_t st) {
   const int vh = head_dim / 8;
-  const RopeArgs A = {(const __half*)cos_t, (const __half*)sin_t, positions, tokens * heads * vh, tokens * heads_z * vh, tokens,
-                      Divisor((uint32_t)heads * vh), Divisor((uint32_t)std::max(1, heads_z * vh)), Divisor((uint32_t)vh), max_seq, linear, scale, offset, early ? nullptr : status, early};
+  const RopeArgs A = {(const __half*)cos_t, (const __half*)sin_t, positions, tokens * heads * vh, tokens * heads_z * vh,
+                      Divisor((uint32_t)heads * vh), Divisor((uint32_t)std::max(1, heads_z * vh)), Divisor((uint32_t)vh), max_seq, linear, scale, offset, status};
   const size_t all = A.total + A.total_z;
   cudaLaunchAttribute at;
-  const cudaLaunchConfig_t cfg = overlapped((int)std::min<size_t>((all + 255) / 256, 148 * 8 * 4) + (early ? 1 : 0), 256, st, &at);
+  const cudaLaunchConfig_t cfg = overlapped((int)std::min<size_t>((all + 255) / 256, 148 * 8 * 4), 256, st, &at);
   if (all >> 31) MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rope_vec_kernel<T, true>, (const T*)x, (T*)y, (T*)z, A));
   else MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rope_vec_kernel<T, false>, (const T*)x, (T*)y, (T*)z, A));
   count_launch();
@@ -426,24 +409,19 @@ bool rope_qk_supported(const void* q, const void* k, const uint16_t* cos_t, cons
 }
 int launch_rope_qk(void* q, void* k, const uint16_t* cos_t, const uint16_t* sin_t, const int32_t* positions, size_t tokens, int q_heads, int kv_heads,
                    int head_dim, int max_seq, int offset, int dtype, int* status, cudaStream_t st) {
-  return dtype == MLXR_F16 ? launch_rope_vec<__half>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, nullptr, st)
-                           : launch_rope_vec<__nv_bfloat16>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, nullptr, st);
+  return dtype == MLXR_F16 ? launch_rope_vec<__half>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, st)
+                           : launch_rope_vec<__nv_bfloat16>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, st);
 }
 
 int launch_rope(const void* x, const uint16_t* cos_t, const uint16_t* sin_t,
                 const int32_t* positions, void* y, size_t tokens, int heads, int head_dim,
-                int max_seq, int mode, float scale, int offset, int dtype, int* status, bool* early,
+                int max_seq, int mode, float scale, int offset, int dtype, int* status,
                 cudaStream_t st) {
-  const bool want_early = early && *early;
-  if (early) *early = false;
   const size_t total = tokens * heads * (head_dim / 2);
   if (total == 0) return MLXR_OK;
-  if (rope_vec_ok(x, y, cos_t, sin_t, head_dim, dtype)) {
-    if (early) *early = want_early;
-    int* word = want_early ? status : nullptr;
-    return dtype == MLXR_F16 ? launch_rope_vec<__half>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, word, st)
-                             : launch_rope_vec<__nv_bfloat16>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, word, st);
-  }
+  if (rope_vec_ok(x, y, cos_t, sin_t, head_dim, dtype))
+    return dtype == MLXR_F16 ? launch_rope_vec<__half>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, st)
+                             : launch_rope_vec<__nv_bfloat16>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, st);
   size_t blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   MLXR_DISPATCH_DTYPE(dtype, T, {

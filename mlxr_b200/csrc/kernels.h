@@ -28,11 +28,9 @@ int stream_status_word(cudaStream_t st, int** status);
 int launch_cast_from_f32(const float* x, void* y, size_t n, int dtype, cudaStream_t st);
 int launch_cast_to_f32(const void* x, float* y, size_t n, int dtype, cudaStream_t st);
 int launch_swiglu(const void* g, const void* u, void* o, size_t n, int dtype, cudaStream_t st);
-// early (optional): the caller wants *status (a word in host memory, 0) to become 1 or 2 - all positions valid or not - as soon
-// as they are checked; on return whether the kernel does that (else it becomes 1 if a position is invalid)
 int launch_rope(const void* x, const uint16_t* cos_t, const uint16_t* sin_t,
                 const int32_t* positions, void* y, size_t tokens, int heads, int head_dim,
-                int max_seq, int mode, float scale, int offset, int dtype, int* status, bool* early,
+                int max_seq, int mode, float scale, int offset, int dtype, int* status,
                 cudaStream_t st);
 
 // rope_apply on q and k [tokens, heads, head_dim] in place, one launch; false if their layout needs launch_rope

@@ -201,7 +201,8 @@ def rope_apply(input: torch.Tensor, cos_table: torch.Tensor, sin_table: torch.Te
                scale_factor: float = 1.0, position_offset: int = 0, inplace: bool = False,
                check_positions: bool = True) -> torch.Tensor:
     """rope_apply(), rope_apply_primitive.h:192-197 / .mm:399-475.  input is
-    [tokens, heads, d] or [batch, seq, heads, d]; tables fp16 [max_seq, d/2]."""
+    [tokens, heads, d] or [batch, seq, heads, d]; tables fp16 [max_seq, d/2].  With check_positions the call
+    returns, or raises, when the stream has done the rotation."""
     r = fast.rope_apply(input, cos_table, sin_table, positions, scaling_mode, scale_factor, position_offset, inplace, check_positions)
     if r is not None:
         done(r)
@@ -234,10 +235,7 @@ def rope_apply(input: torch.Tensor, cos_table: torch.Tensor, sin_table: torch.Te
     check(lib.mlxr_rope_apply(_dev(input, "input"), _dev(cos_table, "cos_table"), _dev(sin_table, "sin_table"),
                               _dev(positions, "positions"), out.data_ptr(), batch, seq, heads, hd,
                               cos_table.shape[0], int(scaling_mode), scale_factor, position_offset,
-                              _dtype_code(input), 2 if check_positions else 0, _stream()))
-    if check_positions:
-        for t in (input, cos_table, sin_table, positions):      # the rotation may still run
-            t.record_stream(torch.cuda.current_stream())
+                              _dtype_code(input), 1 if check_positions else 0, _stream()))
     return out
 
 

@@ -301,3 +301,35 @@ def test_checked_rope_behind_a_long_queue():
     pos.fill_(99)
     with pytest.raises(mx._capi.MlxrError):
         mx.rope_apply(x, cos, sin, pos)
+
+
+@pytest.mark.parametrize("route", ["native", "interpreted", "abi"])
+@pytest.mark.parametrize("bad", [False, True])
+def test_checked_rope_has_ended_when_it_returns(route, bad):
+    """A checked call returns, or raises, with the rotation done, whatever the path: its result may be used from another stream and its
+    inputs released or overwritten at once.  In place, on a side stream, 256 MB (0.1 ms of rotation after the last
+    position is known); the bad position is the last token's."""
+    import mlxr_b200 as mx
+
+    class Tagged(torch.Tensor):
+        pass
+
+    tokens, heads, dim = 32768, 32, 128
+    cos, sin = mx.compute_rope_tables(512, dim, 10000.0, device=torch.device("cuda"))
+    x = torch.ones(tokens, heads, dim, device="cuda", dtype=torch.float16)
+    pos = torch.zeros(tokens, device="cuda", dtype=torch.int32)
+    pos[-1] = 512 if bad else 0
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        raised = False
+        if route == "abi":      # any non-zero value of the check argument
+            raised = mx._capi.lib.mlxr_rope_apply(x.data_ptr(), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), x.data_ptr(), tokens, 1, heads, dim,
+                                                  512, 0, 1.0, 0, 0, 2, st.cuda_stream) != 0
+        else:
+            try:
+                mx.rope_apply(x if route == "native" else x.as_subclass(Tagged), cos, sin, pos, inplace=True)
+            except mx._capi.MlxrError:
+                raised = True
+        assert st.query()
+    assert raised == bad and torch.equal(x, torch.ones_like(x))      # a rotation by position 0 changes nothing
