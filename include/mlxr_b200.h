@@ -311,6 +311,10 @@ MLXR_API int mlxr_debug_set_trace_buffer(void* dev_ptr);
 MLXR_API int mlxr_debug_smallm_partition(long long units, int ctas, int cta, long long unit,
                                          long long* begin, long long* end, int* owner);
 
+/* The rule on sizes by which a linear of up to eight tokens goes to the kernel that multiplies whole rows rather than to the one that splits K
+ * (host arithmetic only, for tests): 1 or 0.  rows: weight rows in all; form: 0 one matrix, 1 gate and up, 2 q / k / v. */
+MLXR_API int mlxr_debug_few_tokens_rule(int quant_type, int M, int K, int rows, int form, int dtype);
+
 /* Device addresses of the words a (device, stream) workspace keeps between launches: the counters of parts of shared
  * output tiles (32-bit, zero between calls) and the status word that mlxr_stream_status reports.  For tests; any
  * pointer may be NULL. */

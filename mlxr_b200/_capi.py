@@ -52,6 +52,7 @@ PROTOTYPES = {
     "mlxr_static_status": (_i, [_vp, _vp]),
     "mlxr_debug_set_trace_buffer": (_i, [_vp]),
     "mlxr_debug_smallm_partition": (_i, [C.c_longlong, _i, _i, C.c_longlong, _vp, _vp, _vp]),
+    "mlxr_debug_few_tokens_rule": (_i, [_i, _i, _i, _i, _i, _i]),
     "mlxr_debug_stream_words": (_i, [_vp, _vp, _vp, _vp]),
     "mlxr_set_decode_launch_mode": (_i, [_i]),
     "mlxr_q_gemm_dequant_static": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),

@@ -242,11 +242,11 @@ static int run_linear(const void* x, const void* w, const void* bias, void* y, i
     L.w[0] = w; L.rows[0] = N; L.nmat = 1; L.K = K; L.x = x; L.y[0] = y; L.bias[0] = bias;
     return launch_gemv(L, M, qt, dtype, ws->status, st);
   }
-  // Canonical Q4_K (with more activations than gemv_tokens.cu takes), and NF4 rows that do not start on 16 bytes, have no other
-  // kernel for one or two tokens.  The one NF4 has looks every weight up once per token; from 2^24 weights on the small-batch kernel, which converts
+  // Canonical Q4_K that gemv_tokens.cu does not take (but for one token of the smallest matrices, which the generic kernel
+  // has first: see there), and NF4 rows that do not start on 16 bytes, have no other kernel for one or two tokens.  The one NF4 has looks every weight up once per token; from 2^24 weights on the small-batch kernel, which converts
   // once, is the faster one for two (4096 x 4096: 14.5 us there, 11.6 here; 14336 x 4096: 34.4, 27.9; 4096 x 14336:
   // 40.5, 26.7; 4096 x 2048: 7.6, 8.5).
-  const bool small_only = qt == MLXR_GGML_Q4_K ||
+  const bool small_only = (qt == MLXR_GGML_Q4_K && (M > 1 || K > 512 || N > 1024)) ||
                           (qt == MLXR_NF4 && (!gemv_rows_supported(qt, M, K, x, w) || (M == 2 && (long long)N * K >= (1 << 24))));
   if ((M >= 3 || (M > 0 && small_only)) && N > 0) {
     TcPath path;
@@ -649,6 +649,8 @@ int mlxr_debug_smallm_partition(long long units, int ctas, int cta, long long un
   smallm_partition(units, ctas, cta, unit, begin, end, owner);
   return MLXR_OK;
 }
+
+int mlxr_debug_few_tokens_rule(int qt, int M, int K, int rows, int form, int dtype) { return gemv_tokens_faster(qt, M, K, rows, form, dtype) ? 1 : 0; }
 
 int mlxr_debug_stream_words(void* stream, void** tile_counters, int* n_counters, void** status_word) {
   Workspace* ws = nullptr;

@@ -464,22 +464,45 @@ static size_t layout(int qt, Params* P, int grid) {
   }
 }
 
-// Where this kernel is the faster one (bf16, weights rotating through more than L2, this / smallm.cu in us; Q4_0 is within 10 % of Q4_K):
-//   canonical Q4_K  1 token 14336 x 4096 12.7 / 28.4, 3 tokens 4096 x 14336 18.5 / 27.3, 16384 x 16384 52.6 / 94.0, 8 tokens 4096 x 4096
-//                   8.4 / 11.4, 14336 x 4096 18.6 / 28.6
-//   Q8_0            3 tokens 4096 x 4096 7.8 / 11.0, 16384 x 16384 70.3 / 92.5, 8 tokens 14336 x 4096 25.1 / 28.5, but 5 tokens of
-//                   4096 x 14336, whose activations leave room for one ring stage, 28.3 / 27.1: to 49152 activations
-//   q / k / v       3 tokens of hidden size 4096 12.0 / 15.9, 8192 25.9 / 38.5, 8 tokens 14.8 / 18.3
-//   Q4_K, Q4_0      (one 16-bit part per weight over there) 3 tokens 4096 x 4096 6.2 / 7.1, 14336 x 4096 13.3 / 12.6, 5 tokens 2048 x
-//                   2048 4.3 / 5.5, 4096 x 4096 7.3 / 7.1, 8 tokens 2048 x 2048 4.8 / 5.5: the products decide
+// Where this kernel is the faster one of the two that take these calls (the other: smallm.cu, which splits K over CTAs).  Every CTA
+// here converts all M * K activations and multiplies whole rows, so few rows of many activations are the other's; bf16 ones
+// cost more to convert.  Device times, weights rotating through more than L2, this / the other in us:
+//   canonical Q4_K  bf16 5 tokens 1000 x 4096 6.1 / 6.6, 1000 x 5632 7.6 / 7.5, 1000 x 8192 9.8 / 9.1, 4096 x 8192 15.2 / 17.6, 14336 x 4096 17.4 / 28.5;
+//                   3 tokens 256 x 16384 14.2 / 9.5, 3000 x 14336 21.1 / 20.7, 4096 x 16384 24.2 / 30.6; one 256 x 24576 14.2 / 12.2.  fp16
+//                   6 tokens 1000 x 8192 7.8 / 9.1; 2 tokens 256 x 16384 10.7 / 9.5.  One token of 1000 x 256 3.3 / 3.0 (the generic kernel)
+//   Q8_0            bf16 3 tokens 1000 x 11008 10.8 / 10.9, 1000 x 16384 16.3 / 12.3, 4096 x 14336 25.8 / 28.4; 8 tokens 1000 x 3072 5.8 / 6.8,
+//                   1000 x 5632 9.7 / 7.4, 3000 x 5632 13.9 / 12.3, 4096 x 5632 14.7 / 14.8
+//   Q4_K, Q4_0      (one 16-bit part per weight over there, so the products decide too) Q4_K 3 tokens 1000 x 768 3.6 / 3.3, 4096 x 1024 3.7 / 3.8,
+//                   6144 x 1024 4.4 / 4.0, 4096 x 1536 4.5 / 5.7, 8192 x 1536 5.7 / 5.1, 8192 x 2048 6.8 / 7.6, 1000 x 4096 5.0 / 5.0, 1000 x 8192
+//                   8.0 / 6.3; 8 tokens 1000 x 1024 4.0 / 3.7, 1000 x 2048 4.9 / 5.1, 1000 x 4096 7.2 / 5.3.  Q4_0 5 tokens 1000 x 3072 4.9 / 5.2
+//   gate / up       Q4_K 5 tokens of hidden size 1024: block of 2048 9.7 / 11.4
+//   q / k / v       Q4_K bf16 8 tokens of hidden size 2048 (3072 rows) 0.96 of the other's time, 2560 (3584) 1.10, 4096 (4352) 1.05, (6144) 0.91,
+//                   5120 (5376) 1.08; Q4_0, 6 tokens and fp16 at most 1.04
+// To 2368 rows (16 for each of 148 SMs) a CTA has one tile of rows; from 1800 on the other's CTAs have as much to do as at 2368.
+bool gemv_tokens_faster(int qt, int M, int K, int rows, int form, int dtype) {
+  const long long acts = (long long)M * K;
+  const bool bf16 = dtype == MLXR_BF16, one_full = rows >= 1800 && rows <= 2368, two = rows > 2368;
+  if (form == kTokensStacked) return !(bf16 && qt != MLXR_Q4_0 && M >= 7 && K > 2048 && K < 6144 && 2ll * rows < 3ll * K);
+  if (qt == MLXR_Q4_K || qt == MLXR_Q4_0) {
+    if (form == kTokensPlain && (K < 1024 || (K < 1536 && (rows > 2560 || M > (K < 1280 ? 4 : 6))) || (K < 2048 && rows > 6144))) return false;
+    // a block whose down rows are the other kernel's too: 5 tokens of 1024 x 3584 12.5 us in turns, 11.5 both there
+    if (form == kTokensGateUp && K < 1536 && rows > 4096 && (long long)M * rows > 2 * 12288) return false;
+    return acts * rows <= 3ll << 24 && (qt == MLXR_Q4_0 ? acts <= 14336 || (K <= 4096 && acts <= 16384) : K <= 2048 || acts <= 12288);
+  }
+  if (rows >= 3500) return true;
+  if (qt == MLXR_Q8_0) return acts <= (bf16 ? (one_full ? 38500 : two ? 34000 : 28000 + 3 * rows) : (one_full ? 49152 : two ? 36500 : 38000 + rows));
+  if (M == 1 && K <= 512 && rows <= 1024) return false;
+  if (!bf16) return rows >= 3000 || K <= 8192 || (M + 2ll) * K <= 58000 + 20ll * rows;      // 8192: one stage for each of the 16 warps
+  return acts <= (one_full ? 46000 : two ? 33500 : M == 1 ? 12000 + 12 * rows : 26000 + 4 * rows);
+}
+
 bool gemv_tokens_supported(int qt, int M, int K, int rows, int form, int dtype, const void* x, const void* const* w, int nmat) {
   if (dtype != MLXR_F16 && dtype != MLXR_BF16) return false;
   if (qt != MLXR_GGML_Q4_K && qt != MLXR_Q8_0 && qt != MLXR_Q4_K && qt != MLXR_Q4_0) return false;
   // One linear or gate / up of MLXR's 4-bit formats and fp16 activations multiplies weights in the shader's half arithmetic
   if ((qt == MLXR_Q4_K || qt == MLXR_Q4_0) && dtype == MLXR_F16 && form != kTokensStacked) return false;
   if (M < (qt == MLXR_GGML_Q4_K ? 1 : 3) || M > kTokens || K < 256 || K % 256 != 0 || rows < 1 || rows > (1 << 19)) return false;
-  if (M * (long long)K > 49152) return false;
-  if ((qt == MLXR_Q4_K || qt == MLXR_Q4_0) && form != kTokensStacked && (long long)M * rows * K > 3ll << 24) return false;
+  if (M * (long long)K > 49152 || !gemv_tokens_faster(qt, M, K, rows, form, dtype)) return false;
   int sms = 0;
   if (device_sms(&sms)) return false;
   Params P;

@@ -127,6 +127,7 @@ int launch_stream_gemv(const DecodeLinear& L, int M, int dtype, int* status, cud
 // ---- up to eight tokens of 16-bit activations (gemv_tokens.cu): canonical Q4_K from one token on, Q8_0, Q4_K, Q4_0 from three ----
 // rows: weight rows in all.  w[0 .. nmat): one matrix, gate and up (y[0] = SiLU(X gate^T) * (X up^T), rows[0] columns), or stacked
 enum TokensForm { kTokensPlain = 0, kTokensGateUp = 1, kTokensStacked = 2 };
+bool gemv_tokens_faster(int qt, int M, int K, int rows, int form, int dtype);       // the part of the rule that is about time
 bool gemv_tokens_supported(int qt, int M, int K, int rows, int form, int dtype, const void* x, const void* const* w, int nmat);
 int launch_gemv_tokens(const void* x, const void* const* w, const int* rows, int nmat, int form, const void* bias, void* const* y, int M, int K, int qt, int dtype,
                        int* status, cudaStream_t st);

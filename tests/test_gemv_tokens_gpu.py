@@ -135,7 +135,7 @@ def test_large_activations_that_cancel(qt, dt, M):
     """Every block of 32 has activations 256 and -256 on equal weights; the others are at most 2^-5, in steps of 2^-9.  A block's sums of
     code * x stay below 2^13, so float32 holds them exactly in any order and the large ones leave nothing behind: the
     bounds are those of the small ones alone.  (Sums of 17 bits leave 1 to 3 % of the results.)"""
-    N, K = 130, 512
+    N, K = 130, 512 if qt in (2, 33) else 1536
     p = _weights(N, K, qt, 3).cpu().numpy().reshape(-1, {0: 18, 2: 34, 3: 144, 33: 144}[qt])
     if qt == 33:
         p[:, 16:].reshape(-1, 4, 32)[..., 20] = p[:, 16:].reshape(-1, 4, 32)[..., 2]      # byte i: element i of two blocks
@@ -150,3 +150,42 @@ def test_large_activations_that_cancel(qt, dt, M):
     x[:, 2::32], x[:, 20::32] = 256.0, -256.0
     x = x.to(DT[dt]).cuda()
     _check(_linear(x, w, N, K, qt), x.double() @ d.T, dt, qt)
+
+
+# The rule of sizes sends these here: remainders of rows, warps without work, an odd number of segments, one ring stage, meetings
+# of the warps in the middle of a CTA's tiles
+HERE = [(0, "bf16", 3, 1000, 1280), (3, "bf16", 4, 67, 1536), (0, "bf16", 5, 593, 1792), (3, "bf16", 6, 2369, 1536), (0, "bf16", 8, 130, 2048), (3, "bf16", 8, 2, 2048), (0, "bf16", 3, 41, 4352),
+        (3, "bf16", 3, 3001, 3328), (33, "bf16", 8, 4102, 6144), (33, "f16", 1, 4097, 32768), (33, "bf16", 1, 3501, 24576), (2, "bf16", 3, 4099, 16384), (2, "f16", 8, 4097, 5632),
+        (33, "bf16", 1, 1025, 512), (33, "f16", 2, 5, 768)]
+
+
+@pytest.mark.parametrize("qt,dt,M,N,K", HERE)
+def test_sizes_that_the_rule_sends_here(qt, dt, M, N, K):
+    import mlxr_b200 as mx
+    assert mx._capi.lib.mlxr_debug_few_tokens_rule(qt, M, K, N, 0, {"f16": 0, "bf16": 1}[dt]) == 1
+    w = _weights(N, K, qt, 7 + N)
+    x = make_acts(M, K, 8 + N, DT[dt])[0].cuda()
+    b = make_acts(1, N, 9, DT[dt])[0][0].contiguous().cuda() if N % 2 else None
+    y = _linear(x, w, N, K, qt, b)
+    assert torch.equal(y, _linear(x, w, N, K, qt, b)) and _status() == 0
+    _check(y, x.double() @ _dense(w, N, K, qt).T + (b.double() if b is not None else 0), dt, qt)
+
+
+@pytest.mark.parametrize("qt,M,N,K", [(33, 1, 1024, 512), (33, 3, 700, 14336), (2, 8, 1000, 5632), (3, 3, 4096, 768), (3, 8, 1000, 4096), (0, 4, 2561, 1280)])
+def test_sizes_beyond_the_rule(qt, M, N, K):
+    """The other kernels' sizes next to these.  Q4_K and Q4_0: weights rounded to bf16, 2^-9 each, and the result."""
+    import mlxr_b200 as mx
+    assert mx._capi.lib.mlxr_debug_few_tokens_rule(qt, M, K, N, 0, 1) == 0
+    w = _weights(N, K, qt, 7)
+    x = make_acts(M, K, 8, torch.bfloat16)[0].cuda()
+    y = _linear(x, w, N, K, qt)
+    want = x.double() @ _dense(w, N, K, qt).T
+    assert _status() == 0 and float((y.double() - want).norm() / want.norm()) <= RESULT["bf16"] + (2.0 ** -9 if qt in (0, 3) else 2.0 ** -15)
+
+
+@pytest.mark.parametrize("qt", [0, 3])
+@pytest.mark.parametrize("M,H,I", [(3, 1536, 1280), (8, 2048, 1536)])
+def test_gate_up_of_the_rule(qt, M, H, I):
+    import mlxr_b200 as mx
+    assert mx._capi.lib.mlxr_debug_few_tokens_rule(qt, M, H, 2 * I, 1, 1) == 1
+    test_gate_up(qt, M, H, I)
