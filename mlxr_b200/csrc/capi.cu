@@ -208,13 +208,14 @@ static int run_tc(TcPath path, const WidePlan& wide, const DensePlan& dense, con
 // split-K partial sums; intermediates of the fused entry points start after them.
 // Small matrices of a few tokens: a kernel without copies into shared memory, barriers and partial sums has its result
 // before the others have set themselves up.  bf16, weights from HBM, in us, gemv_rows_kernel / the kernel that larger ones take:
-//   Q8_0  two tokens of 1000 x 1024 4.1 / 4.6, 2048 x 1024 5.1 / 4.6; one token is gemv.cu's (1000 x 1024 4.1 / 3.5, 3000 x 2048 7.1 /
-//         4.4), three and more gemv_tokens.cu's (8 tokens of 1000 x 1024 7.2 / 3.4)
+//   Q8_0  one token 1000 x 1024 2.9 / 3.5, 2048 x 1280 3.4 / 3.7, 5120 x 512 3.4 / 3.6, 6144 x 256 3.9 / 3.6, 4096 x 1024 4.2 / 3.9, 256 x 1536 2.8 /
+//         3.3, 600 x 1536 3.7 / 3.6; two 2048 x 1024 4.0 / 4.7, 4096 x 512 3.9 / 4.7, 5120 x 512 5.4 / 4.8, 256 x 1536 3.9 / 4.7, 64 x 8192 12.3 /
+//         7.4; three and more are gemv_tokens.cu's (8 tokens of 1000 x 1024 7.2 / 3.4)
 //   NF4   3 and 6 tokens of 1000 x 1024 4.6, 6.9 / 7.4; three of 4096 x 1024 6.5 / 7.6, 2048 x 2048 6.7 / 6.8; four of 2048 x 2048 7.5 / 6.9
 static bool rows_kernel_first(int qt, int M, int N, int K, int dtype, const void* x, const void* w) {
   if (dtype == MLXR_F32 || !gemv_rows_supported(qt, M, K, x, w)) return false;
   const long long size = (long long)N * K;
-  if (qt == MLXR_Q8_0) return M == 2 && size <= 1 << 20;
+  if (qt == MLXR_Q8_0) return M <= 2 && ((K <= 1280 && N <= (M == 1 ? 5120 : 4096) && size <= 5 << 19) || (K <= 1536 && size <= 3 << 17));
   return qt == MLXR_NF4 && M >= 3 && (M * size <= 6 << 20 || (M <= 4 && M * K <= 6144 && size <= 1 << 22));
 }
 

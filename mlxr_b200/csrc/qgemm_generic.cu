@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(128) linear_dense_kernel(const T* __restrict__
 
 // ---- small-batch GEMV for the 32-/64-element block formats ----------------------------------------
 // Q4_0, Q4_1, Q8_0 and NF4 at batch <= 8, as far as gemv.cu, gemv_tokens.cu and smallm.cu are not faster: Q4_1, float32 activations, NF4 of
-// one token (of two below 2^24 weights), small NF4 matrices, two tokens of small Q8_0 ones.  HBM-bound: one warp per weight row, eight rows per CTA.  The row is staged into
+// one token (of two below 2^24 weights), small NF4 matrices, one and two tokens of small Q8_0 ones.  HBM-bound: one warp per weight row, eight rows per CTA.  The row is staged into
 // shared memory in chunks of 4096 weights with coalesced 16-byte loads (block boundaries of 18 /
 // 20 / 34 bytes do not line up with vector loads), then the warp walks the chunk 128 weights at a
 // time: lane l takes weights 4l .. 4l+3, so the activations are read conflict-free and the block

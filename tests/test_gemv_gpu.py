@@ -267,3 +267,27 @@ def test_stacked_projections_of_a_small_hidden_size(M, H, QH, KH):
         want = mx.rope_apply(y, cos, sin, pos) if i < 2 else y
         # one ulp of the linear's result at most, 2^-10, where the two sums round to different sides
         assert float((got.double() - want.double()).norm() / want.double().norm()) <= 2.0 ** -11
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 5120, 512), (1, 5121, 512), (1, 2048, 1280), (1, 2049, 1280), (1, 256, 1536), (1, 257, 1536), (2, 4096, 512), (2, 4097, 512), (2, 2560, 1024), (2, 2561, 1024), (2, 256, 1536), (2, 64, 8192)])
+def test_borders_of_small_q8_0(oracle, M, N, K):
+    for dt in ("bf16", "f16"):
+        test_borders_of_the_small_matrices(oracle, 2, dt, M, N, K)
+
+
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("N,K", [(200, 512), (1000, 1024)])
+def test_small_q8_0_multiplies_float32(oracle, M, N, K):
+    """One and two tokens of small Q8_0 matrices: float32 products with the bf16 activations as they are, of any range.  Each segment of 256 has
+    one of 2^20 on weights of zero, the others are 2^-30: to 16 bits of one scale they are lost."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    wf = make_weights(N, K, 3)
+    wf[:, 5::256] = 0.0
+    packed = quantize(wf, 2)
+    x = make_acts(M, K, 4, torch.float32)[0] * 2.0 ** -30
+    x[:, 5::256] = 2.0 ** 20
+    x = x.to(torch.bfloat16).cuda()
+    y = mx.q_gemm_dequant(x, torch.from_numpy(packed).cuda(), M, N, K, mx.QuantType.Q8_0, 32)
+    want = x.double() @ _dense(oracle, packed, N, K, 2).T
+    assert float((y.double() - want).norm() / want.norm()) <= RESULT["bf16"] + WEIGHT[2]
