@@ -100,9 +100,9 @@ __device__ __forceinline__ float swish_f(float x) {
   const float e = expf(-fabsf(x));
   return (x >= 0.0f ? x : x * e) / (1.0f + e);
 }
-// The same for results that are rounded to a 16-bit type, in half the instructions: the denominator lies in [1, 2], so the
-// quotient needs no care for its range, and one residual correction of n * (1 / d) leaves it within a unit of the last
-// place of float32 of the exact one (for every 16-bit x the product with `up` rounds as swish_f's does).
+// The same for x of a 16-bit type, in half the instructions: the denominator lies in [1, 2], so the quotient needs no care for
+// its range, and n * (1 / d) gets one correction by its residual (Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", 1990).  Compared for all 65536 fp16 and all 65536 bf16 x: the float32 quotients are swish_f's.
 __device__ __forceinline__ float swish_h(float x) {
   const float e = expf(-fabsf(x)), d = 1.0f + e, n = x >= 0.0f ? x : x * e;
   float r;

@@ -1,5 +1,5 @@
 // Linears of up to eight tokens of 16-bit activations (canonical ggml Q4_K from one token on, Q8_0, Q4_K and Q4_0 from
-// three), single, stacked along N (q / k / v) or gate / up, with exact products.
+// three), single, stacked along N (q / k / v) or gate / up, with products of the weights as they are.
 //
 // Roofline: HBM, but most of these calls are small and a launch's fixed part decides.  The small-batch kernel (smallm.cu) converts
 // every weight to two 16-bit parts, hands them to tensor memory and two issuers, and adds parked parts of shared
@@ -11,8 +11,9 @@
 //     as the subnormal numbers that they are need no subtraction, but the MMA then aligns its products some seven bits
 //     too high and drops as many bits of the sum: the results of [1, 1536] x [1318, 1536]^T with some activations 1000 times the others
 //     were 7.5e-6 off before their rounding, 4e-7 so.  It takes 5 to 19 % longer: 4 tokens, 7424 x 14336, 24.6 us and 29.2.)
-//   * activations are fp16 as they are, bf16 ones times a power of two per 256 elements (exact: gemv.cu); they are stored so
-//     that a thread's 16 bytes are the B fragments of the eight weights it holds;
+//   * activations are fp16 as they are, bf16 ones times a power of two per 256 elements that brings the largest to 2^14 .. 2^15: exact
+//     down to 2^-31 of it, fewer bits below that, zero below 2^-40 (which shows where the large ones meet weights of zero only);
+//     they are stored so that a thread's 16 bytes are the B fragments of the eight weights it holds;
 //   * a block's sum over its 32 weights is complete in the accumulators of two MMAs: scale, minimum and the sum of the
 //     block's activations are applied in float32, so the products are those of the float32 weights.
 // Sums of the warps meet in shared memory and are added in the order of K.  A sum that is not finite is computed again from

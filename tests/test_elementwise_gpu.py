@@ -333,3 +333,18 @@ def test_checked_rope_has_ended_when_it_returns(route, bad):
                 raised = True
         assert st.query()
     assert raised == bad and torch.equal(x, torch.ones_like(x))      # a rotation by position 0 changes nothing
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_swiglu_quotients_by_many_products(dtype):
+    """Every 16-bit gate times 64 values of up of all magnitudes: the vector kernel's results are those of the IEEE division."""
+    import mlxr_b200 as mx
+    gate = torch.arange(-32768, 32768, dtype=torch.int32, device="cuda").to(torch.int16).view(dtype)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    ups = (torch.randn(64, device="cuda", generator=g) * 2.0 ** torch.randint(-12, 12, (64,), device="cuda", generator=g)).to(dtype)
+    many = mx.swiglu(gate.repeat(64), ups.repeat_interleave(65536)).reshape(64, -1)
+    for i in range(64):
+        few = mx.swiglu(gate, ups[i].expand(65536).contiguous())
+        nan = torch.isnan(few)
+        assert torch.equal(torch.isnan(many[i]), nan)
+        assert torch.equal(many[i].view(torch.int16)[~nan], few.view(torch.int16)[~nan])

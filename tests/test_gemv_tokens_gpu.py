@@ -189,3 +189,91 @@ def test_gate_up_of_the_rule(qt, M, H, I):
     import mlxr_b200 as mx
     assert mx._capi.lib.mlxr_debug_few_tokens_rule(qt, M, H, 2 * I, 1, 1) == 1
     test_gate_up(qt, M, H, I)
+
+
+def _canonical(codes, d, dmin, sc=1, mn=8):
+    """Canonical Q4_K blocks of codes [rows, K] with one scale and minimum: w = d sc code - dmin mn."""
+    c = codes.astype(np.uint8).reshape(-1, 4, 2, 32)
+    head = np.concatenate([np.array([d, dmin], np.float16).view(np.uint8), np.array([sc] * 4 + [mn] * 4 + [sc | (mn << 4)] * 4, np.uint8)])
+    return np.concatenate([np.broadcast_to(head, (c.shape[0], 16)), (c[:, :, 0] | (c[:, :, 1] << 4)).reshape(-1, 128)], 1).reshape(-1)
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+def test_infinite_activation_in_gate_up(dt):
+    """Gate weights that are small multiples of a positive scale, without a minimum: their codes below 8 make infinity minus infinity of an
+    infinite activation in the kernel's arithmetic, infinity in float32.  Up weights of either sign, down weights of up's sign times the
+    output row's: every output is an infinity with the sign of its row."""
+    import mlxr_b200 as mx
+    M, H, I = 4, 512, 1024
+    rng = np.random.Generator(np.random.PCG64(7))
+    gate = rng.integers(1, 16, (I, H))
+    up = rng.choice([3, 5, 11, 14], (I, H))
+    s, t = np.where(up[:, 77] > 8, 1, -1), rng.choice([-1, 1], H)
+    down = np.where(t[:, None] * s[None, :] > 0, 13, 2)
+    wg, wu, wd = (torch.from_numpy(p).cuda() for p in (_canonical(gate, 1e-3, 0.0), _canonical(up, 1e-3, 1e-3), _canonical(down, 1e-3, 1e-3)))
+    assert torch.equal(torch.sign(_dense(wu, I, H, 33)[:, 77]).cpu(), torch.from_numpy(s).double()) and bool((_dense(wg, I, H, 33)[:, 77] > 0).all())
+    x = make_acts(M, H, 2, DT[dt])[0].cuda()
+    run = lambda: mx.mlp_block(x, None, wg, wu, wd, I, mx.QuantType(33), 1e-5)
+    clean = run()
+    x[1, 77] = float("inf")
+    y = run()
+    assert _status() == 0
+    assert np.array_equal(y[1].float().cpu().numpy(), t * np.float32(np.inf))
+    assert torch.equal(y[[0, 2, 3]], clean[[0, 2, 3]])
+
+
+@pytest.mark.parametrize("qt,dt", [(33, "f16"), (33, "bf16"), (0, "f16"), (3, "bf16"), (2, "bf16")])
+def test_infinite_activation_in_stacked_matrices(qt, dt):
+    """v of q / k / v (q and k are rotated: infinity times a sine of zero): the third matrix, whose rows begin inside a CTA's."""
+    import mlxr_b200 as mx
+    M, H, QH, KH, D = 5, 512, 3, 1, 44
+    w = [_weights(n * D, H, qt, i) for i, n in enumerate((QH, KH, KH))]
+    x = make_acts(M, H, 5, DT[dt])[0].cuda()
+    cos, sin = mx.compute_rope_tables(4, D, 10000.0, device=torch.device("cuda"))
+    run = lambda: mx.qkv_rope(x, None, *w, cos, sin, torch.zeros(M, dtype=torch.int32, device="cuda"), QH, KH, D, mx.QuantType(qt), 1e-5)
+    clean = run()
+    x[1, 77] = float("inf")
+    out = run()
+    assert _status() == 0
+    want = float("inf") * _dense(w[2], KH * D, H, qt)[:, 77].float()
+    nan = torch.isnan(want)
+    v = out[2].reshape(M, -1).float()
+    assert torch.equal(torch.isnan(v[1]), nan) and torch.equal(v[1][~nan], want[~nan])
+    for a, b in zip(out, clean):
+        assert torch.equal(a[[0, 2, 3, 4]], b[[0, 2, 3, 4]])
+    assert not torch.isfinite(out[1][1]).any()
+
+
+@pytest.mark.parametrize("qt", [2, 33])
+@pytest.mark.parametrize("scale", [2.0 ** -100, 1.0, 2.0 ** 100])
+def test_small_segments_decide(qt, scale):
+    """Segments of one row 2^12 apart where the large ones are not there (one token has zeros in them) or meet weights of zero (some
+    rows): norms per token and, for those rows, by themselves."""
+    N, K = 200, 1024
+    w = _weights(N, K, qt, 1)
+    if qt == 2:
+        w.view(N, K // 32, 34)[::3, :16, 2:] = 0
+    x = (make_acts(3, K, 2, torch.float32)[0] * scale).to(torch.bfloat16).cuda()
+    x[:, 512:] *= 2.0 ** -12
+    x[1, :512] = 0.0
+    y, want = _linear(x, w, N, K, qt), x.double() @ _dense(w, N, K, qt).T
+    for m in range(3):
+        _check(y[m:m + 1], want[m:m + 1], "bf16", qt)
+    if qt == 2:
+        _check(y[:, ::3].contiguous(), want[:, ::3], "bf16", qt)
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 8])
+def test_neighbours_of_a_large_activation(M):
+    """bf16 activations are fp16 numbers times a power of two per 256 from the large Q8_0 matrices of one token on: exact down to 2^-31 of the segment's
+    largest.  A large one on weights of zero, the others 2^-30 to 2^-29 of it."""
+    from mlxr_b200.quantize import quantize
+    N, K = 600, 2304
+    wf = make_weights(N, K, 3)
+    wf[:, 9::256] = 0.0
+    w = torch.from_numpy(quantize(wf, 2)).cuda()
+    x = make_acts(M, K, 4, torch.float32)[0]
+    x = torch.sign(x) * (1.0 + x.abs().clamp(max=0.99)) * 2.0 ** -20
+    x[:, 9::256] = 2.0 ** 10
+    x = x.to(torch.bfloat16).cuda()
+    _check(_linear(x, w, N, K, 2), x.double() @ _dense(w, N, K, 2).T, "bf16", 2)

@@ -295,3 +295,64 @@ def test_infinite_activation_in_two_parts(qt, dt):
     y = mx.q_gemm_dequant(x, torch.from_numpy(quantize(wf, qt)).cuda(), M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt)).float().cpu()
     assert np.array_equal(y[2].numpy(), np.where(np.arange(N) % 2 == 0, np.inf, -np.inf).astype(np.float32))
     assert torch.isfinite(y[[0, 1, 3]]).all()
+
+
+# The two-part weights of this kernel at few tokens: more activations than the kernel of whole rows takes, or more tokens
+@pytest.mark.parametrize("qt,M,N,K", [(2, 8, 200, 8192), (2, 3, 385, 16640), (33, 9, 200, 768), (33, 12, 385, 4096)])
+def test_weights_beyond_the_range_of_fp16_here(oracle, qt, M, N, K):
+    import mlxr_b200 as mx
+    assert M > 8 or M * K > 49152
+    test_weights_beyond_the_range_of_fp16(oracle, qt, M, N, K)
+
+
+def test_weights_beyond_the_range_of_fp16_in_the_other_forms_here(oracle):
+    """As in ..._in_the_other_forms: gate / up of Q8_0 and v of stacked Q4_0, 8 tokens of hidden size 8192."""
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    M, H, I = 8, 8192, 512
+    g, u, d = (quantize(make_weights(n, k, s), 2) for n, k, s in ((I, H, 1), (I, H, 2), (H, I, 3)))
+    g, u = _with_large_blocks(g, I, 32, 2000.0), _with_large_blocks(u, I, 32, 1500.0)
+    xt = (make_acts(M, H, 4, torch.float32)[0] * 1e-4).half()
+    deq = lambda w, n, k, qt: torch.from_numpy(oracle.dequantize(w, n, k, qt)[0].astype(np.float64).reshape(n, k))
+    half = lambda t: t.half().double()
+    h = half(torch.nn.functional.silu(half(xt.double() @ deq(g, I, H, 2).T)) * half(xt.double() @ deq(u, I, H, 2).T))
+    y = mx.mlp_block(xt.cuda(), None, *(torch.from_numpy(w).cuda() for w in (g, u, d)), I, mx.QuantType.Q8_0)
+    assert oracle.rel_l2(y.float().cpu().numpy(), (h @ deq(d, H, I, 2).T).numpy()) <= 2e-3
+    QH, KH, D = 3, 1, 64
+    packed = [_with_large_blocks(quantize(make_weights(n * D, H, 9 + i), 0), n * D, 32, 20000.0) for i, n in enumerate((QH, KH, KH))]
+    cos, sin = mx.compute_rope_tables(16, D, 10000.0, device=torch.device("cuda"))
+    v = mx.qkv_rope(xt.cuda(), None, *(torch.from_numpy(w).cuda() for w in packed), cos, sin, torch.arange(M, dtype=torch.int32, device="cuda"), QH, KH, D, mx.QuantType.Q4_0)[2]
+    assert oracle.rel_l2(v.float().cpu().numpy().reshape(M, -1), (xt.double() @ deq(packed[2], KH * D, H, 0).T).numpy()) <= 2.0 ** -11
+    assert _status() == 0
+
+
+@pytest.mark.parametrize("qt,dt,M,K", [(2, "bf16", 8, 8192), (2, "f16", 4, 12544), (16, "bf16", 12, 512), (2, "f16", 40, 512)])
+def test_infinite_activation_here(qt, dt, M, K):
+    import mlxr_b200 as mx
+    from mlxr_b200.quantize import quantize
+    N = 300
+    wf = make_weights(N, K, 3)
+    wf[:, 40] = np.where(np.arange(N) % 2 == 0, 0.047, -0.047)
+    x = make_acts(M, K, 4, DT[dt])[0].cuda()
+    x[2, 40] = float("inf")
+    y = mx.q_gemm_dequant(x, torch.from_numpy(quantize(wf, qt)).cuda(), M, N, K, mx.QuantType(qt), mx._capi.lib.mlxr_default_group_size(qt)).float().cpu()
+    assert np.array_equal(y[2].numpy(), np.where(np.arange(N) % 2 == 0, np.inf, -np.inf).astype(np.float32))
+    assert torch.isfinite(y[[m for m in range(M) if m != 2]]).all()
+
+
+@pytest.mark.parametrize("dt,M", [("bf16", 12), ("f16", 40)])
+def test_infinite_activation_canonical(dt, M):
+    """Canonical Q4_K weights of code 0 are their offset, of either sign or zero: what float32 products give."""
+    import mlxr_b200 as mx
+    N, K = 300, 512
+    rng = np.random.Generator(np.random.PCG64(1))
+    b = rng.integers(0, 256, (N * K // 256, 144), dtype=np.uint8)
+    b[:, :4] = rng.uniform(1e-4, 3e-4, (N * K // 256, 2)).astype(np.float16).view(np.uint8)
+    w = torch.from_numpy(b.reshape(-1)).cuda()
+    x = make_acts(M, K, 4, DT[dt])[0].cuda()
+    x[2, 77] = float("inf")
+    y = mx.q_gemm_dequant(x, w, M, N, K, mx.QuantType(33), 256).float()
+    want = x.float()[2, 77] * mx.dequantize(w, N, K, mx.QuantType(33), torch.float32)[:, 77]
+    nan = torch.isnan(want)
+    assert torch.equal(torch.isnan(y[2]), nan) and torch.equal(y[2][~nan], want[~nan])
+    assert torch.isfinite(y[[m for m in range(M) if m != 2]]).all()
