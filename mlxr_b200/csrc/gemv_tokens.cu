@@ -473,28 +473,31 @@ static size_t layout(int qt, Params* P, int grid) {
 //                   6 tokens 1000 x 8192 7.8 / 9.1; 2 tokens 256 x 16384 10.7 / 9.5.  One token of 1000 x 256 3.3 / 3.0 (the generic kernel)
 //   Q8_0            bf16 3 tokens 1000 x 11008 10.8 / 10.9, 1000 x 16384 16.3 / 12.3, 4096 x 14336 25.8 / 28.4; 8 tokens 1000 x 3072 5.8 / 6.8,
 //                   1000 x 5632 9.7 / 7.4, 3000 x 5632 13.9 / 12.3, 4096 x 5632 14.7 / 14.8
-//   Q4_K, Q4_0      (one 16-bit part per weight over there, so the products decide too) Q4_K 3 tokens 1000 x 768 3.6 / 3.3, 4096 x 1024 3.7 / 3.8,
-//                   6144 x 1024 4.4 / 4.0, 4096 x 1536 4.5 / 5.7, 8192 x 1536 5.7 / 5.1, 8192 x 2048 6.8 / 7.6, 1000 x 4096 5.0 / 5.0, 1000 x 8192
-//                   8.0 / 6.3; 8 tokens 1000 x 1024 4.0 / 3.7, 1000 x 2048 4.9 / 5.1, 1000 x 4096 7.2 / 5.3.  Q4_0 5 tokens 1000 x 3072 4.9 / 5.2
+//   Q4_K, Q4_0      (one 16-bit part per weight over there, 1.75 times as far from the exact result: left to it where it gains an eighth and more)
+//                   Q4_K 3 tokens 1000 x 768 3.6 / 3.3, 4096 x 1024 3.7 / 3.8, 6144 x 1024 4.4 / 4.0, 4096 x 1536 4.5 / 5.7, 8192 x 1536 5.7 / 5.1, 8192 x
+//                   2048 6.8 / 7.6, 1000 x 4096 5.0 / 5.1, 1000 x 8192 8.0 / 6.3; 8 tokens 1000 x 1024 4.0 / 3.7, 1000 x 2048 4.9 / 5.1, 1000 x
+//                   4096 7.2 / 5.3.  Q4_0 5 tokens 1000 x 3072 4.9 / 5.3
 //   gate / up       Q4_K 5 tokens of hidden size 1024: block of 2048 9.7 / 11.4
-//   q / k / v       Q4_K bf16 8 tokens of hidden size 2048 (3072 rows) 0.96 of the other's time, 2560 (3584) 1.10, 4096 (4352) 1.05, (6144) 0.91,
-//                   5120 (5376) 1.08; Q4_0, 6 tokens and fp16 at most 1.04
+//   q / k / v       Q4_K bf16 8 tokens of hidden size 2048 (3072 rows) 0.96 of the other's time, 2560 (3584) 1.10, 3072 (4096) 1.04,
+//                   4096 (4352) 1.05, (6144) 0.91, 5120 (5376) 1.08; canonical 5120 (6144) 0.91; Q4_0, 6 tokens and fp16 at most 1.04
 // To 2368 rows (16 for each of 148 SMs) a CTA has one tile of rows; from 1800 on the other's CTAs have as much to do as at 2368.
 bool gemv_tokens_faster(int qt, int M, int K, int rows, int form, int dtype) {
   const long long acts = (long long)M * K;
   const bool bf16 = dtype == MLXR_BF16, one_full = rows >= 1800 && rows <= 2368, two = rows > 2368;
-  if (form == kTokensStacked) return !(bf16 && qt != MLXR_Q4_0 && M >= 7 && K > 2048 && K < 6144 && 2ll * rows < 3ll * K);
+  if (form == kTokensStacked) return !(bf16 && qt != MLXR_Q4_0 && M >= 7 && K > 2048 && K < 4096 && 2ll * rows < 3ll * K);
   if (qt == MLXR_Q4_K || qt == MLXR_Q4_0) {
-    if (form == kTokensPlain && (K < 1024 || (K < 1536 && (rows > 2560 || M > (K < 1280 ? 4 : 6))) || (K < 2048 && rows > 6144))) return false;
-    // a block whose down rows are the other kernel's too: 5 tokens of 1024 x 3584 12.5 us in turns, 11.5 both there
-    if (form == kTokensGateUp && K < 1536 && rows > 4096 && (long long)M * rows > 2 * 12288) return false;
-    return acts * rows <= 3ll << 24 && (qt == MLXR_Q4_0 ? acts <= 14336 || (K <= 4096 && acts <= 16384) : K <= 2048 || acts <= 12288);
+    const long long most = qt == MLXR_Q4_K ? 18432 : 20480;
+    if (form == kTokensPlain && ((K < 1536 && rows > 4096) || (K < 2048 && rows > 6144))) return false;
+    // a block whose down rows are the other kernel's too: 6 tokens of 1024 x 3584 12.6 us in turns, 11.5 both there
+    if (form == kTokensGateUp && K < 1536 && rows > 6144 && (long long)M * rows > 2 * most) return false;
+    return acts * rows <= 3ll << 24 && acts <= most;
   }
   if (rows >= 3500) return true;
-  if (qt == MLXR_Q8_0) return acts <= (bf16 ? (one_full ? 38500 : two ? 34000 : 28000 + 3 * rows) : (one_full ? 49152 : two ? 36500 : 38000 + rows));
+  if (qt == MLXR_Q8_0) return acts <= (bf16 ? (one_full ? 39000 : two ? 34000 : 28000 + 3 * rows) : (one_full ? 49152 : two ? 36500 : 38000 + rows));
   if (M == 1 && K <= 512 && rows <= 1024) return false;
-  if (!bf16) return rows >= 3000 || K <= 8192 || (M + 2ll) * K <= 58000 + 20ll * rows;      // 8192: one stage for each of the 16 warps
-  return acts <= (one_full ? 46000 : two ? 33500 : M == 1 ? 12000 + 12 * rows : 26000 + 4 * rows);
+  if (one_full && M <= 3) return true;
+  if (!bf16) return rows >= 3000 || K <= 8192 || (rows >= 1500 && M <= 2) || (M + 2ll) * K <= 58000 + 20ll * rows;      // 8192: one stage for each of the 16 warps
+  return acts <= (one_full ? 46000 : two ? 33500 : M == 1 ? 13500 + 12 * rows : 26000 + 4 * rows);
 }
 
 bool gemv_tokens_supported(int qt, int M, int K, int rows, int form, int dtype, const void* x, const void* const* w, int nmat) {
