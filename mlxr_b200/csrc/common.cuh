@@ -282,4 +282,18 @@ template <int QT, typename T> __device__ __forceinline__ float exact_sum(const u
   return warp_sum(acc);
 }
 
+// ---- fp16 fragments of mma.sync (gemv.cu, gemv_tokens.cu) ----
+__device__ __forceinline__ void hmma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t sub_half2(uint32_t a, uint32_t b) {
+  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// Bytes 2 J and 2 J + 1 of four signed bytes, plus 128 each, as a pair of fp16 numbers, exactly: 1024 + b is 0x6400 | b
+template <int J> __device__ __forceinline__ uint32_t pair_of_bytes(uint32_t u) {
+  return sub_half2(__byte_perm(u, 0x64646464u, J == 0 ? 0x4140u : 0x4342u), 0x64806480u);
+}
+
 }  // namespace mlxr

@@ -309,16 +309,6 @@ template <int I> __device__ __forceinline__ void block_q80(const uint8_t* r, int
   for (int j = 0; j < 8; j++) v[j] = __funnelshift_rc(t[j], t[j + 1], odd ? 32 : 16);
 }
 
-__device__ __forceinline__ void hmma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// Bytes 2 J and 2 J + 1 of four signed bytes, plus 128 each, as a pair of fp16 numbers, exactly: 1024 + b is 0x6400 | b
-template <int J> __device__ __forceinline__ uint32_t pair_of_bytes(uint32_t u) {
-  const uint32_t b = __byte_perm(u, 0x64646464u, J == 0 ? 0x4140u : 0x4342u), k = 0x64806480u;
-  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&b), *reinterpret_cast<const __half2*>(&k));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
 // Q8_0: thread c feeds block 4 i + c (34 bytes); columns 2 c and 2 c + 1 stand for its two batch rows
 template <bool SCALED, int NT>
 __device__ __forceinline__ void seg_q80(const uint8_t* rl, const uint8_t* rh, const uint8_t* smem, const Params& P, int sg, const Lane& L, float (&tot)[NT][2]) {

@@ -67,17 +67,8 @@ struct Misc {
   int dead, bad;
 };
 
-__device__ __forceinline__ void hmma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 // Byte J of v as a float, exactly: 2^23 + b is 0x4B000000 | b
 template <int J> __device__ __forceinline__ float byte_f(uint32_t v) { return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440u | J)) - 8388608.0f; }
-template <int J> __device__ __forceinline__ uint32_t pair_of_bytes(uint32_t u) {      // signed bytes 2 J, 2 J + 1, plus 128 each -> fp16
-  const uint32_t b = __byte_perm(u, 0x64646464u, J == 0 ? 0x4140u : 0x4342u), k = 0x64806480u;
-  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&b), *reinterpret_cast<const __half2*>(&k));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
 __device__ __forceinline__ float lo_f(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v & 0xFFFFu))); }
 __device__ __forceinline__ float hi_f(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v >> 16))); }
 
@@ -85,13 +76,9 @@ __device__ __forceinline__ float hi_f(uint32_t v) { return __half2float(__ushort
 // a thread's fragments of two MMAs
 template <int QT> constexpr uint32_t kOrder = QT == MLXR_GGML_Q4_K ? 0x75643120u : QT == MLXR_Q8_0 ? 0x76543210u : 0x73516240u;
 
-__device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
-  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
 // The low nibbles of bytes 0 and 2 less 8; their high nibbles, 16 times that
-__device__ __forceinline__ uint32_t codes_lo(uint32_t w) { return sub2((w & 0x000F000Fu) | 0x64006400u, 0x64086408u); }
-__device__ __forceinline__ uint32_t codes_hi(uint32_t w) { return sub2((w & 0x00F000F0u) | 0x64006400u, 0x64806480u); }
+__device__ __forceinline__ uint32_t codes_lo(uint32_t w) { return sub_half2((w & 0x000F000Fu) | 0x64006400u, 0x64086408u); }
+__device__ __forceinline__ uint32_t codes_hi(uint32_t w) { return sub_half2((w & 0x00F000F0u) | 0x64006400u, 0x64806480u); }
 
 // One segment (256 weights) of 16 rows.  rl / rh: this thread's two rows at the segment; x: its token's row at the segment
 // (+ 16 c bytes); s: sums of the activations per block of 32 of its two tokens, [block][8].  a[2 h + t]: row h, token t.
@@ -118,10 +105,10 @@ template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const u
         const uint2 wl = *reinterpret_cast<const uint2*>(rl + 16 + 16 * b + 8 * c), wh = *reinterpret_cast<const uint2*>(rh + 16 + 16 * b + 8 * c);
         const uint4 xa = xblock(b), xb = xblock(b + 1);
         float lo[4] = {}, hi[4] = {};
-        hmma(lo, codes_lo(wl.x), codes_lo(wh.x), codes_lo(wl.x >> 8), codes_lo(wh.x >> 8), xa.x, xa.y);
-        hmma(hi, codes_hi(wl.x), codes_hi(wh.x), codes_hi(wl.x >> 8), codes_hi(wh.x >> 8), xb.x, xb.y);
-        hmma(lo, codes_lo(wl.y), codes_lo(wh.y), codes_lo(wl.y >> 8), codes_lo(wh.y >> 8), xa.z, xa.w);
-        hmma(hi, codes_hi(wl.y), codes_hi(wh.y), codes_hi(wl.y >> 8), codes_hi(wh.y >> 8), xb.z, xb.w);
+        hmma16816(lo, codes_lo(wl.x), codes_lo(wh.x), codes_lo(wl.x >> 8), codes_lo(wh.x >> 8), xa.x, xa.y);
+        hmma16816(hi, codes_hi(wl.x), codes_hi(wh.x), codes_hi(wl.x >> 8), codes_hi(wh.x >> 8), xb.x, xb.y);
+        hmma16816(lo, codes_lo(wl.y), codes_lo(wh.y), codes_lo(wl.y >> 8), codes_lo(wh.y >> 8), xa.z, xa.w);
+        hmma16816(hi, codes_hi(wl.y), codes_hi(wh.y), codes_hi(wl.y >> 8), codes_hi(wh.y >> 8), xb.z, xb.w);
         auto finish = [&](const float (&d)[4], float part, float sl, float sh, float nl, float nh, float2 sm) {
           add(d, sl * part, sh * part, fmaf(8.0f, sl, ml * nl), fmaf(8.0f, sh, mh * nh), sm);
         };
@@ -140,8 +127,8 @@ template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const u
     auto block = [&](int b, float (&d)[4]) {
       const uint32_t wl = *reinterpret_cast<const uint32_t*>(rl + 16 + 16 * b + 4 * c), wh = *reinterpret_cast<const uint32_t*>(rh + 16 + 16 * b + 4 * c);
       const uint4 xv = xblock(b);
-      hmma(d, codes_lo(wl), codes_lo(wh), codes_lo(wl >> 8), codes_lo(wh >> 8), xv.x, xv.y);
-      hmma(d, codes_lo(wl >> 4), codes_lo(wh >> 4), codes_lo(wl >> 12), codes_lo(wh >> 12), xv.z, xv.w);
+      hmma16816(d, codes_lo(wl), codes_lo(wh), codes_lo(wl >> 8), codes_lo(wh >> 8), xv.x, xv.y);
+      hmma16816(d, codes_lo(wl >> 4), codes_lo(wh >> 4), codes_lo(wl >> 12), codes_lo(wh >> 12), xv.z, xv.w);
     };
     auto finish = [&](int p, const float (&d)[4], float2 sm) {
       auto pair = [&](const uint4& h, float& sc, float& of) {
@@ -180,8 +167,8 @@ template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const u
       }
       const uint4 xv = xblock(b);
       float d[4] = {};
-      hmma(d, codes_lo(w[0]), codes_lo(w[1]), codes_lo(w[0] >> 8), codes_lo(w[1] >> 8), xv.x, xv.y);
-      hmma(d, codes_lo(w[0] >> 4), codes_lo(w[1] >> 4), codes_lo(w[0] >> 12), codes_lo(w[1] >> 12), xv.z, xv.w);
+      hmma16816(d, codes_lo(w[0]), codes_lo(w[1]), codes_lo(w[0] >> 8), codes_lo(w[1] >> 8), xv.x, xv.y);
+      hmma16816(d, codes_lo(w[0] >> 4), codes_lo(w[1] >> 4), codes_lo(w[0] >> 12), codes_lo(w[1] >> 12), xv.z, xv.w);
 #pragma unroll
       for (int i = 0; i < 4; i++) a[i] = fmaf(d2[i >> 1], d[i], a[i]);
     }
@@ -200,8 +187,8 @@ template <int QT> __device__ __forceinline__ void seg(const uint8_t* rl, const u
       }
       const uint4 xv = xblock(b);
       float d[4] = {};
-      hmma(d, pair_of_bytes<0>(w[0][0]), pair_of_bytes<0>(w[1][0]), pair_of_bytes<1>(w[0][0]), pair_of_bytes<1>(w[1][0]), xv.x, xv.y);
-      hmma(d, pair_of_bytes<0>(w[0][1]), pair_of_bytes<0>(w[1][1]), pair_of_bytes<1>(w[0][1]), pair_of_bytes<1>(w[1][1]), xv.z, xv.w);
+      hmma16816(d, pair_of_bytes<0>(w[0][0]), pair_of_bytes<0>(w[1][0]), pair_of_bytes<1>(w[0][0]), pair_of_bytes<1>(w[1][0]), xv.x, xv.y);
+      hmma16816(d, pair_of_bytes<0>(w[0][1]), pair_of_bytes<0>(w[1][1]), pair_of_bytes<1>(w[0][1]), pair_of_bytes<1>(w[1][1]), xv.z, xv.w);
 #pragma unroll
       for (int i = 0; i < 4; i++) a[i] = fmaf(d2[i >> 1], d[i], a[i]);
     }
