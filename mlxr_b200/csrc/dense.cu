@@ -228,8 +228,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
           tma_load_2d_pair(dst + kATile, &maps.w, kb * kBK, wrow, cbar);
         }
       }
-      // a give-up: copies in flight must land before either CTA exits; time is given to them (they take microseconds)
-      if (*dead && i > 0) for (int k = 0; k < 100; k++) __nanosleep(2000);
+      if (*dead) {
+        // a give-up: copies in flight must land before either CTA exits; time is given to them (they take microseconds)
+        if (i > 0) for (int k = 0; k < 100; k++) __nanosleep(2000);
+      } else {
+        // the stages' last releases come from the pair's issuer: none may still be on its way when this CTA exits, or it would
+        // arrive in the shared memory of whatever runs here next
+        for (int k = max(0, i - kStages); k < i; k++) mbar_wait(smem_u32(&sh->empty[k % kStages]), (uint32_t)(k / kStages) & 1u, dead);
+      }
     }
   } else if (warp == kWarpMma) {
     if (rank == 0) {
