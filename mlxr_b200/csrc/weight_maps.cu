@@ -76,6 +76,17 @@ int activation_map(const void* x, int M, int K, int dtype, int rows, CUtensorMap
                    CU_TENSOR_MAP_SWIZZLE_128B, out);
 }
 
+int activation_blocks_map(const void* x, int M, int K, int dtype, int rows, int blocks, CUtensorMap* out) {
+  EncodeTiledFn encode = nullptr;
+  if (int r = tensor_map_encoder(&encode)) return r;
+  const cuuint64_t dims[3] = {64, (cuuint64_t)M, (cuuint64_t)(K / 64)}, strides[2] = {(cuuint64_t)K * 2, 128};
+  const cuuint32_t box[3] = {64, (cuuint32_t)rows, (cuuint32_t)blocks}, estr[3] = {1, 1, 1};
+  const CUresult r = encode(out, dtype == MLXR_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(x), dims, strides, box,
+                            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed (%d) for X [%d, %d]", (int)r, M, K); return MLXR_ERR_CUDA; }
+  return MLXR_OK;
+}
+
 int result_map(void* y, int M, int N, int dtype, int box_cols, int box_rows, CUtensorMap* out) {
   return encode_2d(dtype == MLXR_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, y, N, M, (size_t)N * 2, box_cols, box_rows,
                    box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE, out);

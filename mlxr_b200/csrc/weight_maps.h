@@ -15,6 +15,8 @@ int weight_maps(int qt, const void* w, int N, int K, int tile_rows, CUtensorMap*
 int rows_map(const void* w, int rows, size_t row_bytes, int box_bytes, int box_rows, CUtensorMap* out);
 // X [M, K] of a 16-bit type, boxes of 64 x `rows` with the 128-byte swizzle; rows past M read as zero
 int activation_map(const void* x, int M, int K, int dtype, int rows, CUtensorMap* out);
+// The same with `blocks` consecutive 64-wide k-blocks in a box, one [rows][64] tile behind the other: coordinates (0, row, k-block)
+int activation_blocks_map(const void* x, int M, int K, int dtype, int rows, int blocks, CUtensorMap* out);
 // Y [M, N] of a 16-bit type for stores, boxes of box_cols (16: plain, 32: 64-byte swizzle) x box_rows
 int result_map(void* y, int M, int N, int dtype, int box_cols, int box_rows, CUtensorMap* out);
 int device_sms(int* out);

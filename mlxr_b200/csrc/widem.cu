@@ -19,7 +19,7 @@
 // * With few tiles per pair the units are dealt to the pairs in equal contiguous ranges and shared tiles
 //   are added up by the CTA that delivers the last part; with many, every pair takes whole tiles.
 // * Four groups of four producer warps convert a 64-wide k-block of the unit each, double-buffered in
-//   tensor memory; a k-block's weights and its X tile share a stage and with it one barrier each way; one warp of the pair's first CTA issues; X comes a 64-wide k-block at a time.
+//   tensor memory; two k-blocks' weights and X tiles share a stage and with it one barrier each way; one warp of the pair's first CTA issues.
 // * Weights are rounded once to the activation dtype (fp16: the reference shader's half arithmetic).
 // * Waits are bounded and reported as in smallm.cu; every barrier is waited on by one role in phase order.
 #include <cuda.h>
@@ -45,7 +45,13 @@ using namespace wconv;
 constexpr int kRows = 128, kBK = 64;
 constexpr int kGroups = 4;                 // producer groups of four warps; group g converts k-block g of every unit
 constexpr int kSlots = 2;                  // converted k-blocks per group
-constexpr int kStages = kGroups * kSlots;  // k-blocks in flight: stage g * kSlots + (unit & 1) holds k-block g's weights and X tile
+// A stage is half a unit, two k-blocks: their converted weights (two groups' slots) and their X tiles (one copy), with one
+// barrier each way.  What a hand-over costs the warps that copy X and issue MMAs is the same for one k-block as for two:
+// with a stage and a copy for each k-block the copy warp needed 500 cycles for one (time stamps; the conversion 400),
+// 2050 a unit whatever the number of tokens; see the figures in widem_plan.
+constexpr int kBlocks = 2;
+constexpr int kHalves = kGroups / kBlocks;
+constexpr int kStages = kHalves * kSlots;  // stage (unit & 1) * kHalves + half
 constexpr int kSlotCols = kBK / 2;         // tensor-memory columns of one: two 16-bit elements each
 [[maybe_unused]] constexpr int kWarpMma = 0, kWarpRaw = 1, kWarpX = 2, kWarpFix = 3, kWarpEpi0 = 4, kWarpProd0 = 8;
 constexpr int kThreads = (kWarpProd0 + 4 * kGroups) * 32;
@@ -71,7 +77,7 @@ struct Params {
 struct Maps { CUtensorMap x, w[4]; };
 
 struct Shared {
-  uint64_t full[kStages];       // (first CTA) both CTAs' producer warps have written the k-block, both halves of X have landed
+  uint64_t full[kStages];       // (first CTA) both CTAs' producer warps have written their k-blocks, both halves of X have landed
   uint64_t empty[kStages];      // the MMAs that read it are done
   uint64_t raw_full[kMaxRawStages], raw_empty[kMaxRawStages];
   uint64_t acc_full[2], acc_empty[2];
@@ -84,9 +90,9 @@ struct Shared {
 
 template <int QT, int NMAX> struct Rings {
   static constexpr int kRawBytes = kRows * Geo<QT>::kStage;
-  static constexpr int kXTile = NMAX / 2 * kBK * 2;                          // this CTA's half of the tokens; nt / 2 rows are used
+  static constexpr int kXStage = kBlocks * NMAX / 2 * kBK * 2;               // this CTA's half of the tokens, two tiles of nt / 2 rows
   static constexpr int kRawStages = QT != MLXR_Q8_0 ? 4 : 2;
-  static constexpr size_t kBytes = (size_t)kStages * kXTile + (size_t)kRawStages * kRawBytes;
+  static constexpr size_t kBytes = (size_t)kStages * kXStage + (size_t)kRawStages * kRawBytes;
   static constexpr int kBufs = NMAX == 128 ? 2 : 1;
   static constexpr uint32_t kA0 = 256, kCols = 512;                          // accumulators in columns 0 .. 255
 };
@@ -130,11 +136,11 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
   }
   using R = Rings<QT, NMAX>;
-  constexpr int kRawStages = R::kRawStages, kXTile = R::kXTile, kRawBytes = R::kRawBytes;
+  constexpr int kRawStages = R::kRawStages, kXStage = R::kXStage, kRawBytes = R::kRawBytes;
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw & 1023u)) & 1023u;
   uint8_t* xring = smem_raw + pad;
-  uint8_t* rawring = xring + (size_t)kStages * kXTile;
+  uint8_t* rawring = xring + (size_t)kStages * kXStage;
   Shared* sh = reinterpret_cast<Shared*>(rawring + (size_t)kRawStages * kRawBytes);
   volatile int* dead = &sh->dead;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -178,7 +184,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     sh->ntodo = 0;
     sh->epi_fail = 0;
     for (int s = 0; s < kStages; s++) {
-      mbar_init(smem_u32(&sh->full[s]), 4 * 2 + 1);    // four producer warps of both CTAs, the copy warp's byte count
+      mbar_init(smem_u32(&sh->full[s]), kBlocks * 4 * 2 + 1);    // the groups' four warps of both CTAs, the copy warp's byte count
       mbar_init(smem_u32(&sh->empty[s]), 1);
     }
     for (int a = 0; a < 2; a++) {
@@ -206,7 +212,8 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     const int mat_off = (SWIGLU && lane >= 16) ? 64 : 0;
     const int row_off = (kSplitRows ? mat_off + (local & 1) * (mrows / 2) + (local >> 1) : mat_off + local) * Geo<QT>::kStage;
     const uint32_t col = tmem + R::kA0 + (uint32_t)(g * kSlots * kSlotCols) + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint32_t full[2] = {cluster_map(smem_u32(&sh->full[g * kSlots]), 0), cluster_map(smem_u32(&sh->full[g * kSlots + 1]), 0)};
+    const int half = g / kBlocks;
+    const uint32_t full[2] = {cluster_map(smem_u32(&sh->full[half]), 0), cluster_map(smem_u32(&sh->full[kHalves + half]), 0)};
     int r = 0, sb = sb_first;
     uint32_t rpar = 0;
     for (int i = 0; i < nunits; i++) {
@@ -214,7 +221,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->raw_full[r]), rpar, dead))) break;   // warp-uniform
       const uint8_t* row = rawring + (size_t)r * kRawBytes + row_off;
       if constexpr (kSplitRows) row += (136 * sb + ((local & 1) ? P.odd_shift : 0)) & 8;
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty[g * kSlots + q]), (uint32_t)((i >> 1) & 1) ^ 1u, dead))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty[q * kHalves + half]), (uint32_t)((i >> 1) & 1) ^ 1u, dead))) break;
       tc_fence_after();
       convert64<QT, BF, kRound>(row, g, Levels{sh->nf4}, [&](auto H, const uint32_t (&a)[16], const uint32_t (&)[16]) {
         tmem_st16(col + q * kSlotCols + 16 * decltype(H)::value, a);
@@ -232,6 +239,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     const uint32_t idesc = instr_desc(BF, BF, 2 * kRows, P.nt);
     const uint64_t desc_hi = smem_desc_sw128(0);
     const uint32_t x_lo0 = (smem_u32(xring) & 0x3FFFFu) >> 4, tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t x_tile = (uint32_t)P.nt * (kBK >> 4);         // nt / 2 rows of 128 bytes, in units of 16 bytes
     bool ok = true;
     for (int i0 = 0, part = 0, cnt; i0 < nunits && ok; i0 += cnt, part++) {
       cnt = min(part == 0 ? P.nsb - sb_first : P.nsb, nunits - i0);
@@ -241,17 +249,20 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       for (int i = i0; i < i0 + cnt && ok; i++) {
         const int q = i & 1;
 #pragma unroll
-        for (int g = 0; g < kGroups; g++) {
-          const int st = g * kSlots + q;
+        for (int h = 0; h < kHalves; h++) {
+          const int st = q * kHalves + h;
           ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&sh->full[st]), (uint32_t)(i >> 1) & 1u, dead));
           if (!ok) break;
           tc_fence_after();
-          const uint32_t acol = tm + R::kA0 + (uint32_t)(st * kSlotCols);
-          const uint64_t xdesc = desc_hi | (uint64_t)(x_lo0 + (uint32_t)st * (kXTile >> 4));
+          const uint32_t acol = tm + R::kA0 + (uint32_t)((h * kBlocks * kSlots + q) * kSlotCols);
+          const uint64_t xdesc = desc_hi | (uint64_t)(x_lo0 + (uint32_t)st * (kXStage >> 4));
           if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < kBK / kUmmaK; k++)
-              umma_f16_ts_pair(dcol, acol + k * (kUmmaK / 2), xdesc + (uint64_t)(k * (kUmmaK * 2 >> 4)), idesc, (i > i0 || g > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < kBlocks * kBK / kUmmaK; k++) {
+              const int kb = k / (kBK / kUmmaK), kk = k % (kBK / kUmmaK);
+              umma_f16_ts_pair(dcol, acol + kb * kSlots * kSlotCols + kk * (kUmmaK / 2), xdesc + (uint64_t)(kb * x_tile + kk * (kUmmaK * 2 >> 4)), idesc,
+                               (i > i0 || h > 0 || k > 0) ? 1u : 0u);
+            }
             umma_commit_pair(smem_u32(&sh->empty[st]));
           }
           __syncwarp();
@@ -279,24 +290,31 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       }
     }
   } else if (warp == kWarpX) {
-    // ===== activations: this CTA's half of the X tile [nt rows, 64 columns], one per k-block; both halves
-    // complete on the first CTA's barrier =====
-    if (lane == 0) {
-      int issued = 0, t = t_first, kb = 4 * sb_first;
-      int tok = tile_of(P, t).tt * P.nt + rank * (P.nt / 2);
-      asm volatile("griddepcontrol.wait;" ::: "memory");      // X may be the previous kernel's output
-      for (int i = 0; i < 4 * nunits; i++) {
-        const int st = (i & 3) * kSlots + ((i >> 2) & 1);
-        if (!mbar_wait(smem_u32(&sh->empty[st]), (uint32_t)((i >> 3) & 1) ^ 1u, dead)) break;
-        const uint32_t bar = smem_u32(&sh->full[st]);
-        if (rank == 0) mbar_expect_tx(bar, (uint32_t)P.nt * kBK * 2);
-        tma_load_2d_pair(smem_u32(xring + (size_t)st * kXTile), &maps.x, kb * kBK, tok, cluster_map(bar, 0));
-        issued = i + 1;
-        if (++kb == 4 * P.nsb && i + 1 < 4 * nunits) { kb = 0; t++; tok = tile_of(P, t).tt * P.nt + rank * (P.nt / 2); }
+    // ===== activations: this CTA's half of two X tiles [nt rows, 64 columns] per stage, one copy; both CTAs' complete on the
+    // first one's barrier.  The whole warp walks the loop, one elected lane issues. =====
+    int issued = 0, t = t_first, hb = kHalves * sb_first;
+    int tok = tile_of(P, t).tt * P.nt + rank * (P.nt / 2);
+    const uint32_t bytes = kBlocks * (uint32_t)P.nt * kBK * 2;
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // X may be the previous kernel's output
+    for (int i = 0; i < kHalves * nunits; i++) {
+      const int st = i % kStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty[st]), (uint32_t)((i / kStages) & 1) ^ 1u, dead))) break;
+      const uint32_t bar = smem_u32(&sh->full[st]);
+      if (elect_one()) {
+        if (rank == 0) mbar_expect_tx(bar, bytes);
+        tma_load_3d_pair(smem_u32(xring + (size_t)st * kXStage), &maps.x, 0, tok, kBlocks * hb, cluster_map(bar, 0));
       }
+      __syncwarp();
+      issued = i + 1;
+      if (++hb == kHalves * P.nsb && i + 1 < kHalves * nunits) { hb = 0; t++; tok = tile_of(P, t).tt * P.nt + rank * (P.nt / 2); }
+    }
+    if (*dead) {
       // a give-up: copies in flight must land before either CTA exits; their barrier also counts the producers,
       // so time is given to them instead (a copy takes microseconds)
-      if (*dead && issued > 0) for (int i = 0; i < 100; i++) __nanosleep(2000);
+      if (issued > 0) for (int i = 0; i < 100; i++) __nanosleep(2000);
+    } else {
+      // the last releases of the stages come from the other CTA as well: none may be on its way when this one exits
+      for (int i = max(0, issued - kStages); i < issued; i++) mbar_wait(smem_u32(&sh->empty[i % kStages]), (uint32_t)(i / kStages) & 1u, dead);
     }
   } else if (warp == kWarpFix) {
     // ===== shared tiles: once the epilogue has parked a part, count it; the CTA that delivers a tile's
@@ -551,7 +569,7 @@ int launch_widem(const void* x, const void* w, const void* w2, const void* bias,
   widem::Params P;
   memset(&maps, 0, sizeof(maps));
   memset(&P, 0, sizeof(P));
-  if (int r = activation_map(x, M, K, dtype, plan.nt / 2, &maps.x)) return r;
+  if (int r = activation_blocks_map(x, M, K, dtype, plan.nt / 2, widem::kBlocks, &maps.x)) return r;
   const int tile_rows = swiglu ? 64 : widem::kRows;
   if (int r = weight_maps(qt, w, N, K, tile_rows, maps.w, &P.odd_shift)) return r;
   if (swiglu)
