@@ -187,7 +187,7 @@ static int run_tc(TcPath path, const WidePlan& wide, const DensePlan& dense, con
                   int M, int N, int K, int qt, int dtype, cudaStream_t st) {
   int grid = 0, maxc = 0;
   size_t part = path == kTcWide ? wide.partial_bytes : 0;
-  if (path == kTcSmall) { if (int r = smallm_plan(M, w2 ? 2 * N : N, K, &grid, &maxc, &part)) return r; }
+  if (path == kTcSmall) { if (int r = smallm_plan(qt, false, M, w2 ? 2 * N : N, K, &grid, &maxc, &part)) return r; }
   Workspace* ws = nullptr;
   if (int r = get_workspace(st, 0, &ws)) return r;
   {
@@ -751,7 +751,7 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
     // tokens 31 -> 12.6 us; 8192, 64 tokens 49 -> 31; 1280, 36 tokens 27 -> 10.6.
     int grid = 0, maxc = 0;
     size_t part = 0;
-    if (int r = smallm_plan(M, 128 * tiles, hidden, &grid, &maxc, &part)) return r;
+    if (int r = smallm_plan(qt, true, M, 128 * tiles, hidden, &grid, &maxc, &part)) return r;
     {
       std::lock_guard<std::mutex> lk(g_ws_mu);
       if (int r = grow(&ws->part, &ws->part_bytes, part, st)) return r;

@@ -137,7 +137,7 @@ bool smallm_supported(int qt, int M, int N, int K, int dtype, const void* x, con
 void smallm_partition(long long units, int ctas, int cta, long long unit, long long* begin, long long* end, int* owner);
 // grid size, the most CTAs that share one output tile, and the bytes of fp32 partial sums needed;
 // rows = weight rows streamed (N, or 2 N for the gate/up form)
-int smallm_plan(int M, int rows, int K, int* grid, int* maxc, size_t* partial_bytes);
+int smallm_plan(int qt, bool stacked, int M, int rows, int K, int* grid, int* maxc, size_t* partial_bytes);
 // nmat stacked matrices y[i] [M, rows[i]] = X w[i]^T (+ bias, one matrix only), or swiglu: w[0] = gate, w[1] = up
 int launch_smallm(const void* x, const void* const* w, const int* rows, int nmat, bool swiglu, const void* bias, void* const* y, int M, int K, int qt, int dtype,
                   int* status, float* partials, uint32_t* counters, int grid, int maxc, cudaStream_t st);

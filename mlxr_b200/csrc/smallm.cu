@@ -67,7 +67,7 @@ constexpr int kBlockCols = kBK / 2;        // tensor-memory columns of a k-block
 [[maybe_unused]] constexpr int kWarpMma = 0, kWarpRaw = 2, kWarpX = 3, kWarpEpi0 = 4, kWarpProd0 = 8;   // two issuer warps: 0 and 1
 constexpr int kWarpFix = kWarpProd0 + 4 * kGroups;                                     // counts shared tiles
 constexpr int kThreads = (kWarpFix + 1) * 32;
-constexpr int kMaxXStages = 4, kMaxRawStages = 2 * kGroups;
+constexpr int kMaxXStages = 4, kMaxXBars = 6, kMaxRawStages = 2 * kGroups;
 constexpr int kSmemMax = 227 * 1024;
 
 struct Params {
@@ -80,6 +80,7 @@ struct Params {
   int ntiles;          // ceil(rows / 128)
   int maxc;            // most CTAs that share one tile
   int odd_shift;       // NF4: byte offset of odd rows within their tensor map (0 or 8)
+  int vec_stores;      // bit i: rows of y[i] start on 16 bytes
   long long U;         // units = ntiles * nsb
   int* status;
   float* partials;     // [ntiles][maxc][NPAD][128] fp32
@@ -110,11 +111,10 @@ struct Shared {
   // The group's four warps have written the slot.  Consecutive units of a group belong to different
   // issuers, so even and odd units signal through barriers of their own: a barrier is waited on by one
   // issuer, which sees every phase of it in turn.  (With one barrier per slot an issuer a unit ahead
-  // of the other would take the parity of the phase before last for completion.)  The same rule makes
-  // the number of X stages even.
+  // of the other would take the parity of the phase before last for completion.)
   uint64_t full_a[kGroups][kSlots][2];
   uint64_t empty_a[kGroups][kSlots];   // the MMAs that read it are done
-  uint64_t x_full[kMaxXStages];        // the four X tiles of a unit have landed
+  uint64_t x_full[kMaxXBars];          // the four X tiles of a unit have landed
   uint64_t x_empty[kMaxXStages];
   uint64_t raw_full[kMaxRawStages];
   uint64_t raw_empty[kMaxRawStages];
@@ -126,7 +126,24 @@ struct Shared {
   int todo_tile[2], todo_parts[2];
   int epi_fail;
   int bad;                      // kSplit: some sum was not finite
+  alignas(16) uint16_t turn[4][16 * 32];    // epilogue warps: sixteen tokens' results on their way to 16-byte stores
 };
+
+// The table that a format's producers look codes up in, behind the rings: NF4, and 4-bit codes that are multiplied in
+// 16-bit arithmetic.  The latter with a copy per lane leaves three instructions per pair of codes where the arithmetic takes four or
+// five (14336 x 4096 Q4_K, 16 tokens: 12.6 us with arithmetic, 10.6 so), but 64 KB less for the rings: at batch 64 X needs
+// them.  (NF4's pairs are of float32 and take two cycles of shared memory each, which is its limit: a copy per lane gains nothing.)
+struct NoTable {
+  static constexpr int kBytes = 0;
+  __device__ __forceinline__ NoTable(const uint8_t*, int) {}
+  static __device__ __forceinline__ void fill(uint8_t*, int, int) {}
+};
+template <int QT, int BF, int NPAD, int MODE> struct TableOf { using type = NoTable; };
+template <int BF, int NPAD, int MODE> struct TableOf<MLXR_NF4, BF, NPAD, MODE> { using type = PairLevels; };
+template <int BF> struct TableOf<MLXR_Q4_K, BF, 16, kFast> { using type = CodePairs<BF>; };
+template <int BF> struct TableOf<MLXR_Q4_K, BF, 32, kFast> { using type = CodePairs<BF>; };
+template <int BF> struct TableOf<MLXR_Q4_0, BF, 16, kFast> { using type = CodePairs<BF>; };
+template <int BF> struct TableOf<MLXR_Q4_0, BF, 32, kFast> { using type = CodePairs<BF>; };
 
 // first unit of CTA c, and the CTA that owns unit u, when U units are dealt to G CTAs
 __host__ __device__ inline long long unit_begin(long long U, int G, int c) { return (U * c) / G; }
@@ -151,12 +168,15 @@ __device__ __forceinline__ void note_bad(float& t, float v) { t = fmaf(v, 0.0f, 
 
 __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-template <int QT, int NPAD> struct Rings {
+template <int QT, int NPAD, int TABLE> struct Rings {
   static constexpr int kRawBytes = kRows * Geo<QT>::kStage;                 // packed rows of one unit
   static constexpr int kXTile = NPAD * kBK * 2;                             // one k-block of X
   static constexpr int kXUnit = 4 * kXTile;                                 // the four k-blocks of a unit
-  static constexpr int kXStages = NPAD == 64 ? 2 : 4;                // even: see Shared::full_a
-  static constexpr int kTable = QT == MLXR_NF4 ? PairLevels::kBytes : 0;
+  static constexpr int kTable = TABLE;
+  static constexpr int kXStages = NPAD == 64 ? 2 : NPAD == 32 && TABLE > 32768 ? 3 : 4;
+  // barriers of the X stages' arrival: as units alternate between the issuers, an odd number of stages needs two of each (see
+  // Shared::full_a)
+  static constexpr int kXBars = kXStages % 2 ? 2 * kXStages : kXStages;
   static constexpr int kFree = kSmemMax - kXStages * kXUnit - kTable - (int)sizeof(Shared) - 1024;
   // a multiple of the number of groups, so that a stage's barrier is always waited on by one group
   static constexpr int kRawStages = kFree / kRawBytes >= 2 * kGroups ? 2 * kGroups : kGroups;
@@ -177,7 +197,7 @@ template <int QT, typename T, int NPAD, int MODE, int FORM>
 __global__ void __launch_bounds__(kThreads, 1)
 qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
   constexpr bool SWIGLU = FORM == kSwiglu;
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(16) uint8_t smem_raw[];
   constexpr int BF = Fmt<T>::v;
   constexpr bool kSplitRows = QT == MLXR_NF4;                 // even and odd rows come through maps of their own
   // the TMA unit fetches a tensor map on first use: ask for them before anything else
@@ -187,15 +207,15 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     if (threadIdx.x == 6 || threadIdx.x < mats * (kSplitRows ? 2 : 1))
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
   }
-  using R = Rings<QT, NPAD>;
-  constexpr int kXStages = R::kXStages, kRawStages = R::kRawStages, kXTile = R::kXTile, kXUnit = R::kXUnit, kRawBytes = R::kRawBytes;
+  using Tab = typename TableOf<QT, BF, NPAD, MODE>::type;
+  using R = Rings<QT, NPAD, Tab::kBytes>;
+  constexpr int kXStages = R::kXStages, kXBars = R::kXBars, kRawStages = R::kRawStages, kXTile = R::kXTile, kXUnit = R::kXUnit, kRawBytes = R::kRawBytes;
   constexpr int kSteps = MODE == kSplit ? 4 : 2;              // slots filled per unit
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw & 1023u)) & 1023u;       // X tiles need 1024-byte alignment (128-byte swizzle)
-  uint8_t* smem = smem_raw + pad;
-  uint8_t* xring = smem;
+  uint8_t* xring = smem_raw + pad;
   uint8_t* rawring = xring + (size_t)kXStages * kXUnit;
-  [[maybe_unused]] uint8_t* table = rawring + (size_t)kRawStages * kRawBytes;      // NF4
+  uint8_t* table = rawring + (size_t)kRawStages * kRawBytes;       // in front of the rings the tables cost 2 to 5 % of a launch
   Shared* sh = reinterpret_cast<Shared*>(table + R::kTable);
   volatile int* dead = &sh->dead;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -245,10 +265,8 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
         mbar_init(smem_u32(&sh->full_a[g][s][1]), 4);
         mbar_init(smem_u32(&sh->empty_a[g][s]), 1);
       }
-    for (int r = 0; r < kXStages; r++) {
-      mbar_init(smem_u32(&sh->x_full[r]), 1);
-      mbar_init(smem_u32(&sh->x_empty[r]), 1);
-    }
+    for (int r = 0; r < kXBars; r++) mbar_init(smem_u32(&sh->x_full[r]), 1);
+    for (int r = 0; r < kXStages; r++) mbar_init(smem_u32(&sh->x_empty[r]), 1);
     for (int a = 0; a < 2; a++) {
       mbar_init(smem_u32(&sh->acc_full[a]), 2);
       mbar_init(smem_u32(&sh->acc_empty[a]), 4);       // the four epilogue warps
@@ -256,7 +274,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if constexpr (QT == MLXR_NF4) PairLevels::fill(table, tid, kThreads);
+  Tab::fill(table, tid, kThreads);
   if (warp == kWarpMma) tmem_alloc(smem_u32(&sh->tmem_base), R::kCols);
   tc_fence_before();
   __syncthreads();
@@ -279,7 +297,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
     const int row_off = (kSplitRows ? mat_off + (local & 1) * (mrows / 2) + (local >> 1) : mat_off + local) * Geo<QT>::kStage;
     const uint32_t a_col = tmem + R::kA0 + (uint32_t)(g * kSlots * 2 * kBlockCols) + ((uint32_t)((warp & 3) * 32) << 16);
     int r = g;
-    [[maybe_unused]] const PairLevels levels(table, lane);
+    const Tab levels(table, lane);
     uint32_t rpar = 0, use = 0;         // use: how often this group's slots have been filled
     for (int i = g; i < nunits; i += kGroups) {
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->raw_full[r]), rpar, dead))) break;   // warp-uniform
@@ -346,7 +364,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
       for (int i = first; i < i0 + cnt && ok; i += 2) {
         const int g = i % kGroups, xs = i % kXStages;
         const uint32_t use = (uint32_t)(i / kGroups);
-        ok = mbar_wait(smem_u32(&sh->x_full[xs]), (uint32_t)(i / kXStages) & 1u, dead);
+        ok = mbar_wait(smem_u32(&sh->x_full[i % kXBars]), (uint32_t)(i / kXBars) & 1u, dead);
         const uint32_t acol = tm + R::kA0 + (uint32_t)(g * kSlots * 2 * kBlockCols);
         const uint64_t xdesc = desc_hi | (uint64_t)(x_lo0 + (uint32_t)xs * (kXUnit >> 4));
 #pragma unroll
@@ -393,27 +411,28 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
       }
     }
   } else if (warp == kWarpX) {
-    // ===== activations: per unit the four X tiles [NPAD rows, 64 columns] of its super-block =====
-    if (lane == 0) {
-      int issued = 0, sb = sb_first, xs = 0;
-      uint32_t par = 0;
-      asm volatile("griddepcontrol.wait;" ::: "memory");      // X may be the previous kernel's output
-      for (int i = 0; i < nunits; i++) {
-        if (!mbar_wait(smem_u32(&sh->x_empty[xs]), par ^ 1u, dead)) break;
-        const uint32_t bar = smem_u32(&sh->x_full[xs]);
+    // ===== activations: per unit the four X tiles [NPAD rows, 64 columns] of its super-block (one copy of all four
+    // took NF4 at 64 tokens, 4096 x 14336, from 18.9 to 19.8 us).  The whole warp walks the loop, one elected lane issues. =====
+    int issued = 0, sb = sb_first;
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // X may be the previous kernel's output
+    for (int i = 0; i < nunits; i++) {
+      const int xs = i % kXStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->x_empty[xs]), ((uint32_t)(i / kXStages) & 1u) ^ 1u, dead))) break;
+      if (elect_one()) {
+        const uint32_t bar = smem_u32(&sh->x_full[i % kXBars]);
         mbar_expect_tx(bar, kXUnit);
 #pragma unroll
         for (int jj = 0; jj < 4; jj++)
           tma_load_2d(smem_u32(xring + (size_t)xs * kXUnit + (size_t)jj * kXTile), &maps.x, (4 * sb + jj) * kBK, 0, bar);
-        issued = i + 1;
-        if (++sb == P.nsb) sb = 0;
-        if (++xs == kXStages) { xs = 0; par ^= 1u; }
       }
-      if (*dead) {
-        for (int i = max(0, issued - kXStages); i < issued; i++) {
-          const uint32_t bar = smem_u32(&sh->x_full[i % kXStages]);
-          for (uint32_t sp = 0; sp < kSpin; sp++) if (mbar_try(bar, (i / kXStages) & 1)) break;
-        }
+      __syncwarp();
+      issued = i + 1;
+      if (++sb == P.nsb) sb = 0;
+    }
+    if (*dead) {
+      for (int i = max(0, issued - kXStages); i < issued; i++) {
+        const uint32_t bar = smem_u32(&sh->x_full[i % kXBars]);
+        for (uint32_t sp = 0; sp < kSpin; sp++) if (mbar_try(bar, (i / kXBars) & 1)) break;
       }
     }
   } else if (warp == kWarpFix) {
@@ -462,21 +481,14 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
       // output column of this lane: its weight row, or for SWIGLU the gate row that lanes l and l + 16 share
       const Place at = place_of<FORM>(P, t);
       const int N = P.rows[at.mat], n = SWIGLU ? 64 * at.tile + 16 * quarter + (lane & 15) : at.tile * kRows + rt;
-      const bool writer = (!SWIGLU || lane < 16) && n < N;
       T* y = reinterpret_cast<T*>(P.y[at.mat]);
-      // sums of one batch row -> Y: plain (+ bias), or SiLU(gate) * up across the lane pair
-      auto finish = [&](float v, float bv) -> T {
-        if constexpr (SWIGLU) {
-          const float o = __shfl_xor_sync(0xffffffffu, v, 16);        // lanes < 16: v = gate, o = up
-          const float gv = Act<T>::to_f(Act<T>::from_f(v)), uv = Act<T>::to_f(Act<T>::from_f(o));
-          return Act<T>::from_f(swish_fast(gv) * uv);
-        } else {
-          return Act<T>::from_f(v + bv);
-        }
-      };
       const int slot = whole ? 0 : cta - unit_owner(P.U, G, (long long)t * P.nsb);
       float* part = P.partials + (((size_t)t * P.maxc + slot) * NPAD) * kRows + rt;
       const float bv = (!SWIGLU && bias && n < N) ? Act<T>::to_f(bias[n]) : 0.0f;
+      // this warp's first output column; all its columns exist and start on 16 bytes
+      constexpr int kCols = SWIGLU ? 16 : 32;
+      const int nw = SWIGLU ? 64 * at.tile + 16 * quarter : at.tile * kRows + 32 * quarter;
+      const bool vec = ((P.vec_stores >> at.mat) & 1) && nw + kCols <= N;
 #pragma unroll 1
       for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) {
         uint32_t r[16];
@@ -495,13 +507,42 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
           for (int c = 0; c < 16; c++) note_bad(bad, __uint_as_float(r[c]));
         }
         if (whole) {
+          // sixteen tokens x 32 weight rows (gate/up: 16 columns, SiLU of every other token on the upper lanes) turn in shared
+          // memory into 16-byte stores: with a 2-byte store per lane and token a round of sixteen took 1400 cycles
+          uint16_t* turn = sh->turn[quarter];
+          if constexpr (SWIGLU) {
+            const bool up = lane >= 16;
 #pragma unroll
-          for (int c = 0; c < 16; c++) {
-            if (c0 + c < P.M) {             // uniform: every lane takes part in the exchange
-              const T o = finish(__uint_as_float(r[c]), bv);
-              if (writer) y[(size_t)(c0 + c) * N + n] = o;
+            for (int c = 0; c < 16; c += 2) {
+              const float a = __uint_as_float(r[c]), b = __uint_as_float(r[c + 1]);
+              const float o = __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+              const float gv = Act<T>::to_f(Act<T>::from_f(up ? o : a)), uv = Act<T>::to_f(Act<T>::from_f(up ? b : o));
+              const T h = Act<T>::from_f(swish_fast(gv) * uv);
+              turn[(c + (up ? 1 : 0)) * kCols + (lane & 15)] = *reinterpret_cast<const uint16_t*>(&h);
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 16; c++) {
+              const T o = Act<T>::from_f(__uint_as_float(r[c]) + bv);
+              turn[c * kCols + lane] = *reinterpret_cast<const uint16_t*>(&o);
             }
           }
+          __syncwarp();
+          if (vec) {
+            constexpr int kPer = kCols / 8;                                // 16-byte pieces per token
+#pragma unroll
+            for (int e = 0; e < 16 * kPer / 32; e++) {
+              const int piece = e * 32 + lane, tk = piece / kPer, pc = piece % kPer;
+              if (c0 + tk < P.M) *reinterpret_cast<uint4*>(y + (size_t)(c0 + tk) * N + nw + pc * 8) = *reinterpret_cast<const uint4*>(turn + tk * kCols + pc * 8);
+            }
+          } else {
+#pragma unroll 4
+            for (int e = lane; e < 16 * kCols; e += 32) {
+              const int tk = e / kCols, col = nw + e % kCols;
+              if (c0 + tk < P.M && col < N) y[(size_t)(c0 + tk) * N + col] = *reinterpret_cast<const T*>(turn + e);
+            }
+          }
+          __syncwarp();
         } else {
 #pragma unroll
           for (int c = 0; c < 16; c++)
@@ -638,22 +679,29 @@ bool smallm_supported(int qt, int M, int N, int K, int dtype, const void* x, con
   return true;
 }
 
-int smallm_plan(int M, int rows, int K, int* grid, int* maxc, size_t* partial_bytes) {
+int smallm_plan(int qt, bool stacked, int M, int rows, int K, int* grid, int* maxc, size_t* partial_bytes) {
   const int N = rows;
   int sms = 0;
   if (int r = device_sms(&sms)) return r;
   const int nsb = K / 256, ntiles = (N + smallm::kRows - 1) / smallm::kRows;
   const long long U = (long long)ntiles * nsb;
   // Either all SMs get equal ranges, which cross tiles, or every tile gets c CTAs of its own (the same formula with
-  // c * ntiles CTAs).  Measured with Q4_K (a unit of the other formats takes longer, which the plan does not know) at K = 4096, widths 16 and 64 of the padded batch: a unit takes 0.58 / 0.90 us, a
-  // shared tile 1.6 / 2.0 us plus 0.16 / 0.77 per part (parked, counted, read by the CTA that adds them), and
-  // a range that crosses tiles 1.5 more, because its CTA parks two parts (2368 rows, batch 16: 8.4 us with equal
-  // ranges on 148 SMs, 6.7 with four CTAs for each of the 19 tiles; 4096 rows, batch 64: 11.8 and 10.0).
-  const double w = smallm_npad(M), unit = 0.47 + 0.0067 * w, shared = 1.5 + 0.0085 * w, part = 0.012 * w;
+  // c * ntiles CTAs).  Fitted, in us, to 825 measurements (five formats; 12, 32 and 64 tokens; ten sizes from 1500 x 2048 to 14336 x 4096; the
+  // choice by this estimate takes 0.8 % more than the best one in the mean, 24 % at most; by one fitted to Q4_K alone, before the tables,
+  // 2.6 %: 8192 x 2048 Q4_K 64 tokens 22 % with two CTAs a tile instead of one, 11008 x 4096 canonical Q4_K 26 % with one instead of equal
+  // ranges).  A unit takes what its conversion does, and as much as two of them if a CTA has only one (the groups of
+  // producers take units in turn); a shared tile its parts' trip through L2, which all CTAs make at the same time; a range that crosses
+  // tiles 1.35 more, because its CTA parks two parts.
+  const double w = smallm_npad(M);
+  const bool split = qt == MLXR_GGML_Q4_K || (M <= 8 && (stacked || qt == MLXR_Q8_0 || qt == MLXR_NF4));     // weights in two parts
+  const double unit = split ? 1.40 + 0.0028 * w : qt == MLXR_NF4 ? 0.72 + 0.0012 * w : qt == MLXR_Q8_0 ? 0.67 + 0.0014 * w : 0.37 + 0.004 * w;
+  auto units = [&](double n) { return std::max(n, 2.0) * unit; };
+  auto shared = [&](int G) { return 0.18 + w * (0.0292 + 0.0377 * G / sms); };
+  const double part = 0.02 + 0.0013 * w;
   int G = (int)std::min<long long>(sms, U);
-  double best = std::ceil((double)U / G) * unit + (U % G == 0 && U / G % nsb == 0 ? 0.0 : shared + 1.5 + part * ((double)nsb * G / U + 1.0));
+  double best = units(std::ceil((double)U / G)) + (U % G == 0 && U / G % nsb == 0 ? 0.0 : shared(G) + 1.35 + part * ((double)nsb * G / U + 1.0));
   for (int c = 1; c <= nsb && (long long)c * ntiles <= sms; c++) {
-    const double cost = (nsb + c - 1) / c * unit + (c > 1 ? shared + part * c : 0.0);
+    const double cost = units((nsb + c - 1) / c) + (c > 1 ? shared(c * ntiles) + part * c : 0.0);
     if (cost < best) { best = cost; G = c * ntiles; }
   }
   int mc = 1;
@@ -669,7 +717,7 @@ template <int QT, typename T, int NPAD, int MODE, int FORM>
 static int launch_inst(const smallm::Maps& maps, const smallm::Params& P, int grid, cudaStream_t st) {
   using namespace smallm;
   auto kern = qgemm_smallm_kernel<QT, T, NPAD, MODE, FORM>;
-  constexpr size_t smem = Rings<QT, NPAD>::kBytes + sizeof(Shared) + 1024;
+  constexpr size_t smem = Rings<QT, NPAD, TableOf<QT, tc::Fmt<T>::v, NPAD, MODE>::type::kBytes>::kBytes + sizeof(Shared) + 1024;
   static_assert(smem <= (size_t)kSmemMax, "shared memory");
   static std::atomic<bool> attr_done[64] = {};
   int dev = 0;
@@ -711,6 +759,7 @@ int launch_smallm(const void* x, const void* const* w, const int* rows, int nmat
     if (i < (swiglu ? 1 : nmat)) {
       P.rows[i] = rows[i];
       P.y[i] = y[i];
+      if (rows[i] % 8 == 0 && ((uintptr_t)y[i] & 15u) == 0) P.vec_stores |= 1 << i;
       P.ntiles += (rows[i] + tile_rows - 1) / tile_rows;
     }
     P.end[i] = P.ntiles;

@@ -84,6 +84,19 @@ __device__ __forceinline__ void exact8_f16(uint32_t v, uint32_t ss_, uint32_t sm
 
 __device__ __forceinline__ void put(const uint4& v, uint32_t* out) { out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w; }
 
+// Both members times f, one instruction (fmul.f32x2)
+__device__ __forceinline__ float2 mul2(float2 v, float f) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmul.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(v.x), "f"(v.y), "f"(f));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 v, float f, float c) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmov.b64 c, {%5, %5};\n\tfma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(v.x), "f"(v.y), "f"(f), "f"(c));
+  return r;
+}
 // A pair of float32 weights -> one register (kSplit: leading part and residual)
 template <int BF, int MODE>
 __device__ __forceinline__ void emit(float a, float b, uint32_t& hi, uint32_t& lo) {
@@ -137,15 +150,87 @@ __device__ __forceinline__ __half half_of6(uint32_t n) {
   return __hsub(__ushort_as_half((unsigned short)(0x6400u | n)), __ushort_as_half((unsigned short)0x6400));
 }
 
+// Tables in shared memory that turn a byte (two codes) into a pair of numbers, a copy for each lane so that lookups never
+// conflict; rows are 256 bytes apart, so that one byte permute makes the place: the code in byte 1, the lane's copy in byte 0.
+template <int BYTES> struct TableBase {
+  const uint8_t* t;
+  uint32_t mine;
+  __device__ __forceinline__ TableBase(const uint8_t* table, int lane) : t(table), mine(BYTES * (uint32_t)lane) {}
+  template <int J> __device__ __forceinline__ const uint8_t* at(uint32_t v) const {
+    uint32_t o;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(o) : "r"(v), "r"(mine), "n"(0x5504 | (J << 4)));
+    return t + o;
+  }
+};
+// Pairs n0 - 8, n1 - 8 of the two nibbles of a byte, in fp16 (BF 0) or bf16
+template <int BF> struct CodePairs : TableBase<4> {
+  static constexpr int kBytes = 256 * 256;
+  using TableBase<4>::TableBase;
+  template <int J> __device__ __forceinline__ uint32_t pair(uint32_t v) const { return *reinterpret_cast<const uint32_t*>(at<J>(v)); }
+  // by all threads of the CTA; a barrier must follow
+  static __device__ __forceinline__ void fill(uint8_t* table, int tid, int threads) {
+    for (int i = tid; i < 256 * 8; i += threads) {
+      const float a = (float)((i >> 3) & 15) - 8.0f, b = (float)(i >> 7) - 8.0f;
+      uint32_t w;
+      if constexpr (BF == 0) { const __half2 h = __floats2half2_rn(a, b); w = *reinterpret_cast<const uint32_t*>(&h); }
+      else { const __nv_bfloat162 h = __floats2bfloat162_rn(a, b); w = *reinterpret_cast<const uint32_t*>(&h); }
+      *reinterpret_cast<uint4*>(table + (i >> 3) * 256 + (i & 7) * 16) = make_uint4(w, w, w, w);
+    }
+  }
+};
+// The same pairs in float32, for bf16 weights that are rounded once.  Two cycles of shared memory per lookup: only two words of
+// four take the table, the others the arithmetic, so that neither the one nor the other pipe is the limit.
+struct CodePairs32 : TableBase<8> {
+  static constexpr int kBytes = 256 * 256;
+  using TableBase<8>::TableBase;
+  template <int J> __device__ __forceinline__ float2 pair(uint32_t v) const { return *reinterpret_cast<const float2*>(at<J>(v)); }
+  static __device__ __forceinline__ void fill(uint8_t* table, int tid, int threads) {
+    for (int i = tid; i < kBytes / 16; i += threads) {
+      const float a = (float)((i >> 4) & 15) - 8.0f, b = (float)(i >> 8) - 8.0f;
+      reinterpret_cast<float4*>(table)[i] = make_float4(a, b, a, b);
+    }
+  }
+};
+// Eight weights of one word from the table: the same values as fast8_bf16 and exact8_f16 (MIN: the format has a min)
+template <int BF, bool MIN> __device__ __forceinline__ void table8(uint32_t v, uint32_t ss, uint32_t sm, const CodePairs<BF>& t, uint32_t* out) {
+  const uint32_t q[4] = {t.template pair<0>(v), t.template pair<1>(v), t.template pair<2>(v), t.template pair<3>(v)};
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    if constexpr (BF == 0) {
+      __half2 r = __hmul2_rn(as_half2(q[j]), as_half2(ss));
+      if constexpr (MIN) r = __hadd2_rn(r, as_half2(sm));
+      out[j] = *reinterpret_cast<const uint32_t*>(&r);
+    } else {
+      const __nv_bfloat162 r = MIN ? __hfma2(as_bf162(q[j]), as_bf162(ss), as_bf162(sm)) : __hmul2_rn(as_bf162(q[j]), as_bf162(ss));
+      out[j] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+  }
+}
+
 // Eight weights q ss + sm of one word of nibbles (q = n - 8), in the form MODE asks for
-template <int BF, int MODE> struct Scale { uint32_t s, m; };      // packed pair, or float32 bits
+template <int BF, int MODE> struct Scale { uint32_t s, m; float min = 0.0f; };      // packed pair, or float32 bits (kRound in bf16: m = min - 136 s)
 template <int BF, int MODE> __device__ __forceinline__ Scale<BF, MODE> make_scale(__half ss, __half sm) {
   if constexpr (MODE == kSplit) return {__float_as_uint(__half2float(ss)), __float_as_uint(__half2float(sm))};
   else if constexpr (BF == 0) return {dup_f16(ss), dup_f16(sm)};
   else if constexpr (MODE == kFast) return {dup_bf16(__half2float(ss)), dup_bf16(__half2float(sm))};
-  else { const float f = __half2float(ss); return {__float_as_uint(f), __float_as_uint(fmaf(-136.0f, f, __half2float(sm)))}; }
+  else { const float f = __half2float(ss), m = __half2float(sm); return {__float_as_uint(f), __float_as_uint(fmaf(-136.0f, f, m)), m}; }
 }
-template <int BF, int MODE> __device__ __forceinline__ void nibbles8(uint32_t v, const Scale<BF, MODE>& c, uint32_t* out, uint32_t* res) {
+template <int BF, int MODE, bool MIN> __device__ __forceinline__ void nibbles8(int, uint32_t v, const Scale<BF, MODE>& c, const CodePairs<BF>& t, uint32_t* out, uint32_t*) {
+  table8<BF, MIN>(v, c.s, c.m, t, out);
+}
+// i: the word's number in its block, a constant
+template <int BF, int MODE, bool MIN> __device__ __forceinline__ void nibbles8(int i, uint32_t v, const Scale<BF, MODE>& c, const CodePairs32& t, uint32_t* out, uint32_t*) {
+  const float s = __uint_as_float(c.s), m = __uint_as_float(c.m);
+  if (i & 1) return put(dequant8_bf16(v, s, m), out);
+  const float2 q[4] = {t.template pair<0>(v), t.template pair<1>(v), t.template pair<2>(v), t.template pair<3>(v)};
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const float2 w = MIN ? fma2(q[j], s, c.min) : mul2(q[j], s);
+    const __nv_bfloat162 b = __floats2bfloat162_rn(w.x, w.y);
+    out[j] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+}
+template <int BF, int MODE, bool MIN, typename L> __device__ __forceinline__ void nibbles8(int, uint32_t v, const Scale<BF, MODE>& c, const L&, uint32_t* out, uint32_t* res) {
   if constexpr (MODE == kSplit) {
     const uint32_t lo = v & 0x0F0F0F0Fu, hi = (v >> 4) & 0x0F0F0F0Fu;
     const float s = __uint_as_float(c.s), m = __uint_as_float(c.m);
@@ -186,8 +271,22 @@ struct PairLevels {
   }
 };
 
+// PairLevels with a copy for every lane: one instruction for the address instead of two, 64 KB instead of 32
+struct LanePairLevels : TableBase<8> {
+  static constexpr int kBytes = 256 * 256;
+  using TableBase<8>::TableBase;
+  template <int J> __device__ __forceinline__ float2 pair(uint32_t v) const { return *reinterpret_cast<const float2*>(at<J>(v)); }
+  static __device__ __forceinline__ void fill(uint8_t* table, int tid, int threads) {
+    for (int i = tid; i < kBytes / 16; i += threads) {
+      const float lo = kNF4[(i >> 4) & 15], hi = kNF4[i >> 8];
+      reinterpret_cast<float4*>(table)[i] = make_float4(lo, hi, lo, hi);
+    }
+  }
+};
+
 // Weights 64 kb .. 64 kb + 63 of the unit at `row` (shared memory): out(Int<0>, hi, lo) gets the first 32,
-// out(Int<1>, hi, lo) the others (lo only for kSplit).  nf4: Levels or PairLevels.  KB is int or tc::Int.  With a run-time kb the body stays at a few hundred
+// out(Int<1>, hi, lo) the others (lo only for kSplit).  nf4: Levels, PairLevels or LanePairLevels; CodePairs, or else nothing of use, for
+// the other formats.  KB is int or tc::Int.  With a run-time kb the body stays at a few hundred
 // instructions that every producer warp shares; unrolled over a unit of the long conversions (kSplit), or
 // specialised per group, the warps of a scheduler fetch more code than its instruction cache holds and
 // wait for it (the largest stall by far: canonical Q4_K [16, 4096] x [37888, 4096]^T 90.9 us unrolled, 52.5
@@ -208,10 +307,10 @@ __device__ __forceinline__ void convert64(const uint8_t* row, KB KBV, const L& n
     const auto c1 = make_scale<BF, MODE>(__hmul_rn(half_of6(g & 63u), d), __hmul_rn(half_of6((g >> 6) & 63u), dmin));
     const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
-    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[i], c0, a + 4 * i, b + 4 * i);
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE, true>(i, w[i], c0, nf4, a + 4 * i, b + 4 * i);
     out(tc::Int<0>{}, a, b);
 #pragma unroll
-    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[4 + i], c1, a + 4 * i, b + 4 * i);
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE, true>(i, w[4 + i], c1, nf4, a + 4 * i, b + 4 * i);
     out(tc::Int<1>{}, a, b);
   } else if constexpr (QT == MLXR_Q4_0) {       // two 18-byte blocks: fp16 d, 16 bytes of nibbles (q_gemm_dequant.metal:142-161)
     uint32_t w[9];
@@ -219,10 +318,10 @@ __device__ __forceinline__ void convert64(const uint8_t* row, KB KBV, const L& n
     const __half zero = __ushort_as_half((unsigned short)0);
     const auto c0 = make_scale<BF, MODE>(low_half(w[0]), zero), c1 = make_scale<BF, MODE>(high_half(w[4]), zero);
 #pragma unroll
-    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(__funnelshift_r(w[i], w[i + 1], 16), c0, a + 4 * i, b + 4 * i);
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE, false>(i, __funnelshift_r(w[i], w[i + 1], 16), c0, nf4, a + 4 * i, b + 4 * i);
     out(tc::Int<0>{}, a, b);
 #pragma unroll
-    for (int i = 0; i < 4; i++) nibbles8<BF, MODE>(w[5 + i], c1, a + 4 * i, b + 4 * i);
+    for (int i = 0; i < 4; i++) nibbles8<BF, MODE, false>(i, w[5 + i], c1, nf4, a + 4 * i, b + 4 * i);
     out(tc::Int<1>{}, a, b);
   } else if constexpr (QT == MLXR_Q8_0) {       // two 34-byte blocks: fp16 d, 32 int8 (q_gemm_dequant.metal:190-201)
     uint32_t w[17];
