@@ -2,6 +2,7 @@
 // selection.  Nothing here computes on the CPU: every compute entry point launches CUDA
 // kernels or fails.
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -123,6 +124,16 @@ static int give_check_word(int* w) {
   std::lock_guard<std::mutex> lk(g_check_mu);
   g_check_free.push_back(w);
   return v;
+}
+
+// Looks at a word that a kernel writes until it is no longer 0, for so many microseconds at most
+static bool poll_word(const int* w, int us) {
+  const auto end = std::chrono::steady_clock::now() + std::chrono::microseconds(us);
+  do {
+    for (int i = 0; i < 64; i++)
+      if (*reinterpret_cast<const volatile int*>(w)) { std::atomic_thread_fence(std::memory_order_acquire); return true; }
+  } while (std::chrono::steady_clock::now() < end);
+  return false;
 }
 
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -447,15 +458,19 @@ int mlxr_rope_apply(const void* x, const uint16_t* cos_f16, const uint16_t* sin_
   // With `check` the kernel records a violation straight in pinned host memory (under unified addressing the
   // host address is the device address), which saves a copy and a memset per call.
   int* word = ws->status;
+  bool answers = false;
   if (check) if (int r = take_check_word(&word)) return r;
   if (int r = launch_rope(x, cos_f16, sin_f16, positions, y, tokens, heads, head_dim, max_seq_len, mode,
-                          scale_factor, position_offset, dtype, word, st)) {
+                          scale_factor, position_offset, dtype, word, ws->sync + kRopeCount, check ? &answers : nullptr, st)) {
     if (check) give_check_word(word);       // nothing was launched
     return r;
   }
   if (check) {
-    MLXR_CUDA_TRY(cudaStreamSynchronize(st));     // on failure the kernel may still run: the word is not reused
-    if (give_check_word(word) != 0) {
+    // The answer comes when the kernel is done with all its accesses.  It is looked for where the kernel writes it as long as
+    // it may come soon; behind longer work, or from a kernel that has none, the driver waits for the stream.
+    if (!answers || !poll_word(word, 100)) MLXR_CUDA_TRY(cudaStreamSynchronize(st));     // on failure the kernel may still run: the word is not reused
+    const int bad = answers ? 2 : 1;
+    if (give_check_word(word) == bad) {
       set_error("rope_apply: a position (+offset) lies outside [0, max_seq_len)");
       return MLXR_ERR_SHAPE;
     }
@@ -764,10 +779,10 @@ int mlxr_qkv_rope(const void* x, const void* norm_weight, const void* wq, const 
   if (rope_qk_supported(q_out, k_out, cos_f16, sin_f16, head_dim, dtype))
     return launch_rope_qk(q_out, k_out, cos_f16, sin_f16, positions, (size_t)M, q_heads, kv_heads, head_dim, max_seq_len, position_offset, dtype, ws->status, st);
   if (int r = launch_rope(q_out, cos_f16, sin_f16, positions, q_out, (size_t)M, q_heads, head_dim, max_seq_len,
-                          MLXR_ROPE_BASE, 1.0f, position_offset, dtype, ws->status, st))
+                          MLXR_ROPE_BASE, 1.0f, position_offset, dtype, ws->status, nullptr, nullptr, st))
     return r;
   return launch_rope(k_out, cos_f16, sin_f16, positions, k_out, (size_t)M, kv_heads, head_dim, max_seq_len,
-                     MLXR_ROPE_BASE, 1.0f, position_offset, dtype, ws->status, st);
+                     MLXR_ROPE_BASE, 1.0f, position_offset, dtype, ws->status, nullptr, nullptr, st);
 }
 
 // ---- host-buffer variants ---------------------------------------------------------------

@@ -331,27 +331,37 @@ struct Divisor {
   __device__ __forceinline__ uint32_t quot(uint32_t n) const { return (__umulhi(n, mul) + n) >> shift; }
 };
 
-// The same for 16-bit types and heads of a multiple of 8 elements: one thread per four pairs, 128-bit
-// accesses to x and y, 64-bit to the tables; the token's position is checked once per thread.
+// The same for 16-bit types and heads of a multiple of 8 elements: 128-bit accesses to x and y, 64-bit to the tables.  A thread
+// rotates the same four pairs of HP heads of a token: the quotients, the position and the table values are found once for all of them, and
+// HP loads of x are in flight (32 heads of 1111 tokens: a thread per four pairs of one head spent half its instructions on finding them).
 //
-// Two tensors that share the positions (q and k of a layer) can go in one launch: vectors from `total` on are z's,
+// Two tensors that share the positions (q and k of a layer) can go in one launch: units from `total` on are z's,
 // up to total_z.
+//
+// A checked call waits for the answer on the host.  The last CTA to finish writes it straight to pinned memory (1: done, 2: done, with
+// a position outside the table), where the host sees it some 5 us before cudaStreamSynchronize would return; when it is there
+// every CTA has done its last access, and all results are visible (each CTA's barrier and fence before it is counted, the last one's fence
+// for the system before the answer).
 struct RopeArgs {
   const __half *cos_t, *sin_t;
   const int32_t* positions;
   size_t total, total_z;
-  Divisor per, per_z, per_head;          // vectors of a token of x, of z, of a head
+  Divisor per, per_z, per_head;          // units of a token of x, of z, of a group of heads
+  int heads, heads_z;
   int max_seq, linear;
   float scale;
   int offset;
-  int* status;
+  int* status;                           // unchecked: flag for positions outside the table, or null
+  unsigned* count;                       // checked: CTAs finished (+ 2^16 for each that met such a position); the last one clears it
+  volatile int* answer;
 };
-template <typename T, bool WIDE>          // WIDE: 2^31 vectors and more
+template <typename T, int HP, bool WIDE>          // WIDE: 2^31 units and more
 __global__ void __launch_bounds__(256) rope_vec_kernel(const T* x, T* y, T* z, const RopeArgs A) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   using Index = typename std::conditional<WIDE, size_t, uint32_t>::type;
   const Index total = (Index)A.total, all = (Index)(A.total + A.total_z);
+  bool outside = false;
   for (size_t j0 = (size_t)blockIdx.x * 256 + threadIdx.x; j0 < all; j0 += (size_t)gridDim.x * 256) {
     const Index j = (Index)j0;
     const bool first = j < total;
@@ -359,45 +369,77 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(const T* x, T* y, T* z, c
     const Divisor& per = first ? A.per : A.per_z;
     const T* src = first ? x : z;
     T* dst = first ? y : z;
+    const int heads = first ? A.heads : A.heads_z;
     Index tok;
-    uint32_t c, h;
     if constexpr (WIDE) tok = i / per.d; else tok = per.quot(i);
-    c = (uint32_t)(i - tok * per.d);
-    h = A.per_head.quot(c);
-    c -= h * A.per_head.d;
-    const uint4 xv = __ldcg(reinterpret_cast<const uint4*>(src) + i);
+    uint32_t c = (uint32_t)(i - tok * per.d);
+    const uint32_t h = A.per_head.quot(c), vh = A.per_head.d;
+    c -= h * vh;
+    const int have = min(HP, heads - (int)h * HP);
+    const size_t v0 = ((size_t)tok * heads + h * HP) * vh + c;
+    uint4 xv[HP];
+#pragma unroll
+    for (int k = 0; k < HP; k++) if (k < have) xv[k] = __ldcg(reinterpret_cast<const uint4*>(src) + v0 + k * vh);
     const long long pos = (long long)__ldcg(A.positions + tok) + A.offset;
     if (pos < 0 || pos >= A.max_seq) {
-      if (A.status) atomicExch_system(A.status, 1);
+      outside = true;
       continue;
     }
-    const uint2 cv = __ldg(reinterpret_cast<const uint2*>(A.cos_t) + (size_t)pos * A.per_head.d + c);
-    const uint2 sv = __ldg(reinterpret_cast<const uint2*>(A.sin_t) + (size_t)pos * A.per_head.d + c);
-    const T* hx = reinterpret_cast<const T*>(&xv);
+    const uint2 cv = __ldg(reinterpret_cast<const uint2*>(A.cos_t) + (size_t)pos * vh + c);
+    const uint2 sv = __ldg(reinterpret_cast<const uint2*>(A.sin_t) + (size_t)pos * vh + c);
     const __half *hc = reinterpret_cast<const __half*>(&cv), *hs = reinterpret_cast<const __half*>(&sv);
-    float o[8];
+    float cs[4], sn[4];
 #pragma unroll
-    for (int p = 0; p < 4; p++) {
-      const float cs = __half2float(hc[p]), sn = __half2float(hs[p]), xe = Act<T>::to_f(hx[2 * p]), xo = Act<T>::to_f(hx[2 * p + 1]);
-      o[2 * p] = __fsub_rn(__fmul_rn(xe, cs), __fmul_rn(xo, sn));
-      o[2 * p + 1] = __fadd_rn(__fmul_rn(xo, cs), __fmul_rn(xe, sn));
-      if (A.linear) { o[2 * p] *= A.scale; o[2 * p + 1] *= A.scale; }
+    for (int p = 0; p < 4; p++) { cs[p] = __half2float(hc[p]); sn[p] = __half2float(hs[p]); }
+#pragma unroll
+    for (int k = 0; k < HP; k++) {
+      if (k >= have) break;
+      const T* hx = reinterpret_cast<const T*>(&xv[k]);
+      float o[8];
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const float xe = Act<T>::to_f(hx[2 * p]), xo = Act<T>::to_f(hx[2 * p + 1]);
+        o[2 * p] = __fsub_rn(__fmul_rn(xe, cs[p]), __fmul_rn(xo, sn[p]));
+        o[2 * p + 1] = __fadd_rn(__fmul_rn(xo, cs[p]), __fmul_rn(xe, sn[p]));
+        if (A.linear) { o[2 * p] *= A.scale; o[2 * p + 1] *= A.scale; }
+      }
+      store8v(dst + (v0 + k * vh) * 8, o);
     }
-    store8v(dst + (size_t)i * 8, o);
+  }
+  if (!A.answer) {
+    if (outside && A.status) atomicExch_system(A.status, 1);
+    return;
+  }
+  const bool any = __syncthreads_or(outside);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const unsigned mine = 1u + (any ? 1u << 16 : 0u), sum = atomicAdd(A.count, mine) + mine;
+    if ((sum & 0xFFFFu) == gridDim.x) {
+      *A.count = 0u;
+      __threadfence_system();
+      *A.answer = sum >> 16 ? 2 : 1;
+    }
   }
 }
 
+// word: checked ? where the answer goes, with ctl a zeroed word of device memory : flag for positions outside the table
 template <typename T>
 static int launch_rope_vec(const void* x, const uint16_t* cos_t, const uint16_t* sin_t, const int32_t* positions, void* y, size_t tokens, int heads,
-                           void* z, int heads_z, int head_dim, int max_seq, int linear, float scale, int offset, int* status, cudaStream_t st) {
+                           void* z, int heads_z, int head_dim, int max_seq, int linear, float scale, int offset, int* word, uint32_t* ctl, cudaStream_t st) {
   const int vh = head_dim / 8;
-  const RopeArgs A = {(const __half*)cos_t, (const __half*)sin_t, positions, tokens * heads * vh, tokens * heads_z * vh,
-                      Divisor((uint32_t)heads * vh), Divisor((uint32_t)std::max(1, heads_z * vh)), Divisor((uint32_t)vh), max_seq, linear, scale, offset, status};
+  const size_t vectors = tokens * ((size_t)heads + heads_z) * vh;
+  // four heads a thread as long as that leaves three CTAs per SM, or two (8 heads of 1111 tokens: one)
+  const int hp = vectors >= (size_t)148 * 3 * 256 * 4 ? 4 : vectors >= (size_t)148 * 3 * 256 * 2 ? 2 : 1;
+  const int gx = (heads + hp - 1) / hp, gz = (heads_z + hp - 1) / hp;
+  const RopeArgs A = {(const __half*)cos_t, (const __half*)sin_t, positions, tokens * gx * vh, tokens * gz * vh,
+                      Divisor((uint32_t)gx * vh), Divisor((uint32_t)std::max(1, gz * vh)), Divisor((uint32_t)vh), heads, heads_z, max_seq, linear, scale, offset,
+                      ctl ? nullptr : word, ctl, ctl ? word : nullptr};
   const size_t all = A.total + A.total_z;
   cudaLaunchAttribute at;
   const cudaLaunchConfig_t cfg = overlapped((int)std::min<size_t>((all + 255) / 256, 148 * 8 * 4), 256, st, &at);
-  if (all >> 31) MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rope_vec_kernel<T, true>, (const T*)x, (T*)y, (T*)z, A));
-  else MLXR_CUDA_TRY(cudaLaunchKernelEx(&cfg, rope_vec_kernel<T, false>, (const T*)x, (T*)y, (T*)z, A));
+  auto launch = [&](auto kern) { return cudaLaunchKernelEx(&cfg, kern, (const T*)x, (T*)y, (T*)z, A); };
+  if (all >> 31) MLXR_CUDA_TRY(launch(rope_vec_kernel<T, 4, true>));
+  else MLXR_CUDA_TRY(launch(hp == 4 ? rope_vec_kernel<T, 4, false> : hp == 2 ? rope_vec_kernel<T, 2, false> : rope_vec_kernel<T, 1, false>));
   count_launch();
   return MLXR_OK;
 }
@@ -409,19 +451,22 @@ bool rope_qk_supported(const void* q, const void* k, const uint16_t* cos_t, cons
 }
 int launch_rope_qk(void* q, void* k, const uint16_t* cos_t, const uint16_t* sin_t, const int32_t* positions, size_t tokens, int q_heads, int kv_heads,
                    int head_dim, int max_seq, int offset, int dtype, int* status, cudaStream_t st) {
-  return dtype == MLXR_F16 ? launch_rope_vec<__half>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, st)
-                           : launch_rope_vec<__nv_bfloat16>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, st);
+  return dtype == MLXR_F16 ? launch_rope_vec<__half>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, nullptr, st)
+                           : launch_rope_vec<__nv_bfloat16>(q, cos_t, sin_t, positions, q, tokens, q_heads, k, kv_heads, head_dim, max_seq, 0, 1.0f, offset, status, nullptr, st);
 }
 
 int launch_rope(const void* x, const uint16_t* cos_t, const uint16_t* sin_t,
                 const int32_t* positions, void* y, size_t tokens, int heads, int head_dim,
                 int max_seq, int mode, float scale, int offset, int dtype, int* status,
-                cudaStream_t st) {
+                uint32_t* ctl, bool* answers, cudaStream_t st) {
   const size_t total = tokens * heads * (head_dim / 2);
+  if (answers) *answers = false;
   if (total == 0) return MLXR_OK;
-  if (rope_vec_ok(x, y, cos_t, sin_t, head_dim, dtype))
-    return dtype == MLXR_F16 ? launch_rope_vec<__half>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, st)
-                             : launch_rope_vec<__nv_bfloat16>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, st);
+  if (rope_vec_ok(x, y, cos_t, sin_t, head_dim, dtype)) {
+    if (answers) *answers = true; else ctl = nullptr;
+    return dtype == MLXR_F16 ? launch_rope_vec<__half>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, ctl, st)
+                             : launch_rope_vec<__nv_bfloat16>(x, cos_t, sin_t, positions, y, tokens, heads, nullptr, 0, head_dim, max_seq, mode == MLXR_ROPE_LINEAR, scale, offset, status, ctl, st);
+  }
   size_t blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   MLXR_DISPATCH_DTYPE(dtype, T, {

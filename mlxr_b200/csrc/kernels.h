@@ -10,6 +10,7 @@ namespace mlxr {
 // Zero-initialised 32-bit words per workspace for counters and barriers.
 constexpr int kSyncWords = 4096;
 constexpr int kTileCounters = 16;      // the first of the words that count the parts of shared output tiles
+constexpr int kRopeCount = 2;          // the word that counts the CTAs of a checked rotation
 
 int launch_dequantize(const void* w, void* out, int N, int K, int qt, int out_dtype, int flags,
                       cudaStream_t st);
@@ -28,10 +29,12 @@ int stream_status_word(cudaStream_t st, int** status);
 int launch_cast_from_f32(const float* x, void* y, size_t n, int dtype, cudaStream_t st);
 int launch_cast_to_f32(const void* x, float* y, size_t n, int dtype, cudaStream_t st);
 int launch_swiglu(const void* g, const void* u, void* o, size_t n, int dtype, cudaStream_t st);
+// answers (checked calls): set if the kernel will write 1 (done) or 2 (done, a position outside the table) to *status, pinned host memory, when it
+// is done with all its accesses, counting its CTAs in ctl, a zeroed word of device memory; else, and without it, *status becomes 1 for such a position
 int launch_rope(const void* x, const uint16_t* cos_t, const uint16_t* sin_t,
                 const int32_t* positions, void* y, size_t tokens, int heads, int head_dim,
                 int max_seq, int mode, float scale, int offset, int dtype, int* status,
-                cudaStream_t st);
+                uint32_t* ctl, bool* answers, cudaStream_t st);
 
 // rope_apply on q and k [tokens, heads, head_dim] in place, one launch; false if their layout needs launch_rope
 bool rope_qk_supported(const void* q, const void* k, const uint16_t* cos_t, const uint16_t* sin_t, int head_dim, int dtype);

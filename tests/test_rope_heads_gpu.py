@@ -1,0 +1,47 @@
+"""rope_apply where a thread rotates several heads of a token (csrc/elementwise.cu: four or two from about 450,000 or 230,000 vectors of eight on) and
+where the kernel answers a checked call itself."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _want(x, cos, sin, pos):
+    c, s = cos[pos.long()].float()[:, None], sin[pos.long()].float()[:, None]
+    e, o = x[..., 0::2].float(), x[..., 1::2].float()
+    return torch.stack((e * c - o * s, o * c + e * s), -1).flatten(-2).to(x.dtype)
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("tokens,heads,d", [(3, 5, 64), (6000, 5, 64), (11500, 5, 64), (4100, 7, 128), (2100, 7, 128), (120, 1, 8)])
+def test_heads_of_a_thread(dt, tokens, heads, d):
+    """Head counts that four and two do not divide.  float32 products and one rounding on both sides: the same values."""
+    import mlxr_b200 as mx
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    cos, sin = mx.compute_rope_tables(512, d, 10000.0, device=torch.device("cuda"))
+    x = torch.randn(tokens, heads, d, device="cuda", generator=g).to(dt)
+    pos = torch.randint(0, 512, (tokens,), device="cuda", generator=g, dtype=torch.int32)
+    want = _want(x, cos, sin, pos)
+    for check in (True, False):
+        assert torch.equal(mx.rope_apply(x, cos, sin, pos, check_positions=check), want)
+    # a position outside the table: reported, the other tokens rotated; the next call finds clean words
+    pos[tokens // 2] = 512
+    y = x.clone()
+    with pytest.raises(Exception):
+        mx.rope_apply(y, cos, sin, pos, inplace=True)
+    want[tokens // 2] = x[tokens // 2]
+    assert torch.equal(y, want)
+    pos[tokens // 2] = 0
+    assert torch.equal(mx.rope_apply(x, cos, sin, pos), _want(x, cos, sin, pos))
+
+
+def test_answer_behind_longer_work():
+    """A checked call behind work that takes longer than the host looks for the answer itself."""
+    import mlxr_b200 as mx
+    cos, sin = mx.compute_rope_tables(64, 64, 10000.0, device=torch.device("cuda"))
+    x = torch.randn(100, 4, 64, device="cuda").half()
+    pos = torch.randint(0, 64, (100,), device="cuda", dtype=torch.int32)
+    a = torch.randn(4096, 4096, device="cuda")
+    for _ in range(10):
+        a = torch.nn.functional.normalize(a @ a)
+    assert torch.equal(mx.rope_apply(x, cos, sin, pos), _want(x, cos, sin, pos))
