@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
             const int j = 2 * e + k;
             if constexpr (SWIGLU) {
               const float g = Act<T>::to_f(Act<T>::from_f(__uint_as_float(r[j]))), u = Act<T>::to_f(Act<T>::from_f(__uint_as_float(r[16 + j])));
-              v[k] = Act<T>::from_f(swish_f(g) * u);
+              v[k] = Act<T>::from_f(swish_h(g) * u);
             } else {
               v[k] = Act<T>::from_f(__uint_as_float(r[j]) + (bias && n0 + j < P.N ? Act<T>::to_f(bias[n0 + j]) : 0.0f));
             }

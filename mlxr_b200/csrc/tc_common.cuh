@@ -108,6 +108,9 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
   return r;
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// The same without an order of memory: for a meeting before which everything that one CTA sends into the other's shared memory
+// has been waited for there
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Default (CTA) scope on purpose: what these barriers order is tensor memory and the async proxy, through the
 // tcgen05 fences on both sides; release and acquire at cluster scope flush the SM's memory pipe each time.

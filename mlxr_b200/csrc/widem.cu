@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 
 #include "common.cuh"
@@ -84,15 +85,30 @@ struct Shared {
   uint32_t tmem_base;
   int dead, epi_fail;
   int ntodo, todo_tile[2], todo_first[2], todo_parts[2];
-  float nf4[16];
-  alignas(16) uint16_t turn[4][16 * 32];    // epilogue warps: sixteen tokens' results on their way to 16-byte stores
+  alignas(16) uint32_t turn[4][16 * 32];    // epilogue warps: 32 tokens' results on their way to 16-byte stores
 };
 
-template <int QT, int NMAX> struct Rings {
+// The table that a format's producers look codes up in (weight_convert.cuh), behind the rings.  Up to 128 tokens a
+// tile the conversion sets the pace (1530 cycles a unit of fp16 Q4_0 with arithmetic alone, 128 tokens' MMAs 1024); the
+// wider tiles' X leaves no room for a table, and their MMAs take 2048.
+struct LevelTable : Levels {
+  static constexpr int kBytes = 64;
+  __device__ __forceinline__ LevelTable(const uint8_t* table, int) : Levels{reinterpret_cast<const float*>(table)} {}
+  static __device__ __forceinline__ void fill(uint8_t* table, int tid, int) { if (tid < 16) reinterpret_cast<float*>(table)[tid] = kNF4[tid]; }
+};
+template <int QT, int BF, int NMAX> struct TableOf { using type = LevelTable; };
+template <int BF> struct TableOf<MLXR_NF4, BF, 128> { using type = LanePairLevels; };
+template <> struct TableOf<MLXR_Q4_K, 0, 128> { using type = CodePairs<0>; };
+template <> struct TableOf<MLXR_Q4_0, 0, 128> { using type = CodePairs<0>; };
+template <> struct TableOf<MLXR_Q4_K, 1, 128> { using type = CodePairs32; };
+template <> struct TableOf<MLXR_Q4_0, 1, 128> { using type = CodePairs32; };
+
+template <int QT, int BF, int NMAX> struct Rings {
   static constexpr int kRawBytes = kRows * Geo<QT>::kStage;
   static constexpr int kXStage = kBlocks * NMAX / 2 * kBK * 2;               // this CTA's half of the tokens, two tiles of nt / 2 rows
   static constexpr int kRawStages = QT != MLXR_Q8_0 ? 4 : 2;
-  static constexpr size_t kBytes = (size_t)kStages * kXStage + (size_t)kRawStages * kRawBytes;
+  using Tab = typename TableOf<QT, BF, NMAX>::type;
+  static constexpr size_t kBytes = Tab::kBytes + (size_t)kStages * kXStage + (size_t)kRawStages * kRawBytes;
   static constexpr int kBufs = NMAX == 128 ? 2 : 1;
   static constexpr uint32_t kA0 = 256, kCols = 512;                          // accumulators in columns 0 .. 255
 };
@@ -109,7 +125,13 @@ template <typename T, int FAR> __device__ __forceinline__ Pair<T> swiglu_pair(fl
   const bool up = (lane & FAR) != 0;
   const float o = __shfl_xor_sync(0xffffffffu, up ? a : b, FAR);
   const float g = Act<T>::to_f(Act<T>::from_f(up ? o : a)), u = Act<T>::to_f(Act<T>::from_f(up ? b : o));
-  return {Act<T>::from_f(swish_f(g) * u), up ? 1 : 0};
+  return {Act<T>::from_f(swish_h(g) * u), up ? 1 : 0};
+}
+
+// two values rounded to T in one word, the first in its low half
+template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b) {
+  if constexpr (Act<T>::kDtype == MLXR_F16) { const __half2 v = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t*>(&v); }
+  else { const __nv_bfloat162 v = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const uint32_t*>(&v); }
 }
 
 // weight tile and token tile of tile t
@@ -127,7 +149,7 @@ __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" 
 template <int QT, typename T, int NMAX, bool SWIGLU>
 __global__ void __launch_bounds__(kThreads, 1)
 qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(16) uint8_t smem_raw[];
   constexpr int BF = Fmt<T>::v;
   constexpr bool kSplitRows = QT == MLXR_NF4;
   if (threadIdx.x < 5) {
@@ -135,13 +157,15 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     if (threadIdx.x == 4 || threadIdx.x < (SWIGLU ? 2 : 1) * (kSplitRows ? 2 : 1))
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
   }
-  using R = Rings<QT, NMAX>;
+  using R = Rings<QT, BF, NMAX>;
+  using Tab = typename R::Tab;
   constexpr int kRawStages = R::kRawStages, kXStage = R::kXStage, kRawBytes = R::kRawBytes;
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw & 1023u)) & 1023u;
   uint8_t* xring = smem_raw + pad;
   uint8_t* rawring = xring + (size_t)kStages * kXStage;
-  Shared* sh = reinterpret_cast<Shared*>(rawring + (size_t)kRawStages * kRawBytes);
+  uint8_t* table = rawring + (size_t)kRawStages * kRawBytes;
+  Shared* sh = reinterpret_cast<Shared*>(table + Tab::kBytes);
   volatile int* dead = &sh->dead;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int rank = (int)cluster_rank(), G = gridDim.x >> 1, pair = blockIdx.x >> 1, cta = blockIdx.x;
@@ -194,7 +218,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (QT == MLXR_NF4 && tid >= 128 && tid < 144) sh->nf4[tid - 128] = kNF4[tid - 128];
+  Tab::fill(table, tid, kThreads);
   if (warp == kWarpMma) tmem_alloc_pair(smem_u32(&sh->tmem_base), R::kCols);
   tc_fence_before();
   __syncthreads();
@@ -214,6 +238,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     const uint32_t col = tmem + R::kA0 + (uint32_t)(g * kSlots * kSlotCols) + ((uint32_t)((warp & 3) * 32) << 16);
     const int half = g / kBlocks;
     const uint32_t full[2] = {cluster_map(smem_u32(&sh->full[half]), 0), cluster_map(smem_u32(&sh->full[kHalves + half]), 0)};
+    const Tab levels(table, lane);
     int r = 0, sb = sb_first;
     uint32_t rpar = 0;
     for (int i = 0; i < nunits; i++) {
@@ -223,7 +248,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       if constexpr (kSplitRows) row += (136 * sb + ((local & 1) ? P.odd_shift : 0)) & 8;
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh->empty[q * kHalves + half]), (uint32_t)((i >> 1) & 1) ^ 1u, dead))) break;
       tc_fence_after();
-      convert64<QT, BF, kRound>(row, g, Levels{sh->nf4}, [&](auto H, const uint32_t (&a)[16], const uint32_t (&)[16]) {
+      convert64<QT, BF, kRound>(row, g, levels, [&](auto H, const uint32_t (&a)[16], const uint32_t (&)[16]) {
         tmem_st16(col + q * kSlotCols + 16 * decltype(H)::value, a);
       });
       tmem_wait_st();
@@ -313,7 +338,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       // so time is given to them instead (a copy takes microseconds)
       if (issued > 0) for (int i = 0; i < 100; i++) __nanosleep(2000);
     } else {
-      // the last releases of the stages come from the other CTA as well: none may be on its way when this one exits
+      // the last releases of the stages come from the pair's issuer: none may be on its way when this CTA exits
       for (int i = max(0, issued - kStages); i < issued; i++) mbar_wait(smem_u32(&sh->empty[i % kStages]), (uint32_t)(i / kStages) & 1u, dead);
     }
   } else if (warp == kWarpFix) {
@@ -345,6 +370,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     const int quarter = warp & 3, rt = quarter * 32 + lane;
     const T* bias = reinterpret_cast<const T*>(P.bias);
     const uint32_t acc_free[2] = {cluster_map(smem_u32(&sh->acc_empty[0]), 0), cluster_map(smem_u32(&sh->acc_empty[1]), 0)};
+    const int nparts = (sb_first + nunits + P.nsb - 1) / P.nsb;      // tiles that the range touches
     int t = t_first, g = 0, fix_bar = 2;
     asm volatile("griddepcontrol.wait;" ::: "memory");        // Y, the partial sums and the tile counters
     for (int i = 0, cnt; i < nunits; i += cnt, t++, g++) {
@@ -363,68 +389,81 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       const int wt = 2 * tile.wt + rank, tok0 = tile.tt * P.nt, ntok = min(P.nt, P.M - tok0);
       const int n = SWIGLU ? 64 * wt + 16 * quarter + (lane & 15) : wt * kRows + rt;
       float* part = P.partials + ((size_t)(2 * cta + (i > 0 ? 1 : 0)) * P.nt) * kRows + rt;
-      T* y = reinterpret_cast<T*>(P.y) + (size_t)tok0 * P.N + n;
       const float bv = (!SWIGLU && bias && n < P.N) ? Act<T>::to_f(bias[n]) : 0.0f;
       // this warp's first output column; all its columns exist and start on 16 bytes
       const int nw = SWIGLU ? 64 * wt + 16 * quarter : wt * kRows + 32 * quarter;
-      const bool vec = P.vec_stores && nw + (SWIGLU ? 16 : 32) <= P.N;
+      constexpr int kCols = SWIGLU ? 16 : 32;
+      const bool vec = P.vec_stores && nw + kCols <= P.N;
       T* yv = reinterpret_cast<T*>(P.y) + (size_t)tok0 * P.N + nw;
 #pragma unroll 1
-      for (int c0 = 0; c0 < ntok; c0 += 16) {
-        uint32_t r[16];
-        tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * NMAX + c0), r);
-        if (whole && vec) {
-          // sixteen tokens x 32 weight rows (gate/up: 16 columns) turn in shared memory into 16-byte stores
-          constexpr int kCols = SWIGLU ? 16 : 32;
-          uint16_t* turn = sh->turn[quarter];
+      for (int c0 = 0; c0 < ntok; c0 += 32) {      // past nt: columns of the other buffer or of converted weights, not stored
+        uint32_t r[32];
+        tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * NMAX + c0), r);
+        if (whole) {
+          // 32 tokens x 32 weight rows (gate/up: 16 columns) turn in shared memory into 16-byte stores.  Beside busy producers
+          // every instruction here counts: a tile of 256 tokens whose results leave one 2-byte word each took 6.4 us of a
+          // tile's 24 (K = 4096), and the next tile's MMAs wait for it.
           if constexpr (SWIGLU) {
+            uint16_t* turn = reinterpret_cast<uint16_t*>(sh->turn[quarter]);
 #pragma unroll
-            for (int c = 0; c < 16; c += 2) {
+            for (int c = 0; c < 32; c += 2) {
               const Pair<T> h = swiglu_pair<T, 16>(__uint_as_float(r[c]), __uint_as_float(r[c + 1]), lane);
               turn[(c + h.second) * kCols + (lane & 15)] = *reinterpret_cast<const uint16_t*>(&h.value);
             }
-          } else {
+            __syncwarp();
+            if (vec) {
 #pragma unroll
-            for (int c = 0; c < 16; c++) {
-              const T o = Act<T>::from_f(__uint_as_float(r[c]) + bv);
-              turn[c * kCols + lane] = *reinterpret_cast<const uint16_t*>(&o);
+              for (int e = 0; e < 2; e++) {
+                const int piece = e * 32 + lane, tk = piece >> 1, pc = piece & 1;
+                if (c0 + tk < ntok) *reinterpret_cast<uint4*>(yv + (size_t)(c0 + tk) * P.N + pc * 8) = *reinterpret_cast<const uint4*>(turn + tk * kCols + pc * 8);
+              }
+            } else {
+#pragma unroll 4
+              for (int e = lane; e < 32 * kCols; e += 32) {
+                const int tk = e / kCols, col = e % kCols;
+                if (c0 + tk < ntok && nw + col < P.N) yv[(size_t)(c0 + tk) * P.N + col] = *reinterpret_cast<const T*>(turn + e);
+              }
+            }
+          } else {
+            uint32_t* turn = sh->turn[quarter];                            // [pair of tokens][row]: two tokens of a row per word
+#pragma unroll
+            for (int c = 0; c < 16; c++) turn[c * 32 + lane] = pack2<T>(__uint_as_float(r[2 * c]) + bv, __uint_as_float(r[2 * c + 1]) + bv);
+            __syncwarp();
+            if (vec) {
+#pragma unroll
+              for (int e = 0; e < 2; e++) {
+                const int piece = e * 32 + lane, tk = 2 * (piece >> 2), pc = piece & 3;
+                const uint4* w = reinterpret_cast<const uint4*>(turn + (piece >> 2) * 32 + pc * 8);
+                const uint4 u = w[0], v = w[1];
+                T* at = yv + (size_t)(c0 + tk) * P.N + pc * 8;
+                if (c0 + tk < ntok) *reinterpret_cast<uint4*>(at) = make_uint4(__byte_perm(u.x, u.y, 0x5410), __byte_perm(u.z, u.w, 0x5410), __byte_perm(v.x, v.y, 0x5410), __byte_perm(v.z, v.w, 0x5410));
+                if (c0 + tk + 1 < ntok) *reinterpret_cast<uint4*>(at + P.N) = make_uint4(__byte_perm(u.x, u.y, 0x7632), __byte_perm(u.z, u.w, 0x7632), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x7632));
+              }
+            } else {
+#pragma unroll 4
+              for (int tk = 0; tk < 32; tk++)
+                if (c0 + tk < ntok && nw + lane < P.N) yv[(size_t)(c0 + tk) * P.N + lane] = reinterpret_cast<const T*>(turn)[((tk >> 1) * 32 + lane) * 2 + (tk & 1)];
             }
           }
           __syncwarp();
-          constexpr int kPer = kCols / 8;                                  // 16-byte pieces per token
-#pragma unroll
-          for (int e = 0; e < 16 * kPer / 32; e++) {
-            const int piece = e * 32 + lane, tk = piece / kPer, pc = piece % kPer;
-            if (c0 + tk < ntok) *reinterpret_cast<uint4*>(yv + (size_t)(c0 + tk) * P.N + pc * 8) = *reinterpret_cast<const uint4*>(turn + tk * kCols + pc * 8);
-          }
-          __syncwarp();
-        } else if (whole) {
-          if constexpr (SWIGLU) {
-#pragma unroll
-            for (int c = 0; c < 16; c += 2) {
-              const Pair<T> h = swiglu_pair<T, 16>(__uint_as_float(r[c]), __uint_as_float(r[c + 1]), lane);
-              if (n < P.N && c0 + c + h.second < ntok) y[(size_t)(c0 + c + h.second) * P.N] = h.value;
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < 16; c++)
-              if (n < P.N && c0 + c < ntok) y[(size_t)(c0 + c) * P.N] = Act<T>::from_f(__uint_as_float(r[c]) + bv);
-          }
         } else {
 #pragma unroll
-          for (int c = 0; c < 16; c++)
+          for (int c = 0; c < 32; c++)
             if (c0 + c < ntok) __stcg(part + (size_t)(c0 + c) * kRows, __uint_as_float(r[c]));
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(acc_free[ab]);
+      if (lane == 0 && g + R::kBufs < nparts) mbar_arrive_cluster(acc_free[ab]);      // nobody waits for the last ones
       if (!whole) { asm volatile("bar.arrive %0, 160;" ::"r"(fix_bar) : "memory"); fix_bar++; }
     }
   }
   tc_fence_before();
   __syncthreads();
-  cluster_arrive();         // neither CTA's memory is read or signalled by the other any more
+  // neither CTA's memory is read or signalled by the other any more: each signal has been waited for where it arrives (the stages'
+  // releases by the copy warps, accumulators by the epilogues and, but for the last ones, which are not sent, the issuer), so the
+  // meeting need not wait for this CTA's stores (release: 0.7 us)
+  if (sh->dead) cluster_arrive(); else cluster_arrive_relaxed();
   cluster_wait();
   if (warp == kWarpMma) {
     tc_fence_after();
@@ -534,7 +573,7 @@ template <int QT, typename T, int NMAX, bool SWIGLU>
 static int launch_wide_inst(const widem::Maps& maps, const widem::Params& P, int grid, cudaStream_t st) {
   using namespace widem;
   auto kern = qgemm_widem_kernel<QT, T, NMAX, SWIGLU>;
-  constexpr size_t smem = Rings<QT, NMAX>::kBytes + sizeof(Shared) + 1024;
+  constexpr size_t smem = Rings<QT, Fmt<T>::v, NMAX>::kBytes + sizeof(Shared) + 1024;
   static_assert(smem <= (size_t)kSmemMax, "shared memory");
   static std::atomic<bool> attr_done[64] = {};
   int dev = 0;
