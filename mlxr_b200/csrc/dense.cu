@@ -4,8 +4,8 @@
 //   Y[M, N] = X[M, K] * dequant(W)[N, K]^T (+ bias),  X, Y fp16 or bf16, W in MLXR's Q4_K, Q4_0 or Q8_0
 //   layout or NF4; or Y = SiLU(X gate^T) * (X up^T).
 //
-// The kernels that convert inside the GEMM (widem.cu) convert every weight once per 256 tokens beside the
-// MMAs and are bound by that; from 1040 tokens on (14336 x 4096; 1790 for 4096 x 14336), one pass that writes 16-bit
+// The kernel that converts inside the GEMM (widem.cu) converts every weight once per 256 tokens beside the
+// MMAs and draws power for it; from about 2000 tokens on (14336 x 4096; 4096 x 14336 never), one pass that writes 16-bit
 // weights (2.6 bytes of traffic per weight: 27 us for 14336 x 4096, 23 at HBM's rate) costs less than the conversions it saves, and
 // the GEMM behind it leaves the CUDA cores to the epilogue and runs at the tensor pipe's rate, which
 // under the power cap also means a higher clock.  It takes the rows in slices of at most kSliceBytes so

@@ -153,7 +153,7 @@ struct WidePlan {
   double cost_us;          // the plan's own estimate
 };
 bool widem_supported(int qt, int M, int N, int K, int dtype, const void* x, const void* w);
-int widem_plan(int M, int rows, int K, WidePlan* out);     // rows = weight rows streamed (N, or 2 N for the gate/up form)
+int widem_plan(int qt, int dtype, int M, int rows, int K, WidePlan* out);     // rows = weight rows streamed (N, or 2 N for the gate/up form)
 int launch_widem(const void* x, const void* w, const void* w2, const void* bias, void* y, int M, int N, int K, int qt, int dtype,
                  int* status, float* partials, uint32_t* counters, const WidePlan& plan, cudaStream_t st);
 

@@ -1,4 +1,4 @@
-// Quantized linear for 65 and more tokens, as long as dense.cu is not faster (14336 x 4096: to 1040), on the 5th-generation
+// Quantized linear for 65 and more tokens, as long as dense.cu is not faster (14336 x 4096: to about 2000), on the 5th-generation
 // tensor cores, every weight converted once per 256 tokens:
 //
 //   Y[M, N] = X[M, K] * dequant(W)[N, K]^T (+ bias),  X, Y fp16 or bf16, W in MLXR's Q4_K, Q4_0 or
@@ -14,7 +14,9 @@
 // * Tiles are (256 weight rows) x (nt tokens), nt a multiple of 16 chosen with the number of token
 //   tiles so that the last one is not padding (333 tokens: two tiles of 176, not 512 rows of which 179
 //   are empty).  Work units are (tile, 256-wide super-block of K), weight tile-major with token tiles
-//   inside, so a weight tile's second reading comes from L2.
+//   inside, so a weight tile's second reading comes from L2.  (Taken back: tiles of up to 384 tokens, which convert a weight once for 333 tokens, 70.1 us
+//   instead of 65.4 on 22016 x 4096 Q4_0; the last wave's tiles shared by up to six pairs, 67.8: under the power cap idle SMs cost
+//   little, parts' trips through L2 more.)
 //   Token tiles go in groups of eight, weight tiles inside a group, so that a group's X stays in L2.
 // * With few tiles per pair the units are dealt to the pairs in equal contiguous ranges and shared tiles
 //   are added up by the CTA that delivers the last part; with many, every pair takes whole tiles.
@@ -532,31 +534,40 @@ bool widem_supported(int qt, int M, int N, int K, int dtype, const void* x, cons
   return ((((uintptr_t)x) | ((uintptr_t)w)) & 15u) == 0;
 }
 
-// Token tile, grid and dealing of the units.  Fitted to measurements (Q4_K, 65 to 2048 tokens, 14336 x 4096 and 4096 x
-// 14336): a unit takes about 2000 cycles (the conversion of its 65536 weights and the turn-around of a stage)
-// plus 4.3 per token of the tile, a launch 14000 before and after its units; a shared tile costs its parts'
-// trip through L2 at the end; a whole tile per pair needs none of that but leaves SMs idle in the last wave.
-int widem_plan(int M, int rows, int K, WidePlan* out) {
+// Token tile, grid and dealing of the units.  Fitted, in us, to 4210 measurements (Q4_K, Q4_0, Q8_0, NF4; 65 to 1500 tokens; six sizes from
+// 1500 x 2048 to 22016 x 4096; tiles of 48 to 256 tokens; equal ranges, whole tiles, two to four pairs per tile; the choice by this estimate takes
+// 1.3 % more than the best of them in the mean, 17 % at most).  A unit takes its MMAs (8 cycles a token at the clock that the power cap
+// leaves) or its conversion, which is shorter with a table: to 128 tokens.  A tile costs its results' way out beside that, with two
+// accumulators (to 128 tokens) less; a shared tile its parts' trip through L2 at the end; equal ranges also the
+// parts that a pair parks between two tiles.  Whole tiles need none of that but leave SMs idle in the last wave; above 192 tokens equal ranges take
+// 12 % more than a few passes show once the power cap holds (thousands of passes of 22016 x 4096 Q4_0, 333 tokens: tiles of 176, equal ranges 71.2 us,
+// whole 65.4; 112, 75.1 and 71.9).
+int widem_plan(int qt, int dtype, int M, int rows, int K, WidePlan* out) {
   int sms = 0;
   if (int r = device_sms(&sms)) return r;
   const int nsb = K / 256, wtiles = (rows + 2 * widem::kRows - 1) / (2 * widem::kRows), pairs = sms / 2;
+  const bool f16 = dtype == MLXR_F16;
+  const double convert128 = qt == MLXR_Q8_0 ? 1.21 : qt == MLXR_NF4 ? 1.07 : f16 ? 0.75 : 0.86;
+  const double convert256 = qt == MLXR_Q8_0 ? 1.36 : qt == MLXR_NF4 ? 1.47 : !f16 ? 1.12 : qt == MLXR_Q4_0 ? 0.89 : 1.04;
   double best = 1e300;
-  for (int ntt = (M + 255) / 256; ntt <= (M + 255) / 256 + 4; ntt++) {
+  for (int ntt = (M + 255) / 256;; ntt++) {
     const int nt = ((M + ntt - 1) / ntt + 15) / 16 * 16;
-    if (nt < 16 || nt > 256) continue;
+    if (nt < (M <= 1024 ? 48 : 112) && best < 1e300) break;
     const long long ntiles = (long long)wtiles * ((M + nt - 1) / nt), U = ntiles * nsb;
-    const double unit = 2000.0 + 4.3 * nt, drain = nt > 128 ? 1200.0 + 8.0 * nt : 600.0;
+    const double unit = nt <= 128 ? std::max(convert128, 0.31 + 0.0054 * nt) : std::max(convert256, 0.31 + 0.0046 * nt);
+    const double drain = nt <= 128 ? 2.15 : 0.0303 * nt - 1.72, shared = 0.023 * nt, part = 0.63 + 0.0017 * nt, parked = 0.0375 * nt;
     // split 0: equal ranges of units for all pairs; else so many pairs for each tile (1: whole tiles, any number of them)
-    for (int split = 0; split == 0 || split == 1 || (split <= nsb && split * ntiles <= pairs); split++) {
+    for (int split = 0; split < 2 || (split <= nsb && split * ntiles <= pairs); split++) {
       if (split != 1 && 2 * ntiles > kSyncWords - kTileCounters) continue;        // two counters per tile
       const int G = (int)(split == 0 ? std::min<long long>(pairs, U) : split == 1 ? std::min<long long>(pairs, ntiles) : split * ntiles);
       double c;
       if (split == 0) {
         const double units = (double)((U + G - 1) / G);
-        c = units * unit + units / nsb * drain + 2500.0 + 20.0 * nt + 1200.0 * (double)((nsb + units - 1) / units) + 2500.0;
+        c = units * unit + units / nsb * drain + shared + part * std::floor((nsb + units - 1) / units) + parked;
+        if (M > 192) c *= 1.12;
       } else {
         const double tiles = (double)((ntiles + G - 1) / G);
-        c = tiles * ((nsb + split - 1) / split * unit + drain) + (split > 1 ? 2500.0 + 20.0 * nt + 1200.0 * split : 0.0);
+        c = split == 1 ? tiles * (nsb * unit + drain) : (nsb + split - 1) / split * unit + drain + shared + part * split;
       }
       if (c < best) {
         best = c;
@@ -564,8 +575,9 @@ int widem_plan(int M, int rows, int K, WidePlan* out) {
         out->partial_bytes = split == 1 ? 0 : (size_t)2 * G * 2 * nt * widem::kRows * sizeof(float);
       }
     }
+    if (nt <= 16) break;
   }
-  out->cost_us = (14000.0 + best) / 1750.0;
+  out->cost_us = 4.05 + best;
   return MLXR_OK;
 }
 
