@@ -167,8 +167,8 @@ MLXR_API int mlxr_swiglu(const void* gate, const void* up, void* out, size_t n, 
  * (y may equal x: in place).  positions: int32 [batch] when seq == 1 else [batch, seq];
  * every position + position_offset must lie in [0, max_seq_len) -- checked on the
  * device, a violation leaves that token's output untouched and the call's status word
- * set (reported by mlxr_rope_apply's return value only when `check` is non-zero, which
- * synchronises the stream). */
+ * set (reported by mlxr_rope_apply's return value only when `check` is non-zero: the call
+ * then returns when the rotation, and with it all earlier work of the stream, is done). */
 MLXR_API int mlxr_rope_apply(const void* x, const uint16_t* cos_f16, const uint16_t* sin_f16,
                              const int32_t* positions, void* y, int batch, int seq,
                              int heads, int head_dim, int max_seq_len, int mode,
