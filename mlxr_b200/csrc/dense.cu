@@ -190,11 +190,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  __syncthreads();
+  cluster_arrive();       // both CTAs run and have their barriers before either signals the other or allocates in both SMs' tensor memory
+  cluster_wait();
   if (warp == kWarpMma) tmem_alloc_pair(smem_u32(&sh->tmem_base), 512);
   tc_fence_before();
   __syncthreads();
-  cluster_arrive();
-  cluster_wait();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -345,6 +346,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
     tc_fence_after();
     tmem_dealloc_pair(tmem, 512);
   }
+  __syncwarp();
+  cluster_arrive();         // and neither leaves while the other still frees columns in both SMs
+  cluster_wait();
   if (tid == 0 && sh->dead) atomicExch(P.status, MLXR_ERR_TIMEOUT);
 }
 

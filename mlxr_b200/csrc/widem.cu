@@ -221,11 +221,12 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   Tab::fill(table, tid, kThreads);
+  __syncthreads();
+  cluster_arrive();       // both CTAs run and have their barriers before either signals the other or allocates in both SMs' tensor memory
+  cluster_wait();
   if (warp == kWarpMma) tmem_alloc_pair(smem_u32(&sh->tmem_base), R::kCols);
   tc_fence_before();
   __syncthreads();
-  cluster_arrive();       // both CTAs' barriers exist before either signals the other
-  cluster_wait();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -471,6 +472,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     tc_fence_after();
     tmem_dealloc_pair(tmem, R::kCols);
   }
+  cluster_arrive_relaxed();       // and neither leaves while the other still frees columns in both SMs
   if (tid == 0 && sh->dead) atomicExch(P.status, MLXR_ERR_TIMEOUT);
   // ===== shared tiles of which this CTA delivered the last part: all warps, four tokens each at a time,
   // four weight rows per lane, two parts in flight, added in CTA order =====
@@ -522,6 +524,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       }
     }
   }
+  cluster_wait();
 }
 
 }  // namespace widem
