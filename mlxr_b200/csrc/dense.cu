@@ -21,7 +21,7 @@
 //   both factors of its outputs.
 // * Waits on mbarriers are bounded and reported as in the other tensor-core kernels; every barrier is waited on by one
 //   role in phase order.  `dead` is a CTA's own: a CTA whose partner has given up runs into its own limits, once per role.
-//   Without a limit: the two cluster barriers (a cluster's CTAs start together, and each role's loop ends by its last tile or its
+//   Without a limit: the cluster barriers (a cluster's CTAs start together, and each role's loop ends by its last tile or its
 //   first give-up), tcgen05.alloc (the shared memory leaves room for one such CTA per SM, and one that leaves has freed its
 //   columns), tcgen05.wait::ld (its own loads), cp.async.bulk.wait_group (its own stores), griddepcontrol.wait (the previous kernel's end;
 //   all of a launch's CTAs have started before the next launch's may, so none waits for room that a later launch holds).
