@@ -472,6 +472,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
     tc_fence_after();
     tmem_dealloc_pair(tmem, R::kCols);
   }
+  __syncwarp();                   // the meetings want whole warps
   cluster_arrive_relaxed();       // and neither leaves while the other still frees columns in both SMs
   if (tid == 0 && sh->dead) atomicExch(P.status, MLXR_ERR_TIMEOUT);
   // ===== shared tiles of which this CTA delivered the last part: all warps, four tokens each at a time,
@@ -524,6 +525,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       }
     }
   }
+  __syncwarp();
   cluster_wait();
 }
 
