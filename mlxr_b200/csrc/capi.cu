@@ -98,32 +98,42 @@ int stream_status_word(cudaStream_t st, int** status) {
   return MLXR_OK;
 }
 
-// Words of pinned host memory that the kernels of checked rope_apply calls report into, one per call in flight: callers
-// that share a stream never see one another's.  As many as were ever in flight at once, rounded up to a page;
-// freed by mlxr_release_workspaces().
+// What a checked rope_apply call has to itself: a word of pinned host memory into which its kernel reports, and a word of
+// device memory, 0 between calls, in which the kernel counts its CTAs.  One slot per call in flight, so that callers never see one another's,
+// whether they share a stream or only a handle (cudaStreamPerThread).  As many as were ever in flight on the device at
+// once, rounded up to a page; freed by mlxr_release_workspaces().
+struct CheckSlot { int* word; uint32_t* count; };
+struct CheckPool { std::vector<CheckSlot> free, pages; };
 static std::mutex g_check_mu;
-static std::vector<int*> g_check_free, g_check_pages;
+static std::map<int, CheckPool> g_check;      // by device
 constexpr size_t kCheckPage = 4096 / sizeof(int);
-static int take_check_word(int** out) {
+static int take_check_slot(int* dev, CheckSlot* out) {
+  MLXR_CUDA_TRY(cudaGetDevice(dev));
   std::lock_guard<std::mutex> lk(g_check_mu);
-  if (g_check_free.empty()) {
-    int* page = nullptr;
-    MLXR_CUDA_TRY(cudaHostAlloc(&page, kCheckPage * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
-    memset(page, 0, kCheckPage * sizeof(int));
-    g_check_pages.push_back(page);
-    for (size_t i = 0; i < kCheckPage; i++) g_check_free.push_back(page + i);
+  CheckPool& pool = g_check[*dev];
+  if (pool.free.empty()) {
+    CheckSlot page = {};
+    MLXR_CUDA_TRY(cudaHostAlloc(&page.word, kCheckPage * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    memset(page.word, 0, kCheckPage * sizeof(int));
+    cudaError_t e = cudaMalloc(&page.count, kCheckPage * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemcpy(page.count, page.word, kCheckPage * sizeof(uint32_t), cudaMemcpyHostToDevice);     // done when it returns, unlike cudaMemset
+    if (e != cudaSuccess) {
+      if (page.count) cudaFree(page.count);
+      cudaFreeHost(page.word);
+      return cuda_fail(e, "take_check_slot");
+    }
+    pool.pages.push_back(page);
+    for (size_t i = 0; i < kCheckPage; i++) pool.free.push_back({page.word + i, page.count + i});
   }
-  *out = g_check_free.back();
-  g_check_free.pop_back();
+  *out = pool.free.back();
+  pool.free.pop_back();
   return MLXR_OK;
 }
-// the word's value; the word must not be in use by a kernel any more
-static int give_check_word(int* w) {
-  const int v = *reinterpret_cast<volatile int*>(w);
-  *reinterpret_cast<volatile int*>(w) = 0;
+// The slot must not be in use by a kernel any more
+static void give_check_slot(int dev, const CheckSlot& slot) {
+  *reinterpret_cast<volatile int*>(slot.word) = 0;
   std::lock_guard<std::mutex> lk(g_check_mu);
-  g_check_free.push_back(w);
-  return v;
+  g_check[dev].free.push_back(slot);
 }
 
 // Looks at a word that a kernel writes until it is no longer 0, for so many microseconds at most
@@ -462,27 +472,33 @@ int mlxr_rope_apply(const void* x, const uint16_t* cos_f16, const uint16_t* sin_
   if (tokens * heads == 0) return MLXR_OK;
   if (!x || !y || !cos_f16 || !sin_f16 || !positions) { set_error("null pointer"); return MLXR_ERR_INVALID_ARGUMENT; }
   cudaStream_t st = (cudaStream_t)stream;
-  Workspace* ws = nullptr;
-  if (int r = get_workspace(st, 0, &ws)) return r;
-  // With `check` the kernel records a violation straight in pinned host memory (under unified addressing the
-  // host address is the device address), which saves a copy and a memset per call.
-  int* word = ws->status;
+  if (!check) {
+    Workspace* ws = nullptr;
+    if (int r = get_workspace(st, 0, &ws)) return r;
+    return launch_rope(x, cos_f16, sin_f16, positions, y, tokens, heads, head_dim, max_seq_len, mode, scale_factor, position_offset, dtype, ws->status, nullptr, nullptr, st);
+  }
+  // With `check` the kernel reports straight into pinned host memory (under unified addressing the host address is the
+  // device address), which saves a copy and a memset per call.
+  int dev = 0;
+  CheckSlot slot;
   bool answers = false;
-  if (check) if (int r = take_check_word(&word)) return r;
-  if (int r = launch_rope(x, cos_f16, sin_f16, positions, y, tokens, heads, head_dim, max_seq_len, mode,
-                          scale_factor, position_offset, dtype, word, ws->sync + kRopeCount, check ? &answers : nullptr, st)) {
-    if (check) give_check_word(word);       // nothing was launched
+  if (int r = take_check_slot(&dev, &slot)) return r;
+  if (int r = launch_rope(x, cos_f16, sin_f16, positions, y, tokens, heads, head_dim, max_seq_len, mode, scale_factor, position_offset, dtype, slot.word, slot.count, &answers, st)) {
+    give_check_slot(dev, slot);       // nothing was launched
     return r;
   }
-  if (check) {
-    // The answer comes when the kernel is done with all its accesses.  It is looked for where the kernel writes it as long as
-    // it may come soon; behind longer work, or from a kernel that has none, the driver waits for the stream.
-    if (!answers || !poll_word(word, 100)) MLXR_CUDA_TRY(cudaStreamSynchronize(st));     // on failure the kernel may still run: the word is not reused
-    const int bad = answers ? 2 : 1;
-    if (give_check_word(word) == bad) {
-      set_error("rope_apply: a position (+offset) lies outside [0, max_seq_len)");
-      return MLXR_ERR_SHAPE;
-    }
+  // The answer comes when the kernel is done with all its accesses.  It is looked for where the kernel writes it as long as
+  // it may come soon; behind longer work, or from a kernel that has none, the driver waits for the stream.
+  if (!answers || !poll_word(slot.word, 100)) MLXR_CUDA_TRY(cudaStreamSynchronize(st));     // on failure the kernel may still run: the slot is not reused
+  const int answer = *reinterpret_cast<volatile int*>(slot.word);
+  if (answers && answer == 0) {       // the count has gone wrong: neither the slot nor the rotation is to be relied on
+    set_error("rope_apply: the rotation ended without an answer");
+    return MLXR_ERR_CUDA;
+  }
+  give_check_slot(dev, slot);
+  if (answer == (answers ? 2 : 1)) {
+    set_error("rope_apply: a position (+offset) lies outside [0, max_seq_len)");
+    return MLXR_ERR_SHAPE;
   }
   return MLXR_OK;
 }
@@ -880,10 +896,16 @@ int mlxr_release_workspaces(void) {
   g_ws.clear();
   {
     std::lock_guard<std::mutex> check_lk(g_check_mu);
-    if (g_check_free.size() == g_check_pages.size() * kCheckPage) {      // no call in flight
-      for (int* page : g_check_pages) cudaFreeHost(page);
-      g_check_pages.clear();
-      g_check_free.clear();
+    for (auto& kv : g_check) {
+      CheckPool& pool = kv.second;
+      if (pool.free.size() != pool.pages.size() * kCheckPage) continue;      // calls in flight
+      cudaError_t e;
+      for (const CheckSlot& page : pool.pages) {
+        if ((e = cudaFree(page.count)) != cudaSuccess && first == cudaSuccess) first = e;
+        cudaFreeHost(page.word);
+      }
+      pool.pages.clear();
+      pool.free.clear();
     }
   }
   if (first != cudaSuccess) return cuda_fail(first, "mlxr_release_workspaces");

@@ -10,7 +10,6 @@ namespace mlxr {
 // Zero-initialised 32-bit words per workspace for counters and barriers.
 constexpr int kSyncWords = 4096;
 constexpr int kTileCounters = 16;      // the first of the words that count the parts of shared output tiles
-constexpr int kRopeCount = 2;          // the word that counts the CTAs of a checked rotation
 
 int launch_dequantize(const void* w, void* out, int N, int K, int qt, int out_dtype, int flags,
                       cudaStream_t st);

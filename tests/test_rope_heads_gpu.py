@@ -45,3 +45,39 @@ def test_answer_behind_longer_work():
     for _ in range(10):
         a = torch.nn.functional.normalize(a @ a)
     assert torch.equal(mx.rope_apply(x, cos, sin, pos), _want(x, cos, sin, pos))
+
+
+def test_threads_that_share_a_stream_handle():
+    """Two threads that both pass cudaStreamPerThread share the handle, not the stream: each call's answer and rotation are its own, whatever
+    the other's number of CTAs (4 and 1200), and the rotation is done when the call returns."""
+    import threading
+    import mlxr_b200 as mx
+    from mlxr_b200._capi import ERR_SHAPE, OK, lib
+    per_thread, D, P = 2, 64, 512
+    cos, sin = mx.compute_rope_tables(P, D, 10000.0, device=torch.device("cuda"))
+    wrong = []
+
+    def run(tokens, heads):
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            x = torch.randn(tokens, heads, D, device="cuda").half()
+            good = torch.randint(0, P, (tokens,), device="cuda", dtype=torch.int32)
+            bad = good.clone()
+            bad[-1] = P
+            want, y = _want(x, cos, sin, good), torch.empty_like(x)
+            for i in range(300):
+                pos, code = (bad, ERR_SHAPE) if i % 3 == 1 else (good, OK)
+                y.zero_()
+                side.synchronize()
+                r = lib.mlxr_rope_apply(x.data_ptr(), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), y.data_ptr(), 1, tokens, heads, D, P, 0, 1.0, 0, 0, 1, per_thread)
+                n = tokens - 1 if pos is bad else tokens
+                if r != code or not torch.equal(y[:n], want[:n]):
+                    wrong.append((tokens, i, r))
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=run, args=a) for a in ((16, 8), (9600, 16), (16, 8))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
