@@ -398,11 +398,22 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       constexpr int kCols = SWIGLU ? 16 : 32;
       const bool vec = P.vec_stores && nw + kCols <= P.N;
       T* yv = reinterpret_cast<T*>(P.y) + (size_t)tok0 * P.N + nw;
+      // a part is parked sixteen tokens at a time: 32 took 1.8 us more for a part of 256 tokens (MMAs of the next tile wait for it: 20480 x 1280
+      // Q8_0, 256 tokens, equal ranges 32.2 us, so 27.7)
+      if (!whole) {
 #pragma unroll 1
-      for (int c0 = 0; c0 < ntok; c0 += 32) {      // past nt: columns of the other buffer or of converted weights, not stored
-        uint32_t r[32];
-        tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * NMAX + c0), r);
-        if (whole) {
+        for (int c0 = 0; c0 < ntok; c0 += 16) {
+          uint32_t r[16];
+          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * NMAX + c0), r);
+#pragma unroll
+          for (int c = 0; c < 16; c++)
+            if (c0 + c < ntok) __stcg(part + (size_t)(c0 + c) * kRows, __uint_as_float(r[c]));
+        }
+      } else {
+#pragma unroll 1
+        for (int c0 = 0; c0 < ntok; c0 += 32) {      // past nt: columns of the other buffer, not stored
+          uint32_t r[32];
+          tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * NMAX + c0), r);
           // 32 tokens x 32 weight rows (gate/up: 16 columns) turn in shared memory into 16-byte stores.  Beside busy producers
           // every instruction here counts: a tile of 256 tokens whose results leave one 2-byte word each took 6.4 us of a
           // tile's 24 (K = 4096), and the next tile's MMAs wait for it.
@@ -449,10 +460,6 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
             }
           }
           __syncwarp();
-        } else {
-#pragma unroll
-          for (int c = 0; c < 32; c++)
-            if (c0 + c < ntok) __stcg(part + (size_t)(c0 + c) * kRows, __uint_as_float(r[c]));
         }
       }
       tc_fence_before();
