@@ -399,7 +399,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
       const bool vec = P.vec_stores && nw + kCols <= P.N;
       T* yv = reinterpret_cast<T*>(P.y) + (size_t)tok0 * P.N + nw;
       // a part is parked sixteen tokens at a time: 32 took 1.8 us more for a part of 256 tokens (MMAs of the next tile wait for it: 20480 x 1280
-      // Q8_0, 256 tokens, equal ranges 32.2 us, so 27.7)
+      // Q8_0, 256 tokens, equal ranges 31.8 us, so 26.6)
       if (!whole) {
 #pragma unroll 1
         for (int c0 = 0; c0 < ntok; c0 += 16) {
@@ -408,6 +408,18 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
 #pragma unroll
           for (int c = 0; c < 16; c++)
             if (c0 + c < ntok) __stcg(part + (size_t)(c0 + c) * kRows, __uint_as_float(r[c]));
+        }
+      } else if (!SWIGLU && !vec) {
+        // rows that start anywhere, and the ragged end of the others: straight from the registers (turned in shared memory first,
+        // 12363 x 2304 Q8_0, 515 tokens, took 43.5 us, so 41.5)
+        T* y = yv + lane;
+#pragma unroll 1
+        for (int c0 = 0; c0 < ntok; c0 += 16) {
+          uint32_t r[16];
+          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * NMAX + c0), r);
+#pragma unroll
+          for (int c = 0; c < 16; c++)
+            if (n < P.N && c0 + c < ntok) y[(size_t)(c0 + c) * P.N] = Act<T>::from_f(__uint_as_float(r[c]) + bv);
         }
       } else {
 #pragma unroll 1
@@ -443,20 +455,14 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
 #pragma unroll
             for (int c = 0; c < 16; c++) turn[c * 32 + lane] = pack2<T>(__uint_as_float(r[2 * c]) + bv, __uint_as_float(r[2 * c + 1]) + bv);
             __syncwarp();
-            if (vec) {
 #pragma unroll
-              for (int e = 0; e < 2; e++) {
-                const int piece = e * 32 + lane, tk = 2 * (piece >> 2), pc = piece & 3;
-                const uint4* w = reinterpret_cast<const uint4*>(turn + (piece >> 2) * 32 + pc * 8);
-                const uint4 u = w[0], v = w[1];
-                T* at = yv + (size_t)(c0 + tk) * P.N + pc * 8;
-                if (c0 + tk < ntok) *reinterpret_cast<uint4*>(at) = make_uint4(__byte_perm(u.x, u.y, 0x5410), __byte_perm(u.z, u.w, 0x5410), __byte_perm(v.x, v.y, 0x5410), __byte_perm(v.z, v.w, 0x5410));
-                if (c0 + tk + 1 < ntok) *reinterpret_cast<uint4*>(at + P.N) = make_uint4(__byte_perm(u.x, u.y, 0x7632), __byte_perm(u.z, u.w, 0x7632), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x7632));
-              }
-            } else {
-#pragma unroll 4
-              for (int tk = 0; tk < 32; tk++)
-                if (c0 + tk < ntok && nw + lane < P.N) yv[(size_t)(c0 + tk) * P.N + lane] = reinterpret_cast<const T*>(turn)[((tk >> 1) * 32 + lane) * 2 + (tk & 1)];
+            for (int e = 0; e < 2; e++) {
+              const int piece = e * 32 + lane, tk = 2 * (piece >> 2), pc = piece & 3;
+              const uint4* w = reinterpret_cast<const uint4*>(turn + (piece >> 2) * 32 + pc * 8);
+              const uint4 u = w[0], v = w[1];
+              T* at = yv + (size_t)(c0 + tk) * P.N + pc * 8;
+              if (c0 + tk < ntok) *reinterpret_cast<uint4*>(at) = make_uint4(__byte_perm(u.x, u.y, 0x5410), __byte_perm(u.z, u.w, 0x5410), __byte_perm(v.x, v.y, 0x5410), __byte_perm(v.z, v.w, 0x5410));
+              if (c0 + tk + 1 < ntok) *reinterpret_cast<uint4*>(at + P.N) = make_uint4(__byte_perm(u.x, u.y, 0x7632), __byte_perm(u.z, u.w, 0x7632), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x7632));
             }
           }
           __syncwarp();
