@@ -692,22 +692,29 @@ int smallm_plan(int qt, bool stacked, int M, int rows, int K, int* grid, int* ma
   const int nsb = K / 256, ntiles = (N + smallm::kRows - 1) / smallm::kRows;
   const long long U = (long long)ntiles * nsb;
   // Either all SMs get equal ranges, which cross tiles, or every tile gets c CTAs of its own (the same formula with
-  // c * ntiles CTAs).  Fitted, in us, to 825 measurements (five formats; 12, 32 and 64 tokens; ten sizes from 1500 x 2048 to 14336 x 4096; the
-  // choice by this estimate takes 0.8 % more than the best one in the mean, 24 % at most; by one fitted to Q4_K alone, before the tables,
-  // 2.6 %: 8192 x 2048 Q4_K 64 tokens 22 % with two CTAs a tile instead of one, 11008 x 4096 canonical Q4_K 26 % with one instead of equal
-  // ranges).  A unit takes what its conversion does, and as much as two of them if a CTA has only one (the groups of
-  // producers take units in turn); a shared tile its parts' trip through L2, which all CTAs make at the same time; a range that crosses
-  // tiles 1.35 more, because its CTA parks two parts.
-  const double w = smallm_npad(M);
+  // c * ntiles CTAs).  Fitted, in us, to 13700 measurements of 2524 linears (five formats; 3 to 64 tokens; 256 to 22016 rows of 1024 to
+  // 16384; the choice by this estimate takes 0.6 % more than the best one in the mean, 13 % at most; by one fitted to 1500 and more rows of 2048 and
+  // more, 2.5 % and up to 58 %: 8192 x 1024 Q8_0, 16 tokens, 6.4 us with two CTAs a tile, 4.2 with one).  A unit takes what its conversion does, about half as much
+  // again if a CTA has only one (the groups of producers take units in turn), and more from the seventh on: the first six's bytes have come while the
+  // previous kernel ended.  A shared tile costs its parts' trip through L2, which all CTAs make at the same time, and something for
+  // each part; a range that crosses tiles more, because its CTA parks two parts.
+  struct Costs { double unit[4], late[4], one, shared, together, ranges, part; };      // unit, late: 4-bit, Q8_0, NF4, weights in two parts
+  static constexpr Costs kCosts[3] = {{{0.40, 0.52, 0.64, 1.20}, {0.1, 0.3, 0.0, 0.1}, 1.34, 1.93, 1.12, 0.57, 0.063},        // to 16 tokens
+                                      {{0.44, 0.52, 0.71, 1.42}, {0.1, 0.3, 0.1, 0.2}, 1.54, 2.15, 1.18, 0.95, 0.109},        // to 32
+                                      {{0.62, 0.62, 0.66, 1.57}, {0.1, 0.2, 0.1, 0.0}, 1.46, 2.48, 1.15, 1.18, 0.196}};       // to 64
+  const Costs& k = kCosts[M <= 16 ? 0 : M <= 32 ? 1 : 2];
   const bool split = qt == MLXR_GGML_Q4_K || (M <= 8 && (stacked || qt == MLXR_Q8_0 || qt == MLXR_NF4));     // weights in two parts
-  const double unit = split ? 1.40 + 0.0028 * w : qt == MLXR_NF4 ? 0.72 + 0.0012 * w : qt == MLXR_Q8_0 ? 0.67 + 0.0014 * w : 0.37 + 0.004 * w;
-  auto units = [&](double n) { return std::max(n, 2.0) * unit; };
-  auto shared = [&](int G) { return 0.18 + w * (0.0292 + 0.0377 * G / sms); };
-  const double part = 0.02 + 0.0013 * w;
+  const int f = split ? 3 : qt == MLXR_NF4 ? 2 : qt == MLXR_Q8_0 ? 1 : 0;
+  auto units = [&](double n) { return std::max(n, k.one) * k.unit[f] + std::max(n - 6.0, 0.0) * k.late[f]; };
+  auto shared = [&](int G, double parts) { return k.shared + k.together * G / sms + k.part * parts; };
+  // q/k/v: RMSNorm before it and RoPE behind it set themselves up beside it on the SMs that it leaves to them, if it leaves one for each
+  // token, to 18 (hidden size 3584, 24 tokens of NF4: 15.6 us with 144 CTAs, 11.9 with 108; 2560, five tokens 10.6 with 140, 11.9 with 112)
+  const double need = std::min(18, M);
+  auto crowded = [&](int G) { return stacked ? 3.0 * std::max((G - (sms - need)) / need, 0.0) : 0.0; };
   int G = (int)std::min<long long>(sms, U);
-  double best = units(std::ceil((double)U / G)) + (U % G == 0 && U / G % nsb == 0 ? 0.0 : shared(G) + 1.35 + part * ((double)nsb * G / U + 1.0));
+  double best = units(std::ceil((double)U / G)) + (U % G == 0 && U / G % nsb == 0 ? 0.0 : shared(G, (double)nsb * G / U + 1.0) + k.ranges) + crowded(G);
   for (int c = 1; c <= nsb && (long long)c * ntiles <= sms; c++) {
-    const double cost = units((nsb + c - 1) / c) + (c > 1 ? shared(c * ntiles) + part * c : 0.0);
+    const double cost = units((nsb + c - 1) / c) + (c > 1 ? shared(c * ntiles, c) : 0.0) + crowded(c * ntiles);
     if (cost < best) { best = cost; G = c * ntiles; }
   }
   int mc = 1;
