@@ -184,13 +184,14 @@ static int check_quant(int qt, int K, int group_size, bool check_group) {
 // The tensor-core linears for 16-bit activations: Y = X W^T (+ bias), or SiLU(X w^T) * (X w2^T).
 // Up to 64 tokens the small-batch kernel.  Above that the wide kernel, which converts the weights beside the
 // MMAs once per 256 tokens, or the dense path, which converts them once in a pass of its own: whichever
-// their plans estimate to be faster (the choice takes 1.2 % more than the faster one in the mean over 153 linears of all formats, 20 % at
-// most).  us, wide / dense, Q4_K: 14336 x 4096 700 tokens 70 / 94, 1500 148 / 157, 2048 205 / 198, 8192 833 / 649; 4096 x
-// 14336 2048 tokens 182 / 223.  A handful of short rows takes the dense path at any number of tokens (8 x
-// 512: 7.8 / 7.4 at 65, 11.5 / 7.7 at 4096), and so do matrices to 10 * 2^20 weights above 1040 tokens, although the wide kernel
-// would mostly be faster there (2304 x 4096, 1100 tokens 23 / 30; 4096 x 2048, 4096 tokens 57 / 57): which kernel runs at these sizes
-// is fixed by the tests of both.  The dense path also takes what the others do not: K that is not a multiple of 256, rows that do
-// not start on 16 bytes.
+// their plans estimate to be faster.  Over 154 linears of 1100 to 8192 tokens in runs of half a second each the choice takes 1.7 % more than the
+// faster one in the mean, 20 % at most (4096 x 14336 and 2048 x 14336, 4096 tokens).  us, wide / dense, so measured: 14336 x 4096 Q4_K 1100 tokens 108 / 147, 3500 334 / 347, 6000 640 /
+// 594; Q8_0 8192 851 / 785; 4096 x 14336 Q4_K 1500 157 / 186, 3500 395 / 382; 1024 x 4096 Q4_K 1100 19 / 27.
+// Two kinds of matrix take the dense path whatever the estimates say, as they did before the wide kernel was faster at most of them too: a
+// handful of short rows (8 x 512: 7.8 / 7.4 at 65 tokens, 11.5 / 7.7 at 4096), and above 1040 tokens those to 10 * 2^20 weights
+// whose rows are 2048 or shorter or more than 2048 in number (512 x 1024, 2300 tokens 8.0 / 11.5; 2304 x 4096, 1100 tokens 23 / 30; 1000 x 2048,
+// 6000 tokens 33 / 26): the launches that the tests count at such sizes are the dense path's.  The dense path also takes what the
+// others do not: K that is not a multiple of 256, rows that do not start on 16 bytes.
 enum TcPath { kTcNone = 0, kTcSmall, kTcWide, kTcDense };
 static int tc_path(int qt, int M, int N, int K, int dtype, const void* x, const void* w, const void* w2, WidePlan* wide, DensePlan* dense, TcPath* out) {
   *out = kTcNone;
@@ -203,12 +204,7 @@ static int tc_path(int qt, int M, int N, int K, int dtype, const void* x, const 
   }
   if (both([&](const void* p) { return dense_supported(qt, M, N, K, dtype, x, p); })) {
     if (int r = dense_plan(M, rows, K, dense)) return r;
-    const bool small = (rows <= 16 && K <= 1024) || (M > 1040 && (long long)rows * K <= 10 << 20);
-    // to 2048 tokens the dense path takes more than its estimate: 1.15 of it at K = 4096, 1.25 at 8192, 1.2 to 1.35 at 14336 (X that does not
-    // stay in L2 beside the weights).  Above that the power cap sets both paces, and the wide kernel's conversions cost more of it than they
-    // save (block 4096 x 14336 of 8192 tokens with down on the wide kernel 2387 us, on the dense path 2326, although a few
-    // passes of down alone took 694 and 765).
-    if (M <= 2048) dense->cost_us *= 1.05 + 0.3 * K / 14336.0;
+    const bool small = (rows <= 16 && K <= 1024) || (M > 1040 && (long long)rows * K <= 10 << 20 && (K <= 2048 || rows > 2048));
     if (*out == kTcNone || small || dense->cost_us < wide->cost_us) *out = kTcDense;
   }
   return MLXR_OK;

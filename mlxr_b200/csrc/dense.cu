@@ -5,7 +5,8 @@
 //   layout or NF4; or Y = SiLU(X gate^T) * (X up^T).
 //
 // The kernel that converts inside the GEMM (widem.cu) converts every weight once per 256 tokens beside the
-// MMAs and draws power for it; from about 2000 tokens on (14336 x 4096; 4096 x 14336 never), one pass that writes 16-bit
+// MMAs and draws power for it; from some number of tokens on (14336 x 4096: 2000 of Q8_0, 2500 of Q4_K, 3100 of NF4; 4096 x 14336: 2200 of Q8_0,
+// 4400 of Q4_K, 5600 of Q4_0), one pass that writes 16-bit
 // weights (2.6 bytes of traffic per weight: 27 us for 14336 x 4096, 23 at HBM's rate) costs less than the conversions it saves, and
 // the GEMM behind it leaves the CUDA cores to the epilogue and runs at the tensor pipe's rate, which
 // under the power cap also means a higher clock.  It takes the rows in slices of at most kSliceBytes so
@@ -31,6 +32,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 
 #include "common.cuh"
@@ -387,7 +389,11 @@ int dense_plan(int M, int rows, int K, DensePlan* out) {
   }
   out->slice = slice;
   out->bytes = (size_t)slice * row_bytes;
-  out->cost_us = slices * (best / 1700.0 + 3.0) + (double)rows * K * 2.6 / 5.0e6 + 3.0;
+  // short launches take less than the sum of their parts, which overlap; long ones more, at the clock that the power cap leaves and with X
+  // that does not stay in L2 (to 20 us 0.95 to 1.0 of it, 100 us 1.2, 250 us 1.3, 800 us 1.37 in runs of half a second each).  Rows that do not start
+  // on 16 bytes leave by plain stores
+  const double us = slices * (best / 1700.0 + 3.0) + (double)rows * K * 2.6 / 5.0e6 + 3.0;
+  out->cost_us = us * (0.65 + 0.1 * std::log(us)) * (rows % 8 ? 1.1 : 1.0);
   return MLXR_OK;
 }
 

@@ -1,4 +1,4 @@
-// Quantized linear for 65 and more tokens, as long as dense.cu is not faster (14336 x 4096: to about 2000), on the 5th-generation
+// Quantized linear for 65 and more tokens, as long as dense.cu is not faster (14336 x 4096: to 2000 .. 3000, by format), on the 5th-generation
 // tensor cores, every weight converted once per 256 tokens:
 //
 //   Y[M, N] = X[M, K] * dequant(W)[N, K]^T (+ bias),  X, Y fp16 or bf16, W in MLXR's Q4_K, Q4_0 or
@@ -51,7 +51,7 @@ constexpr int kSlots = 2;                  // converted k-blocks per group
 // A stage is half a unit, two k-blocks: their converted weights (two groups' slots) and their X tiles (one copy), with one
 // barrier each way.  What a hand-over costs the warps that copy X and issue MMAs is the same for one k-block as for two:
 // with a stage and a copy for each k-block the copy warp needed 500 cycles for one (time stamps; the conversion 400),
-// 2050 a unit whatever the number of tokens; see the figures in widem_plan.
+// 2050 a unit whatever the number of tokens.
 constexpr int kBlocks = 2;
 constexpr int kHalves = kGroups / kBlocks;
 constexpr int kStages = kHalves * kSlots;  // stage (unit & 1) * kHalves + half
@@ -121,7 +121,7 @@ __device__ inline int unit_owner(long long U, int G, long long u) { return (int)
 
 // SiLU(gate) * up of two outputs held by a pair of lanes FAR apart: the lower lane has both gates, the upper one both ups.
 // Each of the two computes one output (the upper lane the second): with SiLU on one lane for both the block of 333 tokens,
-// 4096 x 11008, took 138 us, so 127.
+// 4096 x 11008, took 9 % more when that was measured (138 us and 127, of the 107 it takes now).
 template <typename T> struct Pair { T value; int second; };
 template <typename T, int FAR> __device__ __forceinline__ Pair<T> swiglu_pair(float a, float b, int lane) {
   const bool up = (lane & FAR) != 0;
@@ -552,40 +552,43 @@ bool widem_supported(int qt, int M, int N, int K, int dtype, const void* x, cons
   return ((((uintptr_t)x) | ((uintptr_t)w)) & 15u) == 0;
 }
 
-// Token tile, grid and dealing of the units.  Fitted, in us, to 4210 measurements (Q4_K, Q4_0, Q8_0, NF4; 65 to 1500 tokens; six sizes from
-// 1500 x 2048 to 22016 x 4096; tiles of 48 to 256 tokens; equal ranges, whole tiles, two to four pairs per tile; the choice by this estimate takes
-// 1.3 % more than the best of them in the mean, 17 % at most).  A unit takes its MMAs (8 cycles a token at the clock that the power cap
-// leaves) or its conversion, which is shorter with a table: to 128 tokens.  A tile costs its results' way out beside that, with two
-// accumulators (to 128 tokens) less; a shared tile its parts' trip through L2 at the end; equal ranges also the
-// parts that a pair parks between two tiles.  Whole tiles need none of that but leave SMs idle in the last wave; above 192 tokens equal ranges take
-// 12 % more than a few passes show once the power cap holds (thousands of passes of 22016 x 4096 Q4_0, 333 tokens: tiles of 176, equal ranges 71.2 us,
-// whole 65.4; 112, 75.1 and 71.9).
+// Token tile, grid and dealing of the units.  Fitted, in us, to 29000 measurements of 2365 linears (65 to 8192 tokens; 256 to 22016 rows of
+// 1024 to 16384; tiles of 32 to 256 tokens; equal ranges, whole tiles, two to 32 pairs per tile; bursts of 4 ms, weights from HBM): the choice
+// by this estimate takes 2 % more than the best of them in the mean.  A unit takes its MMAs or its conversion, whichever is longer.  A tile costs its results' way out beside
+// that, with two accumulators (to 128 tokens) less, and more if its rows start anywhere (2-byte stores); a shared tile its parts' trip through
+// L2 at the end; equal ranges also the parts that a pair parks between two tiles.  Whole tiles need none of that but leave SMs idle in the last
+// wave.  A launch on more than half of the pairs cannot set itself up beside its predecessor's end.  Long launches run at
+// the lower clock that the power cap leaves: the last line.
 int widem_plan(int qt, int dtype, int M, int rows, int K, WidePlan* out) {
   int sms = 0;
   if (int r = device_sms(&sms)) return r;
   const int nsb = K / 256, wtiles = (rows + 2 * widem::kRows - 1) / (2 * widem::kRows), pairs = sms / 2;
-  const bool f16 = dtype == MLXR_F16;
-  const double convert128 = qt == MLXR_Q8_0 ? 1.21 : qt == MLXR_NF4 ? 1.07 : f16 ? 0.75 : 0.86;
-  const double convert256 = qt == MLXR_Q8_0 ? 1.36 : qt == MLXR_NF4 ? 1.47 : !f16 ? 1.12 : qt == MLXR_Q4_0 ? 0.89 : 1.04;
+  // a unit's conversion with tiles to 128 and to 256 tokens, its MMAs per token with either, what a tile's way out costs beside them
+  struct Costs { double convert128, convert256, mma128, mma256, out; };
+  static constexpr Costs kQ8 = {0.93, 1.10, 0.0070, 0.0043, 0.65}, kNf4 = {0.87, 1.21, 0.0064, 0.0024, 0.92}, kQ40[2] = {{0.76, 0.66, 0.0060, 0.0035, 0.95}, {0.71, 0.99, 0.0051, 0.0036, 0.96}},
+                         kQ4K[2] = {{0.59, 0.84, 0.0037, 0.0036, 1.30}, {0.77, 0.98, 0.0053, 0.0038, 0.71}};      // fp16, bf16
+  const int bf = dtype == MLXR_F16 ? 0 : 1;
+  const Costs& k = qt == MLXR_Q8_0 ? kQ8 : qt == MLXR_NF4 ? kNf4 : qt == MLXR_Q4_0 ? kQ40[bf] : kQ4K[bf];
   double best = 1e300;
   for (int ntt = (M + 255) / 256;; ntt++) {
     const int nt = ((M + ntt - 1) / ntt + 15) / 16 * 16;
     if (nt < (M <= 1024 ? 48 : 112) && best < 1e300) break;
     const long long ntiles = (long long)wtiles * ((M + nt - 1) / nt), U = ntiles * nsb;
-    const double unit = nt <= 128 ? std::max(convert128, 0.31 + 0.0054 * nt) : std::max(convert256, 0.31 + 0.0046 * nt);
-    const double drain = nt <= 128 ? 2.15 : 0.0303 * nt - 1.72, shared = 0.023 * nt, part = 0.63 + 0.0017 * nt, parked = 0.0375 * nt;
+    const double unit = nt <= 128 ? std::max(k.convert128, 0.32 + k.mma128 * nt) : std::max(k.convert256, 0.32 + k.mma256 * nt);
+    const double drain = (nt <= 128 ? 0.68 : 0.0169 * nt - 0.91) * k.out, whole = drain + (rows % 8 ? 0.016 * nt : 0.0);
+    const double shared = 1.56 + 0.0164 * nt, part = 0.07 + 0.0023 * nt, parked = 0.38 + 0.014 * nt;
     // split 0: equal ranges of units for all pairs; else so many pairs for each tile (1: whole tiles, any number of them)
     for (int split = 0; split < 2 || (split <= nsb && split * ntiles <= pairs); split++) {
       if (split != 1 && 2 * ntiles > kSyncWords - kTileCounters) continue;        // two counters per tile
       const int G = (int)(split == 0 ? std::min<long long>(pairs, U) : split == 1 ? std::min<long long>(pairs, ntiles) : split * ntiles);
-      double c;
+      double c = 1.55 * std::max(2.0 * G / pairs - 1.0, 0.0);
       if (split == 0) {
         const double units = (double)((U + G - 1) / G);
-        c = units * unit + units / nsb * drain + shared + part * std::floor((nsb + units - 1) / units) + parked;
-        if (M > 192) c *= 1.12;
+        c += units * unit + std::max(units / nsb - 1.0, 0.0) * whole + drain + shared + part * std::floor((nsb + units - 1) / units) + parked;
+        c *= 1.0 + 0.02 * std::min(M / 2048.0, 2.0);       // runs of half a second: 4096 x 14336 Q4_K, 4096 tokens, 502 us
       } else {
         const double tiles = (double)((ntiles + G - 1) / G);
-        c = split == 1 ? tiles * (nsb * unit + drain) : (nsb + split - 1) / split * unit + drain + shared + part * split;
+        c += split == 1 ? tiles * (nsb * unit + whole) : (nsb + split - 1) / split * unit + drain + shared + part * split;
       }
       if (c < best) {
         best = c;
@@ -595,7 +598,8 @@ int widem_plan(int qt, int dtype, int M, int rows, int K, WidePlan* out) {
     }
     if (nt <= 16) break;
   }
-  out->cost_us = 4.05 + best;
+  best += 4.29;
+  out->cost_us = best * (0.54 + 0.1435 * std::log(best));
   return MLXR_OK;
 }
 
