@@ -489,9 +489,8 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
       constexpr int kCols = SWIGLU ? 16 : 32;
       const int nw = SWIGLU ? 64 * at.tile + 16 * quarter : at.tile * kRows + 32 * quarter;
       const bool vec = ((P.vec_stores >> at.mat) & 1) && nw + kCols <= N;
-#pragma unroll 1
-      for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) {
-        uint32_t r[16];
+      // the sums of sixteen tokens: both issuers' accumulators
+      auto sums = [&](int c0, uint32_t (&r)[16]) {
         const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + R::kAcc0 + (uint32_t)(ab * 2 * NPAD + c0);
         if (cnt == 1) {
           tmem_ld16(acc + (uint32_t)((i & 1) * NPAD), r);
@@ -506,15 +505,32 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
 #pragma unroll
           for (int c = 0; c < 16; c++) note_bad(bad, __uint_as_float(r[c]));
         }
-        if (whole && !SWIGLU && !vec) {
-          // rows that start anywhere, and the ragged end of the others (turned in shared memory first, 3333 x 1536 Q4_0, 64 tokens, took
-          // 9.2 us, so 8.6)
+      };
+      // A loop for each way out: with the three in one, parking took 1 to 2 % of a short launch more
+      if (!whole) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) {
+          uint32_t r[16];
+          sums(c0, r);
 #pragma unroll
           for (int c = 0; c < 16; c++)
-            if (c0 + c < P.M && n < N) y[(size_t)(c0 + c) * N + n] = Act<T>::from_f(__uint_as_float(r[c]) + bv);
-        } else if (whole) {
-          // sixteen tokens x 32 weight rows (gate/up: 16 columns, SiLU of every other token on the upper lanes) turn in shared
-          // memory into 16-byte stores: with a 2-byte store per lane and token a round of sixteen took 1400 cycles
+            if (c0 + c < P.M) __stcg(part + (size_t)(c0 + c) * kRows, __uint_as_float(r[c]));
+        }
+      } else {
+#pragma unroll 1
+        for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) {
+          uint32_t r[16];
+          sums(c0, r);
+          if (!SWIGLU && !vec) {
+            // rows that start anywhere, and the ragged end of the others (turned in shared memory first, 3333 x 1536 Q4_0, 64 tokens, took
+            // 9.2 us, so 8.6)
+#pragma unroll
+            for (int c = 0; c < 16; c++)
+              if (c0 + c < P.M && n < N) y[(size_t)(c0 + c) * N + n] = Act<T>::from_f(__uint_as_float(r[c]) + bv);
+            continue;
+          }
+          // sixteen tokens x 32 weight rows (gate/up: 16 columns, SiLU of every other token on the upper lanes; a warp's columns there all exist or
+          // none does) turn in shared memory into 16-byte stores: with a 2-byte store per lane and token a round of sixteen took 1400 cycles
           uint16_t* turn = sh->turn[quarter];
           if constexpr (SWIGLU) {
             const bool up = lane >= 16;
@@ -541,18 +557,8 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
               const int piece = e * 32 + lane, tk = piece / kPer, pc = piece % kPer;
               if (c0 + tk < P.M) *reinterpret_cast<uint4*>(y + (size_t)(c0 + tk) * N + nw + pc * 8) = *reinterpret_cast<const uint4*>(turn + tk * kCols + pc * 8);
             }
-          } else {
-#pragma unroll 4
-            for (int e = lane; e < 16 * kCols; e += 32) {
-              const int tk = e / kCols, col = nw + e % kCols;
-              if (c0 + tk < P.M && col < N) y[(size_t)(c0 + tk) * N + col] = *reinterpret_cast<const T*>(turn + e);
-            }
           }
           __syncwarp();
-        } else {
-#pragma unroll
-          for (int c = 0; c < 16; c++)
-            if (c0 + c < P.M) __stcg(part + (size_t)(c0 + c) * kRows, __uint_as_float(r[c]));
         }
       }
       tc_fence_before();
@@ -777,6 +783,7 @@ int launch_smallm(const void* x, const void* const* w, const int* rows, int nmat
     }
     P.end[i] = P.ntiles;
   }
+  if (swiglu && (rows[0] % 16 || !P.vec_stores)) { set_error("small-batch kernel: gate / up wants outputs of a multiple of 16 columns, on 16 bytes"); return MLXR_ERR_UNSUPPORTED; }
   P.bias = bias;
   P.M = M; P.K = K;
   P.nsb = K / 256;

@@ -443,7 +443,7 @@ qgemm_widem_kernel(const __grid_constant__ Maps maps, const Params P) {
                 const int piece = e * 32 + lane, tk = piece >> 1, pc = piece & 1;
                 if (c0 + tk < ntok) *reinterpret_cast<uint4*>(yv + (size_t)(c0 + tk) * P.N + pc * 8) = *reinterpret_cast<const uint4*>(turn + tk * kCols + pc * 8);
               }
-            } else {
+            } else {      // nothing to store today: a warp's columns all exist or none does, and h starts on 16 bytes; without these lines the block takes 1.2 % longer
 #pragma unroll 4
               for (int e = lane; e < 32 * kCols; e += 32) {
                 const int tk = e / kCols, col = e % kCols;
