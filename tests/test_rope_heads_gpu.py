@@ -27,7 +27,7 @@ def test_heads_of_a_thread(dt, tokens, heads, d):
     # a position outside the table: reported, the other tokens rotated; the next call finds clean words
     pos[tokens // 2] = 512
     y = x.clone()
-    with pytest.raises(Exception):
+    with pytest.raises(mx._capi.MlxrError):
         mx.rope_apply(y, cos, sin, pos, inplace=True)
     want[tokens // 2] = x[tokens // 2]
     assert torch.equal(y, want)
@@ -81,3 +81,41 @@ def test_threads_that_share_a_stream_handle():
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("tokens,q_heads,kv_heads,d", [(512, 61, 3, 64), (512, 125, 1, 64), (512, 123, 3, 64), (2100, 7, 1, 128), (4100, 7, 2, 128)])
+def test_q_and_k_in_one_launch(tokens, q_heads, kv_heads, d):
+    """Two (the first and fourth sizes) and four heads a thread, of both tensors, with head counts that they do not divide: what the
+    rotation of each by itself gives."""
+    import mlxr_b200 as mx
+    H, qt = 256, mx.QuantType.Q8_0
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, H, device="cuda", generator=g).half()
+    cos, sin = mx.compute_rope_tables(512, d, 10000.0, device=torch.device("cuda"))
+    pos = torch.randint(0, 512, (tokens,), device="cuda", generator=g, dtype=torch.int32)
+
+    def weights(heads):
+        b = torch.randint(0, 256, (heads * d * H // 32, 34), dtype=torch.uint8, device="cuda", generator=g)
+        b[:, :2] = torch.tensor([0, 0x18], dtype=torch.uint8, device="cuda")       # scale 2^-9
+        return b.reshape(-1)
+
+    ws = [weights(h) for h in (q_heads, kv_heads, kv_heads)]
+    got = mx.qkv_rope(x, None, *ws, cos, sin, pos, q_heads, kv_heads, d, qt)
+    lin = [mx.q_gemm_dequant(x, w, tokens, h * d, H, qt, 32).reshape(tokens, h, d) for w, h in zip(ws, (q_heads, kv_heads, kv_heads))]
+    assert torch.equal(got[0], _want(lin[0], cos, sin, pos)) and torch.equal(got[1], _want(lin[1], cos, sin, pos)) and torch.equal(got[2], lin[2])
+
+
+def test_more_work_than_ctas():
+    """80,000 tokens of four heads of 128: 5000 CTAs' worth of units for 4736 CTAs; the position outside the table is among the last ones."""
+    import mlxr_b200 as mx
+    tokens, d = 80000, 128
+    cos, sin = mx.compute_rope_tables(64, d, 10000.0, device=torch.device("cuda"))
+    x = torch.randn(tokens, 4, d, device="cuda").half()
+    pos = torch.randint(0, 64, (tokens,), device="cuda", dtype=torch.int32)
+    want = _want(x, cos, sin, pos)
+    assert torch.equal(mx.rope_apply(x, cos, sin, pos), want)
+    pos[-2] = 64
+    want[-2] = x[-2]          # left as it was
+    with pytest.raises(mx._capi.MlxrError):
+        mx.rope_apply(x, cos, sin, pos, inplace=True)
+    assert torch.equal(x, want)
