@@ -468,11 +468,9 @@ int mlxr_rope_apply(const void* x, const uint16_t* cos_f16, const uint16_t* sin_
   if (tokens * heads == 0) return MLXR_OK;
   if (!x || !y || !cos_f16 || !sin_f16 || !positions) { set_error("null pointer"); return MLXR_ERR_INVALID_ARGUMENT; }
   cudaStream_t st = (cudaStream_t)stream;
-  if (!check) {
-    Workspace* ws = nullptr;
-    if (int r = get_workspace(st, 0, &ws)) return r;
-    return launch_rope(x, cos_f16, sin_f16, positions, y, tokens, heads, head_dim, max_seq_len, mode, scale_factor, position_offset, dtype, ws->status, nullptr, nullptr, st);
-  }
+  Workspace* ws = nullptr;
+  if (int r = get_workspace(st, 0, &ws)) return r;      // checked calls as well: one may be a stream's first call before a capture
+  if (!check) return launch_rope(x, cos_f16, sin_f16, positions, y, tokens, heads, head_dim, max_seq_len, mode, scale_factor, position_offset, dtype, ws->status, nullptr, nullptr, st);
   // With `check` the kernel reports straight into pinned host memory (under unified addressing the host address is the
   // device address), which saves a copy and a memset per call.
   int dev = 0;

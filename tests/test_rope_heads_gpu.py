@@ -119,3 +119,23 @@ def test_more_work_than_ctas():
     with pytest.raises(mx._capi.MlxrError):
         mx.rope_apply(x, cos, sin, pos, inplace=True)
     assert torch.equal(x, want)
+
+
+def test_a_checked_call_readies_its_stream():
+    """A stream whose first call was a checked one can be captured: what calls in it need is there."""
+    import mlxr_b200 as mx
+    cos, sin = mx.compute_rope_tables(64, 64, 10000.0, device=torch.device("cuda"))
+    x = torch.randn(100, 4, 64, device="cuda").half()
+    pos = torch.randint(0, 64, (100,), device="cuda", dtype=torch.int32)
+    y = torch.empty_like(x)
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        mx.rope_apply(x, cos, sin, pos)
+    st.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        y.copy_(mx.rope_apply(x, cos, sin, pos, check_positions=False))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, _want(x, cos, sin, pos))
