@@ -506,60 +506,63 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
           for (int c = 0; c < 16; c++) note_bad(bad, __uint_as_float(r[c]));
         }
       };
-      // A loop for each way out: with the three in one, parking took 1 to 2 % of a short launch more
-      if (!whole) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) {
-          uint32_t r[16];
-          sums(c0, r);
+      auto park = [&](int c0, const uint32_t (&r)[16]) {
+#pragma unroll
+        for (int c = 0; c < 16; c++)
+          if (c0 + c < P.M) __stcg(part + (size_t)(c0 + c) * kRows, __uint_as_float(r[c]));
+      };
+      auto out = [&](int c0, const uint32_t (&r)[16]) {
+        if (!SWIGLU && !vec) {
+          // rows that start anywhere, and the ragged end of the others (turned in shared memory first, 3333 x 1536 Q4_0, 64 tokens, took
+          // 9.2 us, so 8.6)
 #pragma unroll
           for (int c = 0; c < 16; c++)
-            if (c0 + c < P.M) __stcg(part + (size_t)(c0 + c) * kRows, __uint_as_float(r[c]));
+            if (c0 + c < P.M && n < N) y[(size_t)(c0 + c) * N + n] = Act<T>::from_f(__uint_as_float(r[c]) + bv);
+          return;
         }
+        // sixteen tokens x 32 weight rows (gate/up: 16 columns, SiLU of every other token on the upper lanes; a warp's columns there all exist or
+        // none does) turn in shared memory into 16-byte stores: with a 2-byte store per lane and token a round of sixteen took 1400 cycles
+        uint16_t* turn = sh->turn[quarter];
+        if constexpr (SWIGLU) {
+          const bool up = lane >= 16;
+#pragma unroll
+          for (int c = 0; c < 16; c += 2) {
+            const float a = __uint_as_float(r[c]), b = __uint_as_float(r[c + 1]);
+            const float o = __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+            const float gv = Act<T>::to_f(Act<T>::from_f(up ? o : a)), uv = Act<T>::to_f(Act<T>::from_f(up ? b : o));
+            const T h = Act<T>::from_f(swish_fast(gv) * uv);
+            turn[(c + (up ? 1 : 0)) * kCols + (lane & 15)] = *reinterpret_cast<const uint16_t*>(&h);
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 16; c++) {
+            const T o = Act<T>::from_f(__uint_as_float(r[c]) + bv);
+            turn[c * kCols + lane] = *reinterpret_cast<const uint16_t*>(&o);
+          }
+        }
+        __syncwarp();
+        if (vec) {
+          constexpr int kPer = kCols / 8;                                // 16-byte pieces per token
+#pragma unroll
+          for (int e = 0; e < 16 * kPer / 32; e++) {
+            const int piece = e * 32 + lane, tk = piece / kPer, pc = piece % kPer;
+            if (c0 + tk < P.M) *reinterpret_cast<uint4*>(y + (size_t)(c0 + tk) * N + nw + pc * 8) = *reinterpret_cast<const uint4*>(turn + tk * kCols + pc * 8);
+          }
+        }
+        __syncwarp();
+      };
+      // Rounds of sixteen tokens.  Where there are several, a loop for each way out: with both in one, parking took 1 to 2 % of a short launch
+      // more (and with a single round a loop of each takes 1 % of a launch more: 14336 x 4096 NF4, 16 tokens, 16.1 us and 15.9)
+      uint32_t r[16];
+      if constexpr (NPAD == 16) {
+        sums(0, r);
+        if (whole) out(0, r); else park(0, r);
+      } else if (!whole) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) { sums(c0, r); park(c0, r); }
       } else {
 #pragma unroll 1
-        for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) {
-          uint32_t r[16];
-          sums(c0, r);
-          if (!SWIGLU && !vec) {
-            // rows that start anywhere, and the ragged end of the others (turned in shared memory first, 3333 x 1536 Q4_0, 64 tokens, took
-            // 9.2 us, so 8.6)
-#pragma unroll
-            for (int c = 0; c < 16; c++)
-              if (c0 + c < P.M && n < N) y[(size_t)(c0 + c) * N + n] = Act<T>::from_f(__uint_as_float(r[c]) + bv);
-            continue;
-          }
-          // sixteen tokens x 32 weight rows (gate/up: 16 columns, SiLU of every other token on the upper lanes; a warp's columns there all exist or
-          // none does) turn in shared memory into 16-byte stores: with a 2-byte store per lane and token a round of sixteen took 1400 cycles
-          uint16_t* turn = sh->turn[quarter];
-          if constexpr (SWIGLU) {
-            const bool up = lane >= 16;
-#pragma unroll
-            for (int c = 0; c < 16; c += 2) {
-              const float a = __uint_as_float(r[c]), b = __uint_as_float(r[c + 1]);
-              const float o = __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
-              const float gv = Act<T>::to_f(Act<T>::from_f(up ? o : a)), uv = Act<T>::to_f(Act<T>::from_f(up ? b : o));
-              const T h = Act<T>::from_f(swish_fast(gv) * uv);
-              turn[(c + (up ? 1 : 0)) * kCols + (lane & 15)] = *reinterpret_cast<const uint16_t*>(&h);
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < 16; c++) {
-              const T o = Act<T>::from_f(__uint_as_float(r[c]) + bv);
-              turn[c * kCols + lane] = *reinterpret_cast<const uint16_t*>(&o);
-            }
-          }
-          __syncwarp();
-          if (vec) {
-            constexpr int kPer = kCols / 8;                                // 16-byte pieces per token
-#pragma unroll
-            for (int e = 0; e < 16 * kPer / 32; e++) {
-              const int piece = e * 32 + lane, tk = piece / kPer, pc = piece % kPer;
-              if (c0 + tk < P.M) *reinterpret_cast<uint4*>(y + (size_t)(c0 + tk) * N + nw + pc * 8) = *reinterpret_cast<const uint4*>(turn + tk * kCols + pc * 8);
-            }
-          }
-          __syncwarp();
-        }
+        for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) { sums(c0, r); out(c0, r); }
       }
       tc_fence_before();
       __syncwarp();
