@@ -556,7 +556,7 @@ qgemm_smallm_kernel(const __grid_constant__ Maps maps, const Params P) {
       uint32_t r[16];
       if constexpr (NPAD == 16) {
         sums(0, r);
-        if (whole) out(0, r); else park(0, r);
+        if (!whole) park(0, r); else out(0, r);
       } else if (!whole) {
 #pragma unroll 1
         for (int c0 = 0; c0 < NPAD && c0 < P.M; c0 += 16) { sums(c0, r); park(c0, r); }
