@@ -200,6 +200,7 @@ static int tc_path(int qt, int M, int N, int K, int dtype, const void* x, const 
   if (M <= 64 && both([&](const void* p) { return smallm_supported(qt, M, N, K, dtype, x, p); })) { *out = kTcSmall; return MLXR_OK; }
   if (M > 64 && both([&](const void* p) { return widem_supported(qt, M, N, K, dtype, x, p); })) {
     if (int r = widem_plan(qt, dtype, M, rows, K, wide)) return r;
+    if (w2) wide->cost_us *= 1.08;      // SiLU beside the producers: where plain linears of its size break even, gate / up's block takes 1 to 7 % more than with the dense path (1049 to 2848 tokens)
     *out = kTcWide;
   }
   if (both([&](const void* p) { return dense_supported(qt, M, N, K, dtype, x, p); })) {

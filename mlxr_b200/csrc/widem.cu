@@ -585,7 +585,9 @@ int widem_plan(int qt, int dtype, int M, int rows, int K, WidePlan* out) {
       if (split == 0) {
         const double units = (double)((U + G - 1) / G);
         c += units * unit + std::max(units / nsb - 1.0, 0.0) * whole + drain + shared + part * std::floor((nsb + units - 1) / units) + parked;
-        c *= 1.0 + 0.02 * std::min(M / 2048.0, 2.0);       // runs of half a second: 4096 x 14336 Q4_K, 4096 tokens, 502 us
+        // pairs at different places of K share neither X nor weights in L2; in runs of half a second 48 MB of X take 8 % more than whole
+        // tiles' share of it, 96 MB 22 % (4096 x 14336 Q4_K, 4096 tokens, 502 us; the dense path 432); few weight tiles read X few times
+        c *= 1.0 + 0.0025 * std::min(std::max((double)M * K / (1 << 19) - 16.0, 0.0), 120.0) * std::min(wtiles / 8.0, 1.0);
       } else {
         const double tiles = (double)((ntiles + G - 1) / G);
         c += split == 1 ? tiles * (nsb * unit + whole) : (nsb + split - 1) / split * unit + drain + shared + part * split;
