@@ -185,7 +185,7 @@ static int check_quant(int qt, int K, int group_size, bool check_group) {
 // Up to 64 tokens the small-batch kernel.  Above that the wide kernel, which converts the weights beside the
 // MMAs once per 256 tokens, or the dense path, which converts them once in a pass of its own: whichever
 // their plans estimate to be faster.  Over 154 linears of 1100 to 8192 tokens in runs of half a second each the choice takes 1.7 % more than the
-// faster one in the mean, 20 % at most (4096 x 14336 and 2048 x 14336, 4096 tokens).  us, wide / dense, so measured: 14336 x 4096 Q4_K 1100 tokens 108 / 147, 3500 334 / 347, 6000 640 /
+// faster one in the mean, 20 % at most (2048 x 14336, 4096 tokens).  us, wide / dense, so measured: 14336 x 4096 Q4_K 1100 tokens 108 / 147, 3500 334 / 347, 6000 640 /
 // 594; Q8_0 8192 851 / 785; 4096 x 14336 Q4_K 1500 157 / 186, 3500 395 / 382; 1024 x 4096 Q4_K 1100 19 / 27.
 // Two kinds of matrix take the dense path whatever the estimates say, as they did before the wide kernel was faster at most of them too: a
 // handful of short rows (8 x 512: 7.8 / 7.4 at 65 tokens, 11.5 / 7.7 at 4096), and above 1040 tokens those to 10 * 2^20 weights

@@ -5,8 +5,8 @@
 //   layout or NF4; or Y = SiLU(X gate^T) * (X up^T).
 //
 // The kernel that converts inside the GEMM (widem.cu) converts every weight once per 256 tokens beside the
-// MMAs and draws power for it; from some number of tokens on (14336 x 4096: 2000 of Q8_0, 2500 of Q4_K, 3100 of NF4; 4096 x 14336: 2200 of Q8_0,
-// 4400 of Q4_K, 5600 of Q4_0), one pass that writes 16-bit
+// MMAs and draws power for it; from some number of tokens on (14336 x 4096: 1950 of Q8_0, 2500 to 3000 of the other
+// formats, by how the last wave comes out; 4096 x 14336: 2200 to 3500 of Q8_0, 4000 and more of the others), one pass that writes 16-bit
 // weights (2.6 bytes of traffic per weight: 27 us for 14336 x 4096, 23 at HBM's rate) costs less than the conversions it saves, and
 // the GEMM behind it leaves the CUDA cores to the epilogue and runs at the tensor pipe's rate, which
 // under the power cap also means a higher clock.  It takes the rows in slices of at most kSliceBytes so
